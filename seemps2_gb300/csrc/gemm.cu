@@ -4,22 +4,23 @@
 //
 // op = N (as stored), T (transpose) or C (conjugate transpose), the three
 // GemmOrder flags of the reference (cython/gemm.pxi:17-20, :21-122).  GB300
-// runs FP64 on the CUDA cores only, so this is a shared-memory tiled SIMT
-// kernel: 64x64 output tile per CTA, 16-deep K slices, 256 threads holding a
-// 4x4 register tile each; the FP64 pipe is the bound, not HBM (operands are
-// re-read from L2 at most M/64 + N/64 times).  When the output has fewer
-// tiles than the GPU has SMs (the 256..768-sized contractions of a sweep give
-// 16-150 tiles), the K range is split over blockIdx.z: each slice writes its
-// partial tile to a workspace and a second kernel sums the slices in a fixed
-// order (deterministic) and applies alpha / beta.
+// runs FP64 on the CUDA cores only, 2 FMA per clock and SM, so a product is
+// bound by how evenly its multiply-adds are spread over the SMs, not by HBM or
+// by operand reuse; see k_gemm.
+#include <cooperative_groups.h>
+
 #include <algorithm>
+#include <cmath>
 
 #include "kernels.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace sm {
 
 namespace {
 
+// tile of the FP32 kernel k_gemm32
 constexpr int BM = 64, BN = 64, BK = 16, NT = 256;
 
 __device__ __forceinline__ double shfl_xor_T(double v, int o) {
@@ -40,120 +41,130 @@ __device__ __forceinline__ cplx load_op<cplx>(const cplx* p, int op) {
   return op == SM_OP_C ? cplx{v.x, -v.y} : cplx{v.x, v.y};
 }
 
-template <typename T>
-__global__ void __launch_bounds__(NT) k_gemm(int opA, int opB, int M, int N, int K, T alpha,
-                                             const T* __restrict__ A, int lda,
-                                             const T* __restrict__ B, int ldb, T beta,
-                                             T* __restrict__ C, int ldc, int kchunk,
-                                             T* __restrict__ part) {
-  __shared__ T As[BK][BM + 1];
-  __shared__ T Bs[BK][BN + 1];
+// One CTA (128 threads, RM x RN outputs each) per TM x TN tile and K slice; the
+// slices of a tile are the CTAs of one cluster (along z), which add their partial
+// tiles over DSMEM in slice order and write C once.  What bounds it: an FP64
+// warp instruction holds a sub-partition's FP64 pipe for 64 clocks, so the time
+// is the multiply-adds of the fullest SM.  Small tiles and up to 8 slices put
+// the work of the 60..400-sized products of a split on all 152 SMs (a 64 x 64
+// tile with slices of at least 64 left 18 CTAs for 174 x 174 x 190: 116 us, the
+// 32 x 32 tile's 288 CTAs take 21), and the loads of a slab are in flight while the one
+// before it is multiplied.  Warps whose rows all lie beyond M skip the multiply.
+template <typename T, int TM, int TN, int RM, int RN>
+__global__ void __launch_bounds__(128) k_gemm(int opA, int opB, int M, int N, int K, T alpha,
+                                              const T* __restrict__ A, int lda,
+                                              const T* __restrict__ B, int ldb, T beta,
+                                              T* __restrict__ C, int ldc, int kchunk) {
+  constexpr int KS = 16;                    // slab depth
+  constexpr int GM = TM / RM, GN = TN / RN;  // thread grid of the tile
+  static_assert(GM * GN == 128, "128 threads");
+  constexpr int LA = TM * KS / 128, LB = TN * KS / 128;
+  constexpr size_t kSlab = sizeof(T) * KS * (TM + 1 + TN + 1);
+  constexpr size_t kTile = sizeof(T) * TM * TN;
+  __shared__ __align__(16) unsigned char raw[kSlab > kTile ? kSlab : kTile];
+  T(*As)[TM + 1] = reinterpret_cast<T(*)[TM + 1]>(raw);
+  T(*Bs)[TN + 1] = reinterpret_cast<T(*)[TN + 1]>(raw + sizeof(T) * KS * (TM + 1));
   const int tid = threadIdx.x;
-  const int tx = tid % 16, ty = tid / 16;
-  const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  T acc[4][4];
+  const int tx = tid % GN, ty = tid / GN;
+  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+  T acc[RM][RN];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < RM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = S<T>::zero();
-
+    for (int j = 0; j < RN; ++j) acc[i][j] = S<T>::zero();
   const int kbeg = blockIdx.z * kchunk;
   const int kend = min(K, kbeg + kchunk);
-  for (int k0 = kbeg; k0 < kend; k0 += BK) {
+  T ra[LA], rb[LB];
+  auto fetch = [&](int k0) {
 #pragma unroll
-    for (int e = 0; e < (BM * BK) / NT; ++e) {
-      const int idx = tid + e * NT;
-      int mm, kk;
-      if (opA == SM_OP_N) { mm = idx / BK; kk = idx % BK; }
-      else                { kk = idx / BM; mm = idx % BM; }
+    for (int e = 0; e < LA; ++e) {
+      const int idx = tid + e * 128;
+      const int mm = opA == SM_OP_N ? idx / KS : idx % TM;
+      const int kk = opA == SM_OP_N ? idx % KS : idx / TM;
       const int gm = m0 + mm, gk = k0 + kk;
-      T v = S<T>::zero();
+      ra[e] = S<T>::zero();
       if (gm < M && gk < kend)
-        v = opA == SM_OP_N ? load_op(A + (size_t)gm * lda + gk, opA)
-                           : load_op(A + (size_t)gk * lda + gm, opA);
-      As[kk][mm] = v;
+        ra[e] = load_op(opA == SM_OP_N ? A + (size_t)gm * lda + gk : A + (size_t)gk * lda + gm, opA);
     }
 #pragma unroll
-    for (int e = 0; e < (BN * BK) / NT; ++e) {
-      const int idx = tid + e * NT;
-      int nn, kk;
-      if (opB == SM_OP_N) { kk = idx / BN; nn = idx % BN; }
-      else                { nn = idx / BK; kk = idx % BK; }
+    for (int e = 0; e < LB; ++e) {
+      const int idx = tid + e * 128;
+      const int nn = opB == SM_OP_N ? idx % TN : idx / KS;
+      const int kk = opB == SM_OP_N ? idx / TN : idx % KS;
       const int gn = n0 + nn, gk = k0 + kk;
-      T v = S<T>::zero();
+      rb[e] = S<T>::zero();
       if (gn < N && gk < kend)
-        v = opB == SM_OP_N ? load_op(B + (size_t)gk * ldb + gn, opB)
-                           : load_op(B + (size_t)gn * ldb + gk, opB);
-      Bs[kk][nn] = v;
+        rb[e] = load_op(opB == SM_OP_N ? B + (size_t)gk * ldb + gn : B + (size_t)gn * ldb + gk, opB);
     }
-    __syncthreads();
+  };
+  auto stage = [&]() {
 #pragma unroll
-    for (int kk = 0; kk < BK; ++kk) {
-      T a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = S<T>::fma(a[i], b[j], acc[i][j]);
+    for (int e = 0; e < LA; ++e) {
+      const int idx = tid + e * 128;
+      As[opA == SM_OP_N ? idx % KS : idx / TM][opA == SM_OP_N ? idx / KS : idx % TM] = ra[e];
     }
+#pragma unroll
+    for (int e = 0; e < LB; ++e) {
+      const int idx = tid + e * 128;
+      Bs[opB == SM_OP_N ? idx / TN : idx % KS][opB == SM_OP_N ? idx % TN : idx / KS] = rb[e];
+    }
+  };
+  const bool idle = m0 + (tid & ~31) / GN >= M;  // this warp's first row (the others lie below it)
+  if (kbeg < kend) fetch(kbeg);
+  for (int k0 = kbeg; k0 < kend; k0 += KS) {
+    stage();
     __syncthreads();
-  }
-  if (part) {
-    T* p = part + (size_t)blockIdx.z * M * N;
+    if (k0 + KS < kend) fetch(k0 + KS);
+    if (!idle) {
+      const int kn = min(KS, kend - k0);
+#pragma unroll 4
+      for (int kk = 0; kk < kn; ++kk) {
+        T a[RM], b[RN];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int gm = m0 + ty + 16 * i;
-      if (gm >= M) continue;
+        for (int i = 0; i < RM; ++i) a[i] = As[kk][ty + GM * i];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int gn = n0 + tx + 16 * j;
-        if (gn < N) p[(size_t)gm * N + gn] = acc[i][j];
+        for (int j = 0; j < RN; ++j) b[j] = Bs[kk][tx + GN * j];
+#pragma unroll
+        for (int i = 0; i < RM; ++i)
+#pragma unroll
+          for (int j = 0; j < RN; ++j) acc[i][j] = S<T>::fma(a[i], b[j], acc[i][j]);
       }
     }
-    return;
+    __syncthreads();
   }
   const bool use_beta = S<T>::abs2(beta) != 0.0;
+  auto put = [&](int mm, int nn, T v) {
+    const int gm = m0 + mm, gn = n0 + nn;
+    if (gm >= M || gn >= N) return;
+    T* c = C + (size_t)gm * ldc + gn;
+    T r = alpha * v;
+    if (use_beta) r = S<T>::fma(beta, *c, r);
+    *c = r;
+  };
+  const int nz = gridDim.z;
+  if (nz == 1) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gm = m0 + ty + 16 * i;
-    if (gm >= M) continue;
+    for (int i = 0; i < RM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int gn = n0 + tx + 16 * j;
-      if (gn >= N) continue;
-      T* c = C + (size_t)gm * ldc + gn;
-      T v = alpha * acc[i][j];
-      if (use_beta) v = S<T>::fma(beta, *c, v);
-      *c = v;
-    }
+      for (int j = 0; j < RN; ++j) put(ty + GM * i, tx + GN * j, acc[i][j]);
+    return;
   }
-}
-
-// C = alpha * sum_z part[z] + beta * C, slices summed in order z = 0, 1, ...
-// Small products (M N K below 2 Mi multiply-adds: the chain-end
-// contractions and the small splits' refinements): one thread per output
-// element, blocks of 64 threads along N so that even a 64 x 64 output spreads
-// over 64 SMs; GB300's FP64 rate per SM (~2 FMA per cycle) makes spreading the
-// work, not reusing it, what matters at these sizes.
-template <typename T>
-__global__ void __launch_bounds__(64) k_gemm_small(int opA, int opB, int M, int N, int K, T alpha,
-                                                   const T* __restrict__ A, int lda,
-                                                   const T* __restrict__ B, int ldb, T beta,
-                                                   T* __restrict__ C, int ldc) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x, m = blockIdx.y;
-  if (n >= N) return;
-  T acc = S<T>::zero();
-  for (int k = 0; k < K; ++k) {
-    const T a = load_op(opA == SM_OP_N ? A + (size_t)m * lda + k : A + (size_t)k * lda + m, opA);
-    const T b = load_op(opB == SM_OP_N ? B + (size_t)k * ldb + n : B + (size_t)n * ldb + k, opB);
-    acc = S<T>::fma(a, b, acc);
+  cg::cluster_group cluster = cg::this_cluster();
+  T* tile = reinterpret_cast<T*>(raw);  // [TM][TN]: this slice's partial tile
+#pragma unroll
+  for (int i = 0; i < RM; ++i)
+#pragma unroll
+    for (int j = 0; j < RN; ++j) tile[(ty + GM * i) * TN + tx + GN * j] = acc[i][j];
+  cluster.sync();
+  // each slice adds up its share of the tile
+  const int share = (TM * TN + nz - 1) / nz;
+  const int e1 = min(TM * TN, (int)(blockIdx.z + 1) * share);
+  for (int e = blockIdx.z * share + tid; e < e1; e += 128) {
+    T v = S<T>::zero();
+    for (int z = 0; z < nz; ++z) v = v + cluster.map_shared_rank(tile, z)[e];
+    put(e / TN, e % TN, v);
   }
-  T* c = C + (size_t)m * ldc + n;
-  const bool zero_beta = S<T>::abs2(beta) == 0.0;
-  *c = zero_beta ? alpha * acc : alpha * acc + beta * *c;
+  cluster.sync();  // no slice leaves while another reads its tile
 }
 
 // Matrix-vector shapes (N = 1, or M = 1): the Lanczos projections and norms.
@@ -228,7 +239,7 @@ __global__ void k_splitk_reduce(int M, int N, int nz, const T* __restrict__ part
 }
 
 // ---- FP32-arithmetic variant (contractions of the mixed forms) --------------
-// Same tiling as k_gemm; operands are rounded to FP32 (complex: two FP32) when
+// 64 x 64 tile per CTA, 256 threads holding a 4 x 4 register tile each; operands are rounded to FP32 (complex: two FP32) when
 // staged in shared memory and the products accumulate in FP32; alpha, beta
 // and the output stay FP64.  Relative error ~1e-7 |A||B| per entry.
 template <typename T> struct C32;
@@ -334,6 +345,35 @@ __global__ void __launch_bounds__(NT) k_gemm32(int opA, int opB, int M, int N, i
 
 }  // namespace
 
+namespace {
+
+template <typename T, int TM, int TN, int RM, int RN>
+int launch_gemm(cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha, const T* A, int lda,
+                const T* B, int ldb, T beta, T* C, int ldc, int nz) {
+  const int kchunk = ((K + nz - 1) / nz + 15) / 16 * 16;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((N + TN - 1) / TN, (M + TM - 1) / TM, nz);
+  cfg.blockDim = dim3(128);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = nz;
+  cfg.attrs = attr;
+  cfg.numAttrs = nz > 1 ? 1 : 0;
+  if (cfg.gridDim.y > 65535) {
+    set_error("gemm: M too large");
+    return SM_ERR_VALUE;
+  }
+  SM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_gemm<T, TM, TN, RM, RN>, opA, opB, M, N, K, alpha, A, lda,
+                                   B, ldb, beta, C, ldc, kchunk));
+  note_launch();
+  return SM_OK;
+}
+
+}  // namespace
+
 template <typename T>
 int gemm(cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha, const T* A, int lda,
          const T* B, int ldb, T beta, T* C, int ldc) {
@@ -346,40 +386,36 @@ int gemm(cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha, const 
     // C = beta C  (or zero)
     return scale_matrix<T>(st, M, N, beta, C, ldc);
   }
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM);
-  if (grid.y > 65535) {
-    set_error("gemm: M too large");
-    return SM_ERR_VALUE;
+  // The tile and the number of slices whose fullest SM has the least to do: a CTA
+  // takes TM TN kchunk / 2 clocks of its SM's FP64 pipe and some 1500 clocks of
+  // loads and stores that only further CTAs hide, the slices' sum as much again.
+  // (130 x 130 x 256: 25 tiles of 32 in 6 slices, 150 CTAs, against 8 slices, 200
+  // CTAs on 152 SMs: 22 us.)
+  const int sms = 152;
+  double best = 0.0;
+  int best_t = 0, best_z = 1;
+  for (int t = 16; t <= 32; t += 16) {
+    const double tiles = (double)((M + t - 1) / t) * ((N + t - 1) / t);
+    for (int nz = 1; nz <= 8 && (nz == 1 || K > 16 * (nz - 1)); ++nz) {
+      const int kc = ((K + nz - 1) / nz + 15) / 16 * 16;
+      const double cta = 0.5 * t * t * kc * (sizeof(T) == sizeof(double) ? 1.0 : 4.0) + 1500.0;
+      const double cost = std::ceil(tiles * nz / sms) * cta + (nz > 1 ? 1500.0 : 0.0);
+      if (best_t == 0 || cost < best) {
+        best = cost;
+        best_t = t;
+        best_z = nz;
+      }
+    }
   }
-  k_gemm<T><<<grid, NT, 0, st>>>(opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, K,
-                                 nullptr);
-  note_launch();
-  SM_CUDA_CHECK(cudaGetLastError());
-  return SM_OK;
+  if (best_t == 16)
+    return launch_gemm<T, 16, 16, 1, 2>(st, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc,
+                                        best_z);
+  return launch_gemm<T, 32, 32, 2, 4>(st, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc,
+                                      best_z);
 }
 
-// Split-K variant: `nz` K slices (nz > 1) through the workspace `part`
-// (nz * M * N elements).
-template <typename T>
-int gemm_splitk(cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha, const T* A,
-                int lda, const T* B, int ldb, T beta, T* C, int ldc, int nz, T* part) {
-  const int kchunk = ((K + nz - 1) / nz + BK - 1) / BK * BK;
-  nz = (K + kchunk - 1) / kchunk;
-  dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, nz);
-  k_gemm<T><<<grid, NT, 0, st>>>(opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, kchunk,
-                                 part);
-  note_launch();
-  SM_CUDA_CHECK(cudaGetLastError());
-  const size_t mn = (size_t)M * N;
-  const int blocks = (int)std::min<size_t>((mn + 255) / 256, 4096);
-  k_splitk_reduce<T><<<blocks, 256, 0, st>>>(M, N, nz, part, alpha, beta, C, ldc);
-  note_launch();
-  SM_CUDA_CHECK(cudaGetLastError());
-  return SM_OK;
-}
-
-// K slices for an M x N x K product on `sms` SMs: enough CTAs for about two
-// waves, each slice at least 64 deep; 1 = no split.
+// K slices of the FP32 kernel for an M x N x K product on `sms` SMs: enough CTAs
+// for about two waves, each slice at least 64 deep; 1 = no split.
 int splitk_slices(int M, int N, int K, int sms) {
   const long tiles = (long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
   if (tiles >= sms || K < 128) return 1;
@@ -455,27 +491,7 @@ int gemm_ctx_sel(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int 
     SM_CUDA_CHECK(cudaGetLastError());
     return SM_OK;
   }
-  if ((double)M * N * K <= 2.0 * 1024 * 1024 && M <= 65535) {
-    if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev0, st));
-    k_gemm_small<T><<<dim3((N + 63) / 64, M), 64, 0, st>>>(opA, opB, M, N, K, alpha, A, lda, B, ldb,
-                                                           beta, C, ldc);
-    note_launch();
-    SM_CUDA_CHECK(cudaGetLastError());
-    if (ctx.timing) {
-      SM_CUDA_CHECK(cudaEventRecord(ctx.ev1, st));
-      SM_CUDA_CHECK(cudaEventSynchronize(ctx.ev1));
-      float ms = 0.f;
-      SM_CUDA_CHECK(cudaEventElapsedTime(&ms, ctx.ev0, ctx.ev1));
-      ctx.stats.gemm_ms += ms;
-    }
-    return SM_OK;
-  }
-  const int nz = splitk_slices(M, N, K, std::max(1, ctx.num_sms));
-  T* part = nullptr;
-  if (nz > 1) SM_CHECK(ctx.scratch("gemm.splitk", (size_t)nz * M * N, &part));
   auto run = [&]() -> int {
-    if (nz > 1)
-      return gemm_splitk<T>(st, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, nz, part);
     return gemm<T>(st, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
   };
   if (!ctx.timing) return run();
