@@ -124,8 +124,8 @@ struct SplitResult {
 // Control block of one Jacobi iteration: grid-barrier words, convergence
 // status (DevStatus bits) and the sweep count.
 struct JacobiCtl {
-  unsigned int bar_count;
-  unsigned int bar_gen;
+  unsigned int bar_count;  // grid-barrier arrivals so far
+  unsigned int pad;
   unsigned int rot[2];
   int status;
   int sweeps;
@@ -267,6 +267,21 @@ template <typename T>
 int svd_split(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const sm_strategy& strat,
               int left_mode, T* left, int right_mode, T* right, double* s_out,
               SplitResult* res);
+
+// F = 1.5 I - 0.5 M (F may be M), the Newton-Schulz factor of M = V V^H (k x k), and
+// *dev = max(*dev, the largest entry of |M - I|).
+template <typename T>
+int newton_schulz_matrix(cudaStream_t st, const T* M, int k, T* F, double* dev);
+
+// --- svd_precond.cu ----------------------------------------------------------
+// R <- X R (rows k x l, contiguous) with X unitary to FP64 rounding and the rows
+// close to orthogonal; `converged`: every pair passes the FP64 Jacobi's test
+// (tol2, use_floor, defl_rel as k_jacobi's), so that no Jacobi is needed.  Leaves
+// R as it is where the FP32 stage does not take the size or gives no basis.
+constexpr int kPrecondMinRows = 48;
+template <typename T>
+int precondition_rows(Ctx& ctx, cudaStream_t st, T* R, int k, int l, double tol2, int use_floor,
+                      double defl_rel, bool* converged);
 
 // --- mlp.cu ----------------------------------------------------------------
 // The SM_RANK_FEATURES features of a split of size k about to be made.

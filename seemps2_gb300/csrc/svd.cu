@@ -34,37 +34,36 @@ namespace sm {
 
 namespace {
 
-// Grid-wide barrier with a bounded spin: one arrival counter and a generation
-// word (measured on GB300: ~2.3 us for 16-256 CTAs, cheaper than per-CTA
-// arrival flags gathered by one CTA).  Returns false (and sets the status
-// flag) if the wait exceeded the spin limit.
-__device__ bool grid_sync(JacobiCtl* ctl) {
+// Grid-wide barrier with a bounded spin: one counter that only grows, so that a
+// CTA arrives with a single release add and then polls with acquire loads until
+// all CTAs of this barrier (the `epoch`-th of the launch) have added; nothing is
+// reset, and no fence stands apart from the two accesses (a counter that the
+// last CTA resets and a generation word behind full fences took 2.3 us on 16..256
+// CTAs).  bar_count is zeroed by the caller before the launch.  Returns false
+// (and sets the status flag) if the wait exceeded the spin limit.
+__device__ bool grid_sync(JacobiCtl* ctl, unsigned int& epoch) {
   __shared__ int ok;
   __syncthreads();
   if (threadIdx.x == 0) {
     ok = 1;
     if (gridDim.x > 1) {
-      volatile unsigned int* vgen = &ctl->bar_gen;
-      volatile int* vstatus = &ctl->status;
-      const unsigned int gen = *vgen;
-      __threadfence();
-      const unsigned int arrived = atomicAdd(&ctl->bar_count, 1u);
-      if (arrived == gridDim.x - 1) {
-        atomicExch(&ctl->bar_count, 0u);
-        __threadfence();
-        atomicAdd(&ctl->bar_gen, 1u);
-      } else {
-        long long it = 0;
-        while (*vgen == gen) {
-          if (++it > kSpinLimit || (*vstatus & DEV_BARRIER_TIMEOUT)) {
-            atomicOr(&ctl->status, DEV_BARRIER_TIMEOUT);
-            ok = 0;
-            break;
-          }
-          __nanosleep(32);
+      const unsigned int target = ++epoch * gridDim.x;
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->bar_count) : "memory");
+      long long it = 0;
+      while (true) {
+        unsigned int seen;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];"
+                     : "=r"(seen)
+                     : "l"(&ctl->bar_count)
+                     : "memory");
+        if ((int)(seen - target) >= 0) break;
+        if (++it > kSpinLimit ||
+            ((it & 255) == 0 && (*(volatile int*)&ctl->status & DEV_BARRIER_TIMEOUT))) {
+          atomicOr(&ctl->status, DEV_BARRIER_TIMEOUT);
+          ok = 0;
+          break;
         }
       }
-      __threadfence();
     }
   }
   __syncthreads();
@@ -149,6 +148,93 @@ template <> struct Rot<cplx> {
   }
 };
 
+// 1 / sqrt(x) by Newton's iteration y <- y (1.5 - 0.5 x y^2) from an FP32 start
+// (error ~1e-7, squared twice); outside the FP32 range by division.  A chain of a
+// dozen FP64 operations is what a reflector waits for: each holds the pipe for 64
+// clocks, and the library's sqrt and division took half of a step.
+__device__ __forceinline__ double rsqrt_newton(double x) {
+  if (!(x > 1e-30 && x < 1e30)) return 1.0 / sqrt(x);
+  double y = (double)rsqrtf((float)x);
+  const double hx = -0.5 * x;
+  y = y * fma(hx * y, y, 1.5);
+  return y * fma(hx * y, y, 1.5);
+}
+// 1 / x likewise, y <- y (2 - x y)
+__device__ __forceinline__ double recip_newton(double x) {
+  if (!(x > 1e-30 && x < 1e30)) return 1.0 / x;
+  double y = (double)__frcp_rn((float)x);
+  y = y * fma(-x, y, 2.0);
+  return y * fma(-x, y, 2.0);
+}
+
+// Jacobi rotation of a pair of rows with squared norms a, b and overlap g = gr + i gi
+// (g2 = |g|^2): cosine c, sine sn, phase (er, ei) of g, and the norms after it.
+template <bool kCplx>
+__device__ __forceinline__ void jacobi_angle(double a, double b, double gr, double gi, double g2,
+                                             double& c, double& sn, double& er, double& ei,
+                                             double& na, double& nb) {
+  // Angle in FP32 on values scaled by a power of two so that a + b
+  // lands in [1, 2): zeta = (b - a) / 2|g|, t = sign(zeta) /
+  // (|zeta| + sqrt(1 + zeta^2)).  The (c, s) pair (and the complex
+  // phase) are then brought to unit norm in FP64 with a two-term
+  // correction f = 1 - d/2 + 3d^2/8, d = c^2 + s^2 - 1 ~ 1e-7, which
+  // leaves c^2 + s^2 - 1 = O(d^3): each rotation is unitary to FP64
+  // rounding whatever the accuracy of the angle.
+  // An FP32 angle annihilates the overlap only to ~1e-7 of itself.
+  // Far from convergence that is harmless (the next sweep finishes
+  // the job), but once the pair's cosine |g|/sqrt(ab) is small the
+  // residual no longer shrinks quadratically, and inside a cluster
+  // of (nearly) equal singular values the iteration stalls at the
+  // FP32 level.  So the FP32 angle is only taken while the cosine is
+  // at least 1e-4; the last sweeps' few rotations use FP64.
+  const int ex = (__double2hiint(a + b) >> 20) & 0x7ff;
+  const double sc = __hiloint2double((2046 - ex) << 20, 0);     // 2^(1023 - ex)
+  const float as = (float)(a * sc), bs = (float)(b * sc);
+  // |g| and its phase (complex: brought near 1 by a power of two before squaring)
+  double gabs = fabs(gr);
+  er = gr >= 0.0 ? 1.0 : -1.0;  // the phase of a real overlap is its sign
+  ei = 0.0;
+  if constexpr (kCplx) {
+    const int eg = (__double2hiint(fmax(gabs, fabs(gi))) >> 20) & 0x7ff;
+    const double sg = eg > 0 && eg < 2046 ? __hiloint2double((2046 - eg) << 20, 0) : 1.0;
+    const double xr = gr * sg, xi = gi * sg, x2 = fma(xr, xr, xi * xi);
+    const double rn = rsqrt_newton(x2);
+    er = xr * rn;
+    ei = xi * rn;
+    gabs = x2 * rn * (eg > 0 && eg < 2046 ? __hiloint2double(eg << 20, 0) : 1.0);
+  }
+  double tt;
+  float zf = 0.0f;
+  const float gabs_f = (float)(gabs * sc);
+  const bool fp32_ok = ex > 0 && ex < 2046 && gabs_f > 1e-30f && g2 >= 1e-8 * a * b;
+  if (fp32_ok) zf = 0.5f * (bs - as) / gabs_f;
+  if (fp32_ok && fabsf(zf) < 1e18f) {
+    const float az = fabsf(zf);
+    const float tf = copysignf(1.0f / (az + sqrtf(fmaf(az, az, 1.0f))), zf);
+    const float cf = rsqrtf(fmaf(tf, tf, 1.0f));
+    const double c64 = (double)cf, s64 = (double)(cf * tf);
+    const double d = fma(c64, c64, fma(s64, s64, -1.0));
+    const double f = fma(d, fma(0.375, d, -0.5), 1.0);
+    c = c64 * f;
+    sn = s64 * f;
+    tt = (double)tf;
+  } else {
+    // small cosines, extremely graded pairs: tan = 2|g| / (|b - a| + root), the root
+    // and the quotient by Newton's iteration in FP64
+    const bool in_range = ex > 0 && ex < 2046;
+    const double ds = in_range ? (b - a) * sc : b - a, hs = 2.0 * (in_range ? gabs * sc : gabs);
+    const double q = fma(ds, ds, hs * hs);
+    const double r = q > 0.0 ? q * rsqrt_newton(q) : 0.0;
+    tt = r > 0.0 ? copysign(hs * recip_newton(fabs(ds) + r), ds) : 1.0;
+    c = rsqrt_newton(fma(tt, tt, 1.0));
+    sn = c * tt;
+  }
+  // closed-form norm update (approximate; exact norms return at the
+  // first round of the next sweep)
+  na = fma(-tt, gabs, a);
+  nb = fma(tt, gabs, b);
+}
+
 // One CTA (NT threads, NT/32 warps) per pair, so that every SM sub-partition's
 // FP64 unit works on a pair (GB300 FP64 is latency-bound with one warp per
 // pair).  Each row is [w | x]: the l entries of the vector being
@@ -192,6 +278,7 @@ __global__ void __launch_bounds__(NT) k_jacobi(T* Wx, int ld, int k, int l, int 
   // rows whose squared norm falls to thr or below are deflated: the
   // truncation rule certainly discards them, so they leave the round-robin
   const double thr = defl_abs > 0.0 ? fmin(defl_rel * frob2, defl_abs) : defl_rel * frob2;
+  unsigned int epoch = 0;  // grid barriers so far
   int it = 0;  // pair iterations of this CTA (selects the smem buffer)
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     // exact squared norms at the start of every sweep
@@ -209,7 +296,7 @@ __global__ void __launch_bounds__(NT) k_jacobi(T* Wx, int ld, int k, int l, int 
       }
       __syncthreads();
     }
-    if (!grid_sync(ctl)) return;
+    if (!grid_sync(ctl, epoch)) return;
     // every CTA read the previous sweep's rotation flag before this barrier
     if (sweep > 0 && blockIdx.x == 0 && tid == 0) vflag[(sweep + 1) & 1] = 0;
     // active rows, in ascending order, compacted by CTA 0
@@ -232,7 +319,7 @@ __global__ void __launch_bounds__(NT) k_jacobi(T* Wx, int ld, int k, int l, int 
       }
       if (tid == 0) ((volatile int*)&ctl->nact)[0] = base;
     }
-    if (!grid_sync(ctl)) return;
+    if (!grid_sync(ctl, epoch)) return;
     if (tid == 0) snact = ((volatile int*)&ctl->nact)[0];
     __syncthreads();
     const int ka = snact;
@@ -319,73 +406,8 @@ __global__ void __launch_bounds__(NT) k_jacobi(T* Wx, int ld, int k, int l, int 
         const bool rot = g2 > tiny2 && g2 > tol2 * a * b;
         double na = a, nb = b;
         if (rot) {
-          // Angle in FP32 on values scaled by a power of two so that a + b
-          // lands in [1, 2): zeta = (b - a) / 2|g|, t = sign(zeta) /
-          // (|zeta| + sqrt(1 + zeta^2)).  The (c, s) pair (and the complex
-          // phase) are then brought to unit norm in FP64 with a two-term
-          // correction f = 1 - d/2 + 3d^2/8, d = c^2 + s^2 - 1 ~ 1e-7, which
-          // leaves c^2 + s^2 - 1 = O(d^3): each rotation is unitary to FP64
-          // rounding whatever the accuracy of the angle.
-          // An FP32 angle annihilates the overlap only to ~1e-7 of itself.
-          // Far from convergence that is harmless (the next sweep finishes
-          // the job), but once the pair's cosine |g|/sqrt(ab) is small the
-          // residual no longer shrinks quadratically, and inside a cluster
-          // of (nearly) equal singular values the iteration stalls at the
-          // FP32 level.  So the FP32 angle is only taken while the cosine is
-          // at least 1e-4; the last sweeps' few rotations use FP64.
-          const int ex = (__double2hiint(a + b) >> 20) & 0x7ff;
-          const double sc = __hiloint2double((2046 - ex) << 20, 0);     // 2^(1023 - ex)
-          const double sc_inv = __hiloint2double(ex << 20, 0);           // 2^(ex - 1023)
-          const float as = (float)(a * sc), bs = (float)(b * sc);
-          const float grs = (float)(gr * sc), gis = kCplx ? (float)(gi * sc) : 0.0f;
-          const float gabs_f = kCplx ? sqrtf(fmaf(grs, grs, gis * gis)) : fabsf(grs);
-          double tt, c, sn;
-          float zf = 0.0f;
-          const bool fp32_ok = ex > 0 && ex < 2046 && gabs_f > 1e-30f && g2 >= 1e-8 * a * b;
-          if (fp32_ok) zf = 0.5f * (bs - as) / gabs_f;
-          if (fp32_ok && fabsf(zf) < 1e18f) {
-            const float az = fabsf(zf);
-            const float tf = copysignf(1.0f / (az + sqrtf(fmaf(az, az, 1.0f))), zf);
-            const float cf = rsqrtf(fmaf(tf, tf, 1.0f));
-            const double c64 = (double)cf, s64 = (double)(cf * tf);
-            const double d = fma(c64, c64, fma(s64, s64, -1.0));
-            const double f = fma(d, fma(0.375, d, -0.5), 1.0);
-            c = c64 * f;
-            sn = s64 * f;
-            tt = (double)tf;
-          } else {
-            // extremely graded pair (|g| below 1e-30 (a + b) or |zeta| >= 1e18):
-            // the whole angle in FP64, rare
-            const double zeta = 0.5 * (b - a) / sqrt(g2);
-            const double az = fabs(zeta);
-            tt = az < 1e150 ? 1.0 / (az + sqrt(fma(az, az, 1.0))) : 0.5 / az;
-            tt = copysign(tt, zeta);
-            c = 1.0 / sqrt(fma(tt, tt, 1.0));
-            sn = c * tt;
-          }
-          double er, ei;
-          if constexpr (kCplx) {
-            if (fp32_ok) {
-              const float inv = 1.0f / gabs_f;
-              const double e_r = (double)(grs * inv), e_i = (double)(gis * inv);
-              const double de = fma(e_r, e_r, fma(e_i, e_i, -1.0));
-              const double fe = fma(de, fma(0.375, de, -0.5), 1.0);
-              er = e_r * fe;
-              ei = e_i * fe;
-            } else {
-              const double inv = 1.0 / sqrt(g2);
-              er = gr * inv;
-              ei = gi * inv;
-            }
-          } else {
-            er = gr >= 0.0 ? 1.0 : -1.0;  // the phase of a real overlap is its sign
-            ei = 0.0;
-          }
-          // closed-form norm update (approximate; exact norms return at the
-          // first round of the next sweep)
-          const double gabs = fp32_ok ? (double)gabs_f * sc_inv : sqrt(g2);
-          na = fma(-tt, gabs, a);
-          nb = fma(tt, gabs, b);
+          double c, sn, er, ei;
+          jacobi_angle<kCplx>(a, b, gr, gi, g2, c, sn, er, ei, na, nb);
           Rot<T> R;
           R.set(c, sn, er, ei);
           if constexpr (E > 0) {
@@ -413,7 +435,7 @@ __global__ void __launch_bounds__(NT) k_jacobi(T* Wx, int ld, int k, int l, int 
           __stcg(nrm + q, nb);
         }
       }
-      if (!grid_sync(ctl)) return;
+      if (!grid_sync(ctl, epoch)) return;
     }
     if (tid == 0) sflag = vflag[sweep & 1];
     __syncthreads();
@@ -816,12 +838,12 @@ int truncate_device(Ctx& ctx, cudaStream_t st, const double* s_dev, int n,
 // ---------------------------------------------------------------------------
 struct QrCtl {
   JacobiCtl bar;  // barrier words and status, shared layout with the Jacobi kernel
-  int steps;      // reflections performed (the rank estimate)
-  int pad;
+  int steps;      // rows of R above the stopping threshold (the rank estimate)
+  int done;       // reflections performed (>= steps)
   double tau[2];  // tau of the published reflector, by step parity
 };
 
-__device__ bool qr_grid_sync(QrCtl* ctl) { return grid_sync(&ctl->bar); }
+__device__ bool qr_grid_sync(QrCtl* ctl, unsigned int& epoch) { return grid_sync(&ctl->bar, epoch); }
 
 // Reflector for x = Wt[c][j:k]: v = x + nu e1, nu = (x0/|x0|) |x|,
 // tau = 1 / (|x| (|x| + |x0|)); writes v (v0 = x0 + nu) to vdst[j:k] and sets
@@ -861,6 +883,7 @@ __global__ void __launch_bounds__(NT) k_house_qr(T* Wt, int k, int l, double thr
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gw = blockIdx.x * NW + warp, nw = gridDim.x * NW;
   const int nmax = k < l ? k : l;
+  unsigned int epoch = 0;
   // |W|_F^2
   {
     double a = 0.0;
@@ -878,7 +901,7 @@ __global__ void __launch_bounds__(NT) k_house_qr(T* Wt, int k, int l, double thr
     // reflector 0 from column 0
     if (gw == 0) qr_reflector<T>(Wt, 0, k, vbuf, &ctl->tau[0]);
   }
-  if (!qr_grid_sync(ctl)) return;
+  if (!qr_grid_sync(ctl, epoch)) return;
   // per-CTA partials summed by every warp in the same order (lane-strided,
   // then a fixed shuffle tree): a serial FP64 sum over 100+ CTAs costs
   // microseconds on GB300's FP64 unit
@@ -931,7 +954,7 @@ __global__ void __launch_bounds__(NT) k_house_qr(T* Wt, int k, int l, double thr
       for (int w = 0; w < NW; ++w) t += wpart[w];
       __stcg(part + blockIdx.x, t);
     }
-    if (!qr_grid_sync(ctl)) return;
+    if (!qr_grid_sync(ctl, epoch)) return;
     if (warp == 0) {
       double tot = 0.0;
       for (int b = lane; b < (int)gridDim.x; b += 32) tot += __ldcg(part + b);
@@ -945,15 +968,214 @@ __global__ void __launch_bounds__(NT) k_house_qr(T* Wt, int k, int l, double thr
       break;
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) ctl->steps = steps;
+  if (blockIdx.x == 0 && threadIdx.x == 0) ctl->steps = ctl->done = steps;
 }
 
-// Wx[i][c] = R[i][c] from Wt after `steps` reflections: row i < steps is the
+// The same factorisation with every column in the registers of one warp (lane i
+// holds rows i, i + 32, ...: E >= k / 32), for the whole of it: a step reads only
+// the reflector.  gridDim.x * NT / 32 >= l.  The trailing weights are summed once
+// per kQrBatch steps, for all of them (a later reflection leaves the weight below
+// an earlier step unchanged); the factorisation stops at the first batch that
+// holds a step whose trailing block is at most thr_rel |W|_F^2, and that step is
+// the rank.  What bounds a step is its chain: the barrier, the reflector through
+// L2, two passes over the column and two FP64 warp sums, one reciprocal root.
+// 174 x 190: 0.84 ms with columns streamed through L2 and a test per step, see
+// the launcher for the time now.
+constexpr int kQrBatch = 4;
+template <typename T, int NT, int E>
+__global__ void __launch_bounds__(NT) k_house_qr_reg(T* Wt, int k, int l, double thr_rel, T* vbuf,
+                                                     double* part, QrCtl* ctl) {
+  constexpr int NW = NT / 32;
+  __shared__ double wpart[kQrBatch][NW];
+  __shared__ int below[kQrBatch];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int c = blockIdx.x * NW + warp;
+  const int nmax = k < l ? k : l;
+  unsigned int epoch = 0;
+  T y[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = lane + 32 * e;
+    y[e] = (c < l && i < k) ? ldcg(Wt + (size_t)c * k + i) : S<T>::zero();
+  }
+  // sum over the CTA's warps of NV values each into wpart, then into part[value][block]
+  auto publish_sums = [&](const double* v, int n, int slot) {
+#pragma unroll
+    for (int s = 0; s < kQrBatch; ++s) {
+      if (s >= n) break;
+      double a = v[s];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+      if (lane == 0) wpart[s][warp] = a;
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < n) {
+      double t = 0.0;
+      for (int w = 0; w < NW; ++w) t += wpart[threadIdx.x][w];
+      __stcg(part + (size_t)(slot + threadIdx.x) * gridDim.x + blockIdx.x, t);
+    }
+  };
+  // sum of part[s][*] over the grid, by one warp
+  auto grid_sum = [&](int s) {
+    double t = 0.0;
+    for (int b = lane; b < (int)gridDim.x; b += 32) t += __ldcg(part + (size_t)s * gridDim.x + b);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    return t;
+  };
+  // reflector of this warp's column for pivot row j (its rows >= j), published by
+  // the step's parity; the column's rows below j become those of R (zero)
+  auto reflector = [&](int j) {
+    double n2 = 0.0;
+    T x0 = S<T>::zero();
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int i = lane + 32 * e;
+      if (32 * e + 31 < j) continue;
+      if (i >= j) n2 += S<T>::abs2(y[e]);
+      if (i == j) x0 = y[e];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+    if constexpr (sizeof(T) == sizeof(double)) {
+      x0 = __shfl_sync(0xffffffffu, x0, j & 31);
+    } else {
+      x0 = cplx{__shfl_sync(0xffffffffu, x0.re, j & 31), __shfl_sync(0xffffffffu, x0.im, j & 31)};
+    }
+    T nu = S<T>::zero();
+    double tau = 0.0;
+    if (n2 > 0.0) {
+      const double nx = n2 * rsqrt_newton(n2);
+      double a0;
+      if constexpr (sizeof(T) == sizeof(double)) {
+        a0 = fabs(x0);
+        nu = copysign(nx, x0);
+      } else {
+        const double x2 = S<T>::abs2(x0);
+        const double r = x2 > 0.0 ? rsqrt_newton(x2) : 0.0;
+        a0 = x2 * r;
+        nu = x2 > 0.0 ? S<T>::scale(x0, nx * r) : S<T>::from_real(nx);
+      }
+      tau = recip_newton(fma(nx, a0, n2));
+    }
+    T* v = vbuf + (size_t)(j & 1) * k;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const int i = lane + 32 * e;
+      if (32 * e + 31 < j) continue;
+      if (i >= j && i < k) stcg(v + i, i == j ? y[e] + nu : y[e]);
+      if (i == j) y[e] = S<T>::scale(nu, -1.0);
+      else if (i > j) y[e] = S<T>::zero();
+    }
+    if (lane == 0) __stcg(&ctl->tau[j & 1], tau);
+  };
+  double thr;
+  {
+    double a = 0.0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) a += S<T>::abs2(y[e]);
+    // the last slot: no batch writes it before a barrier has passed (a one-step
+    // batch writes slot 0 right away)
+    publish_sums(&a, 1, kQrBatch - 1);
+    if (c == 0) reflector(0);
+    if (!qr_grid_sync(ctl, epoch)) return;
+    thr = thr_rel * grid_sum(kQrBatch - 1);
+  }
+  int steps = nmax, done = nmax;
+  for (int j = 0; j < nmax; ++j) {
+    if (c > j) {
+      const T* v = vbuf + (size_t)(j & 1) * k;
+      const double tau = __ldcg(&ctl->tau[j & 1]);
+      T vv[E];
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int i = lane + 32 * e;
+        vv[e] = S<T>::zero();
+        if (32 * e + 31 >= j && i >= j && i < k) vv[e] = ldcg(v + i);
+      }
+      T w = S<T>::zero();
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        if (32 * e + 31 >= j) w = S<T>::cfma(vv[e], y[e], w);
+      double wr, wi;
+      gamma_parts(w, wr, wi);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        wr += __shfl_xor_sync(0xffffffffu, wr, o);
+        if constexpr (sizeof(T) != sizeof(double)) wi += __shfl_xor_sync(0xffffffffu, wi, o);
+      }
+      T tw;  // y -= tau (v^H y) v
+      if constexpr (sizeof(T) == sizeof(double)) tw = -tau * wr;
+      else tw = cplx{-tau * wr, -tau * wi};
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        if (32 * e + 31 >= j) y[e] = S<T>::fma(tw, vv[e], y[e]);
+    }
+    const int first = j - j % kQrBatch, n = j - first + 1;  // steps of this batch
+    const bool last = n == kQrBatch || j + 1 == nmax;
+    if (last) {
+      double sum[kQrBatch];
+#pragma unroll
+      for (int s = 0; s < kQrBatch; ++s) sum[s] = 0.0;
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const int i = lane + 32 * e;
+        if (32 * e + 31 < first) continue;
+        const double a = S<T>::abs2(y[e]);
+        if (i > j) {
+          sum[kQrBatch - 1] += a;
+        } else {
+#pragma unroll
+          for (int s = 0; s < kQrBatch - 1; ++s)
+            if (i == first + 1 + s) sum[s] += a;
+        }
+      }
+      // sum[s] = the weight below step first + s: the tail, and the rows between
+      double run = sum[kQrBatch - 1];
+#pragma unroll
+      for (int s = kQrBatch - 1; s >= 0; --s) {
+        if (s < kQrBatch - 1) run += first + 1 + s <= j ? sum[s] : 0.0;
+        sum[s] = c > first + s ? run : 0.0;
+      }
+      publish_sums(sum, n, 0);
+    }
+    // the next reflector: this column is up to date
+    if (c == j + 1 && j + 1 < nmax) reflector(j + 1);
+    if (!qr_grid_sync(ctl, epoch)) return;
+    if (last) {
+      for (int s = warp; s < n; s += NW) {
+        const double t = grid_sum(s);
+        if (lane == 0) below[s] = t <= thr;
+      }
+      __syncthreads();
+      int stop = -1;
+      for (int s = n - 1; s >= 0; --s)
+        if (below[s]) stop = s;
+      __syncthreads();  // `below` is written again four steps later
+      if (stop >= 0) {
+        steps = first + stop + 1;
+        done = j + 1;
+        break;
+      }
+    }
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    ctl->steps = steps;
+    ctl->done = done;
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const int i = lane + 32 * e;
+    if (c < l && i < k) stcg(Wt + (size_t)c * k + i, y[e]);
+  }
+}
+
+// Wx[i][c] = R[i][c] from Wt after `steps` (ctl->done) reflections: row i < steps is the
 // upper-triangular row of R; rows i >= steps are the trailing block rows.
 template <typename T>
 __global__ void k_qr_extract(const T* __restrict__ Wt, int k, int l, int kk, const QrCtl* ctl,
                              T* __restrict__ Wx, JacobiCtl* jctl) {
-  const int steps = ctl->steps;
+  const int steps = ctl->done;
   // a QR barrier timeout is reported through the Jacobi status word
   if (blockIdx.x == 0 && threadIdx.x == 0 && ctl->bar.status)
     atomicOr(&jctl->status, ctl->bar.status);
@@ -964,6 +1186,50 @@ __global__ void k_qr_extract(const T* __restrict__ Wt, int k, int l, int kk, con
     const int first = i < steps ? i : steps;
     Wx[e] = c >= first ? Wt[(size_t)c * k + i] : S<T>::zero();
   }
+}
+
+// Launches the factorisation: columns in registers where a warp per column fits the
+// GPU at once and a lane's share of a column its registers, else (and for a
+// context that shares the device, whose grid is one CTA) streamed through L2.
+template <typename T>
+int house_qr(Ctx& ctx, cudaStream_t st, T* Wt, int kw, int l, double thr_rel, T* vbuf, QrCtl* qctl) {
+  constexpr int NT = 128;
+  const int cols = (l + NT / 32 - 1) / (NT / 32);  // CTAs at a warp per column
+  auto per_sm_of = [&](const void* fn) {
+    const auto it = ctx.coop_blocks.find(fn);
+    if (it != ctx.coop_blocks.end()) return it->second;
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, fn, NT, 0) != cudaSuccess) n = 1;
+    return ctx.coop_blocks[fn] = std::max(1, n);
+  };
+  const int sms = std::max(1, ctx.num_sms);
+  const void* fn = nullptr;
+  if (!ctx.concurrent) {
+    const int e = (kw + 31) / 32;
+    constexpr bool real = sizeof(T) == sizeof(double);
+    if (e <= 2) fn = reinterpret_cast<const void*>(k_house_qr_reg<T, NT, 2>);
+    else if (e <= 4) fn = reinterpret_cast<const void*>(k_house_qr_reg<T, NT, 4>);
+    else if (e <= 6) fn = reinterpret_cast<const void*>(k_house_qr_reg<T, NT, 6>);
+    else if (e <= 8) fn = reinterpret_cast<const void*>(k_house_qr_reg<T, NT, 8>);
+    else if (e <= 12) fn = reinterpret_cast<const void*>(k_house_qr_reg<T, NT, 12>);
+    else if (e <= 16) fn = reinterpret_cast<const void*>(k_house_qr_reg<T, NT, 16>);
+    if constexpr (real) {
+      if (e > 16 && e <= 24) fn = reinterpret_cast<const void*>(k_house_qr_reg<T, NT, 24>);
+      else if (e > 24 && e <= 32) fn = reinterpret_cast<const void*>(k_house_qr_reg<T, NT, 32>);
+    }
+    if (fn && cols > per_sm_of(fn) * sms) fn = nullptr;
+  }
+  int grid = cols;
+  if (!fn) {
+    fn = reinterpret_cast<const void*>(k_house_qr<T, NT>);
+    grid = ctx.concurrent ? 1 : std::max(1, std::min(cols, per_sm_of(fn) * sms));
+  }
+  double* part;
+  SM_CHECK(ctx.scratch("svd.qpart", (size_t)kQrBatch * grid, &part));
+  void* args[] = {&Wt, &kw, &l, &thr_rel, &vbuf, &part, &qctl};
+  SM_CHECK(coop_launch(fn, dim3(grid), dim3(NT), args, st));
+  note_launch();
+  return SM_OK;
 }
 
 // Split where only one factor must be an isometry: U for (OUT_U, OUT_SVT)
@@ -985,7 +1251,7 @@ int svd_split_xfree(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   const int k = std::min(kw, l);  // rows of R, = min(m, n) singular values
   const int ld = l;
   T *Wt, *Wx, *vbuf;
-  double *nrm, *nrm0, *s_sorted, *errors, *qpart;
+  double *nrm, *nrm0, *s_sorted, *errors;
   int *perm, *act;
   JacobiCtl* ctl;
   QrCtl* qctl;
@@ -1004,6 +1270,15 @@ int svd_split_xfree(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   SM_CHECK(ctx.scratch("svd.res", 1, &res));
   int* wexp;
   SM_CHECK(ctx.scratch("svd.wexp", 1, &wexp));
+  double drel, dabs;
+  deflation(strat, k, &drel, &dabs);
+  const double eps = DBL_EPSILON;
+  bool use_floor = false;
+  if (strat.method == SM_RELATIVE_NORM_SQUARED_ERROR)
+    use_floor = strat.tolerance >= 64.0 * k * (double)l * eps * eps;
+  else if (strat.method == SM_RELATIVE_SINGULAR_VALUE)
+    use_floor = strat.tolerance >= 16.0 * std::sqrt((double)k * l) * eps;
+  const double tol = std::sqrt((double)l) * DBL_EPSILON;
   // Wt = W^T (l x kw): A itself for U, A^T for V; then scaled to O(1) entries
   if (want_u) {
     SM_CUDA_CHECK(cudaMemcpyAsync(Wt, A, sizeof(T) * (size_t)m * n, cudaMemcpyDeviceToDevice, st));
@@ -1011,31 +1286,10 @@ int svd_split_xfree(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
     SM_CHECK(transpose<T>(st, m, n, A, n, Wt, m));
   }
   SM_CHECK(prescale<T>(st, Wt, l, kw, kw, wexp));
-  double drel, dabs;
-  deflation(strat, k, &drel, &dabs);
   // rank-revealing QR preconditioner: W = Q R, R has k rows
   {
-    constexpr int QNT = 128;
-    auto fn = k_house_qr<T, QNT>;
-    const void* key = reinterpret_cast<const void*>(fn);
-    int per_sm = 0;
-    const auto it = ctx.coop_blocks.find(key);
-    if (it != ctx.coop_blocks.end()) per_sm = it->second;
-    else {
-      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, QNT, 0) != cudaSuccess) per_sm = 1;
-      per_sm = std::max(1, per_sm);
-      ctx.coop_blocks[key] = per_sm;
-    }
-    const int grid =
-        ctx.concurrent
-            ? 1  // one CTA: no grid barrier to wait on (see run_jacobi)
-            : std::max(1, std::min((l + QNT / 32 - 1) / (QNT / 32), per_sm * std::max(1, ctx.num_sms)));
-    SM_CHECK(ctx.scratch("svd.qpart", (size_t)grid, &qpart));
     SM_CUDA_CHECK(cudaMemsetAsync(qctl, 0, sizeof(QrCtl), st));
-    int kk = kw, ll = l;
-    void* args[] = {&Wt, &kk, &ll, &drel, &vbuf, &qpart, &qctl};
-    SM_CHECK(coop_launch(reinterpret_cast<const void*>(fn), dim3(grid), dim3(QNT), args, st));
-    note_launch();
+    SM_CHECK(house_qr<T>(ctx, st, Wt, kw, l, drel, vbuf, qctl));
     const size_t tot = (size_t)k * l;
     const int blocks = (int)std::max<size_t>(1, std::min<size_t>((tot + 255) / 256, 4096));
     SM_CUDA_CHECK(cudaMemsetAsync(ctl, 0, sizeof(JacobiCtl), st));
@@ -1043,20 +1297,26 @@ int svd_split_xfree(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
     note_launch();
     SM_CUDA_CHECK(cudaGetLastError());
   }
-  const double eps = DBL_EPSILON;
-  bool use_floor = false;
-  if (strat.method == SM_RELATIVE_NORM_SQUARED_ERROR)
-    use_floor = strat.tolerance >= 64.0 * k * (double)l * eps * eps;
-  else if (strat.method == SM_RELATIVE_SINGULAR_VALUE)
-    use_floor = strat.tolerance >= 16.0 * std::sqrt((double)k * l) * eps;
   if (k >= 2) {
     k_row_norms<T><<<(k + 7) / 8, 256, 0, st>>>(Wx, ld, k, l, nrm0, 1);
     note_launch();
     SM_CUDA_CHECK(cudaGetLastError());
-    const double tol = std::sqrt((double)l) * DBL_EPSILON;
     if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev0, st));
-    SM_CHECK(run_jacobi<T>(ctx, st, Wx, ld, k, l, l, tol * tol, use_floor ? 1 : 0, drel, dabs, nrm,
-                           nrm0, act, ctl));
+    // the rows of R (the QR's steps; the rows below them are discarded weight)
+    // through the FP32 start; the Jacobi only where that leaves pairs to rotate
+    bool converged = false;
+    if (k >= kPrecondMinRows) {
+      QrCtl* hq = reinterpret_cast<QrCtl*>(ctx.pinned);
+      SM_CUDA_CHECK(cudaMemcpyAsync(hq, qctl, sizeof(QrCtl), cudaMemcpyDeviceToHost, st));
+      SM_CUDA_CHECK(cudaStreamSynchronize(st));
+      const int steps = hq->steps;
+      if (hq->bar.status == 0)
+        SM_CHECK(precondition_rows<T>(ctx, st, Wx, steps, l, tol * tol, use_floor ? 1 : 0, drel,
+                                      &converged));
+    }
+    if (!converged)
+      SM_CHECK(run_jacobi<T>(ctx, st, Wx, ld, k, l, l, tol * tol, use_floor ? 1 : 0, drel, dabs, nrm,
+                             nrm0, act, ctl));
     if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev1, st));
     ctx.stats.jacobi_launches += 1;
     ctx.stats.jacobi_flops += (4.0 * std::max(m, n) * (double)k * k + 8.0 * (double)k * k * k) *
@@ -1257,15 +1517,14 @@ __global__ void k_refine_matrix(const T* __restrict__ G, const T* __restrict__ M
 // dev = max |M - I| over the grid (atomic max on the bits of the non-negative
 // double; dev must be zero beforehand).
 template <typename T>
-__global__ void __launch_bounds__(256) k_ns_matrix(const T* __restrict__ M, int k,
-                                                   T* __restrict__ F, double* dev) {
+__global__ void __launch_bounds__(256) k_ns_matrix(const T* M, int k, T* F, double* dev) {
   __shared__ double red[8];
   const size_t tot = (size_t)k * k;
   double worst = 0.0;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot;
        e += (size_t)gridDim.x * blockDim.x) {
-    T f = S<T>::scale(M[e], -0.5);
     T d = M[e];
+    T f = S<T>::scale(d, -0.5);
     if (e / k == e % k) {
       f = f + S<T>::from_real(1.5);
       d = d - S<T>::one();
@@ -1515,6 +1774,16 @@ double allowed_discard(const sm_strategy& st, double norm2, double s0, int k, in
 }
 
 }  // namespace
+
+template <typename T>
+int newton_schulz_matrix(cudaStream_t st, const T* M, int k, T* F, double* dev) {
+  k_ns_matrix<T><<<grid_for((size_t)k * k), 256, 0, st>>>(M, k, F, dev);
+  note_launch();
+  SM_CUDA_CHECK(cudaGetLastError());
+  return SM_OK;
+}
+template int newton_schulz_matrix<double>(cudaStream_t, const double*, int, double*, double*);
+template int newton_schulz_matrix<cplx>(cudaStream_t, const cplx*, int, cplx*, double*);
 
 // rf_k > 0 (real operands): instead of factoring W, the cluster factors
 // BH = W^T Q (l x rf_k) of a randomized range finder (rangefinder.cu) sized by

@@ -318,8 +318,10 @@ __global__ void __launch_bounds__(kCNT, 1)
   const double nrm = sqrt(norm2);
   const double scale = nrm > 0.0 ? 1.0 / nrm : 1.0;
   // stop once the trailing block holds at most max(thr_rel |W|^2, thr_abs)
+  // (thr_rel < 0: only at an empty trailing block, so that all kmax rows come out)
   const float thr =
-      fmaxf((float)fmax(thr_rel, norm2 > 0.0 ? thr_abs / norm2 : 0.0), kQrFloor);
+      thr_rel < 0.0 ? 0.f
+                    : fmaxf((float)fmax(thr_rel, norm2 > 0.0 ? thr_abs / norm2 : 0.0), kQrFloor);
   for (int s = warp; s < ncs; s += kCNW) {
     const int c = col_of(s);
     if (c >= l) break;
