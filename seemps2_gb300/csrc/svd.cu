@@ -1232,6 +1232,258 @@ int house_qr(Ctx& ctx, cudaStream_t st, T* Wt, int kw, int l, double thr_rel, T*
   return SM_OK;
 }
 
+// ---------------------------------------------------------------------------
+// Small splits: the whole of the FP64 path above (scaling, Householder QR, Jacobi,
+// sorting, truncation) in one CTA with the matrix in shared memory.  The splits at
+// the ends of a chain have 2..48 rows; on the kernels above they pay a launch for
+// each phase and a grid barrier for each reflector and each round (32 x 32: 1.4 ms),
+// while one SM's FP64 pipe does a round of them in about a microsecond.
+//
+// A pair of rows (and a column of the QR) belongs to 8 lanes: four pairs share the
+// FP64 instructions of a warp, so that their sums take three shuffle levels and the
+// angle's scalar chain is paid once for the four (each FP64 instruction holds the
+// pipe for 64 clocks whatever its active lanes).  256 threads take 32 pairs at once.
+// ---------------------------------------------------------------------------
+constexpr int kSmallNT = 256;
+constexpr int kSmallRows = 48;           // rows of R at most
+constexpr size_t kSmallBytes = 160 * 1024;  // W in shared memory at most
+constexpr double kSmallWork = 2e5;       // k^2 l (real) at most: a sweep of ~0.1 ms on one SM
+
+// Fits the kernel: W (kw x l) with its odd row stride in shared memory, and no
+// more work than one SM does in the time the grid's rounds take.
+template <typename T>
+bool small_split_fits(int kw, int l) {
+  const int k = std::min(kw, l);
+  const double work = (double)k * k * l * (sizeof(T) == sizeof(double) ? 1.0 : 4.0);
+  return k <= kSmallRows && work <= kSmallWork &&
+         sizeof(T) * (size_t)kw * (l | 1) <= kSmallBytes;
+}
+
+// sum over the 8 lanes of a group
+__device__ __forceinline__ double sum8(double x) {
+  x += __shfl_xor_sync(0xffffffffu, x, 4);
+  x += __shfl_xor_sync(0xffffffffu, x, 2);
+  return x + __shfl_xor_sync(0xffffffffu, x, 1);
+}
+
+// W (kw x l) = A^T (trans) or A (m x n row-major).  Writes the k = min(kw, l) rows
+// s_i v_i 2^-e to Wx (row-major, ld = l), the sorted values, their order, the rank
+// and the scaling exponent e; no grid barrier, no other CTA.
+template <typename T>
+__global__ void __launch_bounds__(kSmallNT)
+    k_split_small(const T* __restrict__ A, int n_a, int trans, int kw, int l, double tol2,
+                  int use_floor, double defl_rel, int max_sweeps, sm_strategy strat,
+                  T* __restrict__ Wx, int* __restrict__ perm, double* __restrict__ s_sorted,
+                  SplitResult* res, int* __restrict__ wexp) {
+  constexpr bool kCplx = sizeof(T) != sizeof(double);
+  extern __shared__ __align__(16) unsigned char small_raw[];
+  T* W = reinterpret_cast<T*>(small_raw);
+  const int ld = l | 1;  // odd: the lanes of a column walk all banks
+  __shared__ double nrm[kSmallRows], ss[kSmallRows], er[kSmallRows + 1], red[kSmallNT / 32];
+  __shared__ unsigned long long keys[kSmallRows];
+  __shared__ T v0;
+  __shared__ double tau;
+  __shared__ int act[kSmallRows], nact, rotated, emax;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g8 = tid >> 3, l8 = tid & 7;  // group of 8 lanes, lane in it
+  constexpr int NG = kSmallNT / 8;
+  const int k = kw < l ? kw : l;
+  // ---- load, and scale by 2^-e, e the exponent of the largest entry ----------
+  if (tid == 0) emax = INT_MIN;
+  __syncthreads();
+  {
+    int best = INT_MIN;
+    for (int f = tid; f < kw * l; f += kSmallNT) {
+      // consecutive threads read consecutive entries of A
+      const int i = trans ? f % kw : f / l, c = trans ? f / kw : f % l;
+      const T x = A[trans ? (size_t)c * n_a + i : (size_t)i * n_a + c];
+      W[i * ld + c] = x;
+      double a;
+      if constexpr (kCplx) a = fmax(fabs(x.re), fabs(x.im));
+      else a = fabs(x);
+      if (a > 0.0 && isfinite(a)) best = max(best, ilogb(a));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+    if (lane == 0 && best != INT_MIN) atomicMax(&emax, best);
+  }
+  __syncthreads();
+  const int e2 = (emax < -1100 || emax > 1100) ? 0 : emax;
+  if (e2 != 0) {
+    for (int f = tid; f < kw * l; f += kSmallNT) {
+      T& x = W[(f / l) * ld + f % l];
+      if constexpr (kCplx) x = T{ldexp(x.re, -e2), ldexp(x.im, -e2)};
+      else x = ldexp(x, -e2);
+    }
+  }
+  __syncthreads();
+  // ---- Householder QR: R in the upper rows -----------------------------------
+  for (int j = 0; j < k; ++j) {
+    if (warp == 0) {  // reflector of column j, left in its rows below j and in v0, tau
+      double n2 = 0.0;
+      for (int i = j + lane; i < kw; i += 32) n2 += S<T>::abs2(W[i * ld + j]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+      const T x0 = W[j * ld + j];
+      T nu = S<T>::zero();
+      double t = 0.0;
+      if (n2 > 0.0) {
+        const double nx = n2 * rsqrt_newton(n2);
+        double a0;
+        if constexpr (kCplx) {
+          const double x2 = S<T>::abs2(x0);
+          const double r = x2 > 0.0 ? rsqrt_newton(x2) : 0.0;
+          a0 = x2 * r;
+          nu = x2 > 0.0 ? S<T>::scale(x0, nx * r) : S<T>::from_real(nx);
+        } else {
+          a0 = fabs(x0);
+          nu = copysign(nx, x0);
+        }
+        t = recip_newton(fma(nx, a0, n2));
+      }
+      __syncwarp();
+      if (lane == 0) {
+        v0 = x0 + nu;
+        tau = t;
+        W[j * ld + j] = S<T>::neg(nu);
+      }
+    }
+    __syncthreads();
+    // columns j + 1 ..: one per group, y -= tau (v^H y) v
+    for (int c0 = j + 1; c0 < l; c0 += NG) {
+      const int c = c0 + g8;
+      const bool on = c < l;
+      T w = S<T>::zero();
+      for (int i = j + l8; i < kw; i += 8)
+        if (on) w = S<T>::cfma(i == j ? v0 : W[i * ld + j], W[i * ld + c], w);
+      double wr, wi;
+      gamma_parts(w, wr, wi);
+      wr = sum8(wr);
+      if constexpr (kCplx) wi = sum8(wi);
+      T tw;
+      if constexpr (kCplx) tw = cplx{-tau * wr, -tau * wi};
+      else tw = -tau * wr;
+      for (int i = j + l8; i < kw; i += 8)
+        if (on) W[i * ld + c] = S<T>::fma(tw, i == j ? v0 : W[i * ld + j], W[i * ld + c]);
+    }
+    __syncthreads();
+  }
+  for (int f = tid; f < k * l; f += kSmallNT)
+    if (f % l < f / l) W[(f / l) * ld + f % l] = S<T>::zero();
+  __syncthreads();
+  // squared norm of row i by its group
+  auto row_norm = [&](int i) {
+    double a = 0.0;
+    if (i < k)
+      for (int x = l8; x < l; x += 8) a += S<T>::abs2(W[i * ld + x]);
+    return sum8(a);
+  };
+  // ---- one-sided Jacobi (as k_jacobi) ------------------------------------------
+  int status = k >= 2 ? DEV_NOT_CONVERGED : 0, sweeps = 0;
+  double thr = 0.0, tiny2 = 0.0;
+  for (int sweep = 0; k >= 2 && sweep < max_sweeps; ++sweep) {
+    for (int i0 = 0; i0 < k; i0 += NG) {
+      const double a = row_norm(i0 + g8);
+      if (l8 == 0 && i0 + g8 < k) nrm[i0 + g8] = a;
+    }
+    if (tid == 0) rotated = 0;
+    __syncthreads();
+    if (warp == 0) {  // rows above the deflation threshold, in order
+      if (sweep == 0) {
+        double f = (lane < k ? nrm[lane] : 0.0) + (lane + 32 < k ? nrm[lane + 32] : 0.0);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+        if (lane == 0) red[0] = f;
+        thr = defl_rel * f;
+      }
+      const bool on0 = lane < k && nrm[lane] > thr, on1 = lane + 32 < k && nrm[lane + 32] > thr;
+      const unsigned b0 = __ballot_sync(0xffffffffu, on0), b1 = __ballot_sync(0xffffffffu, on1);
+      const unsigned below = (1u << lane) - 1u;
+      if (on0) act[__popc(b0 & below)] = lane;
+      if (on1) act[__popc(b0) + __popc(b1 & below)] = lane + 32;
+      if (lane == 0) nact = __popc(b0) + __popc(b1);
+    }
+    __syncthreads();
+    if (sweep == 0 && use_floor) {
+      const double tiny = 16.0 * l * DBL_EPSILON * DBL_EPSILON * red[0];
+      tiny2 = tiny * tiny;
+    }
+    const int ka = nact, kp = ka + (ka & 1), npairs = kp / 2;
+    for (int r = 0; r + 1 < kp; ++r) {
+      if (4 * warp < npairs) {  // npairs <= 24: one pass of the 32 groups
+        const int t = g8;
+        int p = t == 0 ? kp - 1 : (r + t) % (kp - 1);
+        int q = t == 0 ? r : (r + kp - 1 - t) % (kp - 1);
+        const bool on = t < npairs && p < ka && q < ka;
+        p = on ? act[p] : 0;
+        q = on ? act[q] : 0;
+        if (p > q) { const int tmp = p; p = q; q = tmp; }
+        T* rp = W + p * ld;
+        T* rq = W + q * ld;
+        T g = S<T>::zero();
+        for (int x = l8; x < l; x += 8)
+          if (on) g = S<T>::cfma(rp[x], rq[x], g);
+        double gr, gi;
+        gamma_parts(g, gr, gi);
+        gr = sum8(gr);
+        if constexpr (kCplx) gi = sum8(gi);
+        const double a = nrm[p], b = nrm[q];
+        const double g2 = kCplx ? fma(gr, gr, gi * gi) : gr * gr;
+        const bool rot = on && g2 > tiny2 && g2 > tol2 * a * b;
+        if (__any_sync(0xffffffffu, rot)) {
+          double c = 1.0, sn = 0.0, e_r = 1.0, e_i = 0.0, na = a, nb = b;
+          if (rot) {
+            jacobi_angle<kCplx>(a, b, gr, gi, g2, c, sn, e_r, e_i, na, nb);
+            Rot<T> R;
+            R.set(c, sn, e_r, e_i);
+            for (int x = l8; x < l; x += 8) {
+              T u = rp[x], v = rq[x];
+              R.apply(u, v);
+              rp[x] = u;
+              rq[x] = v;
+            }
+            if (l8 == 0) {
+              nrm[p] = na;
+              nrm[q] = nb;
+              rotated = 1;
+            }
+          }
+        }
+      }
+      __syncthreads();
+    }
+    sweeps = sweep + 1;
+    const int any = rotated;
+    __syncthreads();
+    if (!any) {
+      status = 0;
+      break;
+    }
+  }
+  // ---- values, order, rank -----------------------------------------------------
+  for (int i0 = 0; i0 < k; i0 += NG) {
+    const double a = row_norm(i0 + g8);
+    if (l8 == 0 && i0 + g8 < k)
+      keys[i0 + g8] = (unsigned long long)__double_as_longlong(ldexp(sqrt(a), e2));
+  }
+  __syncthreads();
+  rank_sort(keys, k, perm, s_sorted, ss);
+  for (int f = tid; f < k * l; f += kSmallNT) Wx[f] = W[(f / l) * ld + f % l];
+  __syncthreads();
+  if (tid == 0) {
+    int D;
+    double e;
+    truncate_rule(ss, k, strat, er, &D, &e);
+    for (int i = 0; i < k; ++i)
+      if (!(ss[i] == ss[i]) || ss[i] > DBL_MAX) status |= DEV_NONFINITE;
+    res->D = D;
+    res->err2 = e;
+    res->status = status;
+    res->sweeps = sweeps;
+    *wexp = emax;
+  }
+}
+
 // Split where only one factor must be an isometry: U for (OUT_U, OUT_SVT)
 // (left_orth_2site, right canonical update) and V for (OUT_US, OUT_VT).
 // The Jacobi iteration then orthogonalises the vectors of that side -- the
@@ -1279,53 +1531,69 @@ int svd_split_xfree(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   else if (strat.method == SM_RELATIVE_SINGULAR_VALUE)
     use_floor = strat.tolerance >= 16.0 * std::sqrt((double)k * l) * eps;
   const double tol = std::sqrt((double)l) * DBL_EPSILON;
-  // Wt = W^T (l x kw): A itself for U, A^T for V; then scaled to O(1) entries
-  if (want_u) {
-    SM_CUDA_CHECK(cudaMemcpyAsync(Wt, A, sizeof(T) * (size_t)m * n, cudaMemcpyDeviceToDevice, st));
-  } else {
-    SM_CHECK(transpose<T>(st, m, n, A, n, Wt, m));
-  }
-  SM_CHECK(prescale<T>(st, Wt, l, kw, kw, wexp));
-  // rank-revealing QR preconditioner: W = Q R, R has k rows
-  {
-    SM_CUDA_CHECK(cudaMemsetAsync(qctl, 0, sizeof(QrCtl), st));
-    SM_CHECK(house_qr<T>(ctx, st, Wt, kw, l, drel, vbuf, qctl));
-    const size_t tot = (size_t)k * l;
-    const int blocks = (int)std::max<size_t>(1, std::min<size_t>((tot + 255) / 256, 4096));
-    SM_CUDA_CHECK(cudaMemsetAsync(ctl, 0, sizeof(JacobiCtl), st));
-    k_qr_extract<T><<<blocks, 256, 0, st>>>(Wt, kw, l, k, qctl, Wx, ctl);
-    note_launch();
-    SM_CUDA_CHECK(cudaGetLastError());
-  }
-  if (k >= 2) {
-    k_row_norms<T><<<(k + 7) / 8, 256, 0, st>>>(Wx, ld, k, l, nrm0, 1);
-    note_launch();
-    SM_CUDA_CHECK(cudaGetLastError());
+  if (small_split_fits<T>(kw, l)) {
+    const size_t smem = sizeof(T) * (size_t)kw * (l | 1);
+    SM_CHECK(raise_smem_limit(k_split_small<T>, smem));
     if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev0, st));
-    // the rows of R (the QR's steps; the rows below them are discarded weight)
-    // through the FP32 start; the Jacobi only where that leaves pairs to rotate
-    bool converged = false;
-    if (k >= kPrecondMinRows) {
-      QrCtl* hq = reinterpret_cast<QrCtl*>(ctx.pinned);
-      SM_CUDA_CHECK(cudaMemcpyAsync(hq, qctl, sizeof(QrCtl), cudaMemcpyDeviceToHost, st));
-      SM_CUDA_CHECK(cudaStreamSynchronize(st));
-      const int steps = hq->steps;
-      if (hq->bar.status == 0)
-        SM_CHECK(precondition_rows<T>(ctx, st, Wx, steps, l, tol * tol, use_floor ? 1 : 0, drel,
-                                      &converged));
-    }
-    if (!converged)
-      SM_CHECK(run_jacobi<T>(ctx, st, Wx, ld, k, l, l, tol * tol, use_floor ? 1 : 0, drel, dabs, nrm,
-                             nrm0, act, ctl));
+    k_split_small<T><<<1, kSmallNT, smem, st>>>(A, n, want_u ? 1 : 0, kw, l, tol * tol,
+                                                use_floor ? 1 : 0, drel, kMaxSweeps, strat, Wx, perm,
+                                                s_sorted, res, wexp);
     if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev1, st));
-    ctx.stats.jacobi_launches += 1;
-    ctx.stats.jacobi_flops += (4.0 * std::max(m, n) * (double)k * k + 8.0 * (double)k * k * k) *
-                              (sizeof(T) == sizeof(double) ? 1.0 : 4.0);
+    note_launch();
+    SM_CUDA_CHECK(cudaGetLastError());
+    ctx.stats.jacobi_launches += k >= 2;
+    if (k >= 2)
+      ctx.stats.jacobi_flops += (4.0 * std::max(m, n) * (double)k * k + 8.0 * (double)k * k * k) *
+                                (sizeof(T) == sizeof(double) ? 1.0 : 4.0);
+  } else {
+    // Wt = W^T (l x kw): A itself for U, A^T for V; then scaled to O(1) entries
+    if (want_u) {
+      SM_CUDA_CHECK(cudaMemcpyAsync(Wt, A, sizeof(T) * (size_t)m * n, cudaMemcpyDeviceToDevice, st));
+    } else {
+      SM_CHECK(transpose<T>(st, m, n, A, n, Wt, m));
+    }
+    SM_CHECK(prescale<T>(st, Wt, l, kw, kw, wexp));
+    // rank-revealing QR preconditioner: W = Q R, R has k rows
+    {
+      SM_CUDA_CHECK(cudaMemsetAsync(qctl, 0, sizeof(QrCtl), st));
+      SM_CHECK(house_qr<T>(ctx, st, Wt, kw, l, drel, vbuf, qctl));
+      const size_t tot = (size_t)k * l;
+      const int blocks = (int)std::max<size_t>(1, std::min<size_t>((tot + 255) / 256, 4096));
+      SM_CUDA_CHECK(cudaMemsetAsync(ctl, 0, sizeof(JacobiCtl), st));
+      k_qr_extract<T><<<blocks, 256, 0, st>>>(Wt, kw, l, k, qctl, Wx, ctl);
+      note_launch();
+      SM_CUDA_CHECK(cudaGetLastError());
+    }
+    if (k >= 2) {
+      k_row_norms<T><<<(k + 7) / 8, 256, 0, st>>>(Wx, ld, k, l, nrm0, 1);
+      note_launch();
+      SM_CUDA_CHECK(cudaGetLastError());
+      if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev0, st));
+      // the rows of R (the QR's steps; the rows below them are discarded weight)
+      // through the FP32 start; the Jacobi only where that leaves pairs to rotate
+      bool converged = false;
+      if (k >= kPrecondMinRows) {
+        QrCtl* hq = reinterpret_cast<QrCtl*>(ctx.pinned);
+        SM_CUDA_CHECK(cudaMemcpyAsync(hq, qctl, sizeof(QrCtl), cudaMemcpyDeviceToHost, st));
+        SM_CUDA_CHECK(cudaStreamSynchronize(st));
+        const int steps = hq->steps;
+        if (hq->bar.status == 0)
+          SM_CHECK(precondition_rows<T>(ctx, st, Wx, steps, l, tol * tol, use_floor ? 1 : 0, drel,
+                                        &converged));
+      }
+      if (!converged)
+        SM_CHECK(run_jacobi<T>(ctx, st, Wx, ld, k, l, l, tol * tol, use_floor ? 1 : 0, drel, dabs, nrm,
+                               nrm0, act, ctl));
+      if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev1, st));
+      ctx.stats.jacobi_launches += 1;
+      ctx.stats.jacobi_flops += (4.0 * std::max(m, n) * (double)k * k + 8.0 * (double)k * k * k) *
+                                (sizeof(T) == sizeof(double) ? 1.0 : 4.0);
+    }
+    k_row_norms<T><<<(k + 7) / 8, 256, 0, st>>>(Wx, ld, k, l, nrm, 0, wexp);
+    note_launch();
+    SM_CUDA_CHECK(cudaGetLastError());
+    SM_CHECK(sort_truncate(st, nrm, k, strat, perm, s_sorted, errors, ctl, res));
   }
-  k_row_norms<T><<<(k + 7) / 8, 256, 0, st>>>(Wx, ld, k, l, nrm, 0, wexp);
-  note_launch();
-  SM_CUDA_CHECK(cudaGetLastError());
-  SM_CHECK(sort_truncate(st, nrm, k, strat, perm, s_sorted, errors, ctl, res));
   SplitResult* h = reinterpret_cast<SplitResult*>(ctx.pinned);
   SM_CUDA_CHECK(cudaMemcpyAsync(h, res, sizeof(SplitResult), cudaMemcpyDeviceToHost, st));
   SM_CUDA_CHECK(cudaStreamSynchronize(st));
