@@ -294,27 +294,29 @@ int rank_predict(Ctx& ctx, cudaStream_t st, int k, const sm_strategy& strat, int
 int rank_predict_dev(Ctx& ctx, cudaStream_t st, int k, const sm_strategy& strat, double useful,
                      int* out);
 
-// --- svd_mixed.cu ------------------------------------------------------------
-// Whether the 16-CTA cluster factorisation holds W (kw x l) on this GPU.
+// --- svd_cluster_qr.cu, svd_cluster_jacobi.cu ----------------------------------
+// Whether the FP32 stage (a rank-revealing QR and a one-sided Jacobi, each in one
+// thread-block cluster) takes W (kw x l).
 // Splits with min(m, n) below this stay on the FP64 path in the mixed forms.
 constexpr int kMixedMinRank = 24;
 template <typename T>
 bool split_cluster_size_ok(int kw, int l);
 template <typename T>
 bool split_cluster_fits(int kw, int l);
-// FP32 rank-revealing QR + one-sided Jacobi of W = (want_u ? A^T : A) in one
-// cluster.  Writes kcap rows (FP64, ld = l, zero past the iteration's rows)
-// and their norms; ctl receives status / sweeps / nact = rows of R kept;
+// FP32 rank-revealing QR + one-sided Jacobi of W = (want_u ? A^T : A).  Writes kcap
+// rows (FP64, ld = l, zero past the iteration's rows) and their norms; ctl (zeroed by
+// the caller) receives status / sweeps / nact = rows of R kept;
 // info[0] = |A|_F^2 (FP64), info[1] = trailing weight dropped by the QR.
 // qr_cap > 0 stops the QR after that many steps (a predicted rank) even if
 // the trailing weight is still above the threshold; info[1] then holds the
-// weight it left behind.  info needs 7 doubles; vbuf (device) needs
-// split_cluster_vbuf_floats(kw) floats, kw = n when U is wanted, else m.
+// weight it left behind; thr_rel < 0 lets it stop at an empty trailing block only.
+// info needs 7 doubles; rbuf (device) needs split_cluster_rbuf_bytes(kw, l) bytes,
+// kw = n, l = m when U is wanted, else kw = m, l = n.
 template <typename T>
 int split_cluster_f32(cudaStream_t st, const T* A, int m, int n, bool want_u, double thr_rel,
                       double thr_abs, int max_sweeps, T* out_rows, double* out_nrm, int kcap,
-                      JacobiCtl* ctl, double* info, int qr_cap, float* vbuf, bool pivot = true,
+                      JacobiCtl* ctl, double* info, int qr_cap, void* rbuf, bool pivot = true,
                       const int* cap_dev = nullptr);
-size_t split_cluster_vbuf_floats(int kw);
+size_t split_cluster_rbuf_bytes(int kw, int l);
 
 }  // namespace sm

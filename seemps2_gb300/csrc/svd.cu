@@ -1676,13 +1676,11 @@ int svd_split_xfree(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
 
 // ---------------------------------------------------------------------------
 // Mixed-precision split (SM_PRECISION_MIXED): the cluster kernel of
-// svd_mixed.cu gives the right singular vectors of W to FP32 accuracy; FP64
+// the FP32 stage gives the right singular vectors of W to FP32 accuracy; FP64
 // GEMMs then refine them with the exact matrix:
 //   1. the rows, normalised, are approximate eigenvectors of W^H W within the
 //      row space the FP32 QR kept (it drops at most 1% of the weight the
-//      tolerance allows).  A power step (rows of V W^H W) is NOT used: rows
-//      whose sigma is below FP64 resolution relative to sigma_max would turn
-//      into rounding-level copies of the dominant directions.
+//      tolerance allows).
 //   2. refinement of the approximate eigenvectors of W^H W (Ogita & Aishima,
 //      "Iterative refinement for symmetric eigenvalue decomposition", Japan J.
 //      Indust. Appl. Math. 35 (2018)): with G = V W^H W V^H and M = V V^H,
@@ -1692,6 +1690,8 @@ int svd_split_xfree(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
 //      and V <- (I + E)^H V.  Each step squares the error for separated pairs;
 //      nearly degenerate pairs are only re-orthonormalised, which leaves the
 //      subspace they span unchanged.
+//      A power step V <- V W^H W on the rows that FP32 resolves then takes the FP32
+//      error out of the span they moved in.
 //   3. sigma_i = |W v_i^H| from the final C = W V^H.  For the relative-norm
 //      rule D is the smallest rank whose exact discarded weight
 //      |A|_F^2 - sum_{kept} sigma_i^2 is within tolerance (this stays exact
@@ -1744,6 +1744,25 @@ __global__ void k_scale_rows(T* __restrict__ X, int k, int l, const double* __re
 __device__ __forceinline__ double re_of(double x) { return x; }
 __device__ __forceinline__ double re_of(cplx x) { return x.re; }
 
+// Row i of V (block i) becomes that of P = V W^H W, normalised, where its value
+// lambda_i = G_ii / M_ii (of the refinement step before; row 0 has the largest) is at
+// least blind2 lambda_0; the other rows stay.  (|P_i| would not tell: a row of noise
+// that leans towards the dominant directions has a large one.)
+template <typename T>
+__global__ void __launch_bounds__(128) k_power_rows(const T* __restrict__ P, int k, int l,
+                                                    const double* __restrict__ nrm,
+                                                    const T* __restrict__ G, const T* __restrict__ M,
+                                                    double blind2, T* __restrict__ V) {
+  const int i = blockIdx.x;
+  const double m00 = re_of(M[0]), mii = re_of(M[(size_t)i * k + i]);
+  const double l0 = m00 > 0.0 ? re_of(G[0]) / m00 : 0.0;
+  const double li = mii > 0.0 ? re_of(G[(size_t)i * k + i]) / mii : 0.0;
+  const double n = nrm[i];
+  if (!(n > 0.0 && li >= blind2 * l0)) return;
+  for (int x = threadIdx.x; x < l; x += blockDim.x)
+    V[(size_t)i * l + x] = S<T>::scale(P[(size_t)i * l + x], 1.0 / n);
+}
+
 // F = (I + E)^H from G and M (k x k, Hermitian), E as described above.
 // Pairs of rows that are both below FP32 resolution (lambda < blind2 *
 // lambda_0; row 0 has the largest norm) are only re-orthonormalised
@@ -1783,17 +1802,22 @@ __global__ void k_refine_matrix(const T* __restrict__ G, const T* __restrict__ M
 
 // F = 1.5 I - 0.5 M: one Newton-Schulz step X <- F X towards orthonormal rows;
 // dev = max |M - I| over the grid (atomic max on the bits of the non-negative
-// double; dev must be zero beforehand).
+// double; dev must be zero beforehand).  `ordered`: each row is corrected against the
+// rows before it only, by their whole overlap (first order Gram-Schmidt, as exact to
+// second order): where the rows are in descending order of their singular values and
+// it is the small ones that lean towards the large ones, those stay untouched.
 template <typename T>
-__global__ void __launch_bounds__(256) k_ns_matrix(const T* M, int k, T* F, double* dev) {
+__global__ void __launch_bounds__(256) k_ns_matrix(const T* M, int k, T* F, double* dev,
+                                                   int ordered) {
   __shared__ double red[8];
   const size_t tot = (size_t)k * k;
   double worst = 0.0;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot;
        e += (size_t)gridDim.x * blockDim.x) {
     T d = M[e];
-    T f = S<T>::scale(d, -0.5);
-    if (e / k == e % k) {
+    const int fi = (int)(e / k), fj = (int)(e % k);
+    T f = S<T>::scale(d, !ordered || fi == fj ? -0.5 : fi > fj ? -1.0 : 0.0);
+    if (fi == fj) {
       f = f + S<T>::from_real(1.5);
       d = d - S<T>::one();
     }
@@ -2045,7 +2069,7 @@ double allowed_discard(const sm_strategy& st, double norm2, double s0, int k, in
 
 template <typename T>
 int newton_schulz_matrix(cudaStream_t st, const T* M, int k, T* F, double* dev) {
-  k_ns_matrix<T><<<grid_for((size_t)k * k), 256, 0, st>>>(M, k, F, dev);
+  k_ns_matrix<T><<<grid_for((size_t)k * k), 256, 0, st>>>(M, k, F, dev, 0);
   note_launch();
   SM_CUDA_CHECK(cudaGetLastError());
   return SM_OK;
@@ -2099,8 +2123,8 @@ int svd_split_mixed(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   SM_CHECK(ctx.scratch("mx.perm", (size_t)kcap, &perm));
   SM_CHECK(ctx.scratch("mx.info", 16, &info));
   SM_CHECK(ctx.scratch("mx.ctl", 1, &ctl));
-  float* vbuf;
-  SM_CHECK(ctx.scratch("mx.vbuf", split_cluster_vbuf_floats(ckw), &vbuf));
+  unsigned char* rbuf;
+  SM_CHECK(ctx.scratch("mx.rbuf", split_cluster_rbuf_bytes(ckw, cl), &rbuf));
   SM_CHECK(ctx.scratch("mx.res", 1, &res));
   // RRQR stop: drop at most 1% of what the tolerance allows (never more than
   // 1e-10 of |A|^2, which the power step then suppresses further)
@@ -2134,7 +2158,7 @@ int svd_split_mixed(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
       // no column pivoting here: W^T Q's columns come in the sketch's order, and
       // pivoting them cost the range finder a redo per split (measured)
       SM_CHECK(split_cluster_f32<T>(st, BH, l, rf_k, false, thr_rel, thr_abs, 40, rows, nrm,
-                                    kcap, ctl, info, 0, vbuf, false));
+                                    kcap, ctl, info, 0, rbuf, false));
       if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev1, st));
       SM_CHECK(vdot<T>(ctx, st, (size_t)m * n, A, A, a2));
       SM_CUDA_CHECK(cudaMemcpyAsync(info, a2, sizeof(double), cudaMemcpyDeviceToDevice, st));
@@ -2143,7 +2167,7 @@ int svd_split_mixed(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   if (rf_k == 0) {
     if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev0, st));
     SM_CHECK(split_cluster_f32<T>(st, A, m, n, want_u, thr_rel, thr_abs, 40, rows, nrm, kcap, ctl,
-                                  info, qr_cap, vbuf, true, cap_dev));
+                                  info, qr_cap, rbuf, true, cap_dev));
     if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev1, st));
   }
   struct Head {
@@ -2258,6 +2282,22 @@ int svd_split_mixed(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
     SM_CHECK(gemm_ctx<T>(ctx, st, SM_OP_N, SM_OP_N, cnt, l, cnt, one, Fb, cnt, V, l, zero, Vn, l));
     std::swap(V, Vn);
   }
+  // Power step on the resolved rows, V <- V W^H W normalised: refinement moves rows
+  // within their span only, and that span is off by the FP32 stage's error (1e-6 |W|:
+  // it limited the truncated product to 7e-7).  After it the rows above the FP32
+  // resolution are separated well enough not to turn towards the dominant ones (a
+  // 384 x 384 case: overlaps of 4e-9, the product of the kept rows exact to 1e-9).
+  if (rf_k == 0) {  // (a sketch's rows come from U_B^T B, a power step of their own)
+    SM_CHECK(w_vh(V, Cb));
+    if (want_u)
+      SM_CHECK(gemm_ctx<T>(ctx, st, SM_OP_C, SM_OP_T, cnt, m, n, one, Cb, cnt, A, n, zero, Vn, m));
+    else
+      SM_CHECK(gemm_ctx<T>(ctx, st, SM_OP_C, SM_OP_N, cnt, n, m, one, Cb, cnt, A, n, zero, Vn, n));
+    k_row_norms<T><<<(cnt + 7) / 8, 256, 0, st>>>(Vn, l, cnt, l, cn, 0);
+    k_power_rows<T><<<cnt, 128, 0, st>>>(Vn, cnt, l, cn, Gb, Mb, kMixedBlind * kMixedBlind, V);
+    note_launch(2);
+    SM_CUDA_CHECK(cudaGetLastError());
+  }
   // Newton-Schulz steps V <- (1.5 I - 0.5 V V^H) V take the largest
   // deviation e of V V^H from I to about 1.5 e^2.  Two refinement steps leave
   // e below kMixedNsOne for resolved rows (one step then reaches FP64 level);
@@ -2276,7 +2316,8 @@ int svd_split_mixed(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   for (int ns = 0; ns < kMixedNsMax; ++ns) {
     SM_CUDA_CHECK(cudaMemsetAsync(info + 8, 0, sizeof(double), st));
     SM_CHECK(gemm_ctx<T>(ctx, st, SM_OP_N, SM_OP_C, cnt, cnt, l, one, V, l, V, l, zero, Mb, cnt));
-    k_ns_matrix<T><<<grid_for((size_t)cnt * cnt), 256, 0, st>>>(Mb, cnt, Fb, info + 8);
+    k_ns_matrix<T><<<grid_for((size_t)cnt * cnt), 256, 0, st>>>(Mb, cnt, Fb, info + 8,
+                                                                rf_k == 0 && ns == 0 ? 1 : 0);
     note_launch();
     SM_CUDA_CHECK(cudaGetLastError());
     SM_CUDA_CHECK(cudaMemcpyAsync(hdev, info + 8, sizeof(double), cudaMemcpyDeviceToHost, st));

@@ -8,7 +8,7 @@
 // mixed-precision Jacobi SVD of Gao, Ma and Shao (arXiv 2209.04626), an FP32
 // SVD supplies X to FP32 accuracy and FP64 matrix products do the rest:
 //
-//   1. the cluster kernel of svd_mixed.cu factors R^T in FP32; its rows are
+//   1. the FP32 stage (svd_cluster_*.cu) factors R^T; its rows are
 //      s_i u_i^T, so their normalised conjugates are X0 ~ U^H;
 //   2. Newton-Schulz steps X <- (1.5 I - 0.5 X X^H) X make X unitary to FP64
 //      rounding (X0 is off by ~1e-6: two steps), and W = X R is then an exact
@@ -168,13 +168,13 @@ int precondition_rows(Ctx& ctx, cudaStream_t st, T* R, int k, int l, double tol2
   double *nrm, *info;
   JacobiCtl* ctl;
   PrecondStat* stat;
-  float* vbuf;
+  unsigned char* rbuf;
   SM_CHECK(ctx.scratch("pc.rows", (size_t)cap * k, &rows));
   SM_CHECK(ctx.scratch("pc.nrm", (size_t)cap, &nrm));
   SM_CHECK(ctx.scratch("pc.info", 16, &info));
   SM_CHECK(ctx.scratch("pc.ctl", 1, &ctl));
   SM_CHECK(ctx.scratch("pc.stat", 1, &stat));
-  SM_CHECK(ctx.scratch("pc.vbuf", split_cluster_vbuf_floats(l), &vbuf));
+  SM_CHECK(ctx.scratch("pc.rbuf", split_cluster_rbuf_bytes(l, k), &rbuf));
   SM_CHECK(ctx.scratch("pc.X", kk, &X));
   SM_CHECK(ctx.scratch("pc.Xn", kk, &Xn));
   SM_CHECK(ctx.scratch("pc.M", kk, &M));
@@ -237,7 +237,7 @@ int precondition_rows(Ctx& ctx, cudaStream_t st, T* R, int k, int l, double tol2
     SM_CUDA_CHECK(cudaMemsetAsync(ctl, 0, sizeof(JacobiCtl), st));
     SM_CUDA_CHECK(cudaMemsetAsync(stat, 0, sizeof(PrecondStat), st));
     SM_CHECK(split_cluster_f32<T>(st, src, k, l, true, -1.0, 0.0, 40, rows, nrm, cap, ctl, info, 0,
-                                  vbuf));
+                                  rbuf, false));
     k_rows_to_basis<T><<<cap, 128, 0, st>>>(rows, nrm, cap, k, ctl, X, stat);
     note_launch();
     SM_CUDA_CHECK(cudaGetLastError());
