@@ -133,6 +133,7 @@ struct JacobiCtl {
   int nkeep;  // mixed split: FP32 rows heavy enough to take into the FP64 refinement
   int cap;    // mixed split: the QR cap the cluster kernel used (0: none)
   int pred;   // mixed split: the predicted rank behind a device-side cap (0: none)
+  int plateau;  // mixed split: the QR stopped at the FP32 noise level, above its threshold
 };
 
 // Output forms of the two factors of a split A = U diag(s) Vt.
@@ -310,13 +311,15 @@ bool split_cluster_fits(int kw, int l);
 // qr_cap > 0 stops the QR after that many steps (a predicted rank) even if
 // the trailing weight is still above the threshold; info[1] then holds the
 // weight it left behind; thr_rel < 0 lets it stop at an empty trailing block only.
+// `plateau` also lets it stop where the trailing weight is FP32 noise (ctl->plateau = 1:
+// the caller checks the weight outside the rows' span in FP64).
 // info needs 7 doubles; rbuf (device) needs split_cluster_rbuf_bytes(kw, l) bytes,
 // kw = n, l = m when U is wanted, else kw = m, l = n.
 template <typename T>
 int split_cluster_f32(cudaStream_t st, const T* A, int m, int n, bool want_u, double thr_rel,
                       double thr_abs, int max_sweeps, T* out_rows, double* out_nrm, int kcap,
                       JacobiCtl* ctl, double* info, int qr_cap, void* rbuf, bool pivot = true,
-                      const int* cap_dev = nullptr);
+                      const int* cap_dev = nullptr, bool plateau = false);
 size_t split_cluster_rbuf_bytes(int kw, int l);
 
 }  // namespace sm

@@ -2139,6 +2139,7 @@ int svd_split_mixed(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   // workload at tol 1e-12 did).  The redo of such a split (qr_cap = min(m, n))
   // therefore runs the full QR.
   if (qr_cap >= std::min(m, n)) thr_rel = thr_abs = 0.0;
+  const bool exact = strat.method == SM_RELATIVE_NORM_SQUARED_ERROR;
   SM_CUDA_CHECK(cudaMemsetAsync(ctl, 0, sizeof(JacobiCtl), st));
   // a predicted rank caps the rank-revealing QR (qr_cap rows of R), or sizes
   // the range finder
@@ -2167,7 +2168,8 @@ int svd_split_mixed(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   if (rf_k == 0) {
     if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev0, st));
     SM_CHECK(split_cluster_f32<T>(st, A, m, n, want_u, thr_rel, thr_abs, 40, rows, nrm, kcap, ctl,
-                                  info, qr_cap, rbuf, true, cap_dev));
+                                  info, qr_cap, rbuf, true, cap_dev,
+                                  exact && qr_cap < std::min(m, n)));
     if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev1, st));
   }
   struct Head {
@@ -2177,7 +2179,7 @@ int svd_split_mixed(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   // FP32 singular values: sorted, and the rank the rule gives on them; for the
   // singular-value rules a cut below the FP32 resolution sends the split to
   // the FP64 path right away
-  const bool exact_rule = strat.method == SM_RELATIVE_NORM_SQUARED_ERROR;
+  const bool exact_rule = exact;
   k_mixed_sort<<<1, 1024, 3 * sizeof(double) * (size_t)kcap, st>>>(
       nrm, kcap, strat, exact_rule ? 1 : 0, ctl, kMixedRowFloor, perm, s_sorted, res, info);
   note_launch();
@@ -2308,7 +2310,8 @@ int svd_split_mixed(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   // parallel: the split goes to FP64.
   // a capped QR (the predicted rank, or the range finder's k) that missed
   // weight the rank needs is redone by the caller with the full QR
-  const bool capped = qr_cap > 0 && qr_cap < k;
+  // (and so is a QR that took its trailing weight for noise)
+  const bool capped = (qr_cap > 0 && qr_cap < k) || hc.plateau != 0;
   SM_CHECK(normalise(V));
   double e_ns = 0.0;
   bool ns_done = false;
@@ -2371,7 +2374,9 @@ int svd_split_mixed(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   // a capped QR that left weight the rank may need: more than 1% of what the
   // tolerance allows (and more than 1e-12 of |A|^2) outside the rows' span,
   // computed exactly after the refinement
-  const bool missed = capped && hs[5] > std::max(1e-12, 1e-2 * strat.tolerance) * norm2;
+  // (a stop at the noise level: more than 1e-13, well above FP64's rounding of the sum)
+  const bool missed = capped && hs[5] > std::max(hc.plateau ? 1e-13 : 1e-12,
+                                                 1e-2 * strat.tolerance) * norm2;
   const bool coupled = !(cut_angle <= kMixedCutAmp);
   const bool over_tol = r.err2 > allowed_discard(strat, norm2, s0, k, D) * (1.0 + 1e-12);
   const bool over = D < strat.max_bond_dimension && D < k && over_tol;

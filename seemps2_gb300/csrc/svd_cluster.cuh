@@ -193,11 +193,12 @@ int qr_row_pad(int kw);
 template <typename T>
 bool qr_cluster_ok(int kw, int l);
 // Rank-revealing Householder QR of W = (trans ? A^T : A) (kw x l) / |W|_F: R into Rg,
-// ctl->nact = its rows, info[0] = |W|_F^2 (FP64), info[1] the weight below them.
+// ctl->nact = its rows, ctl->plateau = 1 if it stopped at the FP32 noise level,
+// info[0] = |W|_F^2 (FP64), info[1] the weight below the rows.
 template <typename T>
 int qr_cluster(cudaStream_t st, const T* A, int n_a, int trans, int kw, int l, double thr_rel,
                double thr_abs, typename F32<T>::type* Rg, JacobiCtl* ctl, double* info, int qr_cap,
-               const int* cap_dev, int pivot);
+               const int* cap_dev, int pivot, int plateau);
 // One-sided Jacobi on the ctl->nact (<= kmax) rows of R (length l): kcap rows (FP64,
 // times sqrt(info[0])) and their norms.
 template <typename T>

@@ -16,8 +16,8 @@
 //   * only the overlap is summed in a local round; the rows' norms are taken afresh
 //     once per block round and follow the rotations within it;
 //   * four warps share a scheduler, so instructions count as much as latency: FP32
-//     arithmetic is issued in pairs (f32x2), the angle takes one reciprocal and two
-//     reciprocal roots of the SFU, and convergence is a flag (did a rotation start
+//     arithmetic is issued in pairs (f32x2), the angle takes two reciprocal roots of
+//     the SFU, and convergence is a flag (did a rotation start
 //     above the stopping cosine), not a maximum;
 //   * after the last local round each warp copies its two rows into the next CTAs'
 //     buffers (bulk copies), and a CTA waits on its own mbarrier for the bytes of
@@ -25,10 +25,10 @@
 //     has sent round g's rows only after all its warps are done with the buffers of
 //     round g - 1, and its neighbours send into those only after they have received
 //     those rows (so a copy's source is free as well).
-// The cluster meets once per sweep, to agree on that flag.  The earlier
-// kernel (16 CTAs always, three sums per pair, copies through mailboxes and a cluster
-// barrier per block round) took 84 us per sweep on 157 rows of 256, 2.7 ms for ten
-// sweeps on 340 rows of 512; the times now stand at the launcher.
+// The cluster meets once per sweep, to agree on that flag.  A sweep takes 29 us on 64
+// rows of 64, 61 us on 153 rows of 256 and 206 us on 337 rows of 512 (with 16 CTAs
+// always, three sums per pair, copies through mailboxes and a cluster barrier per
+// block round: 56, 93 and 268 us).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -447,13 +447,13 @@ template <typename T>
 int split_cluster_f32(cudaStream_t st, const T* A, int m, int n, bool want_u, double thr_rel,
                       double thr_abs, int max_sweeps, T* out_rows, double* out_nrm, int kcap,
                       JacobiCtl* ctl, double* info, int qr_cap, void* rbuf, bool pivot,
-                      const int* cap_dev) {
+                      const int* cap_dev, bool plateau) {
   using F = typename F32<T>::type;
   // W = A^T (kw = n, l = m) when U is wanted, else W = A (kw = m, l = n)
   const int kw = want_u ? n : m, l = want_u ? m : n;
   F* Rg = reinterpret_cast<F*>(rbuf);
   SM_CHECK(qr_cluster<T>(st, A, n, want_u ? 1 : 0, kw, l, thr_rel, thr_abs, Rg, ctl, info, qr_cap,
-                         cap_dev, pivot ? 1 : 0));
+                         cap_dev, pivot ? 1 : 0, plateau ? 1 : 0));
   const int kmax = qr_cap > 0 ? std::min(std::min(kw, l), qr_cap) : std::min(kw, l);
   return jacobi_cluster<T>(st, Rg, qr_row_pad<T>(kw), kmax, l, max_sweeps, out_rows, out_nrm, kcap,
                            ctl, info);
@@ -465,9 +465,9 @@ template bool split_cluster_fits<double>(int, int);
 template bool split_cluster_fits<cplx>(int, int);
 template int split_cluster_f32<double>(cudaStream_t, const double*, int, int, bool, double,
                                        double, int, double*, double*, int, JacobiCtl*, double*,
-                                       int, void*, bool, const int*);
+                                       int, void*, bool, const int*, bool);
 template int split_cluster_f32<cplx>(cudaStream_t, const cplx*, int, int, bool, double, double,
                                      int, cplx*, double*, int, JacobiCtl*, double*, int, void*,
-                                     bool, const int*);
+                                     bool, const int*, bool);
 
 }  // namespace sm

@@ -40,6 +40,8 @@ constexpr int kRing = 8;  // steps per cluster barrier
 // range; the QR also stops once the trailing weight is below kQrFloor
 constexpr float kTinyCol = 1e-15f;
 constexpr float kQrFloor = 1e-24f;
+constexpr float kNoise = 1e-11f;  // trailing weight that FP32 noise does not exceed
+constexpr float kFlat = 0.75f;    // its ratio over 8 pivots from which it counts as noise
 
 struct QrShared {
   uint64_t full[kRing];
@@ -89,7 +91,8 @@ template <typename T, int NV, int NC>
 __global__ void __launch_bounds__(kCNT, 1)
     k_qr_cluster(const T* __restrict__ A, int n_a, int trans, int kw, int l, double thr_rel,
                  double thr_abs, typename F32<T>::type* __restrict__ Rg, JacobiCtl* ctl_out,
-                 double* __restrict__ info, int qr_cap, const int* __restrict__ cap_dev, int pivot) {
+                 double* __restrict__ info, int qr_cap, const int* __restrict__ cap_dev, int pivot,
+                 int plateau) {
   using F = typename F32<T>::type;
   constexpr int VW = 16 / (int)sizeof(F);
   constexpr int VR = 32 * VW;        // rows of one vector index over the lanes
@@ -286,8 +289,8 @@ __global__ void __launch_bounds__(kCNT, 1)
     cluster.sync();
     select(1);
   }
-  int keff = qsteps;
-  float trail = 0.f;
+  int keff = qsteps, level = 0;
+  float trail = 0.f, before = 0.f;
   for (int b = 0; b * kRing < qsteps; ++b) {
     const int first = b * kRing, nb = min(kRing, qsteps - first), jl = first + nb - 1;
     const int par = b & 1;
@@ -396,8 +399,18 @@ __global__ void __launch_bounds__(kCNT, 1)
       if (tid < 128) post_mine(par);
     }
     cluster.sync();
+    before = trail;
     trail = 0.f;
     for (int r = 0; r < nc; ++r) trail += sh.part[par][r][0];
+    // A trailing block below kNoise whose weight 8 more pivots hardly reduce is the
+    // rounding noise of FP32 around a matrix of lower rank (a spectrum that decays
+    // towards the threshold falls faster): its rows hold nothing, and the Jacobi and
+    // the FP64 products after it would take them along (337 rows for a rank of 258).
+    if (plateau && trail > thr && trail < kNoise && trail > kFlat * before && b > 0) {
+      keff = jl + 1;
+      level = 1;
+      break;
+    }
     if (trail <= thr) {
       // the rank lies in this batch: the weight below each of its steps (the rows
       // between a step and the batch's last are R's and keep that weight)
@@ -454,6 +467,7 @@ __global__ void __launch_bounds__(kCNT, 1)
   if (rank == 0 && tid == 0) {
     ctl_out->nact = keff;
     ctl_out->cap = qr_cap;
+    ctl_out->plateau = level;
     ctl_out->pred = cap_dev ? cap_dev[1] : 0;
     info[0] = norm2;
     info[1] = (double)trail * norm2;
@@ -484,7 +498,7 @@ inline int qr_ctas(int l) { return l <= 4 * kCNW ? 4 : l <= 8 * kCNW ? 8 : kCWMa
 template <typename T, int NV, int NC>
 int launch_qr(cudaStream_t st, int nc, const T* A, int n_a, int trans, int kw, int l, double thr_rel,
               double thr_abs, typename F32<T>::type* Rg, JacobiCtl* ctl, double* info, int qr_cap,
-              const int* cap_dev, int pivot) {
+              const int* cap_dev, int pivot, int plateau) {
   using F = typename F32<T>::type;
   auto fn = k_qr_cluster<T, NV, NC>;
   const size_t smem = (size_t)2 * kRing * (16 + NV * 512);
@@ -503,7 +517,7 @@ int launch_qr(cudaStream_t st, int nc, const T* A, int n_a, int trans, int kw, i
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   SM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fn, A, n_a, trans, kw, l, thr_rel, thr_abs, Rg, ctl, info,
-                                   qr_cap, cap_dev, pivot));
+                                   qr_cap, cap_dev, pivot, plateau));
   note_launch();
   return SM_OK;
 }
@@ -524,12 +538,12 @@ bool qr_cluster_ok(int kw, int l) {
 template <typename T>
 int qr_cluster(cudaStream_t st, const T* A, int n_a, int trans, int kw, int l, double thr_rel,
                double thr_abs, typename F32<T>::type* Rg, JacobiCtl* ctl, double* info, int qr_cap,
-               const int* cap_dev, int pivot) {
+               const int* cap_dev, int pivot, int plateau) {
   const int nc = qr_ctas(l), cols = (l + nc * kCNW - 1) / (nc * kCNW), nv = nv_bucket<T>(kw);
 #define SM_QR(NVV, NCC)                                                                           \
   if (nv == NVV && cols == NCC)                                                                   \
   return launch_qr<T, NVV, NCC>(st, nc, A, n_a, trans, kw, l, thr_rel, thr_abs, Rg, ctl, info,    \
-                                qr_cap, cap_dev, pivot)
+                                qr_cap, cap_dev, pivot, plateau)
   SM_QR(1, 1);
   SM_QR(1, 2);
   SM_QR(2, 1);
@@ -560,8 +574,8 @@ template int qr_row_pad<cplx>(int);
 template bool qr_cluster_ok<double>(int, int);
 template bool qr_cluster_ok<cplx>(int, int);
 template int qr_cluster<double>(cudaStream_t, const double*, int, int, int, int, double, double,
-                                float*, JacobiCtl*, double*, int, const int*, int);
+                                float*, JacobiCtl*, double*, int, const int*, int, int);
 template int qr_cluster<cplx>(cudaStream_t, const cplx*, int, int, int, int, double, double, float2*,
-                              JacobiCtl*, double*, int, const int*, int);
+                              JacobiCtl*, double*, int, const int*, int, int);
 
 }  // namespace sm
