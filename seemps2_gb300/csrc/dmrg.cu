@@ -22,41 +22,96 @@ namespace sm {
 
 namespace {
 
-// X2[a][ko][lo][dd][f] = sum_{c,k,l} X1[a][c][k][l][f] H[c][ko][k][lo][l][dd].
-// One thread per (a, f), lanes along f (coalesced reads of X1 and writes of
-// X2); H (c p1 p1 p2 p2 e entries) in shared memory.
-// Acc is the accumulation type (T).
-template <typename T, typename Acc>
-__global__ void k_h12_apply(const T* __restrict__ X1, const T* __restrict__ H, int A, int Cc,
-                            int p1, int p2, int E, int F, T* __restrict__ X2) {
-  extern __shared__ unsigned char sraw[];
-  T* Hs = reinterpret_cast<T*>(sraw);
-  const int nh = Cc * p1 * p1 * p2 * p2 * E;
-  for (int i = threadIdx.x + blockDim.x * threadIdx.y; i < nh; i += blockDim.x * blockDim.y)
-    Hs[i] = H[i];
-  __syncthreads();
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  const int a = blockIdx.y * blockDim.y + threadIdx.y;
-  if (f >= F || a >= A) return;
-  const size_t sx = (size_t)F;  // stride of l in X1
-  const T* x = X1 + (size_t)a * Cc * p1 * p2 * F + f;
-  T* out = X2 + (size_t)a * p1 * p2 * E * F + f;
-  for (int ko = 0; ko < p1; ++ko)
-    for (int lo = 0; lo < p2; ++lo)
-      for (int dd = 0; dd < E; ++dd) {
-        Acc acc{};
-        for (int c = 0; c < Cc; ++c)
-          for (int k = 0; k < p1; ++k)
-            for (int l = 0; l < p2; ++l) {
-              const T h = Hs[((((c * p1 + ko) * p1 + k) * p2 + lo) * p2 + l) * E + dd];
-              if (S<T>::abs2(h) == 0.0) continue;  // zero blocks of the MPO (warp-uniform)
-              const T xv = x[(((size_t)c * p1 + k) * p2 + l) * sx];
-              if constexpr (sizeof(Acc) == sizeof(T)) acc = S<T>::fma(h, xv, acc);
-              else acc = fmaf((float)S<T>::real(h), (float)S<T>::real(xv), acc);
-            }
-        if constexpr (sizeof(Acc) == sizeof(T)) out[(((size_t)ko * p2 + lo) * E + dd) * F] = acc;
-        else out[(((size_t)ko * p2 + lo) * E + dd) * F] = S<T>::from_real((double)acc);
+// One pass of the two-site MPO over a block's outputs: block (32, 8) takes 32 values
+// of f, 8 of a, one (ko, lo) and up to kH12Out values of dd; thread (f, a) gets the
+// sums acc[dd] = sum_{c,k,l} H[c][ko][k][lo][l][dd] X1[a][c][k][l][f] in that order.
+// The nonzero entries of each output are listed in shared memory first (warp w lists
+// output w, chunks of kH12In inputs): a bulk site of the Heisenberg chain has 36 of 400,
+// and testing each entry where it is used cost more than everything else (an FP64
+// comparison holds the FP64 pipe for 64 clocks; at a = f = 108, D = 5 96 us, in FP32 at
+// 256 56 us).  Bound by the traffic of X1 and X2 through L2.
+constexpr int kH12Out = 8, kH12In = 256;
+template <typename T, typename V>
+struct H12Shared {
+  V h[kH12Out][kH12In];
+  short in[kH12Out][kH12In];
+  int cnt[kH12Out];
+};
+__device__ __forceinline__ bool h12_zero(double x) { return x == 0.0; }
+__device__ __forceinline__ bool h12_zero(cplx x) { return x.re == 0.0 && x.im == 0.0; }
+template <typename T>
+__device__ __forceinline__ void h12_put(T& d, T x) { d = x; }
+__device__ __forceinline__ void h12_put(float& d, double x) { d = (float)x; }
+template <typename T>
+__device__ __forceinline__ T h12_fma(T h, T x, T acc) { return S<T>::fma(h, x, acc); }
+__device__ __forceinline__ float h12_fma(float h, float x, float acc) { return fmaf(h, x, acc); }
+
+template <typename T, typename V>
+__device__ __forceinline__ void h12_sums(const V* __restrict__ X1, const T* __restrict__ H, int A,
+                                         int Cc, int p1, int p2, int E, int F, int ko, int lo,
+                                         int d0, int nd, int a, int f, V (&acc)[kH12Out],
+                                         H12Shared<T, V>& sh) {
+  const int nin = Cc * p1 * p2;
+  const int warp = threadIdx.y, lane = threadIdx.x;
+  const bool on = a < A && f < F;
+  const V* x = X1 + (size_t)(on ? a : 0) * nin * F + (on ? f : 0);
+  for (int i0 = 0; i0 < nin; i0 += kH12In) {
+    const int ni = min(kH12In, nin - i0);
+    __syncthreads();  // the previous chunk has been used
+    if (warp < nd) {
+      int n = 0;
+      for (int j = 0; j < ni; j += 32) {
+        const int i = i0 + j + lane;
+        bool put = false;
+        T h{};
+        if (j + lane < ni) {
+          const int c = i / (p1 * p2), k = i / p2 % p1, l = i % p2;
+          h = H[((((size_t)(c * p1 + ko) * p1 + k) * p2 + lo) * p2 + l) * E + d0 + warp];
+          put = !h12_zero(h);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, put);
+        if (put) {
+          const int at = n + __popc(m & ((1u << lane) - 1u));
+          h12_put(sh.h[warp][at], h);
+          sh.in[warp][at] = (short)(j + lane);
+        }
+        n += __popc(m);
       }
+      if (lane == 0) sh.cnt[warp] = n;
+    }
+    __syncthreads();
+    const V* xc = x + (size_t)i0 * F;
+#pragma unroll
+    for (int d = 0; d < kH12Out; ++d) {
+      if (d >= nd) break;
+      const int n = sh.cnt[d];
+      for (int i = 0; i < n; ++i)
+        if (on) acc[d] = h12_fma(sh.h[d][i], xc[(size_t)sh.in[d][i] * F], acc[d]);
+    }
+  }
+}
+inline dim3 h12_grid(int a, int p1, int p2, int e, int f) {
+  return dim3((f + 31) / 32, (a + 7) / 8, p1 * p2 * ((e + kH12Out - 1) / kH12Out));
+}
+
+// X2[a][ko][lo][dd][f] = sum_{c,k,l} X1[a][c][k][l][f] H[c][ko][k][lo][l][dd].
+template <typename T>
+__global__ void __launch_bounds__(256) k_h12_apply(const T* __restrict__ X1, const T* __restrict__ H,
+                                                   int A, int Cc, int p1, int p2, int E, int F,
+                                                   T* __restrict__ X2) {
+  __shared__ H12Shared<T, T> sh;
+  const int nch = (E + kH12Out - 1) / kH12Out, kl = blockIdx.z / nch;
+  const int d0 = blockIdx.z % nch * kH12Out, nd = min(kH12Out, E - d0);
+  const int f = blockIdx.x * 32 + threadIdx.x, a = blockIdx.y * 8 + threadIdx.y;
+  T acc[kH12Out];
+#pragma unroll
+  for (int d = 0; d < kH12Out; ++d) acc[d] = S<T>::zero();
+  h12_sums<T, T>(X1, H, A, Cc, p1, p2, E, F, kl / p2, kl % p2, d0, nd, a, f, acc, sh);
+  if (a >= A || f >= F) return;
+  T* out = X2 + (((size_t)a * p1 * p2 + kl) * E + d0) * F + f;
+#pragma unroll
+  for (int d = 0; d < kH12Out; ++d)
+    if (d < nd) out[(size_t)d * F] = acc[d];
 }
 
 template <typename T>
@@ -92,12 +147,9 @@ int two_site_matvec(Ctx& ctx, cudaStream_t st, int a, int c, int b, int p1, int 
   SM_CHECK(ctx.scratch("mv.X2", (size_t)a * p1 * p2 * e * f, &X2));
   SM_CHECK(product<T>(ctx, st, precision, SM_OP_N, SM_OP_N, a * c, p1 * p2 * f, b, L, b, v,
                       p1 * p2 * f, X1, p1 * p2 * f));
-  const size_t hs = sizeof(T) * (size_t)c * p1 * p1 * p2 * p2 * e;
-  const dim3 blk(32, 8), grd((f + 31) / 32, (a + 7) / 8);
   // FP64 arithmetic at every precision: the intermediates are FP64, and
   // converting them to FP32 costs GB300's FP64 pipe as much as the FMAs
-  if (hs > 48 * 1024) SM_CHECK(raise_smem_limit(k_h12_apply<T, T>, hs));
-  k_h12_apply<T, T><<<grd, blk, hs, st>>>(X1, H, a, c, p1, p2, e, f, X2);
+  k_h12_apply<T><<<h12_grid(a, p1, p2, e, f), dim3(32, 8), 0, st>>>(X1, H, a, c, p1, p2, e, f, X2);
   note_launch();
   SM_CUDA_CHECK(cudaGetLastError());
   return product<T>(ctx, st, precision, SM_OP_N, SM_OP_T, a * p1 * p2, g, e * f, X2, e * f, R,
@@ -128,43 +180,33 @@ __device__ __forceinline__ float tf32_round(float x) {
 // X2[(a, ko, lo)][(dd, f)] = sum_{c,k,l} X1[a][c][k][l][f] H[c][ko][k][lo][l][dd]
 // in FP32, written as K-contiguous operand rows of kp entries (the caller
 // zeroes the columns past E F): one BF16 plane, or TF32 hi = rna(x) and
-// lo = x - hi.  One thread per (a, f), lanes along f; H (FP64) converted into
-// shared memory.
+// lo = x - hi.  Blocks as k_h12_apply's; H (FP64) is converted as it is listed.
 template <bool BF16>
-__global__ void k_h12_planes(const float* __restrict__ X1, const double* __restrict__ H, int A,
-                             int Cc, int p1, int p2, int E, int F, int kp, void* __restrict__ hi,
-                             float* __restrict__ lo) {
-  extern __shared__ float hs[];
-  const int nh = Cc * p1 * p1 * p2 * p2 * E;
-  for (int i = threadIdx.x + blockDim.x * threadIdx.y; i < nh; i += blockDim.x * blockDim.y)
-    hs[i] = (float)H[i];
-  __syncthreads();
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
-  const int a = blockIdx.y * blockDim.y + threadIdx.y;
+__global__ void __launch_bounds__(256)
+    k_h12_planes(const float* __restrict__ X1, const double* __restrict__ H, int A, int Cc, int p1,
+                 int p2, int E, int F, int kp, void* __restrict__ hi, float* __restrict__ lo) {
+  __shared__ H12Shared<double, float> sh;
+  const int nch = (E + kH12Out - 1) / kH12Out, kl = blockIdx.z / nch;
+  const int d0 = blockIdx.z % nch * kH12Out, nd = min(kH12Out, E - d0);
+  const int f = blockIdx.x * 32 + threadIdx.x, a = blockIdx.y * 8 + threadIdx.y;
+  float acc[kH12Out];
+#pragma unroll
+  for (int d = 0; d < kH12Out; ++d) acc[d] = 0.f;
+  h12_sums<double, float>(X1, H, A, Cc, p1, p2, E, F, kl / p2, kl % p2, d0, nd, a, f, acc, sh);
   if (a >= A || f >= F) return;
-  const float* x = X1 + (size_t)a * Cc * p1 * p2 * F + f;
-  for (int ko = 0; ko < p1; ++ko)
-    for (int lo2 = 0; lo2 < p2; ++lo2) {
-      const size_t row = ((size_t)a * p1 + ko) * p2 + lo2;
-      for (int dd = 0; dd < E; ++dd) {
-        float acc = 0.f;
-        for (int c = 0; c < Cc; ++c)
-          for (int k = 0; k < p1; ++k)
-            for (int l = 0; l < p2; ++l) {
-              const float h = hs[((((c * p1 + ko) * p1 + k) * p2 + lo2) * p2 + l) * E + dd];
-              if (h == 0.f) continue;  // zero blocks of the MPO (warp-uniform)
-              acc = fmaf(h, x[(((size_t)c * p1 + k) * p2 + l) * F], acc);
-            }
-        const size_t o = row * kp + (size_t)dd * F + f;
-        if (BF16) {
-          reinterpret_cast<__nv_bfloat16*>(hi)[o] = __float2bfloat16_rn(acc);
-        } else {
-          const float h = tf32_round(acc);
-          reinterpret_cast<float*>(hi)[o] = h;
-          lo[o] = acc - h;
-        }
-      }
+  const size_t row = ((size_t)a * p1 * p2 + kl) * kp + (size_t)d0 * F + f;
+#pragma unroll
+  for (int d = 0; d < kH12Out; ++d) {
+    if (d >= nd) break;
+    const size_t o = row + (size_t)d * F;
+    if (BF16) {
+      reinterpret_cast<__nv_bfloat16*>(hi)[o] = __float2bfloat16_rn(acc[d]);
+    } else {
+      const float h = tf32_round(acc[d]);
+      reinterpret_cast<float*>(hi)[o] = h;
+      lo[o] = acc[d] - h;
     }
+  }
 }
 
 }  // namespace
@@ -234,15 +276,11 @@ int two_site_matvec_prepared(Ctx& ctx, cudaStream_t st, const double* H, const d
     SM_CUDA_CHECK(cudaMemsetAsync(x2h, 0, es * (size_t)m3 * mp.kpR, st));
     if (!bf16) SM_CUDA_CHECK(cudaMemsetAsync(x2l, 0, sizeof(float) * (size_t)m3 * mp.kpR, st));
   }
-  const size_t hs = sizeof(float) * (size_t)c * p1 * p1 * p2 * p2 * e;
-  const dim3 blk(32, 8), grd((f + 31) / 32, (a + 7) / 8);
-  if (bf16) {
-    if (hs > 48 * 1024) SM_CHECK(raise_smem_limit(k_h12_planes<true>, hs));
-    k_h12_planes<true><<<grd, blk, hs, st>>>(X1, H, a, c, p1, p2, e, f, mp.kpR, x2h, x2l);
-  } else {
-    if (hs > 48 * 1024) SM_CHECK(raise_smem_limit(k_h12_planes<false>, hs));
-    k_h12_planes<false><<<grd, blk, hs, st>>>(X1, H, a, c, p1, p2, e, f, mp.kpR, x2h, x2l);
-  }
+  const dim3 grd = h12_grid(a, p1, p2, e, f);
+  if (bf16)
+    k_h12_planes<true><<<grd, dim3(32, 8), 0, st>>>(X1, H, a, c, p1, p2, e, f, mp.kpR, x2h, x2l);
+  else
+    k_h12_planes<false><<<grd, dim3(32, 8), 0, st>>>(X1, H, a, c, p1, p2, e, f, mp.kpR, x2h, x2l);
   note_launch();
   SM_CUDA_CHECK(cudaGetLastError());
   return gemm_tc_planes<double>(ctx, st, m3, g, mp.kpR, bf16, x2h, x2l, mp.Rh, mp.Rl, 1.0, 0.0,
