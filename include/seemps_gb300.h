@@ -451,6 +451,17 @@ int sm_two_site_prepare(void* ctx, const int* dims, const void* L, const void* R
 int sm_two_site_matvec_prepared(void* ctx, const void* H, const void* v, void* out,
                                 void* stream);
 
+/* At most m Lanczos steps (real FP64 basis, every new vector re-orthogonalised twice)
+ * on the two-site operator from x0: the matvec of sm_two_site_matvec with `precision`,
+ * or with `prepared` != 0 the prepared operator (sm_two_site_prepare with the same L and
+ * R).  V (m x n, device, n = the vector's size) receives the basis, alpha and beta (host,
+ * m each) the tridiagonal matrix; *steps <= m counts the steps up to a breakdown
+ * (beta <= 1e-14 max |alpha|).  Counterpart of the eigsh call of
+ * optimization/dmrg.py:15-23, whose small eigenproblem stays with the caller. */
+int sm_two_site_lanczos(void* ctx, const int* dims, const void* L, const void* H, const void* R,
+                        const void* x0, int m, int precision, int prepared, void* V, double* alpha,
+                        double* beta, int* steps, void* stream);
+
 /* Upper bound on the bond dimensions a simplify of these kets can produce:
  * min(max_bond_dimension, summed ket bond); fills cap_bonds (L+1). */
 int sm_simplify_bond_caps(int L, const int* phys, int nterms, const int* ket_bonds,

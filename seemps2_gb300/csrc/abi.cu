@@ -513,6 +513,25 @@ int sm_two_site_matvec_prepared(void* ctx, const void* H, const void* v, void* o
   return tc_status_check(c, s);
 }
 
+int sm_two_site_lanczos(void* ctx, const int* dims, const void* L, const void* H, const void* R,
+                        const void* x0, int m, int precision, int prepared, void* V, double* alpha,
+                        double* beta, int* steps, void* stream) {
+  SM_GUARD_CTX(ctx);
+  if (!dims || !L || !H || !R || !x0 || !V || !alpha || !beta || !steps || m < 1 ||
+      precision < SM_MATVEC_FP64 || precision > SM_MATVEC_BF16) {
+    set_error("two_site_lanczos: null argument, no steps or unknown precision");
+    return SM_ERR_VALUE;
+  }
+  for (int i = 0; i < 8; ++i)
+    if (dims[i] <= 0) {
+      set_error("two_site_lanczos: non-positive dimension");
+      return SM_ERR_VALUE;
+    }
+  return lanczos_run(*as_ctx(ctx), as_stream(stream), dims, (const double*)L, (const double*)H,
+                     (const double*)R, precision, prepared != 0, (const double*)x0, m, (double*)V,
+                     alpha, beta, steps);
+}
+
 int sm_ctx_set_rank_cap(void* ctx, double margin, int extra) {
   SM_GUARD_CTX(ctx);
   if (!(margin >= 1.0) || extra < 0) {

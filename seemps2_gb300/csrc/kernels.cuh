@@ -219,6 +219,14 @@ int two_site_prepare(Ctx& ctx, cudaStream_t st, int a, int c, int b, int p1, int
 int two_site_matvec_prepared(Ctx& ctx, cudaStream_t st, const double* H, const double* v,
                              double* out);
 
+// --- lanczos.cu ---------------------------------------------------------------
+// At most m Lanczos steps from x0 on the two-site operator (dims a c b p1 p2 e g f),
+// or on the prepared one: V (m x n, device) receives the basis, alpha and beta (host, m
+// each) the tridiagonal matrix, *steps the steps up to m or a breakdown.
+int lanczos_run(Ctx& ctx, cudaStream_t st, const int* dims, const double* L, const double* H,
+                const double* R, int precision, bool prepared, const double* x0, int m, double* V,
+                double* alpha, double* beta, int* steps);
+
 // --- mpo_env.cu --------------------------------------------------------------
 // Three-leg MPO environments (bra A (a, j, d), MPO O (c, j, i, e), ket B (b, i, f)):
 // left rho (a, c, b) -> out (d, e, f); right rho (d, e, f) -> out (a, c, b).

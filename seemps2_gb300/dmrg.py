@@ -89,6 +89,11 @@ class TwoSiteOperator:
             _lib.stream_handle()))
         TwoSiteOperator._current[_ctx_key(ctx)] = id(self)
 
+    def ensure_prepared(self):
+        """Make this the operator whose planes the context holds."""
+        if TwoSiteOperator._current.get(_ctx_key(_lib.context())) != id(self):
+            self._prepare()
+
     def matvec(self, v, out=None):
         import torch
 
@@ -97,8 +102,7 @@ class TwoSiteOperator:
             raise ValueError("TwoSiteOperator.matvec: v has the wrong shape")
         if out is None:
             out = torch.empty(self.out_shape, dtype=torch.float64, device=v.device)
-        if TwoSiteOperator._current.get(_ctx_key(_lib.context())) != id(self):
-            self._prepare()
+        self.ensure_prepared()
         _lib.check(_lib.load().sm_two_site_matvec_prepared(
             _lib.context(), _lib.ptr(self.H), _lib.ptr(v), _lib.ptr(out), _lib.stream_handle()))
         return out
@@ -112,50 +116,42 @@ def _gemm(opA, opB, M, N, K, A, lda, B, ldb, Cm, ldc, alpha=1.0, beta=0.0):
         _lib.stream_handle()))
 
 
-def _lanczos_cycle(apply, x0, m: int):
-    """One Lanczos run of at most m steps from x0 (real, FP64 basis): every new vector is
-    re-orthogonalised against the basis twice (classical Gram-Schmidt with the library's
-    FP64 GEMM); the tridiagonal problem is solved on the host.  Returns (lowest Ritz value,
-    Ritz vector shaped like x0, residual norm estimate beta_m |y_m|, steps)."""
+def _lanczos_cycle(L, H, R, precision: str, op, x0, m: int):
+    """One Lanczos run of at most m steps from x0 (real, FP64 basis): one library call
+    (``sm_two_site_lanczos``), every new vector re-orthogonalised against the basis twice
+    (classical Gram-Schmidt); the tridiagonal problem is solved on the host.  ``op`` is
+    the TwoSiteOperator to use, or None for matvecs in ``precision``.  Returns (lowest Ritz
+    value, Ritz vector shaped like x0, residual norm estimate beta_m |y_m|, steps)."""
     import torch
 
     shape = tuple(x0.shape)
     n = x0.numel()
     m = max(1, min(m, n))
     dev = x0.device
+    if precision not in PRECISIONS:
+        raise ValueError(f"precision must be one of {sorted(PRECISIONS)}")
+    a, c, b = L.shape
+    c2, p1, k1, p2, k2, e = H.shape
+    g, e2, f = R.shape
+    if (c2, k1, k2, e2) != (c, p1, p2, e) or shape != (b, p1, p2, f) or (a, g) != (b, f):
+        raise ValueError("lanczos: inconsistent shapes")
     V = torch.empty((m, n), dtype=torch.float64, device=dev)
-    coef = torch.empty((m, 1), dtype=torch.float64, device=dev)
-    s = torch.empty((1, 1), dtype=torch.float64, device=dev)
-    one = torch.ones((1, 1), dtype=torch.float64, device=dev)
-    w = torch.empty(shape, dtype=torch.float64, device=dev)
-    alpha, beta = [], []
-    q = x0.reshape(-1)
-    _gemm(0, 0, 1, 1, n, q, n, q, 1, s, 1)
-    _gemm(0, 0, n, 1, 1, q, 1, one, 1, V[0], 1, alpha=1.0 / float(s.sqrt().item()))
-    steps, b = 0, 0.0
-    for j in range(m):
-        apply(V[j].reshape(shape), w)
-        wf = w.reshape(-1)
-        _gemm(0, 0, j + 1, 1, n, V, n, wf, 1, coef, 1)
-        alpha.append(float(coef[j].item()))
-        for rep in range(2):
-            if rep:
-                _gemm(0, 0, j + 1, 1, n, V, n, wf, 1, coef, 1)
-            _gemm(1, 0, n, 1, j + 1, V, n, coef, 1, wf, 1, alpha=-1.0, beta=1.0)
-        _gemm(0, 0, 1, 1, n, wf, n, wf, 1, s, 1)
-        b = float(s.sqrt().item())
-        steps = j + 1
-        # an invariant subspace (breakdown) ends the run: the Ritz pair is then exact
-        if j + 1 == m or b <= 1e-14 * max(abs(a) for a in alpha):
-            break
-        beta.append(b)
-        _gemm(0, 0, n, 1, 1, wf, 1, one, 1, V[j + 1], 1, alpha=1.0 / b)
-    T = np.diag(alpha) + np.diag(beta[: steps - 1], 1) + np.diag(beta[: steps - 1], -1)
+    alpha, beta = (C.c_double * m)(), (C.c_double * m)()
+    count = C.c_int()
+    if op is not None:
+        op.ensure_prepared()
+    _lib.check(_lib.load().sm_two_site_lanczos(
+        _lib.context(), _lib.int_array([a, c, b, p1, p2, e, g, f]), _lib.ptr(L), _lib.ptr(H),
+        _lib.ptr(R), _lib.ptr(x0), m, PRECISIONS[precision], int(op is not None), _lib.ptr(V), alpha,
+        beta, C.byref(count), _lib.stream_handle()))
+    steps = count.value
+    al, be = np.array(alpha[:steps]), np.array(beta[:steps])
+    T = np.diag(al) + np.diag(be[:-1], 1) + np.diag(be[:-1], -1)
     evals, evecs = np.linalg.eigh(T)
     y = torch.from_numpy(np.ascontiguousarray(evecs[:, 0].reshape(1, steps))).to(dev)
     x = torch.empty((1, n), dtype=torch.float64, device=dev)
     _gemm(0, 0, 1, n, steps, y, steps, V, n, x, n)
-    return float(evals[0]), x.reshape(shape), b * abs(float(evecs[steps - 1, 0])), steps
+    return float(evals[0]), x.reshape(shape), be[-1] * abs(float(evecs[steps - 1, 0])), steps
 
 
 def lanczos_ground_state(L, H, R, v0, krylov: int = 30, precision: str = "fp64", tol: float = 0.0,
@@ -176,28 +172,19 @@ def lanczos_ground_state(L, H, R, v0, krylov: int = 30, precision: str = "fp64",
     thr = max(tol, 1e-14)
     op = TwoSiteOperator(L, H, R, precision) if precision in ("tf32x3", "bf16") else None
 
-    def reduced(v, out):
-        if op is not None:
-            op.matvec(v, out=out)
-        else:
-            two_site_matvec(L, H, R, v, precision, out=out)
-
-    def full(v, out):
-        two_site_matvec(L, H, R, v, polish_precision, out=out)
-
     total = 0
     lam = 0.0
     # a reduced-precision operator cannot resolve the residual below its own rounding:
     # one cycle of it, then the FP64-accurate polish
     cycles = 1 if (op is not None and polish > 0) else 1 + max(0, restarts)
     for _ in range(cycles):
-        lam, x, res, steps = _lanczos_cycle(reduced, x, krylov)
+        lam, x, res, steps = _lanczos_cycle(L, H, R, precision, op, x, krylov)
         total += steps
         if res <= thr * max(abs(lam), 1e-300) or steps < krylov:
             break
     if op is not None and polish > 0:
         for _ in range(1 + max(0, restarts)):
-            lam, x, res, steps = _lanczos_cycle(full, x, polish)
+            lam, x, res, steps = _lanczos_cycle(L, H, R, polish_precision, None, x, polish)
             total += steps
             if res <= thr * max(abs(lam), 1e-300) or steps < polish:
                 break
