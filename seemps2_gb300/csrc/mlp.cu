@@ -19,73 +19,16 @@
 #include <cstring>
 #include <vector>
 
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include "kernels.cuh"
 
+namespace cg = cooperative_groups;
+
 namespace sm {
 
 namespace {
-
-constexpr int TB = 64, TK = 16, TNT = 256;
-
-// C[M,N] = op(A)[M,K] op(B)[K,N], FP32, op 0 = as stored, 1 = transposed.
-__global__ void __launch_bounds__(TNT) k_sgemm(int opA, int opB, int M, int N, int K,
-                                               const float* __restrict__ A, int lda,
-                                               const float* __restrict__ B, int ldb,
-                                               float* __restrict__ C, int ldc) {
-  __shared__ float As[TK][TB + 1];
-  __shared__ float Bs[TK][TB + 1];
-  const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
-  const int m0 = blockIdx.y * TB, n0 = blockIdx.x * TB;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += TK) {
-#pragma unroll
-    for (int e = 0; e < (TB * TK) / TNT; ++e) {
-      const int idx = tid + e * TNT;
-      int mm, kk;
-      if (opA == 0) { mm = idx / TK; kk = idx % TK; } else { kk = idx / TB; mm = idx % TB; }
-      const int gm = m0 + mm, gk = k0 + kk;
-      float v = 0.f;
-      if (gm < M && gk < K) v = opA == 0 ? A[(size_t)gm * lda + gk] : A[(size_t)gk * lda + gm];
-      As[kk][mm] = v;
-    }
-#pragma unroll
-    for (int e = 0; e < (TB * TK) / TNT; ++e) {
-      const int idx = tid + e * TNT;
-      int nn, kk;
-      if (opB == 0) { kk = idx / TB; nn = idx % TB; } else { nn = idx / TK; kk = idx % TK; }
-      const int gn = n0 + nn, gk = k0 + kk;
-      float v = 0.f;
-      if (gn < N && gk < K) v = opB == 0 ? B[(size_t)gk * ldb + gn] : B[(size_t)gn * ldb + gk];
-      Bs[kk][nn] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < TK; ++kk) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gm = m0 + ty + 16 * i;
-    if (gm >= M) continue;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int gn = n0 + tx + 16 * j;
-      if (gn < N) C[(size_t)gm * ldc + gn] = acc[i][j];
-    }
-  }
-}
 
 __device__ __forceinline__ float gelu_f(float z) {
   const float c = 0.7978845608028654f;
@@ -98,33 +41,114 @@ __device__ __forceinline__ float gelu_grad(float z) {
   return 0.5f * (1.f + t) + 0.5f * z * (1.f - t * t) * c * (1.f + 3.f * 0.044715f * z * z);
 }
 
-// Z += b (per column); A = gelu(Z) if A != nullptr
-__global__ void k_bias_act(float* __restrict__ Z, const float* __restrict__ b, int M, int N,
-                           float* __restrict__ A) {
-  const size_t tot = (size_t)M * N;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < tot;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const float z = Z[e] + b[e % N];
-    Z[e] = z;
-    if (A) A[e] = gelu_f(z);
+// C[M,N] = op(A)[M,K] op(B)[K,N] in FP32 with the layer's elementwise work in its
+// epilogue.  The training products are small (512 x 256 x 256: 34 MFLOP, well below a
+// microsecond of the chip's FP32 rate), so latency bounds them: 32 x 32 tiles and up to
+// 8 K slices (the CTAs of a cluster, which add their tiles over DSMEM in slice order)
+// put a product on several hundred CTAs with one to four 32-deep slabs each, the next
+// slab's loads in flight during a multiply.  A loss and its gradients on 512 rows
+// took 370 us with 64 x 64 tiles over the whole of K and separate kernels for bias,
+// activation, their gradients and the column sums.
+enum { EPI_LAYER = 0, EPI_DW = 1, EPI_DA = 2 };
+struct Epi {
+  const float* bias = nullptr;  // EPI_LAYER: Z = product + bias
+  float* act = nullptr;         //   A = gelu(Z) (hidden), or Z
+  int hidden = 0;
+  float* out = nullptr;         //   and a copy of A, if given
+  float* colsum = nullptr;      // EPI_DW: sums of op(A)'s rows (the bias gradient)
+  const float* z = nullptr;     // EPI_DA: C = product * gelu'(z)
+};
+
+constexpr int TS = 32, TNT = 128;
+template <int OPA, int OPB, int EPI>
+__global__ void __launch_bounds__(TNT) k_sgemm(int M, int N, int K, const float* __restrict__ A,
+                                               int lda, const float* __restrict__ B, int ldb,
+                                               float* __restrict__ C, int ldc, int kchunk, Epi ep) {
+  __shared__ __align__(16) float As[TS][TS + 2];  // [k][m]: pairs of rows
+  __shared__ __align__(16) float Bs[TS][TS + 4];  // [k][n]: quadruples of columns
+  __shared__ float tile[TS][TS + 1];
+  __shared__ float csum[TS];
+  const int tid = threadIdx.x, tx = tid % 8, ty = tid / 8;
+  const int m0 = blockIdx.x * TS, n0 = blockIdx.y * TS;
+  const int kbeg = blockIdx.z * kchunk, kend = min(K, kbeg + kchunk);
+  float acc[2][4] = {};
+  float ra[8], rb[8], cs = 0.f;
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int idx = tid + e * TNT, hi = idx / TS, lo = idx % TS;  // consecutive threads: lo
+      const int mm = OPA ? lo : hi, ka = OPA ? hi : lo;
+      const int nn = OPB ? hi : lo, kb = OPB ? lo : hi;
+      ra[e] = rb[e] = 0.f;
+      if (m0 + mm < M && k0 + ka < kend)
+        ra[e] = OPA ? A[(size_t)(k0 + ka) * lda + m0 + mm] : A[(size_t)(m0 + mm) * lda + k0 + ka];
+      if (n0 + nn < N && k0 + kb < kend)
+        rb[e] = OPB ? B[(size_t)(n0 + nn) * ldb + k0 + kb] : B[(size_t)(k0 + kb) * ldb + n0 + nn];
+    }
+  };
+  if (kbeg < kend) fetch(kbeg);
+  for (int k0 = kbeg; k0 < kend; k0 += TS) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int idx = tid + e * TNT, hi = idx / TS, lo = idx % TS;
+      As[OPA ? hi : lo][OPA ? lo : hi] = ra[e];
+      Bs[OPB ? lo : hi][OPB ? hi : lo] = rb[e];
+    }
+    __syncthreads();
+    if (k0 + TS < kend) fetch(k0 + TS);
+#pragma unroll
+    for (int kk = 0; kk < TS; ++kk) {
+      const float2 a = *reinterpret_cast<const float2*>(&As[kk][2 * ty]);
+      const float4 b = *reinterpret_cast<const float4*>(&Bs[kk][4 * tx]);
+      acc[0][0] = fmaf(a.x, b.x, acc[0][0]);
+      acc[0][1] = fmaf(a.x, b.y, acc[0][1]);
+      acc[0][2] = fmaf(a.x, b.z, acc[0][2]);
+      acc[0][3] = fmaf(a.x, b.w, acc[0][3]);
+      acc[1][0] = fmaf(a.y, b.x, acc[1][0]);
+      acc[1][1] = fmaf(a.y, b.y, acc[1][1]);
+      acc[1][2] = fmaf(a.y, b.z, acc[1][2]);
+      acc[1][3] = fmaf(a.y, b.w, acc[1][3]);
+    }
+    if (EPI == EPI_DW && n0 == 0 && tid < TS)
+      for (int kk = 0; kk < TS; ++kk) cs += As[kk][tid];
+    __syncthreads();
   }
-}
-
-// dZ = dA * gelu'(Z)
-__global__ void k_gelu_back(const float* __restrict__ dA, const float* __restrict__ Z, size_t n,
-                            float* __restrict__ dZ) {
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n;
-       e += (size_t)gridDim.x * blockDim.x)
-    dZ[e] = dA[e] * gelu_grad(Z[e]);
-}
-
-// db[j] = sum_i dZ[i][j], one thread per column, rows summed in order
-__global__ void k_col_sum(const float* __restrict__ dZ, int M, int N, float* __restrict__ db) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= N) return;
-  float a = 0.f;
-  for (int i = 0; i < M; ++i) a += dZ[(size_t)i * N + j];
-  db[j] = a;
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) tile[2 * ty + i][4 * tx + j] = acc[i][j];
+  if (EPI == EPI_DW && n0 == 0 && tid < TS) csum[tid] = cs;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int nz = gridDim.z;
+  if (nz > 1) cluster.sync();
+  else __syncthreads();
+  // this slice's share of the rows
+  const int rows = (TS + nz - 1) / nz, r1 = min(TS, (int)(blockIdx.z + 1) * rows);
+  for (int e = blockIdx.z * rows * TS + tid; e < r1 * TS; e += TNT) {
+    const int mm = e / TS, nn = e % TS, m = m0 + mm, n = n0 + nn;
+    if (m >= M || n >= N) continue;
+    float v = 0.f;
+    if (nz > 1)
+      for (int z = 0; z < nz; ++z) v += *cluster.map_shared_rank(&tile[mm][nn], z);
+    else v = tile[mm][nn];
+    if (EPI == EPI_LAYER) {
+      v += ep.bias[n];
+      C[(size_t)m * ldc + n] = v;
+      const float a = ep.hidden ? gelu_f(v) : v;
+      ep.act[(size_t)m * N + n] = a;
+      if (ep.out) ep.out[(size_t)m * N + n] = a;
+    } else if (EPI == EPI_DA) {
+      C[(size_t)m * ldc + n] = v * gelu_grad(ep.z[(size_t)m * N + n]);
+    } else {
+      C[(size_t)m * ldc + n] = v;
+    }
+  }
+  if (EPI == EPI_DW && n0 == 0 && blockIdx.z == 0 && tid < TS && m0 + tid < M) {
+    float v = 0.f;
+    for (int z = 0; z < nz; ++z) v += nz > 1 ? *cluster.map_shared_rank(&csum[tid], z) : csum[tid];
+    ep.colsum[m0 + tid] = v;
+  }
+  if (nz > 1) cluster.sync();  // no slice leaves while another reads its tile
 }
 
 // mean squared error: dy = 2 (yhat - y) / B; loss[0] = mean (one block)
@@ -190,13 +214,28 @@ inline int blocks_for(size_t n) {
   return (int)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 4096));
 }
 
-int sgemm(cudaStream_t st, int opA, int opB, int M, int N, int K, const float* A, int lda,
-          const float* B, int ldb, float* C, int ldc) {
-  if (M <= 0 || N <= 0) return SM_OK;
-  dim3 grid((N + TB - 1) / TB, (M + TB - 1) / TB);
-  k_sgemm<<<grid, TNT, 0, st>>>(opA, opB, M, N, K, A, lda, B, ldb, C, ldc);
+template <int OPA, int OPB, int EPI>
+int sgemm(cudaStream_t st, int M, int N, int K, const float* A, int lda, const float* B, int ldb,
+          float* C, int ldc, const Epi& ep) {
+  const long tiles = (long)((N + TS - 1) / TS) * ((M + TS - 1) / TS);
+  // slices of at least one slab, until two CTAs per SM
+  int nz = 1;
+  while (nz < 8 && tiles * nz < 304 && K > TS * nz) nz *= 2;
+  const int kchunk = ((K + nz - 1) / nz + TS - 1) / TS * TS;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((M + TS - 1) / TS, (N + TS - 1) / TS, nz);  // N <= 4096
+  cfg.blockDim = dim3(TNT);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = nz;
+  cfg.attrs = attr;
+  cfg.numAttrs = nz > 1 ? 1 : 0;
+  SM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_sgemm<OPA, OPB, EPI>, M, N, K, A, lda, B, ldb, C, ldc,
+                                   kchunk, ep));
   note_launch();
-  SM_CUDA_CHECK(cudaGetLastError());
   return SM_OK;
 }
 
@@ -379,19 +418,16 @@ int sm_mlp_forward(void* ctx, int n_layers, const int* dims, const float* params
     const float* b = W + (size_t)dout * di;
     float* Z = cache + co;
     float* A = Z + (size_t)batch * dout;
-    SM_CHECK(sgemm(st, 0, 1, batch, dout, di, in, di, W, di, Z, dout));
-    const bool hidden = k + 1 < n_layers;
-    k_bias_act<<<blocks_for((size_t)batch * dout), 256, 0, st>>>(Z, b, batch, dout,
-                                                                 hidden ? A : nullptr);
-    note_launch();
-    if (!hidden)
-      SM_CUDA_CHECK(cudaMemcpyAsync(A, Z, sizeof(float) * batch * dout, cudaMemcpyDeviceToDevice, st));
+    Epi ep;
+    ep.bias = b;
+    ep.act = A;
+    ep.hidden = k + 1 < n_layers;
+    ep.out = ep.hidden ? nullptr : Y;
+    SM_CHECK((sgemm<0, 1, EPI_LAYER>(st, batch, dout, di, in, di, W, di, Z, dout, ep)));
     in = A;
     po += (size_t)dout * di + dout;
     co += 2 * (size_t)batch * dout;
   }
-  SM_CUDA_CHECK(cudaMemcpyAsync(Y, in, sizeof(float) * batch * dims[n_layers],
-                                cudaMemcpyDeviceToDevice, st));
   SM_CUDA_CHECK(cudaGetLastError());
   return SM_OK;
 }
@@ -419,23 +455,22 @@ int sm_mlp_backward(void* ctx, int n_layers, const int* dims, const float* param
     p += (size_t)dims[k + 1] * dims[k] + dims[k + 1];
     q += 2 * (size_t)batch * dims[k + 1];
   }
-  // dZ of the last layer = dY (no activation)
-  SM_CUDA_CHECK(cudaMemcpyAsync(g0, dY, sizeof(float) * batch * dims[n_layers],
-                                cudaMemcpyDeviceToDevice, st));
+  const float* dZ = dY;  // of the last layer: no activation
   for (int k = n_layers - 1; k >= 0; --k) {
     const int di = dims[k], dout = dims[k + 1];
     const float* W = params + po[k];
     float* gW = grads + po[k];
     float* gb = gW + (size_t)dout * di;
     const float* in = k == 0 ? X : cache + co[k - 1] + (size_t)batch * dims[k];  // A_{k-1}
-    SM_CHECK(sgemm(st, 1, 0, dout, di, batch, g0, dout, in, di, gW, di));  // dW = dZ^T X
-    k_col_sum<<<(dout + 127) / 128, 128, 0, st>>>(g0, batch, dout, gb);
-    note_launch();
-    if (k > 0) {
-      SM_CHECK(sgemm(st, 0, 0, batch, di, dout, g0, dout, W, di, g1, di));  // dA = dZ W
-      const float* Zp = cache + co[k - 1];
-      k_gelu_back<<<blocks_for((size_t)batch * di), 256, 0, st>>>(g1, Zp, (size_t)batch * di, g0);
-      note_launch();
+    Epi ep;
+    ep.colsum = gb;
+    SM_CHECK((sgemm<1, 0, EPI_DW>(st, dout, di, batch, dZ, dout, in, di, gW, di, ep)));  // dZ^T X
+    if (k > 0) {  // dZ of the layer below = (dZ W) gelu'(Z)
+      Epi ed;
+      ed.z = cache + co[k - 1];
+      float* g = dZ == g0 ? g1 : g0;
+      SM_CHECK((sgemm<0, 0, EPI_DA>(st, batch, di, dout, dZ, dout, W, di, g, di, ed)));
+      dZ = g;
     }
   }
   SM_CUDA_CHECK(cudaGetLastError());
