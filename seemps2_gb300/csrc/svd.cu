@@ -167,72 +167,99 @@ __device__ __forceinline__ double recip_newton(double x) {
   return y * fma(-x, y, 2.0);
 }
 
-// Jacobi rotation of a pair of rows with squared norms a, b and overlap g = gr + i gi
-// (g2 = |g|^2): cosine c, sine sn, phase (er, ei) of g, and the norms after it.
+// A positive double as an FP32 mantissa in [1, 2) and an exponent, by integer
+// operations alone: a conversion holds the FP64 pipe like any other operation.
+// Zero and denormals have m = 0; infinity and NaN have e = 1024.
+struct FloatExp {
+  float m;
+  int e;
+};
+__device__ __forceinline__ FloatExp split_abs(double x) {
+  const int hi = __double2hiint(x) & 0x7fffffff;
+  const unsigned lo = (unsigned)__double2loint(x);
+  const float m = __int_as_float(0x3f800000 | ((hi & 0xfffff) << 3) | (int)(lo >> 29));
+  return {hi >> 20 ? m : 0.0f, (hi >> 20) - 1023};
+}
+// f 2^e of a normal or zero FP32 f as a double; 0 below the normal range
+__device__ __forceinline__ double join_exp(float f, int e) {
+  const int b = __float_as_int(f), x = ((b >> 23) & 0xff) - 127 + 1023 + e;
+  if ((b & 0x7f800000) == 0 || x <= 0) return 0.0;
+  return __hiloint2double((b & 0x80000000) | x << 20 | (b & 0x7fffff) >> 3, (int)((unsigned)b << 29));
+}
+// 2^e in FP32, 0 below its normal range (e <= 127)
+__device__ __forceinline__ float pow2f(int e) { return e < -126 ? 0.0f : __int_as_float((e + 127) << 23); }
+// x > y
+__device__ __forceinline__ bool greater_exp(FloatExp x, FloatExp y) {
+  const int d = x.e - y.e;
+  if (x.m == 0.0f || y.m == 0.0f) return x.m > y.m;
+  return d > 60 || (d > -60 && x.m * pow2f(d) > y.m);
+}
+
+// Jacobi rotation of a pair of rows with squared norms a, b and overlap g = gr + i gi:
+// whether |g|^2 is above tiny2 and tol2 a b, and if so the cosine c, the sine sn, the
+// phase (er, ei) of g, and the norms after it.
+//
+// What a round waits for is this chain: each FP64 operation holds a sub-partition's
+// pipe for 64 clocks.  So the test, tan = sign(b - a) 2|g| / (|b - a| + root) and the
+// phase are computed in FP32 on mantissas, with their exponents beside them (no range
+// is lost), and FP64 only makes the rotation unitary: c = 1/sqrt(1 + tan^2) by one
+// Newton step of third order from an FP32 start, the phase by the same step.  An
+// angle of FP32 accuracy leaves ~1e-7 of the overlap for the pair's next round.
+// (15 FP64 operations for a real pair, against 30 to 50 with conversions, FP64
+// tests and an FP64 angle for small cosines.)
 template <bool kCplx>
-__device__ __forceinline__ void jacobi_angle(double a, double b, double gr, double gi, double g2,
-                                             double& c, double& sn, double& er, double& ei,
-                                             double& na, double& nb) {
-  // Angle in FP32 on values scaled by a power of two so that a + b
-  // lands in [1, 2): zeta = (b - a) / 2|g|, t = sign(zeta) /
-  // (|zeta| + sqrt(1 + zeta^2)).  The (c, s) pair (and the complex
-  // phase) are then brought to unit norm in FP64 with a two-term
-  // correction f = 1 - d/2 + 3d^2/8, d = c^2 + s^2 - 1 ~ 1e-7, which
-  // leaves c^2 + s^2 - 1 = O(d^3): each rotation is unitary to FP64
-  // rounding whatever the accuracy of the angle.
-  // An FP32 angle annihilates the overlap only to ~1e-7 of itself.
-  // Far from convergence that is harmless (the next sweep finishes
-  // the job), but once the pair's cosine |g|/sqrt(ab) is small the
-  // residual no longer shrinks quadratically, and inside a cluster
-  // of (nearly) equal singular values the iteration stalls at the
-  // FP32 level.  So the FP32 angle is only taken while the cosine is
-  // at least 1e-4; the last sweeps' few rotations use FP64.
-  const int ex = (__double2hiint(a + b) >> 20) & 0x7ff;
-  const double sc = __hiloint2double((2046 - ex) << 20, 0);     // 2^(1023 - ex)
-  const float as = (float)(a * sc), bs = (float)(b * sc);
-  // |g| and its phase (complex: brought near 1 by a power of two before squaring)
-  double gabs = fabs(gr);
-  er = gr >= 0.0 ? 1.0 : -1.0;  // the phase of a real overlap is its sign
-  ei = 0.0;
+__device__ __forceinline__ bool jacobi_rotation(double a, double b, double gr, double gi,
+                                                FloatExp tol2, FloatExp tiny2, double& c,
+                                                double& sn, double& er, double& ei, double& na,
+                                                double& nb) {
+  const FloatExp fa = split_abs(a), fb = split_abs(b), fr = split_abs(gr);
+  int eg = fr.e;  // |g|^2 = g2 4^eg, |g| = gm 2^eg
+  float xr = copysignf(fr.m, __int_as_float(__double2hiint(gr))), xi = 0.0f, g2 = fr.m * fr.m;
+  float gm = fr.m;
   if constexpr (kCplx) {
-    const int eg = (__double2hiint(fmax(gabs, fabs(gi))) >> 20) & 0x7ff;
-    const double sg = eg > 0 && eg < 2046 ? __hiloint2double((2046 - eg) << 20, 0) : 1.0;
-    const double xr = gr * sg, xi = gi * sg, x2 = fma(xr, xr, xi * xi);
-    const double rn = rsqrt_newton(x2);
-    er = xr * rn;
-    ei = xi * rn;
-    gabs = x2 * rn * (eg > 0 && eg < 2046 ? __hiloint2double(eg << 20, 0) : 1.0);
+    const FloatExp fi = split_abs(gi);
+    eg = max(fr.e, fi.e);
+    xr *= pow2f(fr.e - eg);
+    xi = copysignf(fi.m * pow2f(fi.e - eg), __int_as_float(__double2hiint(gi)));
+    g2 = fmaf(xr, xr, xi * xi);
+    gm = sqrtf(g2);
   }
-  double tt;
-  float zf = 0.0f;
-  const float gabs_f = (float)(gabs * sc);
-  const bool fp32_ok = ex > 0 && ex < 2046 && gabs_f > 1e-30f && g2 >= 1e-8 * a * b;
-  if (fp32_ok) zf = 0.5f * (bs - as) / gabs_f;
-  if (fp32_ok && fabsf(zf) < 1e18f) {
-    const float az = fabsf(zf);
-    const float tf = copysignf(1.0f / (az + sqrtf(fmaf(az, az, 1.0f))), zf);
-    const float cf = rsqrtf(fmaf(tf, tf, 1.0f));
-    const double c64 = (double)cf, s64 = (double)(cf * tf);
-    const double d = fma(c64, c64, fma(s64, s64, -1.0));
-    const double f = fma(d, fma(0.375, d, -0.5), 1.0);
-    c = c64 * f;
-    sn = s64 * f;
-    tt = (double)tf;
+  if (fa.e > 1023 || fb.e > 1023 || eg > 1023) return false;  // not finite: no rotation mends it
+  const FloatExp f2 = {g2, 2 * eg};
+  if (!greater_exp(f2, tiny2) ||
+      !greater_exp(f2, FloatExp{fa.m * fb.m * tol2.m, fa.e + fb.e + tol2.e}))
+    return false;
+  const double d = b - a;
+  const FloatExp fd = split_abs(d);
+  const int e = max(fd.e, eg + 1);
+  const float df = fd.m * pow2f(fd.e - e), hf = gm * pow2f(eg + 1 - e);
+  const float den = df + sqrtf(fmaf(df, df, hf * hf));
+  const double t = copysign(join_exp(gm / den, eg + 1 - e), d);
+  const double u = fma(t, t, 1.0);
+  const FloatExp fu = split_abs(u);  // u in [1, 2]
+  const double y = join_exp(rsqrtf(fu.e > 0 ? 2.0f : fu.m), 0);
+  const double r = fma(-u * y, y, 1.0);
+  c = fma(y * r, fma(0.375, r, 0.5), y);
+  sn = c * t;
+  double gabs;
+  if constexpr (kCplx) {
+    const float rg = rsqrtf(g2);
+    er = join_exp(xr * rg, 0);
+    ei = join_exp(xi * rg, 0);
+    const double q = fma(er, er, fma(ei, ei, -1.0));
+    const double f = fma(q, fma(0.375, q, -0.5), 1.0);
+    er *= f;
+    ei *= f;
+    gabs = fma(er, gr, ei * gi);
   } else {
-    // small cosines, extremely graded pairs: tan = 2|g| / (|b - a| + root), the root
-    // and the quotient by Newton's iteration in FP64
-    const bool in_range = ex > 0 && ex < 2046;
-    const double ds = in_range ? (b - a) * sc : b - a, hs = 2.0 * (in_range ? gabs * sc : gabs);
-    const double q = fma(ds, ds, hs * hs);
-    const double r = q > 0.0 ? q * rsqrt_newton(q) : 0.0;
-    tt = r > 0.0 ? copysign(hs * recip_newton(fabs(ds) + r), ds) : 1.0;
-    c = rsqrt_newton(fma(tt, tt, 1.0));
-    sn = c * tt;
+    er = copysign(1.0, gr);
+    ei = 0.0;
+    gabs = fabs(gr);
   }
-  // closed-form norm update (approximate; exact norms return at the
-  // first round of the next sweep)
-  na = fma(-tt, gabs, a);
-  nb = fma(tt, gabs, b);
+  // closed-form norm update (exact norms return with the next sweep)
+  na = fma(-t, gabs, a);
+  nb = fma(t, gabs, b);
+  return true;
 }
 
 // One CTA (NT threads, NT/32 warps) per pair, so that every SM sub-partition's
@@ -243,13 +270,9 @@ __device__ __forceinline__ void jacobi_angle(double a, double b, double gr, doub
 // thread keeps its E elements of both rows in registers between the dot
 // products and the rotation; E == 0 streams the rows twice from L2.
 //
-// Rotation parameters: the convergence test |g|^2 > tol^2 a b needs no root;
-// zeta = (b - a) / 2|g| uses one FP64 rsqrt; t = tan(theta) is evaluated in
-// FP32 (an inexact angle only leaves a slightly larger residual for the next
-// sweep) except for |zeta| >= 1e18 where t = 1/2zeta in FP64; c = 1/sqrt(1+t^2),
-// s = c t and the complex phase g/|g| use FP64 rsqrt, so every applied rotation
-// is unitary to FP64 rounding.  Squared norms are computed exactly in the first
-// round of every sweep and updated in closed form after each rotation.
+// The rotation is jacobi_rotation's: unitary to FP64 rounding, its angle to FP32
+// accuracy.  Squared norms are computed exactly in the first round of every sweep
+// and updated in closed form after each rotation.
 //
 // Pairs whose overlap is below an absolute floor (16 l eps^2 |A|_F^2, just
 // above the rounding-noise level) count as orthogonal when `use_floor` is set:
@@ -275,6 +298,7 @@ __global__ void __launch_bounds__(NT) k_jacobi(T* Wx, int ld, int k, int l, int 
     const double tiny = 16.0 * l * DBL_EPSILON * DBL_EPSILON * frob2;
     tiny2 = tiny * tiny;
   }
+  const FloatExp ftol2 = split_abs(tol2), ftiny2 = split_abs(tiny2);
   // rows whose squared norm falls to thr or below are deflated: the
   // truncation rule certainly discards them, so they leave the round-robin
   const double thr = defl_abs > 0.0 ? fmin(defl_rel * frob2, defl_abs) : defl_rel * frob2;
@@ -402,12 +426,10 @@ __global__ void __launch_bounds__(NT) k_jacobi(T* Wx, int ld, int k, int l, int 
         // form after each rotation
         a = __ldcg(nrm + p);
         b = __ldcg(nrm + q);
-        const double g2 = kCplx ? fma(gr, gr, gi * gi) : gr * gr;
-        const bool rot = g2 > tiny2 && g2 > tol2 * a * b;
-        double na = a, nb = b;
+        double na = a, nb = b, c, sn, er, ei;
+        const bool rot =
+            jacobi_rotation<kCplx>(a, b, gr, gi, ftol2, ftiny2, c, sn, er, ei, na, nb);
         if (rot) {
-          double c, sn, er, ei;
-          jacobi_angle<kCplx>(a, b, gr, gi, g2, c, sn, er, ei, na, nb);
           Rot<T> R;
           R.set(c, sn, er, ei);
           if constexpr (E > 0) {
@@ -1237,7 +1259,8 @@ int house_qr(Ctx& ctx, cudaStream_t st, T* Wt, int kw, int l, double thr_rel, T*
 // sorting, truncation) in one CTA with the matrix in shared memory.  The splits at
 // the ends of a chain have 2..48 rows; on the kernels above they pay a launch for
 // each phase and a grid barrier for each reflector and each round (32 x 32: 1.4 ms),
-// while one SM's FP64 pipe does a round of them in about a microsecond.
+// while one SM's FP64 pipe does a round of them in two microseconds (32 x 32: 0.70
+// ms; 0.91 ms with the angle's conversions, tests and small cosines in FP64).
 //
 // A pair of rows (and a column of the QR) belongs to 8 lanes: four pairs share the
 // FP64 instructions of a warp, so that their sums take three shuffle levels and the
@@ -1380,7 +1403,9 @@ __global__ void __launch_bounds__(kSmallNT)
   };
   // ---- one-sided Jacobi (as k_jacobi) ------------------------------------------
   int status = k >= 2 ? DEV_NOT_CONVERGED : 0, sweeps = 0;
-  double thr = 0.0, tiny2 = 0.0;
+  const FloatExp ftol2 = split_abs(tol2);
+  FloatExp ftiny2 = {0.0f, 0};
+  double thr = 0.0;
   for (int sweep = 0; k >= 2 && sweep < max_sweeps; ++sweep) {
     for (int i0 = 0; i0 < k; i0 += NG) {
       const double a = row_norm(i0 + g8);
@@ -1406,7 +1431,7 @@ __global__ void __launch_bounds__(kSmallNT)
     __syncthreads();
     if (sweep == 0 && use_floor) {
       const double tiny = 16.0 * l * DBL_EPSILON * DBL_EPSILON * red[0];
-      tiny2 = tiny * tiny;
+      ftiny2 = split_abs(tiny * tiny);
     }
     const int ka = nact, kp = ka + (ka & 1), npairs = kp / 2;
     for (int r = 0; r + 1 < kp; ++r) {
@@ -1428,25 +1453,20 @@ __global__ void __launch_bounds__(kSmallNT)
         gr = sum8(gr);
         if constexpr (kCplx) gi = sum8(gi);
         const double a = nrm[p], b = nrm[q];
-        const double g2 = kCplx ? fma(gr, gr, gi * gi) : gr * gr;
-        const bool rot = on && g2 > tiny2 && g2 > tol2 * a * b;
-        if (__any_sync(0xffffffffu, rot)) {
-          double c = 1.0, sn = 0.0, e_r = 1.0, e_i = 0.0, na = a, nb = b;
-          if (rot) {
-            jacobi_angle<kCplx>(a, b, gr, gi, g2, c, sn, e_r, e_i, na, nb);
-            Rot<T> R;
-            R.set(c, sn, e_r, e_i);
-            for (int x = l8; x < l; x += 8) {
-              T u = rp[x], v = rq[x];
-              R.apply(u, v);
-              rp[x] = u;
-              rq[x] = v;
-            }
-            if (l8 == 0) {
-              nrm[p] = na;
-              nrm[q] = nb;
-              rotated = 1;
-            }
+        double c, sn, e_r, e_i, na, nb;
+        if (on && jacobi_rotation<kCplx>(a, b, gr, gi, ftol2, ftiny2, c, sn, e_r, e_i, na, nb)) {
+          Rot<T> R;
+          R.set(c, sn, e_r, e_i);
+          for (int x = l8; x < l; x += 8) {
+            T u = rp[x], v = rq[x];
+            R.apply(u, v);
+            rp[x] = u;
+            rq[x] = v;
+          }
+          if (l8 == 0) {
+            nrm[p] = na;
+            nrm[q] = nb;
+            rotated = 1;
           }
         }
       }

@@ -1,0 +1,82 @@
+"""Splits, products and steps at the sizes where a kernel's tiles or the choice between
+two kernels change (GPU required): one short and one long of each boundary, remainders,
+the smallest and the largest."""
+
+import numpy as np
+import pytest
+
+from oracle import seemps_oracle as so
+from tests.gpu_util import to_np
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA GPU", allow_module_level=True)
+
+import seemps2_gb300 as sg  # noqa: E402
+from seemps2_gb300 import core  # noqa: E402
+
+
+def gaussian(rng, shape, cplx):
+    x = rng.normal(size=shape)
+    return x + 1j * rng.normal(size=shape) if cplx else x
+
+
+def matrix(rng, m, n, s, cplx):
+    """m x n with the singular values s"""
+    q = [np.linalg.qr(gaussian(rng, (r, len(s)), cplx))[0] for r in (m, n)]
+    return (q[0] * s) @ q[1].conj().T
+
+
+def check_split(A, tol=1e-12, maxb=10**6, atol=1e-12):
+    """Both two-site splits of the m x n matrix A against the oracle's: the kept rank, the
+    product, the discarded weight, and the orthogonal factor.  An FP64 split of k rows is
+    some 10 k rotations of each element, 4 roundings each: below 1e-12 for k < 250."""
+    m, n = A.shape
+    st = sg.Strategy(tolerance=tol, max_bond_dimension=maxb)
+    ost = so.Strategy(tolerance=tol, max_bond_dimension=maxb)
+    scale = max(np.linalg.norm(A, 2), 1e-300)
+    for fn, ofn, left in [(core._left_orth_2site, so.left_orth_2site, True),
+                          (core._right_orth_2site, so.right_orth_2site, False)]:
+        L, R, e = fn(A.reshape(m, 1, 1, n), st)
+        oL, oR, oe = ofn(A.reshape(m, 1, 1, n), ost)
+        assert L.shape == oL.shape and R.shape == oR.shape
+        D = L.shape[-1]
+        L, R = to_np(L).reshape(m, D), to_np(R).reshape(D, n)
+        assert np.abs(L @ R - oL.reshape(m, D) @ oR.reshape(D, n)).max() <= atol * scale
+        Q = L.conj().T @ L if left else R @ R.conj().T
+        assert np.abs(Q - np.eye(D)).max() <= atol
+        assert abs(e - oe) <= 1e-9 * max(1e-2 * scale, oe)
+
+
+@pytest.mark.parametrize("m, n, cplx", [
+    (1, 1, False), (1, 1, True), (1, 7, False), (2, 2, True), (3, 2, False), (5, 4, True),
+    (8, 9, False), (31, 33, False), (32, 32, True), (33, 31, False), (47, 64, False),
+    # the last that one CTA takes, and the first that it does not: 48 rows, the
+    # work of 48^2 86 (complex 36^2 38), the shared memory of 9 x 2275
+    (48, 86, False), (87, 48, False), (36, 38, True), (39, 36, True), (49, 49, False),
+    (9, 2275, False), (2277, 9, False),
+])
+def test_small_fp64_splits(m, n, cplx):
+    rng = np.random.default_rng(100 * m + n)
+    k = min(m, n)
+    check_split(matrix(rng, m, n, np.geomspace(1.0, 1e-3, k), cplx))
+    # rows down to 1e-9 of the largest, half of them cut
+    check_split(matrix(rng, m, n, np.geomspace(1.0, 1e-9, k), cplx), maxb=max(1, k // 2))
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+def test_small_fp64_splits_of_odd_matrices(cplx):
+    """Pairs of rows whose norms differ by far more than the FP32 range, equal rows,
+    a zero row, and entries that are not finite."""
+    rng = np.random.default_rng(5)
+    A = gaussian(rng, (6, 20), cplx)
+    graded = A * np.array([[1.0], [1e-30], [1e-60], [1.0], [0.0], [1e-5]])
+    check_split(graded, tol=1e-25)
+    check_split(np.vstack([A[:3], A[:3]]))
+    A[2] = 0
+    check_split(A)
+    A[2, 3] = np.nan
+    with pytest.raises(Exception):
+        core._left_orth_2site(A.reshape(6, 1, 1, 20), sg.Strategy(tolerance=1e-12))
