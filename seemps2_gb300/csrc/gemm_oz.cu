@@ -25,22 +25,26 @@
 // products (i + j >= 8) are below 2^-56 of the row / column maxima, so the
 // result has the accuracy of an FP64 GEMM.
 //
-// One CTA (10 warps) per 128 x 64 output tile and K range (split over
-// blockIdx.z for small outputs):
+// One CTA (10 warps) per 128 x 64 output tile and K range:
 //   warp 8 / lane 0: TMA, one 3-D box per operand and stage holding all 8
 //            slices of a 32-wide K slab (64-byte swizzle), 2 stages;
 //   warp 9 / lane 0: 2 x 36 tcgen05.mma (M=128, N=64, K=16) per slab into
 //            8 x 64 TMEM columns, a commit per stage and per chunk;
 //   warps 0-7: per chunk, tcgen05.ld of the 8 accumulators (warp w owns tile
 //            rows 32 (w % 4) .. +31, columns 32 (w / 4) .. +31) into 32 int64
-//            + 32 FP32 registers per thread; at the end the scaled FP64 tile
-//            (or a split-K partial).
+//            + 32 FP32 registers per thread.
+// The K ranges of a tile are the CTAs of one cluster.  They leave their int64 and
+// FP32 sums in shared memory (where the stages were) and each adds up a share of
+// the tile's rows over the cluster and turns it into FP64.  Besides filling the
+// SMs, the split divides that conversion: three FP64-pipe operations for each
+// element are 6 us on a whole tile, against 1.2 us for a slab's MMAs.
 // Every mbarrier wait is bounded; a timeout sets a bit of the status word
 // shared with the TF32 path (read by tc_status_check), waits for the CTA's
 // copies in flight, frees TMEM and returns.
 #include <algorithm>
 #include <cfloat>
 
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -48,6 +52,8 @@
 #include "kernels.cuh"
 
 namespace sm {
+
+namespace cg = cooperative_groups;
 
 namespace {
 
@@ -60,6 +66,11 @@ constexpr uint32_t kSliceA = OM * OK * 2;  // 8 KB: one slice of A, one slab
 constexpr uint32_t kSliceB = ON * OK * 2;  // 4 KB
 constexpr uint32_t kOzStage = kSlices * (kSliceA + kSliceB);  // 96 KB
 constexpr size_t kOzSmem = (size_t)OS * kOzStage + 1024 + 256;
+constexpr int kOzRow = ON + 1;   // row stride of the sums in shared memory: no bank conflicts
+static_assert((size_t)OM * kOzRow * 12 <= (size_t)OS * kOzStage, "the sums fit where the stages were");
+constexpr int kOzNoExp = -(1 << 28);  // exponent of an all-zero row of an operand
+constexpr int kOzNotFinite = 1 << 28;  // and of one with an infinity or a NaN
+constexpr int kOzCluster = 8;    // K ranges of a tile that share a cluster (portable size)
 constexpr uint32_t kOzCols = 512;  // TMEM allocation: 8 accumulators of 64 columns
 // instruction descriptor: D = F32, A = B = BF16, K-major, N = 64, M = 128
 constexpr uint32_t kOzIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(ON >> 3) << 17) |
@@ -169,7 +180,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * OM, n0 = blockIdx.x * ON;
   const int s0 = blockIdx.z * slabs_per;
-  const int nk = min(nslabs, s0 + slabs_per) - s0;  // >= 1 (host)
+  const int nk = max(0, min(nslabs, s0 + slabs_per) - s0);
   const int nchunks = (nk + kChunkSlabs - 1) / kChunkSlabs;
   if (threadIdx.x == 0) {
     for (int s = 0; s < OS; ++s) {
@@ -306,46 +317,71 @@ __global__ void __launch_bounds__(kOzThreads, 1)
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_empty);
     }
-    if (!ok) {
-      if (lane == 0) atomicOr(status, 128u);
-    } else {
-      const int row = m0 + quad * 32 + lane;
-      if (row < M) {
-        const int er = max(ea[row], -1100) - 14;
+    if (!ok && lane == 0) atomicOr(status, 128u);
+    // the last commit has completed: no copy and no MMA uses the stages any more
+    long long* Ss = reinterpret_cast<long long*>(base);
+    float* Sm = reinterpret_cast<float*>(base + (size_t)OM * kOzRow * 8);
+    const int at = (quad * 32 + lane) * kOzRow + c0;
 #pragma unroll
-        for (int j = 0; j < HC; ++j) {
-          const int col = n0 + c0 + j;
-          if (col < N) {
-            const double acc = fma((double)S[j], 3.725290298461914e-09 /* 2^-28 */,
-                                   (double)small[j]);
-            // 2^e from its exponent bits (one FP64 multiply; GB300's FP64 pipe
-            // makes ldexp's general path expensive), ldexp outside that range
-            const int e = er + max(eb[col], -1100);
-            const double v = (e > -1022 && e < 1024) ? acc * __hiloint2double((e + 1023) << 20, 0)
-                                                     : ldexp(acc, e);
-            if (part) {
-              part[((size_t)blockIdx.z * M + row) * N + col] = v;
-            } else {
-              double* p = C + (size_t)row * ldc + col;
-              *p = beta == 0.0 ? alpha * v : fma(alpha, v, beta * *p);
-            }
-          }
-        }
-      }
+    for (int j = 0; j < HC; ++j) {
+      Ss[at + j] = S[j];
+      Sm[at + j] = small[j];
     }
   }
   tc_fence_before();
-  __syncthreads();
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
   if (warp == 0) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kOzCols)
                  : "memory");
   }
+  // this CTA's share of the tile's rows, lanes along the columns
+  const int nz = (int)cluster.num_blocks(), z = (int)cluster.block_rank();
+  const int mv = min(OM, M - m0), per = (mv + nz - 1) / nz;
+  const int f1 = min(mv, (z + 1) * per) * ON;
+  long long* Ss = reinterpret_cast<long long*>(base);
+  float* Sm = reinterpret_cast<float*>(base + (size_t)OM * kOzRow * 8);
+  double* out = part ? part + (size_t)(blockIdx.z / nz) * M * N : nullptr;
+  for (int f = z * per * ON + threadIdx.x; f < f1; f += kOzThreads) {
+    const int r = f / ON, row = m0 + r, col = n0 + f % ON;
+    if (col >= N) continue;
+    const int at = r * kOzRow + f % ON;
+    long long S = 0;
+    float small = 0.f;
+#pragma unroll
+    for (int y = 0; y < kOzCluster; ++y)
+      if (y < nz) {
+        S += *cluster.map_shared_rank(Ss + at, y);
+        small += *cluster.map_shared_rank(Sm + at, y);
+      }
+    double v = fma((double)S, 3.725290298461914e-09 /* 2^-28 */, (double)small);
+    // times 2^e: on the exponent's bits unless that leaves the normal range
+    const int e = max(ea[row], -1100) - 14 + max(eb[col], -1100);
+    const int hi = __double2hiint(v), x = (hi >> 20) & 0x7ff;
+    if (e > kOzNotFinite / 2)
+      v = __hiloint2double(0x7ff80000, 0);
+    else if (x != 0 && x + e > 0 && x + e < 0x7ff)
+      v = __hiloint2double(hi + (e << 20), __double2loint(v));
+    else
+      v = ldexp(v, e);
+    if (out) {
+      out[(size_t)row * N + col] = v;
+    } else {
+      double* p = C + (size_t)row * ldc + col;
+      if (beta != 0.0) v = fma(alpha, v, beta * *p);
+      else if (alpha != 1.0) v *= alpha;
+      *p = v;
+    }
+  }
+  cluster.sync();  // no CTA leaves while another reads its sums
 }
 
-// One operand of the preparation kernels: op(X) is rows x K with element
+// One operand of the preparation: op(X) is rows x K with element
 // (r, k) = X[r * ldx + k] (trans = 0) or X[k * ldx + r] (trans = 1).
-constexpr int kOzNoExp = (int)0x80808080;  // exponent of an all-zero row
+constexpr int kPrepRows = 8;     // rows of a CTA: a warp each
+constexpr int kPrepCols = 512;   // K entries held in shared memory
+constexpr int kPrepRange = 256;  // K entries of a CTA while the cluster can grow
 
 struct OzOperand {
   const double* X;
@@ -354,95 +390,113 @@ struct OzOperand {
   __nv_bfloat16* out;
 };
 
-// Exponent e (x = f 2^e, f in [0.5, 1)) of the largest |element| of each row
-// of op(X) into ex; the bytes 0x80 (kOzNoExp) for an all-zero (or non-finite)
-// row.  32 x 32 threads per 32 rows over the whole of K; lanes run along the
-// contiguous index; blockIdx.z picks the operand.
-__global__ void __launch_bounds__(1024) k_oz_exp(OzOperand A, OzOperand B, int K) {
+// Exponent e (x = f 2^e, f in [0.5, 1)) of the largest |element| of each row of
+// op(X) into ex (or kOzNoExp, kOzNotFinite), and the 8 slices of
+// op(X) scaled by 2^-ex[r]: out[(i * rows + r) * kp + k] = sign(x) a_i 2^(-7 i)
+// (BF16, exact), zero for k >= K, where a_0 a_1 ... a_7 are the base-128 digits of
+// |x| 2^-ex[r] < 1, i.e. 7-bit fields of the 56-bit fixed-point value
+// F = floor(|x| 2^(56 - ex[r])) taken from the FP64 significand with integer shifts.
+//
+// A CTA has 8 rows and a K range, a cluster (along y) the whole rows; blockIdx.z
+// picks the operand.  The range is read once into shared memory, the maxima go
+// through the cluster, and a warp writes the slices of one row, two entries to a
+// lane.  Only integer and FP32 operations: maxima of doubles alone, at 64 clocks of
+// the FP64 pipe each, took 8 us of the 15 us that separate passes for the exponents
+// and the slices did at 320 x 256.
+__global__ void __launch_bounds__(32 * kPrepRows)
+    k_oz_prep(OzOperand A, OzOperand B, int K, int kp, int range) {
   const OzOperand& o = blockIdx.z ? B : A;
-  __shared__ double red[32][33];
-  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 32
-  const int r0 = blockIdx.x * 32;
-  if (r0 >= o.rows) return;  // uniform over the block
-  const int k0 = 0, k1 = K;
-  double m = 0.0;
-  if (o.trans) {  // tx = row, ty strides over k
-    const int r = r0 + tx;
-    if (r < o.rows)
-      for (int k = k0 + ty; k < k1; k += 32) m = fmax(m, fabs(o.X[(size_t)k * o.ldx + r]));
-    red[ty][tx] = m;
-  } else {  // ty = row, tx strides over k
-    const int r = r0 + ty;
-    if (r < o.rows)
-      for (int k = k0 + tx; k < k1; k += 32) m = fmax(m, fabs(o.X[(size_t)r * o.ldx + k]));
-    red[tx][ty] = m;
-  }
+  __shared__ __align__(16) double X[kPrepRows][kPrepCols + 2];
+  __shared__ unsigned key[kPrepRows];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int r0 = blockIdx.x * kPrepRows;
+  if (r0 >= o.rows) return;  // uniform over the cluster
+  const int k0 = blockIdx.y * range, k1 = min(kp, k0 + range);
+  const int nch = max(1, (k1 - k0 + kPrepCols - 1) / kPrepCols);
+  if (tid < kPrepRows) key[tid] = 0;
   __syncthreads();
-  if (ty == 0) {  // column tx of red: the 32 partial maxima of row r0 + tx
-    double v = 0.0;
-    for (int j = 0; j < 32; ++j) v = fmax(v, red[j][tx]);
-    const int r = r0 + tx;
-    if (r < o.rows) {
-      int e = kOzNoExp;
-      if (v > 0.0 && v <= DBL_MAX) frexp(v, &e);
-      o.ex[r] = e;
-    }
-  }
-}
-
-// The 8 slices of op(X) scaled by 2^-ex[r]: out[(i * rows + r) * kp + k] =
-// sign(x) a_i 2^(-7 i) (BF16, exact), zero for k >= K, where a_0 a_1 ... a_7
-// are the base-128 digits of |x| 2^-ex[r] < 1, i.e. 7-bit fields of the 56-bit
-// fixed-point value F = floor(|x| 2^(56 - ex[r])) taken from the FP64
-// significand with integer shifts.  32 x 32 tiles through shared memory so
-// reads and writes stay coalesced; blockIdx.z picks the operand.
-__global__ void k_oz_slice(OzOperand A, OzOperand B, int K, int kp) {
-  const OzOperand& o = blockIdx.z ? B : A;
-  __shared__ double tile[32][33];
-  const int r0 = blockIdx.y * 32, k0 = blockIdx.x * 32;
-  if (r0 >= o.rows) return;  // uniform over the block
-  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
-  for (int j = ty; j < 32; j += 8) {
-    double v = 0.0;
-    if (o.trans) {
-      const int k = k0 + j, r = r0 + tx;
-      if (k < K && r < o.rows) v = o.X[(size_t)k * o.ldx + r];
+  // columns c0 .. c0 + n - 1 into X, their maximum (high words; 1 for what is
+  // nonzero below them) into key
+  auto load = [&](int c0, int n) {
+    if (o.trans) {  // 8 rows x 4 columns to a warp: 64 contiguous bytes per column
+      const int r = tid & 7;
+      unsigned m = 0;
+      for (int k = tid >> 3; k < n; k += 4 * kPrepRows) {
+        const double x =
+            r0 + r < o.rows && c0 + k < K ? o.X[(size_t)(c0 + k) * o.ldx + r0 + r] : 0.0;
+        X[r][k] = x;
+        m = max(m, (unsigned)(__double2hiint(x) & 0x7fffffff) | (__double2loint(x) != 0));
+      }
+      m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
+      m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
+      if (lane < 8) atomicMax(&key[r], m);
     } else {
-      const int r = r0 + j, k = k0 + tx;
-      if (k < K && r < o.rows) v = o.X[(size_t)r * o.ldx + k];
+      unsigned m = 0;
+      for (int k = lane; k < n; k += 32) {
+        const double x =
+            r0 + warp < o.rows && c0 + k < K ? o.X[(size_t)(r0 + warp) * o.ldx + c0 + k] : 0.0;
+        X[warp][k] = x;
+        m = max(m, (unsigned)(__double2hiint(x) & 0x7fffffff) | (__double2loint(x) != 0));
+      }
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (lane == 0) atomicMax(&key[warp], m);
     }
-    tile[j][tx] = v;
+  };
+  for (int c = 0; c < nch; ++c) {
+    if (c) __syncthreads();
+    load(k0 + c * kPrepCols, min(kPrepCols, k1 - k0 - c * kPrepCols));
   }
-  __syncthreads();
+  cluster.sync();
+  const int r = r0 + warp;
+  unsigned m = 0;
+  for (int y = 0; y < (int)cluster.num_blocks(); ++y)
+    m = max(m, *cluster.map_shared_rank(&key[warp], y));
+  // the bound 2^-1021 of a row of subnormals loses none of their bits
+  const int ex = m == 0 ? kOzNoExp
+                        : m >= 0x7ff00000u ? kOzNotFinite : max((int)(m >> 20), 1) - 1022;
+  if (cluster.block_rank() == 0 && lane == 0 && r < o.rows) o.ex[r] = ex;
   const size_t plane = (size_t)o.rows * kp;
-  for (int j = ty; j < 32; j += 8) {
-    const int r = r0 + j, k = k0 + tx;
-    if (r >= o.rows || k >= kp) continue;
-    const unsigned long long bits =
-        (unsigned long long)__double_as_longlong(o.trans ? tile[tx][j] : tile[j][tx]);
-    const int bexp = (int)((bits >> 52) & 0x7FF);
-    unsigned long long m = bits & ((1ull << 52) - 1);
-    int ev = -1022;  // subnormal
-    if (bexp) {
-      m |= 1ull << 52;
-      ev = bexp - 1023;
+  for (int c = 0; c < nch; ++c) {
+    const int c0 = k0 + c * kPrepCols, n = min(kPrepCols, k1 - c0);
+    if (nch > 1) {
+      __syncthreads();
+      load(c0, n);
+      __syncthreads();
     }
-    unsigned long long F = 0;
-    if (m) {  // |x| = m 2^(ev - 52) < 2^ex[r], so the shift is at most 3
-      const int sh = ev - o.ex[r] + 4;
-      F = sh >= 0 ? m << sh : (sh > -64 ? m >> (-sh) : 0ull);
-    }
-    const bool neg = (bits >> 63) != 0;
-    float scale = 1.f;
+    if (r >= o.rows) continue;
+    for (int k = 2 * lane; k < n; k += 64) {
+      unsigned long long F[2];
+      unsigned sign[2];
 #pragma unroll
-    for (int i = 0; i < kSlices; ++i) {
-      const float a = (float)(unsigned)((F >> (49 - 7 * i)) & 127ull) * scale;
-      o.out[i * plane + (size_t)r * kp + k] = __float2bfloat16_rn(neg ? -a : a);
-      scale *= 0.0078125f;  // 2^-7
+      for (int h = 0; h < 2; ++h) {
+        const unsigned long long bits = (unsigned long long)__double_as_longlong(X[warp][k + h]);
+        const int bexp = (int)((bits >> 52) & 0x7FF);
+        // |x| = f 2^(ev - 52) < 2^ex, so the shift is at most 3
+        const unsigned long long f = (bits & ((1ull << 52) - 1)) | (bexp ? 1ull << 52 : 0ull);
+        const int sh = (bexp ? bexp - 1023 : -1022) - ex + 4;
+        F[h] = f == 0 ? 0ull : sh >= 0 ? f << (sh & 63) : (sh > -64 ? f >> (-sh) : 0ull);
+        sign[h] = (unsigned)(bits >> 32) & 0x80000000u;
+      }
+      float scale = 1.f;
+#pragma unroll
+      for (int i = 0; i < kSlices; ++i) {
+        unsigned w[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {  // the digit as a float: 2^23 + a - 2^23
+          const unsigned a = (unsigned)(F[h] >> (49 - 7 * i)) & 127u;
+          w[h] = __float_as_uint((__uint_as_float(0x4B000000u | a) - 8388608.0f) * scale) | sign[h];
+        }
+        *reinterpret_cast<unsigned*>(o.out + i * plane + (size_t)r * kp + c0 + k) =
+            __byte_perm(w[0], w[1], 0x7632);
+        scale *= 0.0078125f;  // 2^-7
+      }
     }
   }
+  cluster.sync();  // no CTA leaves while another reads its maxima
 }
 
+// C = alpha sum_z part_z + beta C: the clusters of one tile
 __global__ void k_oz_reduce(int M, int N, int nz, const double* __restrict__ part, double alpha,
                             double beta, double* __restrict__ C, int ldc) {
   const size_t mn = (size_t)M * N;
@@ -494,6 +548,29 @@ int make_slice_map(CUtensorMap* map, const __nv_bfloat16* base, int rows, int kp
 
 }  // namespace
 
+namespace {
+
+template <typename... P, typename... Q>
+int cluster_launch(void (*fn)(P...), dim3 grid, dim3 block, dim3 cluster, size_t smem,
+                   cudaStream_t st, Q... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = cluster.x;
+  attr.val.clusterDim.y = cluster.y;
+  attr.val.clusterDim.z = cluster.z;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  SM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fn, args...));
+  return SM_OK;
+}
+
+}  // namespace
+
 bool gemm_oz_eligible(int M, int N, int K) {
   return (double)M * N * K >= 2.0 * 1024 * 1024 && M >= 32 && N >= 32 && K >= 32 &&
          oz_encode_fn() != nullptr;
@@ -515,32 +592,37 @@ int gemm_oz(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, do
   // (N) or B[n][k] (T, C)
   const int ta = opA == SM_OP_N ? 0 : 1, tb = opB == SM_OP_N ? 1 : 0;
   const OzOperand oa{A, lda, M, ta, ea, sa}, ob{B, ldb, N, tb, eb, sb};
-  const int rb = (std::max(M, N) + 31) / 32;
-  k_oz_exp<<<dim3(rb, 1, 2), dim3(32, 32), 0, st>>>(oa, ob, K);
-  k_oz_slice<<<dim3(kp / 32, rb, 2), dim3(32, 8), 0, st>>>(oa, ob, K, kp);
-  note_launch(2);
-  SM_CUDA_CHECK(cudaGetLastError());
+  const int rb = (std::max(M, N) + kPrepRows - 1) / kPrepRows;
+  const int zk = std::min(kOzCluster, (kp + kPrepRange - 1) / kPrepRange);
+  const int range = (nslabs + zk - 1) / zk * OK;
+  SM_CHECK(cluster_launch(k_oz_prep, dim3(rb, zk, 2), dim3(32 * kPrepRows), dim3(1, zk, 1), 0, st,
+                          oa, ob, K, kp, range));
+  note_launch();
   CUtensorMap mA, mB;
   SM_CHECK(make_slice_map(&mA, sa, M, kp, OM));
   SM_CHECK(make_slice_map(&mB, sb, N, kp, ON));
   const int tiles = ((M + OM - 1) / OM) * ((N + ON - 1) / ON);
-  // split K over CTAs while the output has fewer tiles than SMs, in whole
-  // 32-wide slabs, at least two per CTA (each CTA's range is accumulated in
-  // exact chunks of at most 256, so any slab split is exact)
-  int nz = std::max(1, std::min(std::max(1, ctx.num_sms) / tiles, nslabs / 2));
-  const int slabs_per = (nslabs + nz - 1) / nz;
+  // Split K over the CTAs of a cluster while the output has fewer tiles than SMs,
+  // down to one slab each (any split at slabs is exact).  Only beyond 16 slabs a CTA
+  // a tile gets several clusters: their sum is another launch of ~4 us.
+  const int sms = std::max(1, ctx.num_sms);
+  int nz = std::max(1, std::min({kOzCluster, sms / tiles, nslabs}));
+  int slabs_per = (nslabs + nz - 1) / nz;
   nz = (nslabs + slabs_per - 1) / slabs_per;
+  const int nzo =
+      nz < kOzCluster ? 1 : std::max(1, std::min(sms / (tiles * nz), slabs_per / 8));
+  if (nzo > 1) slabs_per = (nslabs + nz * nzo - 1) / (nz * nzo);
   double* part = nullptr;
-  if (nz > 1) SM_CHECK(ctx.scratch("oz.part", (size_t)nz * M * N, &part));
+  if (nzo > 1) SM_CHECK(ctx.scratch("oz.part", (size_t)nzo * M * N, &part));
   SM_CHECK(raise_smem_limit(k_gemm_oz, kOzSmem));
-  const dim3 grid((N + ON - 1) / ON, (M + OM - 1) / OM, nz);
-  k_gemm_oz<<<grid, kOzThreads, kOzSmem, st>>>(mA, mB, ea, eb, M, N, nslabs, slabs_per, alpha,
-                                               beta, C, ldc, part, status);
+  const dim3 grid((N + ON - 1) / ON, (M + OM - 1) / OM, nz * nzo);
+  SM_CHECK(cluster_launch(k_gemm_oz, grid, dim3(kOzThreads), dim3(1, 1, nz), kOzSmem, st, mA, mB,
+                          (const int*)ea, (const int*)eb, M, N, nslabs, slabs_per, alpha, beta, C,
+                          ldc, part, status));
   note_launch();
-  SM_CUDA_CHECK(cudaGetLastError());
-  if (nz > 1) {
+  if (nzo > 1) {
     const size_t mn = (size_t)M * N;
-    k_oz_reduce<<<(int)std::min<size_t>((mn + 255) / 256, 4096), 256, 0, st>>>(M, N, nz, part,
+    k_oz_reduce<<<(int)std::min<size_t>((mn + 255) / 256, 4096), 256, 0, st>>>(M, N, nzo, part,
                                                                                alpha, beta, C, ldc);
     note_launch();
     SM_CUDA_CHECK(cudaGetLastError());
