@@ -25,19 +25,22 @@
 // products (i + j >= 8) are below 2^-56 of the row / column maxima, so the
 // result has the accuracy of an FP64 GEMM.
 //
-// One CTA (10 warps) per 128 x 64 output tile and K range:
+// One CTA (10 warps) per 128 x 64 (128 x 32) output tile and K range:
 //   warp 8 / lane 0: TMA, one 3-D box per operand and stage holding all 8
 //            slices of a 32-wide K slab (64-byte swizzle), 2 stages;
-//   warp 9 / lane 0: 2 x 36 tcgen05.mma (M=128, N=64, K=16) per slab into
-//            8 x 64 TMEM columns, a commit per stage and per chunk;
+//   warp 9 / lane 0: 2 x 12 (2 x 8) tcgen05.mma of N = 256 and less, K = 16,
+//            per slab into 8 accumulators in TMEM, a commit per stage and per
+//            chunk.  (A slice product to an MMA reads A again for each: 4560
+//            clocks a slab, shared memory bound, against 2600 and 1800);
 //   warps 0-7: per chunk, tcgen05.ld of the 8 accumulators (warp w owns tile
-//            rows 32 (w % 4) .. +31, columns 32 (w / 4) .. +31) into 32 int64
-//            + 32 FP32 registers per thread.
+//            rows 32 (w % 4) .. +31, half w / 4 of the columns) into an int64
+//            and an FP32 register per element.
 // The K ranges of a tile are the CTAs of one cluster.  They leave their int64 and
 // FP32 sums in shared memory (where the stages were) and each adds up a share of
 // the tile's rows over the cluster and turns it into FP64.  Besides filling the
-// SMs, the split divides that conversion: three FP64-pipe operations for each
-// element are 6 us on a whole tile, against 1.2 us for a slab's MMAs.
+// SMs, the split divides that conversion, which on a whole 128 x 64 tile takes as
+// long as ten slabs' MMAs.  320 x 128 x 256: 14 us after 5 us of preparation; one
+// CTA a tile, 64-bit conversions and FP64 partial sums were 30 us after 15 us.
 // Every mbarrier wait is bounded; a timeout sets a bit of the status word
 // shared with the TF32 path (read by tc_status_check), waits for the CTA's
 // copies in flight, frees TMEM and returns.
@@ -57,24 +60,31 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int OM = 128, ON = 64, OK = 32, OS = 2;  // tile M, N, K slab (BF16), stages
+constexpr int OM = 128, OK = 32, OS = 2;  // tile M, K slab (BF16), stages
 constexpr int kSlices = 8;
 constexpr int kChunkSlabs = 8;  // 256 of K per exact chunk
 constexpr int kGroups = 8;      // one accumulator per t = i + j
 constexpr int kOzThreads = 320;  // 8 flush warps, TMA, MMA
 constexpr uint32_t kSliceA = OM * OK * 2;  // 8 KB: one slice of A, one slab
-constexpr uint32_t kSliceB = ON * OK * 2;  // 4 KB
-constexpr uint32_t kOzStage = kSlices * (kSliceA + kSliceB);  // 96 KB
-constexpr size_t kOzSmem = (size_t)OS * kOzStage + 1024 + 256;
-constexpr int kOzRow = ON + 1;   // row stride of the sums in shared memory: no bank conflicts
-static_assert((size_t)OM * kOzRow * 12 <= (size_t)OS * kOzStage, "the sums fit where the stages were");
+// Sizes that follow from the tile's N (64, or 32 where that fills more SMs)
+template <int ON>
+struct OzTile {
+  static constexpr uint32_t kSliceB = ON * OK * 2;
+  static constexpr uint32_t kStage = kSlices * (kSliceA + kSliceB);  // 96 KB, 80 KB
+  static constexpr size_t kSmem = (size_t)OS * kStage + 1024 + 256;
+  static constexpr int kRow = ON + 1;  // row stride of the sums in shared memory: no bank conflicts
+  static constexpr uint32_t kCols = kSlices * ON;  // TMEM columns: 8 accumulators
+  static constexpr int kGang = 256 / ON;  // slices of B to an MMA
+  static_assert((size_t)OM * kRow * 12 <= (size_t)OS * kStage, "the sums fit where the stages were");
+};
 constexpr int kOzNoExp = -(1 << 28);  // exponent of an all-zero row of an operand
 constexpr int kOzNotFinite = 1 << 28;  // and of one with an infinity or a NaN
 constexpr int kOzCluster = 8;    // K ranges of a tile that share a cluster (portable size)
-constexpr uint32_t kOzCols = 512;  // TMEM allocation: 8 accumulators of 64 columns
-// instruction descriptor: D = F32, A = B = BF16, K-major, N = 64, M = 128
-constexpr uint32_t kOzIdesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(ON >> 3) << 17) |
-                              ((uint32_t)(OM >> 4) << 24);
+// instruction descriptor: D = F32, A = B = BF16, K-major, M = 128
+__device__ __forceinline__ constexpr uint32_t oz_idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) |
+         ((uint32_t)(OM >> 4) << 24);
+}
 constexpr unsigned long long kOzWaitNs = 1000000000ull;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -137,12 +147,13 @@ __device__ __forceinline__ uint64_t sdesc_sw64(uint32_t saddr) {
   d |= (uint64_t)4 << 61;            // 64-byte swizzle
   return d;
 }
-__device__ __forceinline__ void umma_bf16(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t acc) {
+__device__ __forceinline__ void umma_bf16(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc,
+                                          uint32_t acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(dtmem),
-      "l"(a), "l"(b), "r"(kOzIdesc), "r"(acc)
+      "l"(a), "l"(b), "r"(idesc), "r"(acc)
       : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
@@ -164,21 +175,95 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ uint32_t mapa(uint32_t saddr, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ long long ld_cluster_s64(uint32_t a) {
+  long long v;
+  asm volatile("ld.shared::cluster.s64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t a) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// S 2^(e-28) + small 2^e in three FP64 operations: the words of S are the low bits of
+// 2^56 (the upper one biased by 2^31, i.e. 2^35 here) and of 2^24, small's bits are
+// moved, and 2^e goes onto the exponent's bits unless that leaves the normal range.
+// (Every FP64 operation holds the pipe for 64 clocks, a predicated-off one too: what
+// is rare is out of line.)
+__device__ __noinline__ double oz_outside(double v, int e) {
+  return e > kOzNotFinite / 2 ? __hiloint2double(0x7ff80000, 0) : ldexp(v, e);
+}
+__device__ __noinline__ double oz_axpby(double alpha, double v, double beta, const double* c) {
+  return beta == 0.0 ? alpha * v : fma(alpha, v, beta * *c);
+}
+__device__ __forceinline__ double oz_double(long long S, float small, int e) {
+  const int f = __float_as_int(small), x = (f >> 23) & 0xff;
+  const double s64 = __hiloint2double(x == 0 ? 0 : (f & 0x80000000) | (x + 896) << 20 | (f & 0x7fffff) >> 3,
+                                      x == 0 ? 0 : (int)((unsigned)f << 29));
+  const double shi = __hiloint2double(0x43700000, (int)((unsigned long long)S >> 32) ^ 0x80000000);
+  const double slo = __hiloint2double(0x41700000, (int)S);
+  const double v = ((shi - (72057594037927936.0 + 34359738368.0 + 16777216.0)) + slo) + s64;
+  const int hi = __double2hiint(v), xv = (hi >> 20) & 0x7ff;
+  if (xv == 0 || xv + e <= 0 || xv + e >= 0x7ff) return oz_outside(v, e);
+  return __hiloint2double(hi + (e << 20), __double2loint(v));
+}
+
+// Rows r0 .. r1 - 1 of the tile: the sums of the cluster's NZ CTAs in FP64, stored by
+// lanes along the columns.  add: C = alpha v + beta C (else C = v)
+template <int ON, int NZ>
+__device__ __forceinline__ void oz_store(uint32_t base, const int* et, int r0, int r1, int ncol,
+                                         bool add, double alpha, double beta, double* C, size_t ldc) {
+  uint32_t src[NZ];
+#pragma unroll
+  for (int y = 0; y < NZ; ++y) src[y] = mapa(base, y);
+  const int c = threadIdx.x % ON;
+  if (c >= ncol) return;
+#pragma unroll 2
+  for (int r = r0 + threadIdx.x / ON; r < r1; r += kOzThreads / ON) {
+    const uint32_t at = (uint32_t)(r * OzTile<ON>::kRow + c);
+    long long S = 0;
+    float small = 0.f;
+#pragma unroll
+    for (int y = 0; y < NZ; ++y) {
+      S += ld_cluster_s64(src[y] + at * 8);
+      small += ld_cluster_f32(src[y] + (uint32_t)(OM * OzTile<ON>::kRow * 8) + at * 4);
+    }
+    double v = oz_double(S, small, et[r] + et[OM + c]);
+    double* p = C + (size_t)r * ldc + c;
+    if (add) v = oz_axpby(alpha, v, beta, p);
+    *p = v;
+  }
+}
+
+template <int ON>
 __global__ void __launch_bounds__(kOzThreads, 1)
     k_gemm_oz(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB,
               const int* __restrict__ ea, const int* __restrict__ eb, int M, int N, int nslabs,
               int slabs_per, double alpha, double beta, double* __restrict__ C, int ldc,
               double* __restrict__ part, unsigned int* __restrict__ status) {
+  using Tile = OzTile<ON>;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base =
       reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* full = reinterpret_cast<uint64_t*>(base + (size_t)OS * kOzStage);
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + (size_t)OS * Tile::kStage);
   uint64_t* empty = full + OS;
   uint64_t* acc_full = empty + OS;
   uint64_t* acc_empty = acc_full + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
+  __shared__ int et[OM + ON];  // exponents of the tile's rows and columns
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * OM, n0 = blockIdx.x * ON;
+  if (threadIdx.x < OM) {
+    if (m0 + threadIdx.x < M) et[threadIdx.x] = max(ea[m0 + threadIdx.x], -1100) - 14;
+  } else if (threadIdx.x < OM + ON) {
+    if (n0 + threadIdx.x - OM < N) et[threadIdx.x] = max(eb[n0 + threadIdx.x - OM], -1100);
+  }
   const int s0 = blockIdx.z * slabs_per;
   const int nk = max(0, min(nslabs, s0 + slabs_per) - s0);
   const int nchunks = (nk + kChunkSlabs - 1) / kChunkSlabs;
@@ -195,7 +280,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
-                 "r"(kOzCols)
+                 "r"(Tile::kCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -214,8 +299,8 @@ __global__ void __launch_bounds__(kOzThreads, 1)
           atomicOr(status, 16u);
           break;
         }
-        unsigned char* stg = base + (size_t)s * kOzStage;
-        mbar_expect_tx(&full[s], kOzStage);
+        unsigned char* stg = base + (size_t)s * Tile::kStage;
+        mbar_expect_tx(&full[s], Tile::kStage);
         const int x = (s0 + i) * OK;
         tma_load_3d(stg, &mA, &full[s], x, m0, 0);
         tma_load_3d(stg + kSlices * kSliceA, &mB, &full[s], x, n0, 0);
@@ -244,25 +329,22 @@ __global__ void __launch_bounds__(kOzThreads, 1)
           break;
         }
         tc_fence_after();
-        const uint32_t a0 = smem_u32(base + (size_t)s * kOzStage);
+        const uint32_t a0 = smem_u32(base + (size_t)s * Tile::kStage);
         const uint32_t b0 = a0 + kSlices * kSliceA;
-        bool written[kGroups] = {};
-        if (!first) {
-#pragma unroll
-          for (int g = 0; g < kGroups; ++g) written[g] = true;
-        }
+        // slice ia of A against slices 0 .. 7 - ia of B, which follow one another in
+        // shared memory as their accumulators t = ia .. 7 do in TMEM: up to N = 256
+        // to an MMA
 #pragma unroll
         for (int kk = 0; kk < OK / 16; ++kk) {
 #pragma unroll
-          for (int t = 0; t < kSlices; ++t) {
-            const int g = t;
+          for (int ia = 0; ia < kSlices; ++ia) {
+            const uint64_t da = sdesc_sw64(a0 + ia * kSliceA + kk * 32);
 #pragma unroll
-            for (int ia = 0; ia <= t; ++ia) {
-              const int jb = t - ia;
-              const uint64_t da = sdesc_sw64(a0 + ia * kSliceA + kk * 32);
-              const uint64_t db = sdesc_sw64(b0 + jb * kSliceB + kk * 32);
-              umma_bf16(tmem + (uint32_t)(g * ON), da, db, written[g] ? 1u : 0u);
-              written[g] = true;
+            for (int jb = 0; jb < kSlices - ia; jb += Tile::kGang) {
+              const int n = kSlices - ia - jb < Tile::kGang ? kSlices - ia - jb : Tile::kGang;
+              umma_bf16(tmem + (uint32_t)((ia + jb) * ON), da,
+                        sdesc_sw64(b0 + jb * Tile::kSliceB + kk * 32), oz_idesc(n * ON),
+                        first && kk == 0 && ia == 0 ? 0u : 1u);
             }
           }
         }
@@ -320,8 +402,8 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     if (!ok && lane == 0) atomicOr(status, 128u);
     // the last commit has completed: no copy and no MMA uses the stages any more
     long long* Ss = reinterpret_cast<long long*>(base);
-    float* Sm = reinterpret_cast<float*>(base + (size_t)OM * kOzRow * 8);
-    const int at = (quad * 32 + lane) * kOzRow + c0;
+    float* Sm = reinterpret_cast<float*>(base + (size_t)OM * Tile::kRow * 8);
+    const int at = (quad * 32 + lane) * Tile::kRow + c0;
 #pragma unroll
     for (int j = 0; j < HC; ++j) {
       Ss[at + j] = S[j];
@@ -333,46 +415,22 @@ __global__ void __launch_bounds__(kOzThreads, 1)
   cluster.sync();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kOzCols)
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Tile::kCols)
                  : "memory");
   }
   // this CTA's share of the tile's rows, lanes along the columns
   const int nz = (int)cluster.num_blocks(), z = (int)cluster.block_rank();
   const int mv = min(OM, M - m0), per = (mv + nz - 1) / nz;
-  const int f1 = min(mv, (z + 1) * per) * ON;
-  long long* Ss = reinterpret_cast<long long*>(base);
-  float* Sm = reinterpret_cast<float*>(base + (size_t)OM * kOzRow * 8);
-  double* out = part ? part + (size_t)(blockIdx.z / nz) * M * N : nullptr;
-  for (int f = z * per * ON + threadIdx.x; f < f1; f += kOzThreads) {
-    const int r = f / ON, row = m0 + r, col = n0 + f % ON;
-    if (col >= N) continue;
-    const int at = r * kOzRow + f % ON;
-    long long S = 0;
-    float small = 0.f;
-#pragma unroll
-    for (int y = 0; y < kOzCluster; ++y)
-      if (y < nz) {
-        S += *cluster.map_shared_rank(Ss + at, y);
-        small += *cluster.map_shared_rank(Sm + at, y);
-      }
-    double v = fma((double)S, 3.725290298461914e-09 /* 2^-28 */, (double)small);
-    // times 2^e: on the exponent's bits unless that leaves the normal range
-    const int e = max(ea[row], -1100) - 14 + max(eb[col], -1100);
-    const int hi = __double2hiint(v), x = (hi >> 20) & 0x7ff;
-    if (e > kOzNotFinite / 2)
-      v = __hiloint2double(0x7ff80000, 0);
-    else if (x != 0 && x + e > 0 && x + e < 0x7ff)
-      v = __hiloint2double(hi + (e << 20), __double2loint(v));
-    else
-      v = ldexp(v, e);
-    if (out) {
-      out[(size_t)row * N + col] = v;
-    } else {
-      double* p = C + (size_t)row * ldc + col;
-      if (beta != 0.0) v = fma(alpha, v, beta * *p);
-      else if (alpha != 1.0) v *= alpha;
-      *p = v;
-    }
+  const int r0 = z * per, r1 = min(mv, r0 + per), nc = min(ON, N - n0);
+  const uint32_t sums = smem_u32(base);
+  const bool add = !part && (alpha != 1.0 || beta != 0.0);
+  const size_t ldo = part ? N : ldc;
+  double* out = (part ? part + (size_t)(blockIdx.z / nz) * M * N : C) + (size_t)m0 * ldo + n0;
+  switch (nz) {  // a power of two (host)
+    case 1: oz_store<ON, 1>(sums, et, r0, r1, nc, add, alpha, beta, out, ldo); break;
+    case 2: oz_store<ON, 2>(sums, et, r0, r1, nc, add, alpha, beta, out, ldo); break;
+    case 4: oz_store<ON, 4>(sums, et, r0, r1, nc, add, alpha, beta, out, ldo); break;
+    default: oz_store<ON, kOzCluster>(sums, et, r0, r1, nc, add, alpha, beta, out, ldo); break;
   }
   cluster.sync();  // no CTA leaves while another reads its sums
 }
@@ -419,28 +477,33 @@ __global__ void __launch_bounds__(32 * kPrepRows)
   // columns c0 .. c0 + n - 1 into X, their maximum (high words; 1 for what is
   // nonzero below them) into key
   auto load = [&](int c0, int n) {
-    if (o.trans) {  // 8 rows x 4 columns to a warp: 64 contiguous bytes per column
-      const int r = tid & 7;
-      unsigned m = 0;
-      for (int k = tid >> 3; k < n; k += 4 * kPrepRows) {
-        const double x =
-            r0 + r < o.rows && c0 + k < K ? o.X[(size_t)(c0 + k) * o.ldx + r0 + r] : 0.0;
-        X[r][k] = x;
-        m = max(m, (unsigned)(__double2hiint(x) & 0x7fffffff) | (__double2loint(x) != 0));
+    // trans: 8 rows x 4 columns to a warp, 64 contiguous bytes of each column
+    const int rr = o.trans ? tid & 7 : warp, kt = o.trans ? tid >> 3 : lane;
+    const bool on = r0 + rr < o.rows;
+    const size_t step = o.trans ? o.ldx : 1;
+    const double* src = o.X + (o.trans ? (size_t)(r0 + rr) : (size_t)(r0 + rr) * o.ldx) + c0 * step;
+    unsigned m = 0;
+    for (int ka = kt; ka < n; ka += 8 * 32) {  // eight loads in flight
+      double x[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int k = ka + 32 * i;
+        x[i] = on && k < n && c0 + k < K ? src[k * step] : 0.0;
       }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int k = ka + 32 * i;
+        if (k < n) X[rr][k] = x[i];
+        m = max(m, (unsigned)(__double2hiint(x[i]) & 0x7fffffff) | (__double2loint(x[i]) != 0));
+      }
+    }
+    if (o.trans) {
       m = max(m, __shfl_xor_sync(0xffffffffu, m, 8));
       m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
-      if (lane < 8) atomicMax(&key[r], m);
+      if (lane < 8) atomicMax(&key[rr], m);
     } else {
-      unsigned m = 0;
-      for (int k = lane; k < n; k += 32) {
-        const double x =
-            r0 + warp < o.rows && c0 + k < K ? o.X[(size_t)(r0 + warp) * o.ldx + c0 + k] : 0.0;
-        X[warp][k] = x;
-        m = max(m, (unsigned)(__double2hiint(x) & 0x7fffffff) | (__double2loint(x) != 0));
-      }
       m = __reduce_max_sync(0xffffffffu, m);
-      if (lane == 0) atomicMax(&key[warp], m);
+      if (lane == 0) atomicMax(&key[rr], m);
     }
   };
   for (int c = 0; c < nch; ++c) {
@@ -600,25 +663,30 @@ int gemm_oz(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, do
   note_launch();
   CUtensorMap mA, mB;
   SM_CHECK(make_slice_map(&mA, sa, M, kp, OM));
-  SM_CHECK(make_slice_map(&mB, sb, N, kp, ON));
-  const int tiles = ((M + OM - 1) / OM) * ((N + ON - 1) / ON);
   // Split K over the CTAs of a cluster while the output has fewer tiles than SMs,
   // down to one slab each (any split at slabs is exact).  Only beyond 16 slabs a CTA
   // a tile gets several clusters: their sum is another launch of ~4 us.
-  const int sms = std::max(1, ctx.num_sms);
-  int nz = std::max(1, std::min({kOzCluster, sms / tiles, nslabs}));
+  const int sms = std::max(1, ctx.num_sms), tm = (M + OM - 1) / OM;
+  const int tiles = tm * ((N + 63) / 64);
+  int nz = 1;
+  while (nz < kOzCluster && 2 * nz <= std::min(sms / tiles, nslabs)) nz *= 2;
   int slabs_per = (nslabs + nz - 1) / nz;
-  nz = (nslabs + slabs_per - 1) / slabs_per;
   const int nzo =
       nz < kOzCluster ? 1 : std::max(1, std::min(sms / (tiles * nz), slabs_per / 8));
   if (nzo > 1) slabs_per = (nslabs + nz * nzo - 1) / (nz * nzo);
   double* part = nullptr;
   if (nzo > 1) SM_CHECK(ctx.scratch("oz.part", (size_t)nzo * M * N, &part));
-  SM_CHECK(raise_smem_limit(k_gemm_oz, kOzSmem));
-  const dim3 grid((N + ON - 1) / ON, (M + OM - 1) / OM, nz * nzo);
-  SM_CHECK(cluster_launch(k_gemm_oz, grid, dim3(kOzThreads), dim3(1, 1, nz), kOzSmem, st, mA, mB,
-                          (const int*)ea, (const int*)eb, M, N, nslabs, slabs_per, alpha, beta, C,
-                          ldc, part, status));
+  // Half as wide a tile where twice as many CTAs still find an SM each: half of
+  // everything but the loads of A to a CTA.
+  const bool narrow = 2 * tiles * nz * nzo <= sms && N > 32;
+  const int on = narrow ? 32 : 64;
+  SM_CHECK(make_slice_map(&mB, sb, N, kp, on));
+  const auto kernel = narrow ? k_gemm_oz<32> : k_gemm_oz<64>;
+  const size_t smem = narrow ? OzTile<32>::kSmem : OzTile<64>::kSmem;
+  SM_CHECK(raise_smem_limit(kernel, smem));
+  SM_CHECK(cluster_launch(kernel, dim3((N + on - 1) / on, tm, nz * nzo), dim3(kOzThreads),
+                          dim3(1, 1, nz), smem, st, mA, mB, (const int*)ea, (const int*)eb, M, N,
+                          nslabs, slabs_per, alpha, beta, C, ldc, part, status));
   note_launch();
   if (nzo > 1) {
     const size_t mn = (size_t)M * N;

@@ -80,3 +80,30 @@ def test_small_fp64_splits_of_odd_matrices(cplx):
     A[2, 3] = np.nan
     with pytest.raises(Exception):
         core._left_orth_2site(A.reshape(6, 1, 1, 20), sg.Strategy(tolerance=1e-12))
+
+
+@pytest.mark.parametrize("M, N, K", [
+    # tiles of 128 x 32 and 128 x 64 and their remainders, one slab of K and ragged ones,
+    # clusters of 1, 2, 4 and 8 ranges, ranges left empty, several clusters to a tile
+    (32, 32, 2048), (33, 65, 1000), (127, 33, 512), (129, 64, 300), (256, 257, 32), (257, 2080, 33),
+    (1100, 1100, 64), (640, 640, 96), (300, 500, 288), (128, 32, 4097), (40, 48, 9001),
+])
+def test_sliced_gemm_tiles(M, N, K):
+    """Against numpy's FP64 product, normalised by |A||B|: 8 sqrt(K) u; a row with a NaN or an
+    infinity gives NaN, and only there."""
+    from tests.test_gpu_tc import _gemm_f64tc
+
+    rng = np.random.default_rng(M + N + K)
+    A = rng.normal(size=(M, K)) * np.exp(rng.uniform(-18, 18, size=(M, 1)))
+    B = rng.normal(size=(K, N)) * np.exp(rng.uniform(-18, 18, size=(1, N)))
+    B[:, N // 2] = 0.0
+    ref, scale = A @ B, np.abs(A) @ np.abs(B)
+    scale[:, N // 2] = 1.0
+    for opA, opB in [("N", "N"), ("T", "T")]:
+        a, b = (A, B) if opA == "N" else (A.T.copy(), B.T.copy())
+        assert np.max(np.abs(_gemm_f64tc(opA, opB, a, b, M, N, K) - ref) / scale) <= 8 * np.sqrt(K) * 2.0**-53
+    A[1, 0], A[M - 1, K - 1] = np.nan, np.inf
+    out = _gemm_f64tc("N", "N", A, B, M, N, K)
+    assert np.isnan(out[[1, M - 1]]).all()
+    rest = np.delete(np.arange(M), [1, M - 1])
+    assert np.max((np.abs(out - ref) / scale)[rest]) <= 8 * np.sqrt(K) * 2.0**-53
