@@ -45,35 +45,80 @@ __global__ void k_double_layer(const T* __restrict__ O, int Dl, int q, int p, in
   }
 }
 
+// +0 or -0, by its bits: an FP64 comparison would cost as much as the multiply-add
+__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+__device__ __forceinline__ bool is_zero(cplx x) { return is_zero(x.re) && is_zero(x.im); }
+
 // Out[l][t][al2][be2][o] = sum_{al,be,s} K4[al][be][j][k][al2][be2] In[s][o][al][be][l]
-// with (j, k) = (s, t), or (t, s) when `swap` is set.  One thread per (l, o)
-// pair and output physical index t; lanes run along l, so the loads of In are
-// contiguous; the K4 entries are warp-uniform (zero blocks of the MPO, common
-// in banded operators, are skipped).
+// with (j, k) = (s, t), or (t, s) when `swap` is set.
+//
+// Few entries of K4 are not zero in banded operators, and GB300's FP64 pipe (64 clocks
+// a warp instruction) bounds the rest: a block lists the nonzero entries of its output
+// (t, al2, be2) = z in shared memory and makes only their multiply-adds, for
+// 32 x 32 pairs (l, o), four to a thread.  Lanes run along l for the loads; the tile is
+// transposed in shared memory so that they run along o for the stores.  (One thread for
+// all outputs of a pair, testing every entry in FP64 and storing 8 bytes to a sector:
+// 66 us at bonds of 16, 98 us at 128 x 192.)
+constexpr int kDlIn = 256;  // inputs (s, al, be) listed at a time
+
 template <typename T>
-__global__ void k_double_layer_apply(const T* __restrict__ K4, int Dl, int p, int Dr, int swap,
-                                     const T* __restrict__ In, int no, int nl,
-                                     T* __restrict__ Out) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  const int o = blockIdx.y * blockDim.y + threadIdx.y;
-  if (l >= nl || o >= no) return;
-  const size_t sIn = (size_t)no * Dl * Dl * nl;  // stride of s in In
-  const T* in = In + (size_t)o * Dl * Dl * nl + l;
-  for (int t = 0; t < p; ++t)
-    for (int a2 = 0; a2 < Dr; ++a2)
-      for (int b2 = 0; b2 < Dr; ++b2) {
-        T acc = S<T>::zero();
-        for (int s = 0; s < p; ++s) {
-          const int j = swap ? t : s, k = swap ? s : t;
-          for (int a = 0; a < Dl; ++a)
-            for (int b = 0; b < Dl; ++b) {
-              const T w = K4[(((((size_t)a * Dl + b) * p + j) * p + k) * Dr + a2) * Dr + b2];
-              if (S<T>::abs2(w) == 0.0) continue;
-              acc = S<T>::fma(w, in[(size_t)s * sIn + ((size_t)a * Dl + b) * nl], acc);
-            }
+__global__ void __launch_bounds__(256)
+    k_double_layer_apply(const T* __restrict__ K4, int Dl, int p, int Dr, int swap,
+                         const T* __restrict__ In, int no, int nl, T* __restrict__ Out) {
+  __shared__ T val[kDlIn];
+  __shared__ int at[kDlIn];
+  __shared__ int cnt;
+  __shared__ T tile[32][33];
+  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
+  const int l0 = blockIdx.x * 32, o0 = blockIdx.y * 32;
+  const int r2 = Dr * Dr, dd = Dl * Dl, nin = p * dd;
+  for (int z = blockIdx.z; z < p * r2; z += gridDim.z) {
+    const int ab2 = z % r2, t = z / r2;
+    const T* in[4];
+    T acc[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {  // beyond the edge: the last column, not stored
+      acc[j] = S<T>::zero();
+      in[j] = In + (size_t)min(o0 + ty + 8 * j, no - 1) * dd * nl + min(l0 + tx, nl - 1);
+    }
+    for (int i0 = 0; i0 < nin; i0 += kDlIn) {
+      const int ni = min(kDlIn, nin - i0);
+      __syncthreads();
+      if (ty == 0) {
+        int n = 0;
+        for (int i = 0; i < ni; i += 32) {
+          const int e = i0 + i + tx, s = e / dd, ab = e % dd;
+          T w = S<T>::zero();
+          if (i + tx < ni)
+            w = K4[(((size_t)ab * p + (swap ? t : s)) * p + (swap ? s : t)) * r2 + ab2];
+          const bool put = !is_zero(w);
+          const unsigned m = __ballot_sync(0xffffffffu, put);
+          if (put) {
+            const int k = n + __popc(m & ((1u << tx) - 1u));
+            val[k] = w;
+            at[k] = e;
+          }
+          n += __popc(m);
         }
-        Out[((((size_t)l * p + t) * Dr + a2) * Dr + b2) * no + o] = acc;
+        if (tx == 0) cnt = n;
       }
+      __syncthreads();
+      for (int k = 0; k < cnt; ++k) {
+        const int e = at[k];
+        const size_t off = ((size_t)(e / dd) * no * dd + e % dd) * nl;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[j] = S<T>::fma(val[k], in[j][off], acc[j]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) tile[ty + 8 * j][tx] = acc[j];
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int l = l0 + ty + 8 * j, o = o0 + tx;
+      if (l < nl && o < no) Out[(((size_t)l * p + t) * r2 + ab2) * no + o] = tile[tx][ty + 8 * j];
+    }
+  }
 }
 
 }  // namespace
@@ -125,7 +170,7 @@ int mpo_scprod_impl(Ctx& ctx, cudaStream_t st, int L, const int* dout, const int
       SM_CHECK(gemm_ctx<T>(ctx, st, SM_OP_T, SM_OP_N, p * lead2, N1, lead, one, B[i], p * lead2, E,
                            N1, zero, U, N1));
     // double layer: W[(l,t),(a',b',o')] with l = the other state's left bond
-    dim3 blk(32, 8), grd((other + 31) / 32, (lead2 + 7) / 8);
+    dim3 blk(32, 8), grd((other + 31) / 32, (lead2 + 31) / 32, std::min(p * Dr * Dr, 65535));
     k_double_layer_apply<T><<<grd, blk, 0, st>>>(K4, Dl, p, Dr, even ? 0 : 1, U, lead2, other, W);
     note_launch();
     SM_CUDA_CHECK(cudaGetLastError());

@@ -107,3 +107,24 @@ def test_sliced_gemm_tiles(M, N, K):
     assert np.isnan(out[[1, M - 1]]).all()
     rest = np.delete(np.arange(M), [1, M - 1])
     assert np.max((np.abs(out - ref) / scale)[rest]) <= 8 * np.sqrt(K) * 2.0**-53
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("chi, D, dense", [(33, 3, False), (31, 12, False), (65, 4, True), (1, 17, True)])
+def test_mpo_scprod_lists(chi, D, dense, cplx):
+    """<O a|O b> with tiles of 32 x 32 bonds left ragged and more than 256 inputs to an output
+    (2 x 12^2), mostly zero and dense MPO tensors; sums of about chi^2 D^2 terms."""
+    rng = np.random.default_rng(chi + D)
+    n, d = 4, 2
+    bond = [1] + [chi] * (n - 1) + [1]
+    ob = [1] + [D] * (n - 1) + [1]
+    a, b = ([gaussian(rng, (bond[i], d, bond[i + 1]), cplx) for i in range(n)] for _ in range(2))
+    O = [gaussian(rng, (ob[i], d, d, ob[i + 1]), cplx) for i in range(n)]
+    if not dense:
+        O = [t * (rng.random(t.shape) < 0.2) for t in O]
+    prod = lambda x: [np.einsum("aijb,cjd->acibd", o, t).reshape(o.shape[0] * t.shape[0], d, -1)
+                      for o, t in zip(O, x)]
+    ref = so.scprod(prod(a), prod(b))
+    got = sg.mpo_scprod(sg.MPO(O), sg.MPS(a), sg.MPS(b))
+    norm = np.sqrt(abs(so.scprod(prod(a), prod(a)) * so.scprod(prod(b), prod(b))))
+    assert abs(got - ref) <= 1e-12 * norm
