@@ -5,9 +5,11 @@
 //   op(A) op(B) = (T1 - T2) + i (T3 - T1 - T2):
 // three real GEMMs (6 M N K real flops) instead of the four of the direct form.
 // k_cplx_planes writes op(X) (transposition and conjugation applied) as the
-// three FP64 planes re, im and re + im in one pass; the real products run on
-// the 3xTF32 tensor-core GEMM (FP32 accuracy, the mixed forms' contractions)
-// or on the FP64-accurate BF16-slice GEMM (the mixed forms' FP64 products);
+// three FP64 planes re, im and re + im in one pass for the 3xTF32 tensor-core GEMM
+// (FP32 accuracy, the mixed forms' contractions); the FP64-accurate BF16-slice GEMM
+// (the mixed forms' FP64 products) slices the three parts as it reads X and makes the
+// three products in one launch (128^3: 24 us; planes, slices and products one by one
+// were 63 us in nine launches);
 // k_cplx_combine forms alpha (T1 - T2 + i (T3 - T1 - T2)) + beta C.  The 3M
 // form's cancellation in T3 - T1 - T2 keeps the error normwise: within a few
 // units of the real products' own error times |A| |B|.
@@ -103,22 +105,20 @@ int gemm_cplx_3m(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int 
                  bool fp64_accurate) {
   const size_t mk = (size_t)M * K, kn = (size_t)K * N, mn = (size_t)M * N;
   double *pa, *pb, *t;
-  SM_CHECK(ctx.scratch("c3m.A", 3 * mk, &pa));
-  SM_CHECK(ctx.scratch("c3m.B", 3 * kn, &pb));
   SM_CHECK(ctx.scratch("c3m.T", 3 * mn, &t));
-  // op(A): M x K; op(B): K x N
-  SM_CHECK(planes(st, A, lda, M, K, opA == SM_OP_N ? 0 : 1, opA == SM_OP_C ? 1 : 0, pa, pa + mk,
-                  pa + 2 * mk));
-  SM_CHECK(planes(st, B, ldb, K, N, opB == SM_OP_N ? 0 : 1, opB == SM_OP_C ? 1 : 0, pb, pb + kn,
-                  pb + 2 * kn));
-  for (int p = 0; p < 3; ++p) {
-    const double* a = pa + p * mk;
-    const double* b = pb + p * kn;
-    double* c = t + p * mn;
-    if (fp64_accurate)
-      SM_CHECK(gemm_oz(ctx, st, SM_OP_N, SM_OP_N, M, N, K, 1.0, a, K, b, N, 0.0, c, N));
-    else
-      SM_CHECK(gemm_tc(ctx, st, SM_OP_N, SM_OP_N, M, N, K, 1.0, a, K, b, N, 0.0, c, N));
+  if (fp64_accurate) {
+    SM_CHECK(gemm_oz_3m(ctx, st, opA, opB, M, N, K, A, lda, B, ldb, t));
+  } else {
+    SM_CHECK(ctx.scratch("c3m.A", 3 * mk, &pa));
+    SM_CHECK(ctx.scratch("c3m.B", 3 * kn, &pb));
+    // op(A): M x K; op(B): K x N
+    SM_CHECK(planes(st, A, lda, M, K, opA == SM_OP_N ? 0 : 1, opA == SM_OP_C ? 1 : 0, pa, pa + mk,
+                    pa + 2 * mk));
+    SM_CHECK(planes(st, B, ldb, K, N, opB == SM_OP_N ? 0 : 1, opB == SM_OP_C ? 1 : 0, pb, pb + kn,
+                    pb + 2 * kn));
+    for (int p = 0; p < 3; ++p)
+      SM_CHECK(gemm_tc(ctx, st, SM_OP_N, SM_OP_N, M, N, K, 1.0, pa + p * mk, K, pb + p * kn, N, 0.0,
+                       t + p * mn, N));
   }
   const int blocks = (int)std::max<size_t>(1, std::min<size_t>((mn + 255) / 256, 4096));
   k_cplx_combine<<<blocks, 256, 0, st>>>(M, N, t, t + mn, t + 2 * mn, alpha, beta, C, ldc);

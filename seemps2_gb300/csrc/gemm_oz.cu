@@ -244,8 +244,8 @@ __device__ __forceinline__ void oz_store(uint32_t base, const int* et, int r0, i
 template <int ON>
 __global__ void __launch_bounds__(kOzThreads, 1)
     k_gemm_oz(const __grid_constant__ CUtensorMap mA, const __grid_constant__ CUtensorMap mB,
-              const int* __restrict__ ea, const int* __restrict__ eb, int M, int N, int nslabs,
-              int slabs_per, double alpha, double beta, double* __restrict__ C, int ldc,
+              const int* __restrict__ ea, const int* __restrict__ eb, int M, int N, int tm,
+              int nslabs, int slabs_per, double alpha, double beta, double* __restrict__ C, int ldc,
               double* __restrict__ part, unsigned int* __restrict__ status) {
   using Tile = OzTile<ON>;
   extern __shared__ unsigned char smem_raw[];
@@ -258,11 +258,14 @@ __global__ void __launch_bounds__(kOzThreads, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
   __shared__ int et[OM + ON];  // exponents of the tile's rows and columns
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m0 = blockIdx.y * OM, n0 = blockIdx.x * ON;
+  // product p: rows p M .. of the slices of A, rows p N .. of those of B (a tile's rows
+  // beyond M belong to the next product and are not stored)
+  const int p = blockIdx.y / tm, m0 = blockIdx.y % tm * OM, n0 = blockIdx.x * ON;
   if (threadIdx.x < OM) {
-    if (m0 + threadIdx.x < M) et[threadIdx.x] = max(ea[m0 + threadIdx.x], -1100) - 14;
+    if (m0 + threadIdx.x < M) et[threadIdx.x] = max(ea[p * M + m0 + threadIdx.x], -1100) - 14;
   } else if (threadIdx.x < OM + ON) {
-    if (n0 + threadIdx.x - OM < N) et[threadIdx.x] = max(eb[n0 + threadIdx.x - OM], -1100);
+    if (n0 + threadIdx.x - OM < N)
+      et[threadIdx.x] = max(eb[p * N + n0 + threadIdx.x - OM], -1100);
   }
   const int s0 = blockIdx.z * slabs_per;
   const int nk = max(0, min(nslabs, s0 + slabs_per) - s0);
@@ -302,8 +305,8 @@ __global__ void __launch_bounds__(kOzThreads, 1)
         unsigned char* stg = base + (size_t)s * Tile::kStage;
         mbar_expect_tx(&full[s], Tile::kStage);
         const int x = (s0 + i) * OK;
-        tma_load_3d(stg, &mA, &full[s], x, m0, 0);
-        tma_load_3d(stg + kSlices * kSliceA, &mB, &full[s], x, n0, 0);
+        tma_load_3d(stg, &mA, &full[s], x, p * M + m0, 0);
+        tma_load_3d(stg + kSlices * kSliceA, &mB, &full[s], x, p * N + n0, 0);
         issued[s] += 1;
       }
       for (int s = 0; s < OS; ++s)
@@ -425,7 +428,8 @@ __global__ void __launch_bounds__(kOzThreads, 1)
   const uint32_t sums = smem_u32(base);
   const bool add = !part && (alpha != 1.0 || beta != 0.0);
   const size_t ldo = part ? N : ldc;
-  double* out = (part ? part + (size_t)(blockIdx.z / nz) * M * N : C) + (size_t)m0 * ldo + n0;
+  double* out = (part ? part + (size_t)(blockIdx.z / nz) * (gridDim.y / tm) * M * N : C) +
+                (size_t)(p * M + m0) * ldo + n0;
   switch (nz) {  // a power of two (host)
     case 1: oz_store<ON, 1>(sums, et, r0, r1, nc, add, alpha, beta, out, ldo); break;
     case 2: oz_store<ON, 2>(sums, et, r0, r1, nc, add, alpha, beta, out, ldo); break;
@@ -436,14 +440,16 @@ __global__ void __launch_bounds__(kOzThreads, 1)
 }
 
 // One operand of the preparation: op(X) is rows x K with element
-// (r, k) = X[r * ldx + k] (trans = 0) or X[k * ldx + r] (trans = 1).
+// (r, k) = X[r * ldx + k] (trans = 0) or X[k * ldx + r] (trans = 1).  A complex X
+// (conjugated if sign is -1) becomes three operands of rows x K, one below the other:
+// its real part, its imaginary part, and their sum.
 constexpr int kPrepRows = 8;     // rows of a CTA: a warp each
 constexpr int kPrepCols = 512;   // K entries held in shared memory
 constexpr int kPrepRange = 256;  // K entries of a CTA while the cluster can grow
 
 struct OzOperand {
   const double* X;
-  int ldx, rows, trans;
+  int ldx, rows, trans, sign;
   int* ex;
   __nv_bfloat16* out;
 };
@@ -461,6 +467,7 @@ struct OzOperand {
 // lane.  Only integer and FP32 operations: maxima of doubles alone, at 64 clocks of
 // the FP64 pipe each, took 8 us of the 15 us that separate passes for the exponents
 // and the slices did at 320 x 256.
+template <int kParts>  // 1: real, 3: complex
 __global__ void __launch_bounds__(32 * kPrepRows)
     k_oz_prep(OzOperand A, OzOperand B, int K, int kp, int range) {
   const OzOperand& o = blockIdx.z ? B : A;
@@ -468,7 +475,7 @@ __global__ void __launch_bounds__(32 * kPrepRows)
   __shared__ unsigned key[kPrepRows];
   cg::cluster_group cluster = cg::this_cluster();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int r0 = blockIdx.x * kPrepRows;
+  const int rb = gridDim.x / kParts, p = blockIdx.x / rb, r0 = blockIdx.x % rb * kPrepRows;
   if (r0 >= o.rows) return;  // uniform over the cluster
   const int k0 = blockIdx.y * range, k1 = min(kp, k0 + range);
   const int nch = max(1, (k1 - k0 + kPrepCols - 1) / kPrepCols);
@@ -480,15 +487,22 @@ __global__ void __launch_bounds__(32 * kPrepRows)
     // trans: 8 rows x 4 columns to a warp, 64 contiguous bytes of each column
     const int rr = o.trans ? tid & 7 : warp, kt = o.trans ? tid >> 3 : lane;
     const bool on = r0 + rr < o.rows;
-    const size_t step = o.trans ? o.ldx : 1;
-    const double* src = o.X + (o.trans ? (size_t)(r0 + rr) : (size_t)(r0 + rr) * o.ldx) + c0 * step;
+    constexpr int kWords = kParts == 1 ? 1 : 2;
+    const size_t step = (o.trans ? (size_t)o.ldx : 1) * kWords;
+    const double* src =
+        o.X + (o.trans ? (size_t)(r0 + rr) : (size_t)(r0 + rr) * o.ldx) * kWords + c0 * step;
     unsigned m = 0;
     for (int ka = kt; ka < n; ka += 8 * 32) {  // eight loads in flight
       double x[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int k = ka + 32 * i;
-        x[i] = on && k < n && c0 + k < K ? src[k * step] : 0.0;
+        x[i] = 0.0;
+        if (on && k < n && c0 + k < K) {
+          if (kParts == 1 || p == 0) x[i] = src[k * step];
+          else if (p == 1) x[i] = o.sign < 0 ? -src[k * step + 1] : src[k * step + 1];
+          else x[i] = o.sign < 0 ? src[k * step] - src[k * step + 1] : src[k * step] + src[k * step + 1];
+        }
       }
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -518,8 +532,9 @@ __global__ void __launch_bounds__(32 * kPrepRows)
   // the bound 2^-1021 of a row of subnormals loses none of their bits
   const int ex = m == 0 ? kOzNoExp
                         : m >= 0x7ff00000u ? kOzNotFinite : max((int)(m >> 20), 1) - 1022;
-  if (cluster.block_rank() == 0 && lane == 0 && r < o.rows) o.ex[r] = ex;
-  const size_t plane = (size_t)o.rows * kp;
+  if (cluster.block_rank() == 0 && lane == 0 && r < o.rows) o.ex[p * o.rows + r] = ex;
+  const size_t plane = (size_t)kParts * o.rows * kp;
+  __nv_bfloat16* out = o.out + (size_t)(p * o.rows + r) * kp;
   for (int c = 0; c < nch; ++c) {
     const int c0 = k0 + c * kPrepCols, n = min(kPrepCols, k1 - c0);
     if (nch > 1) {
@@ -550,7 +565,7 @@ __global__ void __launch_bounds__(32 * kPrepRows)
           const unsigned a = (unsigned)(F[h] >> (49 - 7 * i)) & 127u;
           w[h] = __float_as_uint((__uint_as_float(0x4B000000u | a) - 8388608.0f) * scale) | sign[h];
         }
-        *reinterpret_cast<unsigned*>(o.out + i * plane + (size_t)r * kp + c0 + k) =
+        *reinterpret_cast<unsigned*>(out + i * plane + c0 + k) =
             __byte_perm(w[0], w[1], 0x7632);
         scale *= 0.0078125f;  // 2^-7
       }
@@ -639,35 +654,40 @@ bool gemm_oz_eligible(int M, int N, int K) {
          oz_encode_fn() != nullptr;
 }
 
-int gemm_oz(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, double alpha,
-            const double* A, int lda, const double* B, int ldb, double beta, double* C, int ldc) {
+namespace {
+
+// parts products of M x N x K, the p-th at rows p M .. of C
+template <int kParts>
+int products(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, double alpha,
+             const double* A, int lda, const double* B, int ldb, double beta, double* C, int ldc) {
   const int kp = (K + OK - 1) / OK * OK;
   const int nslabs = kp / OK;
   __nv_bfloat16 *sa, *sb;
   int *ea, *eb;
   unsigned int* status;
-  SM_CHECK(ctx.scratch("oz.A", (size_t)kSlices * M * kp, &sa));
-  SM_CHECK(ctx.scratch("oz.B", (size_t)kSlices * N * kp, &sb));
-  SM_CHECK(ctx.scratch("oz.ea", (size_t)M, &ea));
-  SM_CHECK(ctx.scratch("oz.eb", (size_t)N, &eb));
+  SM_CHECK(ctx.scratch("oz.A", (size_t)kSlices * kParts * M * kp, &sa));
+  SM_CHECK(ctx.scratch("oz.B", (size_t)kSlices * kParts * N * kp, &sb));
+  SM_CHECK(ctx.scratch("oz.ea", (size_t)kParts * M, &ea));
+  SM_CHECK(ctx.scratch("oz.eb", (size_t)kParts * N, &eb));
   SM_CHECK(tc_status(ctx, &status));
   // op(A)[m][k] = A[m][k] (N) or A[k][m] (T, C: real); op(B)^T[n][k] = B[k][n]
   // (N) or B[n][k] (T, C)
   const int ta = opA == SM_OP_N ? 0 : 1, tb = opB == SM_OP_N ? 1 : 0;
-  const OzOperand oa{A, lda, M, ta, ea, sa}, ob{B, ldb, N, tb, eb, sb};
+  const OzOperand oa{A, lda, M, ta, opA == SM_OP_C ? -1 : 1, ea, sa};
+  const OzOperand ob{B, ldb, N, tb, opB == SM_OP_C ? -1 : 1, eb, sb};
   const int rb = (std::max(M, N) + kPrepRows - 1) / kPrepRows;
   const int zk = std::min(kOzCluster, (kp + kPrepRange - 1) / kPrepRange);
   const int range = (nslabs + zk - 1) / zk * OK;
-  SM_CHECK(cluster_launch(k_oz_prep, dim3(rb, zk, 2), dim3(32 * kPrepRows), dim3(1, zk, 1), 0, st,
+  SM_CHECK(cluster_launch(k_oz_prep<kParts>, dim3(kParts * rb, zk, 2), dim3(32 * kPrepRows), dim3(1, zk, 1), 0, st,
                           oa, ob, K, kp, range));
   note_launch();
   CUtensorMap mA, mB;
-  SM_CHECK(make_slice_map(&mA, sa, M, kp, OM));
+  SM_CHECK(make_slice_map(&mA, sa, kParts * M, kp, OM));
   // Split K over the CTAs of a cluster while the output has fewer tiles than SMs,
   // down to one slab each (any split at slabs is exact).  Only beyond 16 slabs a CTA
   // a tile gets several clusters: their sum is another launch of ~4 us.
   const int sms = std::max(1, ctx.num_sms), tm = (M + OM - 1) / OM;
-  const int tiles = tm * ((N + 63) / 64);
+  const int tiles = kParts * tm * ((N + 63) / 64);
   int nz = 1;
   while (nz < kOzCluster && 2 * nz <= std::min(sms / tiles, nslabs)) nz *= 2;
   int slabs_per = (nslabs + nz - 1) / nz;
@@ -675,27 +695,39 @@ int gemm_oz(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, do
       nz < kOzCluster ? 1 : std::max(1, std::min(sms / (tiles * nz), slabs_per / 8));
   if (nzo > 1) slabs_per = (nslabs + nz * nzo - 1) / (nz * nzo);
   double* part = nullptr;
-  if (nzo > 1) SM_CHECK(ctx.scratch("oz.part", (size_t)nzo * M * N, &part));
+  if (nzo > 1) SM_CHECK(ctx.scratch("oz.part", (size_t)nzo * kParts * M * N, &part));
   // Half as wide a tile where twice as many CTAs still find an SM each: half of
   // everything but the loads of A to a CTA.
   const bool narrow = 2 * tiles * nz * nzo <= sms && N > 32;
   const int on = narrow ? 32 : 64;
-  SM_CHECK(make_slice_map(&mB, sb, N, kp, on));
+  SM_CHECK(make_slice_map(&mB, sb, kParts * N, kp, on));
   const auto kernel = narrow ? k_gemm_oz<32> : k_gemm_oz<64>;
   const size_t smem = narrow ? OzTile<32>::kSmem : OzTile<64>::kSmem;
   SM_CHECK(raise_smem_limit(kernel, smem));
-  SM_CHECK(cluster_launch(kernel, dim3((N + on - 1) / on, tm, nz * nzo), dim3(kOzThreads),
-                          dim3(1, 1, nz), smem, st, mA, mB, (const int*)ea, (const int*)eb, M, N,
+  SM_CHECK(cluster_launch(kernel, dim3((N + on - 1) / on, kParts * tm, nz * nzo), dim3(kOzThreads),
+                          dim3(1, 1, nz), smem, st, mA, mB, (const int*)ea, (const int*)eb, M, N, tm,
                           nslabs, slabs_per, alpha, beta, C, ldc, part, status));
   note_launch();
   if (nzo > 1) {
-    const size_t mn = (size_t)M * N;
-    k_oz_reduce<<<(int)std::min<size_t>((mn + 255) / 256, 4096), 256, 0, st>>>(M, N, nzo, part,
+    const size_t mn = (size_t)kParts * M * N;
+    k_oz_reduce<<<(int)std::min<size_t>((mn + 255) / 256, 4096), 256, 0, st>>>(kParts * M, N, nzo, part,
                                                                                alpha, beta, C, ldc);
     note_launch();
     SM_CUDA_CHECK(cudaGetLastError());
   }
   return SM_OK;
+}
+
+}  // namespace
+
+int gemm_oz(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, double alpha,
+            const double* A, int lda, const double* B, int ldb, double beta, double* C, int ldc) {
+  return products<1>(ctx, st, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+}
+
+int gemm_oz_3m(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, const cplx* A,
+               int lda, const cplx* B, int ldb, double* T) {
+  return products<3>(ctx, st, opA, opB, M, N, K, 1.0, &A->re, lda, &B->re, ldb, 0.0, T, N);
 }
 
 }  // namespace sm

@@ -189,6 +189,9 @@ int tc_status_check(Ctx& ctx, cudaStream_t st);
 // the operands into 7-bit integer slices); gemm_ctx<double> uses it in the
 // mixed forms (ctx.fp64_tc) for shapes gemm_oz_eligible accepts.
 bool gemm_oz_eligible(int M, int N, int K);
+// the three products of a complex one: T = [Ar Br; Ai Bi; (Ar + Ai)(Br + Bi)], 3 M x N
+int gemm_oz_3m(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, const cplx* A,
+               int lda, const cplx* B, int ldb, double* T);
 int gemm_oz(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, double alpha,
             const double* A, int lda, const double* B, int ldb, double beta, double* C, int ldc);
 

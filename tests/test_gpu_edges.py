@@ -128,3 +128,16 @@ def test_mpo_scprod_lists(chi, D, dense, cplx):
     got = sg.mpo_scprod(sg.MPO(O), sg.MPS(a), sg.MPS(b))
     norm = np.sqrt(abs(so.scprod(prod(a), prod(a)) * so.scprod(prod(b), prod(b))))
     assert abs(got - ref) <= 1e-12 * norm
+
+
+@pytest.mark.parametrize("M, N, K", [(32, 32, 600), (65, 33, 257), (129, 130, 96), (400, 300, 200), (48, 40, 5000)])
+def test_sliced_complex_gemm_tiles(M, N, K):
+    """The three real products of a complex one: 16 sqrt(K) u of |A||B| (the sum of three
+    bounds of 8 sqrt(K) u, each of at most half of |A||B| in the part it enters)."""
+    from tests.test_gpu_tc import _cplx_case, _gemm_c
+
+    for opA, opB in [("N", "N"), ("T", "C"), ("C", "T")]:
+        Aop, Bop, A, B = _cplx_case(M, N, K, opA, opB, M + N + K, scaled=True)
+        out = _gemm_c("sm_gemm_f64tc", opA, opB, A, B, M, N, K)
+        err = np.max(np.abs(out - Aop @ Bop) / (np.abs(Aop) @ np.abs(Bop)))
+        assert err <= 16 * np.sqrt(K) * 2.0**-53
