@@ -25,6 +25,7 @@
 // returns; the sweep reads the status word at its end.
 #include <algorithm>
 
+#include <cooperative_groups.h>
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -33,10 +34,14 @@
 
 namespace sm {
 
+namespace cg = cooperative_groups;
+
 namespace {
 
 constexpr int TM = 128, TN = 128, TS = 3;
 constexpr int kTCThreads = 128;
+constexpr int kTcCluster = 8;   // K ranges of a tile that share a cluster (portable size)
+constexpr int kTcRow = TN + 1;  // row stride of the sums in shared memory: no bank conflicts
 // Per mode: 3xTF32 (FP32 planes hi and lo of both operands, 32-wide K slabs,
 // three tf32 MMAs of K = 8 per 8 of K) or BF16 (one BF16 plane per operand,
 // 64-wide K slabs, one f16-kind MMA of K = 16 per 16 of K).  Either way a
@@ -57,6 +62,8 @@ struct TcMode {
   static constexpr uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) |
                                     ((uint32_t)(TN >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
 };
+static_assert((size_t)TM * kTcRow * 4 <= (size_t)TS * TcMode<true>::stage,
+              "the sums fit where the stages were");
 constexpr unsigned long long kWaitNs = 1000000000ull;  // 1 s per wait
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -154,6 +161,63 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ uint32_t mapa(uint32_t saddr, int rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t a) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+// FP32 to FP64 by integer operations: a conversion holds the FP64 pipe for 64 clocks, a
+// predicated-off one too, so what is rare (subnormal, infinite, NaN) is out of line
+__device__ __noinline__ double tc_widen_rare(float f) { return (double)f; }
+__device__ __forceinline__ double tc_widen(float f) {
+  const unsigned b = __float_as_uint(f), x = (b >> 23) & 0xffu;
+  if ((b << 1) != 0 && (x == 0 || x == 0xffu)) return tc_widen_rare(f);
+  const unsigned hi = (b << 1) == 0 ? b : (b & 0x80000000u) | ((x + 896u) << 20) | ((b & 0x7fffffu) >> 3);
+  return __hiloint2double((int)hi, (int)((b << 1) == 0 ? 0u : b << 29));
+}
+template <typename OutT>
+__device__ __noinline__ void tc_axpby(double alpha, double v, double beta, OutT* c) {
+  *c = beta == 0.0 ? (OutT)(alpha * v) : (OutT)fma(alpha, v, beta * (double)*c);
+}
+
+// Rows r0 .. r1 - 1 of the tile: the sum of the cluster's NZ FP32 tiles, carried as an
+// unevaluated sum of two FP32 (48 bits) so that FP64 adds once, stored by lanes along
+// the columns.  add: C = alpha v + beta C (else C = v)
+template <int NZ, typename OutT>
+__device__ __forceinline__ void tc_store(uint32_t base, int r0, int r1, int ncol, bool add,
+                                         double alpha, double beta, OutT* C, size_t ldc) {
+  uint32_t src[NZ];
+#pragma unroll
+  for (int y = 0; y < NZ; ++y) src[y] = mapa(base, y) + threadIdx.x * 4;
+  const int c = threadIdx.x;  // kTCThreads == TN
+  if (c >= ncol) return;
+#pragma unroll 4
+  for (int r = r0; r < r1; ++r) {
+    float hi = ld_cluster_f32(src[0] + (uint32_t)(r * kTcRow * 4)), lo = 0.f;
+#pragma unroll
+    for (int y = 1; y < NZ; ++y) {
+      const float x = ld_cluster_f32(src[y] + (uint32_t)(r * kTcRow * 4));
+      const float t = hi + x, u = t - hi;
+      lo += (hi - (t - u)) + (x - u);
+      hi = t;
+    }
+    OutT* p = C + (size_t)r * ldc + c;
+    if (NZ > 1 && !(fabsf(lo) <= FLT_MAX)) lo = 0.f;  // an infinity in hi stays one
+    if (add) {
+      tc_axpby<OutT>(alpha, (double)hi + (double)lo, beta, p);
+    } else if constexpr (sizeof(OutT) == 8) {
+      *p = NZ > 1 ? tc_widen(hi) + tc_widen(lo) : tc_widen(hi);
+    } else {
+      *p = hi + lo;
+    }
+  }
+}
+
 template <bool BF16, typename OutT>
 __global__ void __launch_bounds__(kTCThreads, 1)
     k_gemm_tc(const __grid_constant__ CUtensorMap mAh, const __grid_constant__ CUtensorMap mAl,
@@ -174,7 +238,7 @@ __global__ void __launch_bounds__(kTCThreads, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
   const int kt0 = blockIdx.z * kt_per;
-  const int nk = min(ktiles, kt0 + kt_per) - kt0;  // >= 1 (host)
+  const int nk = max(0, min(ktiles, kt0 + kt_per) - kt0);
   if (threadIdx.x == 0) {
     for (int s = 0; s < TS; ++s) {
       mbar_init(&full[s], 1);
@@ -264,38 +328,40 @@ __global__ void __launch_bounds__(kTCThreads, 1)
   const bool ok = mbar_wait(done, 0u, 4 * kWaitNs);
   __syncwarp();
   tc_fence_after();
-  if (ok) {
-    const int row = m0 + warp * 32 + lane;
-    for (int c = 0; c < TN; c += 16) {
-      float v[16];
-      tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
-      if (row < M) {
+  // The accumulators go to shared memory (no copy or MMA uses the stages any more), and
+  // each CTA of the cluster stores a share of the rows.
+  float* sums = reinterpret_cast<float*>(base);
+  if (!ok && threadIdx.x == 0) atomicOr(status, 8u);
+  for (int c = 0; c < TN; c += 16) {
+    float v[16];
+    if (ok && nk > 0) tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int col = n0 + c + j;
-          if (col < N) {
-            if (part) {
-              part[((size_t)blockIdx.z * M + row) * N + col] = (OutT)v[j];
-            } else {
-              OutT* p = C + (size_t)row * ldc + col;
-              *p = beta == 0.0 ? (OutT)(alpha * (double)v[j])
-                               : (OutT)fma(alpha, (double)v[j], beta * (double)*p);
-            }
-          }
-        }
-      }
-    }
-  } else if (threadIdx.x == 0) {
-    atomicOr(status, 8u);
+    for (int j = 0; j < 16; ++j)
+      sums[(warp * 32 + lane) * kTcRow + c + j] = nk > 0 ? v[j] : 0.f;
   }
   tc_fence_before();
-  __syncthreads();
+  cg::cluster_group cluster = cg::this_cluster();
+  cluster.sync();
   if (warp == 0) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
                  "r"((uint32_t)TN)
                  : "memory");
   }
+  const int nz = (int)cluster.num_blocks(), z = (int)cluster.block_rank();
+  const int mv = min(TM, M - m0), per = (mv + nz - 1) / nz;
+  const int r0 = z * per, r1 = min(mv, r0 + per), nc = min(TN, N - n0);
+  const uint32_t at = smem_u32(sums);
+  const bool add = !part && (alpha != 1.0 || beta != 0.0);
+  const size_t ldo = part ? N : ldc;
+  OutT* out = (part ? part + (size_t)(blockIdx.z / nz) * M * N : C) + (size_t)m0 * ldo + n0;
+  switch (nz) {  // a power of two (host)
+    case 1: tc_store<1, OutT>(at, r0, r1, nc, add, alpha, beta, out, ldo); break;
+    case 2: tc_store<2, OutT>(at, r0, r1, nc, add, alpha, beta, out, ldo); break;
+    case 4: tc_store<4, OutT>(at, r0, r1, nc, add, alpha, beta, out, ldo); break;
+    default: tc_store<kTcCluster, OutT>(at, r0, r1, nc, add, alpha, beta, out, ldo); break;
+  }
+  cluster.sync();  // no CTA leaves while another reads its sums
 }
 
 __device__ __forceinline__ float tf32_rna(float x) {
@@ -306,11 +372,22 @@ __device__ __forceinline__ float tf32_rna(float x) {
 
 // hi / lo FP32 parts of op(X) as a rows x kp K-contiguous array: element
 // (r, k) is X[r * ldx + k] (trans = 0) or X[k * ldx + r] (trans = 1), zero for
-// k >= K.  32 x 32 tiles through shared memory so both sides stay coalesced.
-__global__ void k_split_tf32(const double* __restrict__ X, int ldx, int rows, int K, int kp,
-                             int trans, float* __restrict__ hi, float* __restrict__ lo) {
+// k >= K.  32 x 32 tiles through shared memory so both sides stay coalesced;
+// blockIdx.z picks the operand.
+struct TcOperand {
+  const double* X;
+  int ldx, rows, trans;
+  void* hi;
+  float* lo;
+};
+__global__ void k_split_tf32(TcOperand A, TcOperand B, int K, int kp) {
+  const TcOperand& o = blockIdx.z ? B : A;
+  const double* __restrict__ X = o.X;
+  const int ldx = o.ldx, rows = o.rows, trans = o.trans;
+  float *hi = reinterpret_cast<float*>(o.hi), *lo = o.lo;
   __shared__ double tile[32][33];
   const int r0 = blockIdx.y * 32, k0 = blockIdx.x * 32;
+  if (r0 >= rows) return;  // uniform over the block
   const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
   for (int j = ty; j < 32; j += 8) {
     double v = 0.0;
@@ -338,10 +415,14 @@ __global__ void k_split_tf32(const double* __restrict__ X, int ldx, int rows, in
 
 // op(X) rounded to BF16 as a rows x kp K-contiguous array (same tiling and
 // element rule as k_split_tf32).
-__global__ void k_split_bf16(const double* __restrict__ X, int ldx, int rows, int K, int kp,
-                             int trans, __nv_bfloat16* __restrict__ out) {
+__global__ void k_split_bf16(TcOperand A, TcOperand B, int K, int kp) {
+  const TcOperand& o = blockIdx.z ? B : A;
+  const double* __restrict__ X = o.X;
+  const int ldx = o.ldx, rows = o.rows, trans = o.trans;
+  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(o.hi);
   __shared__ double tile[32][33];
   const int r0 = blockIdx.y * 32, k0 = blockIdx.x * 32;
+  if (r0 >= rows) return;  // uniform over the block
   const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
   for (int j = ty; j < 32; j += 8) {
     double v = 0.0;
@@ -425,18 +506,41 @@ bool gemm_tc_eligible(int M, int N, int K) {
 
 int tc_kslab(bool bf16) { return bf16 ? TcMode<true>::TK : TcMode<false>::TK; }
 
-int tc_planes(Ctx& ctx, cudaStream_t st, const double* X, int ldx, int rows, int K, int kp,
-              int trans, bool bf16, void* hi, float* lo) {
-  const dim3 sblk(32, 8), grd(kp / 32, (rows + 31) / 32);
-  if (bf16)
-    k_split_bf16<<<grd, sblk, 0, st>>>(X, ldx, rows, K, kp, trans,
-                                       reinterpret_cast<__nv_bfloat16*>(hi));
-  else
-    k_split_tf32<<<grd, sblk, 0, st>>>(X, ldx, rows, K, kp, trans, reinterpret_cast<float*>(hi),
-                                       lo);
+namespace {
+// the planes of one operand, or of two in one launch
+int split_planes(cudaStream_t st, const TcOperand& a, const TcOperand* b, int K, int kp, bool bf16) {
+  const int rows = std::max(a.rows, b ? b->rows : 0);
+  const dim3 blk(32, 8), grd(kp / 32, (rows + 31) / 32, b ? 2 : 1);
+  if (bf16) k_split_bf16<<<grd, blk, 0, st>>>(a, b ? *b : a, K, kp);
+  else k_split_tf32<<<grd, blk, 0, st>>>(a, b ? *b : a, K, kp);
   note_launch();
   SM_CUDA_CHECK(cudaGetLastError());
   return SM_OK;
+}
+
+template <typename... P, typename... Q>
+int cluster_launch(void (*fn)(P...), dim3 grid, int block, int nz, size_t smem, cudaStream_t st,
+                   Q... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = 1;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = nz;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  SM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fn, args...));
+  return SM_OK;
+}
+}  // namespace
+
+int tc_planes(Ctx&, cudaStream_t st, const double* X, int ldx, int rows, int K, int kp, int trans,
+              bool bf16, void* hi, float* lo) {
+  return split_planes(st, TcOperand{X, ldx, rows, trans, hi, lo}, nullptr, K, kp, bf16);
 }
 
 template <typename OutT>
@@ -458,28 +562,29 @@ int gemm_tc_planes(Ctx& ctx, cudaStream_t st, int M, int N, int kp, bool bf16, c
     SM_CHECK(make_map(&mBl, bl, false, N, kp, TN));
   }
   const int tiles = ((M + TM - 1) / TM) * ((N + TN - 1) / TN);
-  int nz = std::max(1, std::min(std::max(1, ctx.num_sms) / tiles, ktiles / 2));
-  const int kt_per = (ktiles + nz - 1) / nz;
-  nz = (ktiles + kt_per - 1) / kt_per;
+  // K over the CTAs of a cluster while the output has fewer tiles than SMs; beyond 16
+  // slabs a CTA a tile gets several clusters, whose sum is another launch
+  const int sms = std::max(1, ctx.num_sms);
+  int nz = 1;
+  while (nz < kTcCluster && 2 * nz <= std::min(sms / tiles, ktiles)) nz *= 2;
+  int kt_per = (ktiles + nz - 1) / nz;
+  const int nzo =
+      nz < kTcCluster ? 1 : std::max(1, std::min(sms / (tiles * nz), kt_per / 8));
+  if (nzo > 1) kt_per = (ktiles + nz * nzo - 1) / (nz * nzo);
   OutT* part = nullptr;
-  if (nz > 1)
-    SM_CHECK(ctx.scratch(sizeof(OutT) == 8 ? "tc.part" : "tc.part32", (size_t)nz * M * N, &part));
-  const dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM, nz);
-  if (bf16) {
-    SM_CHECK(raise_smem_limit(k_gemm_tc<true, OutT>, TcMode<true>::smem));
-    k_gemm_tc<true, OutT><<<grid, kTCThreads, TcMode<true>::smem, st>>>(
-        mAh, mAl, mBh, mBl, M, N, ktiles, kt_per, alpha, beta, C, ldc, part, status);
-  } else {
-    SM_CHECK(raise_smem_limit(k_gemm_tc<false, OutT>, TcMode<false>::smem));
-    k_gemm_tc<false, OutT><<<grid, kTCThreads, TcMode<false>::smem, st>>>(
-        mAh, mAl, mBh, mBl, M, N, ktiles, kt_per, alpha, beta, C, ldc, part, status);
-  }
+  if (nzo > 1)
+    SM_CHECK(ctx.scratch(sizeof(OutT) == 8 ? "tc.part" : "tc.part32", (size_t)nzo * M * N, &part));
+  const dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM, nz * nzo);
+  const auto kernel = bf16 ? k_gemm_tc<true, OutT> : k_gemm_tc<false, OutT>;
+  const size_t smem = bf16 ? TcMode<true>::smem : TcMode<false>::smem;
+  SM_CHECK(raise_smem_limit(kernel, smem));
+  SM_CHECK(cluster_launch(kernel, grid, kTCThreads, nz, smem, st, mAh, mAl, mBh, mBl, M, N, ktiles,
+                          kt_per, alpha, beta, C, ldc, part, status));
   note_launch();
-  SM_CUDA_CHECK(cudaGetLastError());
-  if (nz > 1) {
+  if (nzo > 1) {
     const size_t mn = (size_t)M * N;
     k_tc_reduce<OutT><<<(int)std::min<size_t>((mn + 255) / 256, 4096), 256, 0, st>>>(
-        M, N, nz, part, alpha, beta, C, ldc);
+        M, N, nzo, part, alpha, beta, C, ldc);
     note_launch();
     SM_CUDA_CHECK(cudaGetLastError());
   }
@@ -510,8 +615,8 @@ int gemm_tc(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, do
     SM_CHECK(ctx.scratch("tc.Al", (size_t)M * kp, &al));
     SM_CHECK(ctx.scratch("tc.Bl", (size_t)N * kp, &bl));
   }
-  SM_CHECK(tc_planes(ctx, st, A, lda, M, K, kp, ta, bf16, ah, al));
-  SM_CHECK(tc_planes(ctx, st, B, ldb, N, K, kp, tb, bf16, bh, bl));
+  const TcOperand oa{A, lda, M, ta, ah, al}, ob{B, ldb, N, tb, bh, bl};
+  SM_CHECK(split_planes(st, oa, &ob, K, kp, bf16));
   return gemm_tc_planes<double>(ctx, st, M, N, kp, bf16, ah, al, bh, bl, alpha, beta, C, ldc);
 }
 
