@@ -9,17 +9,21 @@
 // TF32, lo = the FP32 rest) and the product is hi*hi + hi*lo + lo*hi
 // accumulated in FP32 in tensor memory: the error of an FP32 GEMM.
 //
-// Data path per 128 x 128 output tile (one CTA of 128 threads, K split over
-// blockIdx.z when the output has few tiles):
+// Data path per 128 x 128 output tile (one CTA of 128 threads and K range; the K ranges
+// of a tile are the CTAs of a cluster, taken when the output has few tiles):
 //   * a split kernel writes hi / lo of op(A) as M x Kp and of op(B)^T as
 //     N x Kp FP32 arrays (K contiguous, Kp = K rounded up to 32, zero pad);
 //   * warp 0 / lane 0 streams 32-wide K slices of the four arrays with TMA
 //     (cp.async.bulk.tensor, 128-byte swizzle) into a 3-stage ring;
 //   * warp 1 / lane 0 issues tcgen05.mma kind::tf32 (M=128, N=128, K=8; three
-//     per K step) accumulating in 128 TMEM columns, and tcgen05.commit frees
-//     each stage;
-//   * all four warps read the accumulator back with tcgen05.ld (warp w owns
-//     TMEM lanes 32w..32w+31 = tile rows) and write FP64 results.
+//     per K step) into 4 accumulators of 128 TMEM columns in turn, and
+//     tcgen05.commit frees each stage;
+//   * all four warps read the accumulators back with tcgen05.ld (warp w owns
+//     TMEM lanes 32w..32w+31 = tile rows), leave their sum in shared memory, and
+//     each CTA adds up a share of the rows over the cluster and stores it.
+// 320 x 128 x 256 takes 10 us after 6 us of splitting.  (Planes in a launch for each
+// operand, an epilogue that widened and stored a row to a lane, FP64 partial sums in
+// memory and a pass over them: 15, 12 and 4.5 us.)
 // Every mbarrier wait is bounded (globaltimer): on timeout the CTA records an
 // error bit, waits (bounded) for its own copies in flight, frees its TMEM and
 // returns; the sweep reads the status word at its end.
@@ -55,6 +59,8 @@ struct TcMode {
   static constexpr uint32_t tileB = TN * 128;
   static constexpr uint32_t stage = planes * (tileA + tileB);
   static constexpr size_t smem = (size_t)TS * stage + 1024 + 256;
+  // accumulators that the slabs take turns in
+  static constexpr int acc = BF16 ? 1 : 4;
   // instruction descriptor: D = F32 (bits 4-5 = 1), A and B TF32 (2) or BF16
   // (1) at bits 7-9 and 10-12, both K-major (bits 15, 16 = 0), N >> 3 at bits
   // 17-22, M >> 4 at bits 24-28
@@ -251,7 +257,7 @@ __global__ void __launch_bounds__(kTCThreads, 1)
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(tmem_slot)),
-                 "r"((uint32_t)TN)
+                 "r"((uint32_t)(Md::acc * TN))
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -299,13 +305,14 @@ __global__ void __launch_bounds__(kTCThreads, 1)
       }
       tc_fence_after();
       const uint32_t ah = smem_u32(base + (size_t)s * kStage);
+      const uint32_t d = tmem + (uint32_t)(i % Md::acc * TN);
+      const bool more = i >= Md::acc;
       if constexpr (BF16) {
         const uint32_t bh = ah + kTileA;
 #pragma unroll
         for (int kk = 0; kk < TK / Md::KMMA; ++kk) {
           const uint32_t off = kk * 32;  // 16 BF16 values
-          umma_bf16(tmem, sdesc_sw128(ah + off), sdesc_sw128(bh + off),
-                    (i > 0 || kk > 0) ? 1u : 0u);
+          umma_bf16(d, sdesc_sw128(ah + off), sdesc_sw128(bh + off), (more || kk > 0) ? 1u : 0u);
         }
       } else {
         const uint32_t al = ah + kTileA, bh = ah + 2 * kTileA, bl = bh + kTileB;
@@ -314,9 +321,9 @@ __global__ void __launch_bounds__(kTCThreads, 1)
           const uint32_t off = kk * 32;  // 8 TF32 values
           const uint64_t dah = sdesc_sw128(ah + off), dal = sdesc_sw128(al + off);
           const uint64_t dbh = sdesc_sw128(bh + off), dbl = sdesc_sw128(bl + off);
-          umma_tf32(tmem, dah, dbh, (i > 0 || kk > 0) ? 1u : 0u);
-          umma_tf32(tmem, dah, dbl, 1u);
-          umma_tf32(tmem, dal, dbh, 1u);
+          umma_tf32(d, dah, dbh, (more || kk > 0) ? 1u : 0u);
+          umma_tf32(d, dah, dbl, 1u);
+          umma_tf32(d, dal, dbh, 1u);
         }
       }
       umma_commit(&empty[s]);
@@ -333,11 +340,19 @@ __global__ void __launch_bounds__(kTCThreads, 1)
   float* sums = reinterpret_cast<float*>(base);
   if (!ok && threadIdx.x == 0) atomicOr(status, 8u);
   for (int c = 0; c < TN; c += 16) {
-    float v[16];
-    if (ok && nk > 0) tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c, v);
+    float v[16] = {};
+    if (ok && nk > 0) {
+      const uint32_t t = tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c;
+      tmem_ld16(t, v);
+      for (int q = 1; q < min(nk, Md::acc); ++q) {
+        float w[16];
+        tmem_ld16(t + (uint32_t)(q * TN), w);
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
-      sums[(warp * 32 + lane) * kTcRow + c + j] = nk > 0 ? v[j] : 0.f;
+        for (int j = 0; j < 16; ++j) v[j] += w[j];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) sums[(warp * 32 + lane) * kTcRow + c + j] = v[j];
   }
   tc_fence_before();
   cg::cluster_group cluster = cg::this_cluster();
@@ -345,7 +360,7 @@ __global__ void __launch_bounds__(kTCThreads, 1)
   if (warp == 0) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem),
-                 "r"((uint32_t)TN)
+                 "r"((uint32_t)(Md::acc * TN))
                  : "memory");
   }
   const int nz = (int)cluster.num_blocks(), z = (int)cluster.block_rank();
@@ -562,15 +577,26 @@ int gemm_tc_planes(Ctx& ctx, cudaStream_t st, int M, int N, int kp, bool bf16, c
     SM_CHECK(make_map(&mBl, bl, false, N, kp, TN));
   }
   const int tiles = ((M + TM - 1) / TM) * ((N + TN - 1) / TN);
-  // K over the CTAs of a cluster while the output has fewer tiles than SMs; beyond 16
-  // slabs a CTA a tile gets several clusters, whose sum is another launch
+  // K over the CTAs of a cluster while the output has fewer tiles than SMs.  The tensor
+  // cores truncate as they accumulate, an error that grows with the slabs an accumulator
+  // takes: two slabs to an accumulator, and beyond that several clusters to a tile,
+  // whose sum is another launch.
   const int sms = std::max(1, ctx.num_sms);
-  int nz = 1;
-  while (nz < kTcCluster && 2 * nz <= std::min(sms / tiles, ktiles)) nz *= 2;
-  int kt_per = (ktiles + nz - 1) / nz;
-  const int nzo =
-      nz < kTcCluster ? 1 : std::max(1, std::min(sms / (tiles * nz), kt_per / 8));
-  if (nzo > 1) kt_per = (ktiles + nz * nzo - 1) / (nz * nzo);
+  int nz = 1, nzo = 1, kt_per;
+  if (bf16) {  // ranges of two slabs and more, an accumulator each
+    const int want = std::max(1, std::min(sms / tiles, ktiles / 2));
+    kt_per = (ktiles + want - 1) / want;
+    const int ranges = (ktiles + kt_per - 1) / kt_per;
+    while (nz < kTcCluster && nz < ranges) nz *= 2;
+    nzo = (ranges + nz - 1) / nz;
+  } else {
+    while (nz < kTcCluster && 2 * nz <= std::min(sms / tiles, ktiles)) nz *= 2;
+    kt_per = (ktiles + nz - 1) / nz;
+    constexpr int most = 2 * TcMode<false>::acc;
+    if (nz == kTcCluster)
+      nzo = std::max(1, std::min(sms / (tiles * nz), (kt_per + most - 1) / most));
+    if (nzo > 1) kt_per = (ktiles + nz * nzo - 1) / (nz * nzo);
+  }
   OutT* part = nullptr;
   if (nzo > 1)
     SM_CHECK(ctx.scratch(sizeof(OutT) == 8 ? "tc.part" : "tc.part32", (size_t)nzo * M * N, &part));

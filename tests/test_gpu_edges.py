@@ -141,3 +141,24 @@ def test_sliced_complex_gemm_tiles(M, N, K):
         out = _gemm_c("sm_gemm_f64tc", opA, opB, A, B, M, N, K)
         err = np.max(np.abs(out - Aop @ Bop) / (np.abs(Aop) @ np.abs(Bop)))
         assert err <= 16 * np.sqrt(K) * 2.0**-53
+
+
+@pytest.mark.parametrize("M, N, K", [(64, 64, 1024), (65, 129, 1100), (127, 300, 250), (257, 128, 129), (128, 65, 17000)])
+def test_tf32_gemm_tiles(M, N, K):
+    """Tiles of 128 x 128 left ragged, clusters of 1 to 8 ranges of K and several clusters to a
+    tile: 2e-6 of the norm (three products of 11-bit parts); a row of
+    zeros stays one, and one with an infinity is not finite."""
+    from tests.test_gpu_tc import _gemm_f32
+
+    rng = np.random.default_rng(M + N + K)
+    A, B = rng.normal(size=(M, K)), rng.normal(size=(K, N))
+    A[3] = 0.0
+    ref = A @ B
+    out = _gemm_f32("N", "T", A, B.T.copy(), M, N, K)
+    assert np.linalg.norm(out - ref) <= 2e-6 * np.linalg.norm(ref)
+    assert (out[3] == 0.0).all()
+    A[3, 5] = np.inf
+    out = _gemm_f32("T", "N", A.T.copy(), B, M, N, K)
+    assert not np.isfinite(out[3]).any()
+    rest = np.delete(np.arange(M), 3)
+    assert np.linalg.norm((out - ref)[rest]) <= 2e-6 * np.linalg.norm(ref)
