@@ -1259,8 +1259,8 @@ int house_qr(Ctx& ctx, cudaStream_t st, T* Wt, int kw, int l, double thr_rel, T*
 // sorting, truncation) in one CTA with the matrix in shared memory.  The splits at
 // the ends of a chain have 2..48 rows; on the kernels above they pay a launch for
 // each phase and a grid barrier for each reflector and each round (32 x 32: 1.4 ms),
-// while one SM's FP64 pipe does a round of them in two microseconds (32 x 32: 0.70
-// ms; 0.91 ms with the angle's conversions, tests and small cosines in FP64).
+// while one SM's FP64 pipe does a round of them in two microseconds (32 x 32: 0.91
+// ms, 0.67 ms since the angles are FP32's, 0.52 ms with the FP32 stage).
 //
 // A pair of rows (and a column of the QR) belongs to 8 lanes: four pairs share the
 // FP64 instructions of a warp, so that their sums take three shuffle levels and the
@@ -1270,6 +1270,12 @@ int house_qr(Ctx& ctx, cudaStream_t st, T* Wt, int kw, int l, double thr_rel, T*
 constexpr int kSmallNT = 256;
 constexpr int kSmallRows = 48;           // rows of R at most
 constexpr size_t kSmallBytes = 160 * 1024;  // W in shared memory at most
+// Rows from which the FP32 stage pays: a call takes 114 us with it and without at 4 rows,
+// 135 and 154 at 8, 196 and 241 at 12, 235 and 308 at 16, 0.52 and 0.67 ms at 32, 1.10
+// and 1.59 ms at 48, complex 32 0.80 and 1.21 ms.  (Where the rows span 1e-12 most of
+// them are below FP32's reach: 32 rows 0.83 and 0.80 ms.)
+constexpr int kStageRows = 8;
+constexpr size_t kStageBytes = 220 * 1024;  // shared memory with the FP32 stage's at most
 constexpr double kSmallWork = 2e5;       // k^2 l (real) at most: a sweep of ~0.1 ms on one SM
 
 // Fits the kernel: W (kw x l) with its odd row stride in shared memory, and no
@@ -1289,10 +1295,150 @@ __device__ __forceinline__ double sum8(double x) {
   return x + __shfl_xor_sync(0xffffffffu, x, 1);
 }
 
+struct float2c {
+  float x, y;
+};
+__device__ __forceinline__ float sum8(float x) {
+  x += __shfl_xor_sync(0xffffffffu, x, 4);
+  x += __shfl_xor_sync(0xffffffffu, x, 2);
+  return x + __shfl_xor_sync(0xffffffffu, x, 1);
+}
+
+// Shared memory of the FP32 stage behind W (kw x ld): W2 (k x ld), X and E (k x k | 1),
+// and the FP32 rows [R | X].
+template <typename T>
+__host__ __device__ constexpr size_t small_stage_bytes(int k, int l) {
+  return sizeof(T) * ((size_t)k * (l | 1) + 2 * (size_t)k * (k | 1)) +
+         sizeof(T) / 2 * (size_t)k * ((l + k) | 1);
+}
+
+// W2 = X R for the rows R of W (k x l, stride ld): see k_split_small
+template <typename T>
+__device__ __forceinline__ T* small_fp32_stage(T* W, int ld, int kw, int k, int l) {
+  constexpr bool kCplx = sizeof(T) != sizeof(double);
+  using F = typename std::conditional<kCplx, float2c, float>::type;
+  const int tid = threadIdx.x, warp = tid >> 5, g8 = tid >> 3, l8 = tid & 7;
+  const int lk = k | 1, lf = (l + k) | 1;
+  T* W2 = W + (size_t)kw * ld;
+  T* X = W2 + (size_t)k * ld;
+  T* E = X + (size_t)k * lk;
+  F* R = reinterpret_cast<F*>(E + (size_t)k * lk);
+  __shared__ int wide;
+  for (int f = tid; f < k * (l + k); f += kSmallNT) {
+    const int i = f / (l + k), x = f % (l + k);
+    F v;
+    if constexpr (kCplx)
+      v = x < l ? F{(float)W[i * ld + x].re, (float)W[i * ld + x].im} : F{x - l == i ? 1.f : 0.f, 0.f};
+    else
+      v = x < l ? (float)W[i * ld + x] : (x - l == i ? 1.f : 0.f);
+    R[i * lf + x] = v;
+  }
+  const int kp = k + (k & 1), npairs = kp / 2;
+  for (int sweep = 0; sweep < 10; ++sweep) {
+    if (tid == 0) wide = 0;
+    __syncthreads();
+    for (int r = 0; r + 1 < kp; ++r) {
+      if (4 * warp < npairs) {
+        int p = g8 == 0 ? kp - 1 : (r + g8) % (kp - 1);
+        int q = g8 == 0 ? r : (r + kp - 1 - g8) % (kp - 1);
+        const bool on = g8 < npairs && p < k && q < k;
+        if (!on) p = q = 0;
+        if (p > q) { const int t = p; p = q; q = t; }
+        F* fp = R + p * lf;
+        F* fq = R + q * lf;
+        float a = 0.f, b = 0.f, gr = 0.f, gi = 0.f;
+        for (int x = l8; x < l; x += 8) {
+          const F u = fp[x], v = fq[x];
+          if constexpr (kCplx) {
+            a = fmaf(u.x, u.x, fmaf(u.y, u.y, a));
+            b = fmaf(v.x, v.x, fmaf(v.y, v.y, b));
+            gr = fmaf(u.x, v.x, fmaf(u.y, v.y, gr));
+            gi = fmaf(u.x, v.y, fmaf(-u.y, v.x, gi));
+          } else {
+            a = fmaf(u, u, a);
+            b = fmaf(v, v, b);
+            gr = fmaf(u, v, gr);
+          }
+        }
+        a = sum8(a);
+        b = sum8(b);
+        gr = sum8(gr);
+        if constexpr (kCplx) gi = sum8(gi);
+        const float g2 = fmaf(gr, gr, gi * gi), m = fmaxf(a, b);
+        // above cosine 1e-6 and the FP32 rounding of the larger row
+        if (on && g2 > 1e-12f * (a * b) && g2 > 1e-13f * (m * m) && g2 > 1e-36f) {
+          const float d = b - a, ga = sqrtf(g2);
+          const float t = copysignf(2.f * ga / (fabsf(d) + sqrtf(fmaf(d, d, 4.f * g2))), d);
+          const float c = rsqrtf(fmaf(t, t, 1.f)), sg = c * t / ga, sr = sg * gr, si = sg * gi;
+          for (int x = l8; x < l + k; x += 8) {  // p' = c p - conj(s) q, q' = s p + c q
+            const F u = fp[x], v = fq[x];
+            if constexpr (kCplx) {
+              fp[x] = F{fmaf(c, u.x, -fmaf(sr, v.x, si * v.y)), fmaf(c, u.y, -fmaf(sr, v.y, -si * v.x))};
+              fq[x] = F{fmaf(c, v.x, fmaf(sr, u.x, -si * u.y)), fmaf(c, v.y, fmaf(sr, u.y, si * u.x))};
+            } else {
+              fp[x] = fmaf(c, u, -sr * v);
+              fq[x] = fmaf(c, v, sr * u);
+            }
+          }
+          if (l8 == 0 && g2 > 1e-6f * (a * b)) wide = 1;
+        }
+      }
+      __syncthreads();
+    }
+    const int any = wide;
+    __syncthreads();
+    if (!any) break;  // quadratic: the rows left cosines of ~1e-6
+  }
+  for (int f = tid; f < k * k; f += kSmallNT) {
+    const F v = R[(f / k) * lf + l + f % k];
+    if constexpr (kCplx) X[(f / k) * lk + f % k] = T{(double)v.x, (double)v.y};
+    else X[(f / k) * lk + f % k] = (double)v;
+  }
+  __syncthreads();
+  for (int f = tid; f < k * k; f += kSmallNT) {
+    const int i = f / k, j = f % k;
+    T acc = S<T>::zero();
+    for (int x = 0; x < k; ++x) acc = S<T>::cfma(X[j * lk + x], X[i * lk + x], acc);
+    E[i * lk + j] = S<T>::fma(S<T>::from_real(-1.0), acc, S<T>::from_real(i == j ? 1.0 : 0.0));
+  }
+  __syncthreads();
+  T* Y = W2;  // I + E / 2 + 3/8 E^2, stride lk <= ld
+  for (int f = tid; f < k * k; f += kSmallNT) {
+    const int i = f / k, j = f % k;
+    T acc = S<T>::zero();
+    for (int x = 0; x < k; ++x) acc = S<T>::fma(E[i * lk + x], E[x * lk + j], acc);
+    acc = S<T>::fma(S<T>::from_real(0.5), E[i * lk + j], S<T>::scale(acc, 0.375));
+    Y[i * lk + j] = S<T>::fma(S<T>::from_real(i == j ? 1.0 : 0.0), S<T>::one(), acc);
+  }
+  __syncthreads();
+  for (int f = tid; f < k * k; f += kSmallNT) {
+    const int i = f / k, j = f % k;
+    T acc = S<T>::zero();
+    for (int x = 0; x < k; ++x) acc = S<T>::fma(Y[i * lk + x], X[x * lk + j], acc);
+    E[i * lk + j] = acc;
+  }
+  __syncthreads();
+  for (int f = tid; f < k * l; f += kSmallNT) {
+    const int i = f / l, c = f % l;
+    T acc = S<T>::zero();
+    for (int x = 0; x < k && x <= c; ++x) acc = S<T>::fma(E[i * lk + x], W[x * ld + c], acc);
+    W2[i * ld + c] = acc;
+  }
+  __syncthreads();
+  return W2;
+}
+
 // W (kw x l) = A^T (trans) or A (m x n row-major).  Writes the k = min(kw, l) rows
 // s_i v_i 2^-e to Wx (row-major, ld = l), the sorted values, their order, the rank
 // and the scaling exponent e; no grid barrier, no other CTA.
-template <typename T>
+//
+// The FP64 pipe bounds a round (two microseconds for 16 pairs, 33 operations of 64 clocks
+// and their latencies), so most of the iteration is FP32's: kStage runs the Jacobi on an
+// FP32 copy of R's rows with the rotations accumulated in X (0.25 us a round), makes X
+// orthonormal to FP64, X <- (I + E/2 + 3/8 E^2) X with E = I - X X^H ~ 1e-6, and goes on
+// from W = X R, orthogonal to FP32 level where R's rows are resolved by FP32: three or
+// four FP64 sweeps are left of eight to ten.
+template <typename T, bool kStage>
 __global__ void __launch_bounds__(kSmallNT)
     k_split_small(const T* __restrict__ A, int n_a, int trans, int kw, int l, double tol2,
                   int use_floor, double defl_rel, int max_sweeps, sm_strategy strat,
@@ -1394,6 +1540,7 @@ __global__ void __launch_bounds__(kSmallNT)
   for (int f = tid; f < k * l; f += kSmallNT)
     if (f % l < f / l) W[(f / l) * ld + f % l] = S<T>::zero();
   __syncthreads();
+  if constexpr (kStage) W = small_fp32_stage(W, ld, kw, k, l);
   // squared norm of row i by its group
   auto row_norm = [&](int i) {
     double a = 0.0;
@@ -1552,12 +1699,15 @@ int svd_split_xfree(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
     use_floor = strat.tolerance >= 16.0 * std::sqrt((double)k * l) * eps;
   const double tol = std::sqrt((double)l) * DBL_EPSILON;
   if (small_split_fits<T>(kw, l)) {
-    const size_t smem = sizeof(T) * (size_t)kw * (l | 1);
-    SM_CHECK(raise_smem_limit(k_split_small<T>, smem));
+    const size_t plain = sizeof(T) * (size_t)kw * (l | 1);
+    const size_t staged = plain + small_stage_bytes<T>(k, l);
+    const bool stage = k >= kStageRows && staged <= kStageBytes;
+    const size_t smem = stage ? staged : plain;
+    const auto kernel = stage ? k_split_small<T, true> : k_split_small<T, false>;
+    SM_CHECK(raise_smem_limit(kernel, smem));
     if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev0, st));
-    k_split_small<T><<<1, kSmallNT, smem, st>>>(A, n, want_u ? 1 : 0, kw, l, tol * tol,
-                                                use_floor ? 1 : 0, drel, kMaxSweeps, strat, Wx, perm,
-                                                s_sorted, res, wexp);
+    kernel<<<1, kSmallNT, smem, st>>>(A, n, want_u ? 1 : 0, kw, l, tol * tol, use_floor ? 1 : 0,
+                                      drel, kMaxSweeps, strat, Wx, perm, s_sorted, res, wexp);
     if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev1, st));
     note_launch();
     SM_CUDA_CHECK(cudaGetLastError());
