@@ -290,7 +290,7 @@ int newton_schulz_matrix(cudaStream_t st, const T* M, int k, T* F, double* dev);
 // close to orthogonal; `converged`: every pair passes the FP64 Jacobi's test
 // (tol2, use_floor, defl_rel as k_jacobi's), so that no Jacobi is needed.  Leaves
 // R as it is where the FP32 stage does not take the size or gives no basis.
-constexpr int kPrecondMinRows = 48;
+constexpr int kPrecondMinRows = 24;
 template <typename T>
 int precondition_rows(Ctx& ctx, cudaStream_t st, T* R, int k, int l, double tol2, int use_floor,
                       double defl_rel, bool* converged);

@@ -1276,16 +1276,25 @@ constexpr size_t kSmallBytes = 160 * 1024;  // W in shared memory at most
 // them are below FP32's reach: 32 rows 0.83 and 0.80 ms.)
 constexpr int kStageRows = 8;
 constexpr size_t kStageBytes = 220 * 1024;  // shared memory with the FP32 stage's at most
-constexpr double kSmallWork = 2e5;       // k^2 l (real) at most: a sweep of ~0.1 ms on one SM
+// Work (k^2 l) up to which one CTA is the faster: against the grid's Jacobi, and against
+// the FP32 start (svd_precond.cu) where that takes over.
+constexpr double kSmallWork = 2e5, kSmallWorkPrecond = 5e4;
 
-// Fits the kernel: W (kw x l) with its odd row stride in shared memory, and no
-// more work than one SM does in the time the grid's rounds take.
+// Fits the kernel: W (kw x l) with its odd row stride in shared memory, and no more work
+// than the other path's latencies leave time for.  Against the FP32 start: 24 rows 0.34
+// ms here and 0.49 there, 32 rows 0.49 and 0.54 (spanning 1e-12 0.83 and 0.98, in groups
+// of equal values 0.57 and 1.29), 40 rows 0.77 and 0.60, 48 rows 1.10 and 0.65; complex
+// 24 rows 0.53 and 0.58, 32 rows 0.80 and 0.66.  A context that shares the device has no
+// grid for the FP64 QR before that start and keeps the larger limit.
 template <typename T>
-bool small_split_fits(int kw, int l) {
+bool small_split_fits(const Ctx& ctx, int kw, int l) {
   const int k = std::min(kw, l);
-  const double work = (double)k * k * l * (sizeof(T) == sizeof(double) ? 1.0 : 4.0);
-  return k <= kSmallRows && work <= kSmallWork &&
-         sizeof(T) * (size_t)kw * (l | 1) <= kSmallBytes;
+  const bool cplx_t = sizeof(T) != sizeof(double);
+  const double work = (double)k * k * l;
+  const bool fast = k < kPrecondMinRows || ctx.concurrent
+                        ? work * (cplx_t ? 4.0 : 1.0) <= kSmallWork
+                        : work * (cplx_t ? 2.5 : 1.0) <= kSmallWorkPrecond;
+  return k <= kSmallRows && fast && sizeof(T) * (size_t)kw * (l | 1) <= kSmallBytes;
 }
 
 // sum over the 8 lanes of a group
@@ -1698,7 +1707,7 @@ int svd_split_xfree(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   else if (strat.method == SM_RELATIVE_SINGULAR_VALUE)
     use_floor = strat.tolerance >= 16.0 * std::sqrt((double)k * l) * eps;
   const double tol = std::sqrt((double)l) * DBL_EPSILON;
-  if (small_split_fits<T>(kw, l)) {
+  if (small_split_fits<T>(ctx, kw, l)) {
     const size_t plain = sizeof(T) * (size_t)kw * (l | 1);
     const size_t staged = plain + small_stage_bytes<T>(k, l);
     const bool stage = k >= kStageRows && staged <= kStageBytes;

@@ -53,10 +53,12 @@ def check_split(A, tol=1e-12, maxb=10**6, atol=1e-12):
 @pytest.mark.parametrize("m, n, cplx", [
     (1, 1, False), (1, 1, True), (1, 7, False), (2, 2, True), (3, 2, False), (5, 4, True),
     (8, 9, False), (31, 33, False), (32, 32, True), (33, 31, False), (47, 64, False),
-    # the last that one CTA takes, and the first that it does not: 48 rows, the
-    # work of 48^2 86 (complex 36^2 38), the shared memory of 9 x 2275
+    # the last that one CTA takes, and the first that it does not: the work of 23^2 378
+    # and, where the FP32 start takes over, 36^3 and 24^2 86 (complex 23^2 94, 27^3), the
+    # shared memory of 9 x 2275
+    (23, 378, False), (379, 23, False), (36, 36, False), (37, 37, False), (24, 86, False), (87, 24, False),
+    (23, 94, True), (95, 23, True), (27, 27, True), (28, 28, True), (9, 2275, False), (2277, 9, False),
     (48, 86, False), (87, 48, False), (36, 38, True), (39, 36, True), (49, 49, False),
-    (9, 2275, False), (2277, 9, False),
 ])
 def test_small_fp64_splits(m, n, cplx):
     rng = np.random.default_rng(100 * m + n)
