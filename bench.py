@@ -882,8 +882,8 @@ def main():
     }
     roofline = dict(fp64_roof)
     if stt["cluster_ms"] > kms and stt["mixed_splits"]:
-        # the mixed forms' dominant kernel: the FP32 cluster factorisation, one launch per mixed
-        # split on the 16 SMs of one thread-block cluster; bound by latency (barriers and each
+        # the mixed forms' dominant kernels: the FP32 cluster factorisation, a QR and a Jacobi launch
+        # per mixed split on the SMs of one thread-block cluster; bound by latency (each step's and
         # pair step's dependent chain), so its FP32 rate is reported against the SIMT peak of
         # those 16 SMs and of the whole GPU at the sampled SM clock
         nl = stt["mixed_splits"]
@@ -894,8 +894,8 @@ def main():
         fp32_sm = 128 * 2 * mhz * 1e6  # FP32 FMA lanes per SM x 2 flops x clock
         n_sm = torch.cuda.get_device_properties(0).multi_processor_count
         roofline = {
-            "bound": "latency", "kernel": "k_split_cluster (FP32 blocked QR + block-cyclic "
-                                          "one-sided Jacobi, 16-CTA cluster)",
+            "bound": "latency", "kernel": "k_qr_cluster + k_jacobi_cluster (FP32 QR, "
+                                          "block-cyclic one-sided Jacobi, one cluster)",
             "achieved": alg / 1e12, "peak": n_sm * fp32_sm / 1e12, "unit": "TFLOP/s",
             "frac": alg / (n_sm * fp32_sm),
             "work_convention": "algorithmic SVD flops 4mn^2 + 8n^3 per m x n split (m >= n), "

@@ -187,7 +187,7 @@ int tc_status_check(Ctx& ctx, cudaStream_t st);
 // --- gemm_oz.cu -------------------------------------------------------------
 // Real GEMM at FP64 accuracy on the BF16 tensor cores (error-free slicing of
 // the operands into 7-bit integer slices); gemm_ctx<double> uses it in the
-// mixed forms (ctx.fp64_tc) for shapes gemm_oz_eligible accepts.
+// mixed forms (ctx.fp64_tc) where it is the faster (slices_pay in gemm.cu).
 bool gemm_oz_eligible(int M, int N, int K);
 // the three products of a complex one: T = [Ar Br; Ai Bi; (Ar + Ai)(Br + Bi)], 3 M x N
 int gemm_oz_3m(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, const cplx* A,

@@ -2,8 +2,11 @@
 //
 // The reference calls LAPACK gesdd (cython/svd.pxi:35-83) and then truncates
 // the singular values in place (cython/truncation.pxi:251-334).  Here the SVD
-// is a one-sided (Hestenes) Jacobi iteration in FP64, run as ONE cooperative
-// persistent kernel per matrix:
+// is a one-sided (Hestenes) Jacobi iteration in FP64.  A split's small matrices run
+// it in one CTA (k_split_small); larger ones are reduced by a Householder QR and
+// brought to FP64 orthogonality by an FP32 start and matrix products
+// (svd_precond.cu), and only what that leaves, and the SVD that also wants the
+// short-side vectors, runs it as ONE cooperative persistent kernel per matrix:
 //
 //  * the k = min(m,n) vectors of the short side (rows of A if m <= n, rows of
 //    A^T otherwise) are stored contiguously, k x l with l = max(m,n);
@@ -1001,8 +1004,9 @@ __global__ void __launch_bounds__(NT) k_house_qr(T* Wt, int k, int l, double thr
 // holds a step whose trailing block is at most thr_rel |W|_F^2, and that step is
 // the rank.  What bounds a step is its chain: the barrier, the reflector through
 // L2, two passes over the column and two FP64 warp sums, one reciprocal root.
-// 174 x 190: 0.84 ms with columns streamed through L2 and a test per step, see
-// the launcher for the time now.
+// 174 x 190 0.80 ms, rank 130 of 256 x 256 0.69 ms, complex 128 x 128 0.69 ms (with
+// columns streamed through L2 and a test per step 174 x 190 took 0.84 ms, and more
+// the more rows a column has).
 constexpr int kQrBatch = 4;
 template <typename T, int NT, int E>
 __global__ void __launch_bounds__(NT) k_house_qr_reg(T* Wt, int k, int l, double thr_rel, T* vbuf,

@@ -164,3 +164,104 @@ def test_tf32_gemm_tiles(M, N, K):
     assert not np.isfinite(out[3]).any()
     rest = np.delete(np.arange(M), 3)
     assert np.linalg.norm((out - ref)[rest]) <= 2e-6 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("cplx", [False, True])
+@pytest.mark.parametrize("M, N, K", [(1, 1, 1), (15, 17, 16), (16, 33, 17), (31, 32, 129), (33, 200, 31),
+                                     (174, 174, 190), (300, 7, 2000), (600, 600, 40)])
+def test_fp64_gemm_tiles(M, N, K, cplx):
+    """Tiles of 16 and 32 and one to eight ranges of K, every operand rule: (K + 2) u of |A||B|,
+    twice that for complex products."""
+    rng = np.random.default_rng(M + N + K)
+    A, B = gaussian(rng, (M, K), cplx), gaussian(rng, (K, N), cplx)
+    ref, scale = A @ B, np.abs(A) @ np.abs(B)
+    op = {0: lambda x: x, 1: lambda x: x.T.copy(), 2: lambda x: x.conj().T.copy()}
+    for opA, opB in [(0, 0), (1, 2), (2, 1), (0, 2)]:
+        out = to_np(core._gemm(op[opA](A), opA, op[opB](B), opB))
+        assert np.max(np.abs(out - ref) / scale) <= (2 + 2 * cplx) * (K + 2) * 2.0**-53
+
+
+@pytest.mark.parametrize("m, n, kind, cplx", [
+    (24, 300, "flat", False), (49, 64, "flat", True), (64, 65, "graded", False), (100, 200, "flat", False),
+    (200, 100, "graded", False), (129, 130, "groups", False), (96, 128, "groups", True),
+    (120, 150, "rank", False), (128, 100, "rank", True), (33, 257, "graded", True),
+])
+def test_fp64_splits_through_the_fp32_start(m, n, kind, cplx):
+    """Flat spectra, spectra that span 1e-12 (several FP32 levels), groups of equal values (left
+    to the Jacobi) and rank-deficient matrices, square, wide and tall."""
+    rng = np.random.default_rng(m + n)
+    k = min(m, n)
+    s = {"flat": np.geomspace(1.0, 0.03, k), "graded": np.geomspace(1.0, 1e-12, k),
+         "groups": np.repeat(np.geomspace(1.0, 0.01, k // 8 + 1), 8)[:k],
+         "rank": np.geomspace(1.0, 1e-3, k // 3)}[kind]
+    check_split(matrix(rng, m, n, s, cplx))
+
+
+@pytest.mark.parametrize("m, n, cplx", [
+    (24, 24, False), (64, 65, False), (129, 128, False), (257, 300, False), (96, 700, False), (512, 514, False),
+    (25, 24, True), (128, 129, True), (256, 200, True), (300, 310, True),
+])
+def test_mixed_splits_at_the_cluster_sizes(m, n, cplx):
+    """Where the FP32 stage changes its cluster or its registers: the oracle's rank (a gap of
+    1e-8), an orthogonal factor to 1e-12, and the kept part to 2e-6 (the coupling of a kept and
+    a dropped row that the split accepts is 1e-6)."""
+    rng = np.random.default_rng(m + n)
+    k = min(m, n) // 2
+    A = matrix(rng, m, n, np.concatenate([np.geomspace(1.0, 0.1, k), np.full(k // 2, 1e-9)]), cplx)
+    st = sg.Strategy(tolerance=1e-12, max_bond_dimension=k)
+    ost = so.Strategy(tolerance=1e-12, max_bond_dimension=k)
+    sg.set_precision("mixed")
+    try:
+        L, R, _ = core._left_orth_2site(A.reshape(m, 1, 1, n), st)
+    finally:
+        sg.set_precision("fp64")
+    oL, oR, _ = so.left_orth_2site(A.reshape(m, 1, 1, n), ost)
+    assert L.shape[-1] == oL.shape[-1] == k
+    L, R = to_np(L).reshape(m, k), to_np(R).reshape(k, n)
+    assert np.abs(L.conj().T @ L - np.eye(k)).max() <= 1e-12
+    P = oL.reshape(m, k) @ oR.reshape(k, n)
+    assert np.linalg.norm(L @ R - P) <= 2e-6 * np.linalg.norm(P)
+
+
+@pytest.mark.parametrize("a, g, c, e", [(1, 1, 3, 3), (9, 33, 4, 9), (33, 8, 70, 5), (31, 40, 5, 17)])
+def test_two_site_matvec_lists(a, g, c, e):
+    """More than 8 output bonds, more than 256 inputs to an output (2 x 2 x 70), rectangular
+    environments, sparse MPO tensors: sums of a c p1 p2 e terms, 1e-12 of the largest entry."""
+    from oracle import dmrg_oracle as do
+    from seemps2_gb300 import dmrg
+
+    rng = np.random.default_rng(a + g + c + e)
+    b, f = a + 2, g + 1
+    L, R = rng.normal(size=(a, c, b)), rng.normal(size=(g, e, f))
+    H = rng.normal(size=(c, 2, 2, 2, 2, e)) * (rng.random((c, 2, 2, 2, 2, e)) < 0.3)
+    v = rng.normal(size=(b, 2, 2, f))
+    ref = do.two_site_matvec(L, H, R, v)
+    scale = do.two_site_matvec(abs(L), abs(H), abs(R), abs(v)).max()
+    out = to_np(dmrg.two_site_matvec(L, H, R, v, "fp64"))
+    assert np.abs(out - ref).max() <= 1e-12 * scale
+
+
+def test_lanczos_of_tiny_operators():
+    """Four unknowns and a run of thirty steps (it breaks down at four), and an eigenvector as
+    the start (it breaks down at one): the lowest eigenvalue to 1e-12 of the norm."""
+    from seemps2_gb300 import dmrg
+
+    rng = np.random.default_rng(2)
+    h = rng.normal(size=(4, 4))
+    h = h + h.T
+    H = h.reshape(2, 2, 2, 2).transpose(0, 2, 1, 3).reshape(1, 2, 2, 2, 2, 1)
+    one = np.ones((1, 1, 1))
+    w, u = np.linalg.eigh(h)
+    for start in (rng.normal(size=4), u[:, 0]):
+        ev, vec, _ = dmrg.lanczos_ground_state(one, H, one, start.reshape(1, 2, 2, 1), krylov=30)
+        assert abs(ev - w[0]) <= 1e-12 * np.abs(w).max()
+        assert abs(abs(to_np(vec).ravel() @ u[:, 0]) - 1.0) <= 1e-12
+
+
+@pytest.mark.parametrize("batch", [1, 31, 33, 257])
+def test_mlp_gradients_of_ragged_batches(batch):
+    """One row, and a row short of and beyond the 32 x 32 tiles: the bars of the other gradient
+    tests (1e-4 of the largest entry)."""
+    from tests.test_gpu_learned import test_gradients_match_oracle
+
+    test_gradients_match_oracle(batch)
