@@ -1264,7 +1264,8 @@ int house_qr(Ctx& ctx, cudaStream_t st, T* Wt, int kw, int l, double thr_rel, T*
 // the ends of a chain have 2..48 rows; on the kernels above they pay a launch for
 // each phase and a grid barrier for each reflector and each round (32 x 32: 1.4 ms),
 // while one SM's FP64 pipe does a round of them in two microseconds (32 x 32: 0.91
-// ms, 0.67 ms since the angles are FP32's, 0.52 ms with the FP32 stage).
+// ms, 0.67 ms since the angles are FP32's, 0.52 ms with the FP32 stage, 0.41 ms with a
+// pair's rows in registers).
 //
 // A pair of rows (and a column of the QR) belongs to 8 lanes: four pairs share the
 // FP64 instructions of a warp, so that their sums take three shuffle levels and the
@@ -1275,9 +1276,8 @@ constexpr int kSmallNT = 256;
 constexpr int kSmallRows = 48;           // rows of R at most
 constexpr size_t kSmallBytes = 160 * 1024;  // W in shared memory at most
 // Rows from which the FP32 stage pays: a call takes 114 us with it and without at 4 rows,
-// 135 and 154 at 8, 196 and 241 at 12, 235 and 308 at 16, 0.52 and 0.67 ms at 32, 1.10
-// and 1.59 ms at 48, complex 32 0.80 and 1.21 ms.  (Where the rows span 1e-12 most of
-// them are below FP32's reach: 32 rows 0.83 and 0.80 ms.)
+// 135 and 154 at 8, 165 and 241 at 12, 193 and 308 at 16, 0.41 and 0.67 ms at 32, complex
+// 24 0.50 and 0.75 ms.
 constexpr int kStageRows = 8;
 constexpr size_t kStageBytes = 220 * 1024;  // shared memory with the FP32 stage's at most
 // Work (k^2 l) up to which one CTA is the faster: against the grid's Jacobi, and against
@@ -1285,10 +1285,10 @@ constexpr size_t kStageBytes = 220 * 1024;  // shared memory with the FP32 stage
 constexpr double kSmallWork = 2e5, kSmallWorkPrecond = 5e4;
 
 // Fits the kernel: W (kw x l) with its odd row stride in shared memory, and no more work
-// than the other path's latencies leave time for.  Against the FP32 start: 24 rows 0.34
-// ms here and 0.49 there, 32 rows 0.49 and 0.54 (spanning 1e-12 0.83 and 0.98, in groups
-// of equal values 0.57 and 1.29), 40 rows 0.77 and 0.60, 48 rows 1.10 and 0.65; complex
-// 24 rows 0.53 and 0.58, 32 rows 0.80 and 0.66.  A context that shares the device has no
+// than the other path's latencies leave time for.  Against the FP32 start: 24 rows 0.31
+// ms here and 0.49 there, 32 rows 0.41 and 0.54 (spanning 1e-12 0.59 and 0.98, in groups
+// of equal values 0.48 and 1.29); before the rows went to registers 40 rows 0.77 and 0.60,
+// 48 rows 1.10 and 0.65, complex 24 rows 0.53 and 0.58, 32 rows 0.80 and 0.66.  A context that shares the device has no
 // grid for the FP64 QR before that start and keeps the larger limit.
 template <typename T>
 bool small_split_fits(const Ctx& ctx, int kw, int l) {
@@ -1315,6 +1315,123 @@ __device__ __forceinline__ float sum8(float x) {
   x += __shfl_xor_sync(0xffffffffu, x, 4);
   x += __shfl_xor_sync(0xffffffffu, x, 2);
   return x + __shfl_xor_sync(0xffffffffu, x, 1);
+}
+
+// a / b and 1 / sqrt(a) to a few FP32 roundings (the angle of an FP32 rotation)
+__device__ __forceinline__ float div_fast(float a, float b) { return __fdividef(a, b); }
+
+// One pair of FP32 rows [R | X] on 8 lanes: rotates them (all of l + k entries) if their
+// cosine over the first l is above 1e-6 and the FP32 rounding of the larger row; true if
+// it was above 1e-3.  NE > 0: l + k <= 8 NE, rows in registers from the sums to the stores
+// (read twice and stored entry by entry a round took 1400 clocks whatever the size).
+template <bool kCplx, int NE, typename F>
+__device__ __forceinline__ bool small_pair32(F* fp, F* fq, int l, int n, int l8, bool on) {
+  constexpr int NR = NE > 0 ? NE : 1;
+  F u[NR], v[NR];
+  float a = 0.f, b = 0.f, gr = 0.f, gi = 0.f;
+  auto add = [&](const F& p, const F& q) {
+    if constexpr (kCplx) {
+      a = fmaf(p.x, p.x, fmaf(p.y, p.y, a));
+      b = fmaf(q.x, q.x, fmaf(q.y, q.y, b));
+      gr = fmaf(p.x, q.x, fmaf(p.y, q.y, gr));
+      gi = fmaf(p.x, q.y, fmaf(-p.y, q.x, gi));
+    } else {
+      a = fmaf(p, p, a);
+      b = fmaf(q, q, b);
+      gr = fmaf(p, q, gr);
+    }
+  };
+  if constexpr (NE > 0) {
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      const int x = l8 + 8 * e;
+      u[e] = on && x < n ? fp[x] : F{};
+      v[e] = on && x < n ? fq[x] : F{};
+    }
+#pragma unroll
+    for (int e = 0; e < NE; ++e)
+      if (l8 + 8 * e < l) add(u[e], v[e]);
+  } else {
+    for (int x = l8; on && x < l; x += 8) add(fp[x], fq[x]);
+  }
+  a = sum8(a);
+  b = sum8(b);
+  gr = sum8(gr);
+  if constexpr (kCplx) gi = sum8(gi);
+  const float g2 = fmaf(gr, gr, gi * gi), m = fmaxf(a, b);
+  if (!(on && g2 > 1e-12f * (a * b) && g2 > 1e-13f * (m * m) && g2 > 1e-36f)) return false;
+  const float d = b - a, ig = rsqrtf(g2), q2 = fmaf(d, d, 4.f * g2);
+  const float t = copysignf(div_fast(2.f * g2 * ig, fabsf(d) + q2 * rsqrtf(q2)), d);
+  const float c = rsqrtf(fmaf(t, t, 1.f)), sg = c * t * ig, sr = sg * gr, si = sg * gi;
+  auto turn = [&](F& p, F& q) {  // p' = c p - conj(s) q, q' = s p + c q
+    const F x = p, y = q;
+    if constexpr (kCplx) {
+      p = F{fmaf(c, x.x, -fmaf(sr, y.x, si * y.y)), fmaf(c, x.y, -fmaf(sr, y.y, -si * y.x))};
+      q = F{fmaf(c, y.x, fmaf(sr, x.x, -si * x.y)), fmaf(c, y.y, fmaf(sr, x.y, si * x.x))};
+    } else {
+      p = fmaf(c, x, -sr * y);
+      q = fmaf(c, y, sr * x);
+    }
+  };
+  if constexpr (NE > 0) {
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      const int x = l8 + 8 * e;
+      turn(u[e], v[e]);
+      if (x < n) {
+        fp[x] = u[e];
+        fq[x] = v[e];
+      }
+    }
+  } else {
+    for (int x = l8; x < n; x += 8) turn(fp[x], fq[x]);
+  }
+  return g2 > 1e-6f * (a * b);
+}
+
+// One pair of FP64 rows on 8 lanes likewise (l <= 8 NE in registers): rotates it if the
+// Jacobi's test says so; the norms after it in na, nb.
+template <typename T, int NE>
+__device__ __forceinline__ bool small_pair64(T* rp, T* rq, int l, int l8, bool on, double a,
+                                             double b, FloatExp tol2, FloatExp tiny2, double& na,
+                                             double& nb) {
+  constexpr bool kCplx = sizeof(T) != sizeof(double);
+  constexpr int NR = NE > 0 ? NE : 1;
+  T u[NR], v[NR], g = S<T>::zero();
+  if constexpr (NE > 0) {
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      const int x = l8 + 8 * e;
+      u[e] = on && x < l ? rp[x] : S<T>::zero();
+      v[e] = on && x < l ? rq[x] : S<T>::zero();
+    }
+#pragma unroll
+    for (int e = 0; e < NE; ++e) g = S<T>::cfma(u[e], v[e], g);
+  } else {
+    for (int x = l8; on && x < l; x += 8) g = S<T>::cfma(rp[x], rq[x], g);
+  }
+  double gr, gi, c, sn, e_r, e_i;
+  gamma_parts(g, gr, gi);
+  gr = sum8(gr);
+  if constexpr (kCplx) gi = sum8(gi);
+  if (!(on && jacobi_rotation<kCplx>(a, b, gr, gi, tol2, tiny2, c, sn, e_r, e_i, na, nb)))
+    return false;
+  Rot<T> R;
+  R.set(c, sn, e_r, e_i);
+  if constexpr (NE > 0) {
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      const int x = l8 + 8 * e;
+      R.apply(u[e], v[e]);
+      if (x < l) {
+        rp[x] = u[e];
+        rq[x] = v[e];
+      }
+    }
+  } else {
+    for (int x = l8; x < l; x += 8) R.apply(rp[x], rq[x]);
+  }
+  return true;
 }
 
 // Shared memory of the FP32 stage behind W (kw x ld): W2 (k x ld), X and E (k x k | 1),
@@ -1350,51 +1467,21 @@ __device__ __forceinline__ T* small_fp32_stage(T* W, int ld, int kw, int k, int 
   for (int sweep = 0; sweep < 10; ++sweep) {
     if (tid == 0) wide = 0;
     __syncthreads();
+    int p0 = g8 == 0 ? kp - 1 : g8, q0 = g8 == 0 ? 0 : kp - 1 - g8;  // both advance with r
     for (int r = 0; r + 1 < kp; ++r) {
       if (4 * warp < npairs) {
-        int p = g8 == 0 ? kp - 1 : (r + g8) % (kp - 1);
-        int q = g8 == 0 ? r : (r + kp - 1 - g8) % (kp - 1);
-        const bool on = g8 < npairs && p < k && q < k;
-        if (!on) p = q = 0;
-        if (p > q) { const int t = p; p = q; q = t; }
+        const bool on = g8 < npairs && p0 < k && q0 < k;
+        const int p = on ? min(p0, q0) : 0, q = on ? max(p0, q0) : 0;
         F* fp = R + p * lf;
         F* fq = R + q * lf;
-        float a = 0.f, b = 0.f, gr = 0.f, gi = 0.f;
-        for (int x = l8; x < l; x += 8) {
-          const F u = fp[x], v = fq[x];
-          if constexpr (kCplx) {
-            a = fmaf(u.x, u.x, fmaf(u.y, u.y, a));
-            b = fmaf(v.x, v.x, fmaf(v.y, v.y, b));
-            gr = fmaf(u.x, v.x, fmaf(u.y, v.y, gr));
-            gi = fmaf(u.x, v.y, fmaf(-u.y, v.x, gi));
-          } else {
-            a = fmaf(u, u, a);
-            b = fmaf(v, v, b);
-            gr = fmaf(u, v, gr);
-          }
-        }
-        a = sum8(a);
-        b = sum8(b);
-        gr = sum8(gr);
-        if constexpr (kCplx) gi = sum8(gi);
-        const float g2 = fmaf(gr, gr, gi * gi), m = fmaxf(a, b);
-        // above cosine 1e-6 and the FP32 rounding of the larger row
-        if (on && g2 > 1e-12f * (a * b) && g2 > 1e-13f * (m * m) && g2 > 1e-36f) {
-          const float d = b - a, ga = sqrtf(g2);
-          const float t = copysignf(2.f * ga / (fabsf(d) + sqrtf(fmaf(d, d, 4.f * g2))), d);
-          const float c = rsqrtf(fmaf(t, t, 1.f)), sg = c * t / ga, sr = sg * gr, si = sg * gi;
-          for (int x = l8; x < l + k; x += 8) {  // p' = c p - conj(s) q, q' = s p + c q
-            const F u = fp[x], v = fq[x];
-            if constexpr (kCplx) {
-              fp[x] = F{fmaf(c, u.x, -fmaf(sr, v.x, si * v.y)), fmaf(c, u.y, -fmaf(sr, v.y, -si * v.x))};
-              fq[x] = F{fmaf(c, v.x, fmaf(sr, u.x, -si * u.y)), fmaf(c, v.y, fmaf(sr, u.y, si * u.x))};
-            } else {
-              fp[x] = fmaf(c, u, -sr * v);
-              fq[x] = fmaf(c, v, sr * u);
-            }
-          }
-          if (l8 == 0 && g2 > 1e-6f * (a * b)) wide = 1;
-        }
+        const int n = l + k;
+        const bool w = n <= 16   ? small_pair32<kCplx, 2>(fp, fq, l, n, l8, on)
+                       : n <= 32 ? small_pair32<kCplx, 4>(fp, fq, l, n, l8, on)
+                       : n <= 64 ? small_pair32<kCplx, 8>(fp, fq, l, n, l8, on)
+                                 : small_pair32<kCplx, 0>(fp, fq, l, n, l8, on);
+        if (w && l8 == 0) wide = 1;
+        if (g8 != 0) p0 = p0 + 1 == kp - 1 ? 0 : p0 + 1;
+        q0 = q0 + 1 == kp - 1 ? 0 : q0 + 1;
       }
       __syncthreads();
     }
@@ -1447,7 +1534,7 @@ __device__ __forceinline__ T* small_fp32_stage(T* W, int ld, int kw, int k, int 
 //
 // The FP64 pipe bounds a round (two microseconds for 16 pairs, 33 operations of 64 clocks
 // and their latencies), so most of the iteration is FP32's: kStage runs the Jacobi on an
-// FP32 copy of R's rows with the rotations accumulated in X (0.25 us a round), makes X
+// FP32 copy of R's rows with the rotations accumulated in X (0.3 us a round), makes X
 // orthonormal to FP64, X <- (I + E/2 + 3/8 E^2) X with E = I - X X^H ~ 1e-6, and goes on
 // from W = X R, orthogonal to FP32 level where R's rows are resolved by FP32: three or
 // four FP64 sweeps are left of eight to ten.
@@ -1594,41 +1681,28 @@ __global__ void __launch_bounds__(kSmallNT)
       ftiny2 = split_abs(tiny * tiny);
     }
     const int ka = nact, kp = ka + (ka & 1), npairs = kp / 2;
+    int p0 = g8 == 0 ? kp - 1 : g8, q0 = g8 == 0 ? 0 : kp - 1 - g8;  // both advance with r
     for (int r = 0; r + 1 < kp; ++r) {
       if (4 * warp < npairs) {  // npairs <= 24: one pass of the 32 groups
-        const int t = g8;
-        int p = t == 0 ? kp - 1 : (r + t) % (kp - 1);
-        int q = t == 0 ? r : (r + kp - 1 - t) % (kp - 1);
-        const bool on = t < npairs && p < ka && q < ka;
-        p = on ? act[p] : 0;
-        q = on ? act[q] : 0;
-        if (p > q) { const int tmp = p; p = q; q = tmp; }
+        const bool on = g8 < npairs && p0 < ka && q0 < ka;
+        const int ap = on ? act[p0] : 0, aq = on ? act[q0] : 0;
+        const int p = min(ap, aq), q = max(ap, aq);
         T* rp = W + p * ld;
         T* rq = W + q * ld;
-        T g = S<T>::zero();
-        for (int x = l8; x < l; x += 8)
-          if (on) g = S<T>::cfma(rp[x], rq[x], g);
-        double gr, gi;
-        gamma_parts(g, gr, gi);
-        gr = sum8(gr);
-        if constexpr (kCplx) gi = sum8(gi);
+        double na, nb;
         const double a = nrm[p], b = nrm[q];
-        double c, sn, e_r, e_i, na, nb;
-        if (on && jacobi_rotation<kCplx>(a, b, gr, gi, ftol2, ftiny2, c, sn, e_r, e_i, na, nb)) {
-          Rot<T> R;
-          R.set(c, sn, e_r, e_i);
-          for (int x = l8; x < l; x += 8) {
-            T u = rp[x], v = rq[x];
-            R.apply(u, v);
-            rp[x] = u;
-            rq[x] = v;
-          }
-          if (l8 == 0) {
-            nrm[p] = na;
-            nrm[q] = nb;
-            rotated = 1;
-          }
+        const bool rot =
+            l <= 16   ? small_pair64<T, 2>(rp, rq, l, l8, on, a, b, ftol2, ftiny2, na, nb)
+            : l <= 32 ? small_pair64<T, 4>(rp, rq, l, l8, on, a, b, ftol2, ftiny2, na, nb)
+            : l <= 48 ? small_pair64<T, 6>(rp, rq, l, l8, on, a, b, ftol2, ftiny2, na, nb)
+                      : small_pair64<T, 0>(rp, rq, l, l8, on, a, b, ftol2, ftiny2, na, nb);
+        if (rot && l8 == 0) {
+          nrm[p] = na;
+          nrm[q] = nb;
+          rotated = 1;
         }
+        if (g8 != 0) p0 = p0 + 1 == kp - 1 ? 0 : p0 + 1;
+        q0 = q0 + 1 == kp - 1 ? 0 : q0 + 1;
       }
       __syncthreads();
     }
