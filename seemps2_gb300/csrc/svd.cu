@@ -1288,8 +1288,9 @@ constexpr double kSmallWork = 2e5, kSmallWorkPrecond = 5e4;
 // than the other path's latencies leave time for.  Against the FP32 start: 24 rows 0.31
 // ms here and 0.49 there, 32 rows 0.41 and 0.54 (spanning 1e-12 0.59 and 0.98, in groups
 // of equal values 0.48 and 1.29); before the rows went to registers 40 rows 0.77 and 0.60,
-// 48 rows 1.10 and 0.65, complex 24 rows 0.53 and 0.58, 32 rows 0.80 and 0.66.  A context that shares the device has no
-// grid for the FP64 QR before that start and keeps the larger limit.
+// 48 rows 1.10 and 0.65, complex 24 rows 0.53 and 0.58, 32 rows 0.80 and 0.66.  A
+// context that shares the device has no grid for the FP64 QR before that start and
+// keeps the larger limit.
 template <typename T>
 bool small_split_fits(const Ctx& ctx, int kw, int l) {
   const int k = std::min(kw, l);
