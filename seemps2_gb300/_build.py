@@ -33,7 +33,7 @@ def nvcc() -> str:
 
 
 def _newest_dep() -> float:
-    deps = glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(INCLUDE, "*.h"))
+    deps = [p for d in (CSRC, INCLUDE) for e in ("*.cuh", "*.h") for p in glob.glob(os.path.join(d, e))]
     return max((os.path.getmtime(p) for p in deps), default=0.0)
 
 

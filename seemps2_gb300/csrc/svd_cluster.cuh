@@ -129,6 +129,10 @@ __device__ __forceinline__ void cl_mbar_expect(uint64_t* b, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(cl_smem(b)), "r"(bytes)
                : "memory");
 }
+// one arrival on an mbarrier of any CTA of the cluster (a cl_map'ed address)
+__device__ __forceinline__ void cl_mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ bool cl_mbar_try(uint64_t* b, uint32_t parity) {
   uint32_t ok;
   asm volatile(

@@ -24,7 +24,11 @@
 //     its new blocks: no cluster barrier.  Two buffers per block are enough: a CTA
 //     has sent round g's rows only after all its warps are done with the buffers of
 //     round g - 1, and its neighbours send into those only after they have received
-//     those rows (so a copy's source is free as well).
+//     rows of it.  Those are not always the rows whose place they take (a top goes up
+//     while its place is filled from below), and a copy is known to have read its
+//     source only where it arrives: whoever has received a round's rows tells the CTAs
+//     that write over their sources (an mbarrier each, sync_rules.h), which wait for it
+//     a whole block round later.
 // The cluster meets once per sweep, to agree on that flag.  A sweep takes 29 us on 64
 // rows of 64, 61 us on 153 rows of 256 and 206 us on 337 rows of 512 (with 16 CTAs
 // always, three sums per pair, copies through mailboxes and a cluster barrier per
@@ -35,6 +39,7 @@
 #include <cmath>
 
 #include "svd_cluster.cuh"
+#include "sync_rules.h"
 
 namespace cg = cooperative_groups;
 
@@ -54,6 +59,7 @@ constexpr float kTinyG2 = 1e-36f;
 
 struct JacShared {
   uint64_t bar[2];             // this CTA's new blocks, by the round's parity
+  uint64_t clear[2];           // a round's copies out of the buffers this CTA writes next
   float nB[2][16];             // squared norms of the bottom rows, by the round's parity
   int verdict[2][kCWMax];      // every CTA's rotations of the sweep, by its parity: 1 some
                                //   above the stopping cosine, 2 a wait ran out
@@ -92,6 +98,8 @@ __global__ void __launch_bounds__(kCNT, 1)
   if (tid == 0) {
     cl_mbar_init(&sh.bar[0], 1);
     cl_mbar_init(&sh.bar[1], 1);
+    cl_mbar_init(&sh.clear[0], max(1, jac_reports(rank, nc)));
+    cl_mbar_init(&sh.clear[1], max(1, jac_reports(rank, nc)));
     cl_mbar_fence();
   }
   // ---- the rows of R (column-major in L2; zero rows past keff) ------------------
@@ -194,11 +202,12 @@ __global__ void __launch_bounds__(kCNT, 1)
     }
     return true;
   };
-  // the CTAs the blocks go to: top to the next CTA's top (the last CTA's own bottom),
-  // bottom to the previous CTA's bottom (CTA 1's top from CTA 0, whose top stays)
-  const bool top_stays = rank == 0 || rank + 1 == nc;
-  const int bdst = rank > 0 ? rank - 1 : 1, bhalf = rank > 0 ? 1 : 0;
+  // where the blocks go, and whom this CTA and who to it reports a round's receipt
+  const JacBlock tdst = jac_dest(rank, 0, nc), bdst = jac_dest(rank, 1, nc);
+  const bool top_stays = tdst.cta == rank;
   const uint32_t incoming = (top_stays ? 1u : 2u) * blk;
+  const int report0 = jac_report(rank, 0, nc), report1 = jac_report(rank, 1, nc);
+  const bool reported = jac_reports(rank, nc) > 0;
   bool timeout = false;
   int status = DEV_NOT_CONVERGED, sweeps = max_sweeps;
   unsigned int g = 0;  // block rounds so far; the active buffers have parity g & 1
@@ -266,19 +275,28 @@ __global__ void __launch_bounds__(kCNT, 1)
         // the round's buffers.  CTA 0's top and the last CTA's top (its own bottom
         // next) stay in the CTA: plain stores of the warp that reads them first.
         const uint32_t trow = adr(0, ap) + (uint32_t)warp * kRowBytes;
-        if (top_stays) store_row(adr(rank == 0 ? 0 : 1, np) + (uint32_t)warp * kRowBytes, tr);
-        else store_row(trow, tr);
         store_row(brow, v);
+        if (!top_stays) store_row(trow, tr);
         cl_bulk_fence();
+        // the buffers written now were the sources of the round before
+        if (reported && g > 0 && !timeout && !cl_mbar_wait(&sh.clear[np], ((g - 1) >> 1) & 1))
+          timeout = true;
         __syncwarp();
-        if (lane == 0) {
+        if (top_stays) store_row(adr(tdst.half, np) + (uint32_t)warp * kRowBytes, tr);
+        if (lane == 0 && !timeout) {
           const uint32_t bar = cl_smem(&sh.bar[ap]);
           if (!top_stays)
-            cl_bulk(cl_map(adr(0, np) + (uint32_t)warp * kRowBytes, rank + 1), trow, kRowBytes,
-                    cl_map(bar, rank + 1));
-          cl_bulk(cl_map(adr(bhalf, np) + (brow - B), bdst), brow, kRowBytes, cl_map(bar, bdst));
+            cl_bulk(cl_map(adr(tdst.half, np) + (uint32_t)warp * kRowBytes, tdst.cta), trow, kRowBytes,
+                    cl_map(bar, tdst.cta));
+          cl_bulk(cl_map(adr(bdst.half, np) + (brow - B), bdst.cta), brow, kRowBytes,
+                  cl_map(bar, bdst.cta));
         }
         if (!timeout && !cl_mbar_wait(&sh.bar[ap], (g >> 1) & 1)) timeout = true;
+        if (tid == 0 && !timeout) {
+          const uint32_t clear = cl_smem(&sh.clear[ap]);
+          if (report0 >= 0) cl_mbar_arrive(cl_map(clear, report0));
+          if (report1 >= 0) cl_mbar_arrive(cl_map(clear, report1));
+        }
       }
     } else {
       g += 2 * nc - 1;

@@ -1,0 +1,25 @@
+"""The rules by which CTAs exchange data without a barrier around every access (csrc/sync_rules.h,
+the functions the kernels use), run through random orders of events on the CPU."""
+
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def check(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("sync") / "check")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-I", os.path.join(ROOT, "seemps2_gb300", "csrc"), "-o", exe,
+                    os.path.join(ROOT, "tests", "sync_rules_check.cpp")], check=True)
+    return lambda mode: subprocess.run([exe, mode], check=True, capture_output=True, text=True).stdout.strip()
+
+
+def test_jacobi_block_rounds(check):
+    """Clusters of 2 to 16 CTAs, three sweeps: every pair of blocks meets once a sweep, no block is
+    written over while a copy of it may be in flight or its CTA works on it, and every wait ends.
+    Without the reports of receipt, the check finds the write over a copy's source."""
+    assert check("jacobi") == "ok"
+    assert check("jacobi-blind").endswith("a write over the source of a copy in flight")
