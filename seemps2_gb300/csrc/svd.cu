@@ -32,6 +32,7 @@
 #include <cmath>
 
 #include "kernels.cuh"
+#include "sync_rules.h"
 
 namespace sm {
 
@@ -977,12 +978,13 @@ __global__ void __launch_bounds__(NT) k_house_qr(T* Wt, int k, int l, double thr
     if (threadIdx.x == 0) {
       double t = 0.0;
       for (int w = 0; w < NW; ++w) t += wpart[w];
-      __stcg(part + blockIdx.x, t);
+      __stcg(part + qr_step_slot(j) * gridDim.x + blockIdx.x, t);
     }
     if (!qr_grid_sync(ctl, epoch)) return;
     if (warp == 0) {
       double tot = 0.0;
-      for (int b = lane; b < (int)gridDim.x; b += 32) tot += __ldcg(part + b);
+      const double* sums = part + qr_step_slot(j) * gridDim.x;
+      for (int b = lane; b < (int)gridDim.x; b += 32) tot += __ldcg(sums + b);
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
       if (lane == 0) stop_flag = tot <= thr;
@@ -1007,7 +1009,6 @@ __global__ void __launch_bounds__(NT) k_house_qr(T* Wt, int k, int l, double thr
 // 174 x 190 0.80 ms, rank 130 of 256 x 256 0.69 ms, complex 128 x 128 0.69 ms (with
 // columns streamed through L2 and a test per step 174 x 190 took 0.84 ms, and more
 // the more rows a column has).
-constexpr int kQrBatch = 4;
 template <typename T, int NT, int E>
 __global__ void __launch_bounds__(NT) k_house_qr_reg(T* Wt, int k, int l, double thr_rel, T* vbuf,
                                                      double* part, QrCtl* ctl) {
@@ -1024,7 +1025,7 @@ __global__ void __launch_bounds__(NT) k_house_qr_reg(T* Wt, int k, int l, double
     const int i = lane + 32 * e;
     y[e] = (c < l && i < k) ? ldcg(Wt + (size_t)c * k + i) : S<T>::zero();
   }
-  // sum over the CTA's warps of NV values each into wpart, then into part[value][block]
+  // sum over the CTA's warps of n values each into wpart, then into part[slot + value][block]
   auto publish_sums = [&](const double* v, int n, int slot) {
 #pragma unroll
     for (int s = 0; s < kQrBatch; ++s) {
@@ -1100,12 +1101,10 @@ __global__ void __launch_bounds__(NT) k_house_qr_reg(T* Wt, int k, int l, double
     double a = 0.0;
 #pragma unroll
     for (int e = 0; e < E; ++e) a += S<T>::abs2(y[e]);
-    // the last slot: no batch writes it before a barrier has passed (a one-step
-    // batch writes slot 0 right away)
-    publish_sums(&a, 1, kQrBatch - 1);
+    publish_sums(&a, 1, kQrNormSlot);
     if (c == 0) reflector(0);
     if (!qr_grid_sync(ctl, epoch)) return;
-    thr = thr_rel * grid_sum(kQrBatch - 1);
+    thr = thr_rel * grid_sum(kQrNormSlot);
   }
   int steps = nmax, done = nmax;
   for (int j = 0; j < nmax; ++j) {
@@ -1163,14 +1162,14 @@ __global__ void __launch_bounds__(NT) k_house_qr_reg(T* Wt, int k, int l, double
         if (s < kQrBatch - 1) run += first + 1 + s <= j ? sum[s] : 0.0;
         sum[s] = c > first + s ? run : 0.0;
       }
-      publish_sums(sum, n, 0);
+      publish_sums(sum, n, qr_batch_slot(j));
     }
     // the next reflector: this column is up to date
     if (c == j + 1 && j + 1 < nmax) reflector(j + 1);
     if (!qr_grid_sync(ctl, epoch)) return;
     if (last) {
       for (int s = warp; s < n; s += NW) {
-        const double t = grid_sum(s);
+        const double t = grid_sum(qr_batch_slot(j) + s);
         if (lane == 0) below[s] = t <= thr;
       }
       __syncthreads();
@@ -1251,7 +1250,7 @@ int house_qr(Ctx& ctx, cudaStream_t st, T* Wt, int kw, int l, double thr_rel, T*
     grid = ctx.concurrent ? 1 : std::max(1, std::min(cols, per_sm_of(fn) * sms));
   }
   double* part;
-  SM_CHECK(ctx.scratch("svd.qpart", (size_t)kQrBatch * grid, &part));
+  SM_CHECK(ctx.scratch("svd.qpart", (size_t)kQrBatchSlots * grid, &part));
   void* args[] = {&Wt, &kw, &l, &thr_rel, &vbuf, &part, &qctl};
   SM_CHECK(coop_launch(fn, dim3(grid), dim3(NT), args, st));
   note_launch();

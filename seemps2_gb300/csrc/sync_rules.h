@@ -46,4 +46,19 @@ SM_RULE int jac_reports(int c, int nc) {
   return n;
 }
 
+// ---- k_house_qr, k_house_qr_reg: sums over the grid --------------------------------
+// Each CTA leaves its part of a sum before a step's grid barrier and all CTAs read the
+// parts after it, while the fastest of them may already be in the next step: what a
+// step writes before its barrier must not be what the step before it reads after its
+// own.  Slots (a part per CTA each) by step j:
+// the streaming kernel sums once a step; |W|^2, summed before step 0, is in slot 0
+SM_RULE int qr_step_slot(int j) { return (j + 1) & 1; }
+constexpr int kQrStepSlots = 2;
+// the register kernel sums once per kQrBatch steps, for each of them, and a last batch
+// may be a single step; |W|^2 has the slot after the two batches'
+constexpr int kQrBatch = 4;
+SM_RULE int qr_batch_slot(int j) { return j / kQrBatch % 2 * kQrBatch; }
+constexpr int kQrNormSlot = 2 * kQrBatch, kQrBatchSlots = 2 * kQrBatch + 1;
+static_assert(kQrStepSlots <= kQrBatchSlots, "one buffer serves both");
+
 }  // namespace sm

@@ -1,5 +1,6 @@
 // Runs the rules of csrc/sync_rules.h through random orders of events; prints "ok" or
-// what went wrong. Argument "jacobi-blind" leaves the reports out.
+// what went wrong. "jacobi-blind" leaves the reports out, "qr-step-single" and
+// "qr-batch-single" keep one buffer for the sums.
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -128,6 +129,32 @@ const char* jacobi(int nc, int rounds, bool reports, unsigned seed) {
   return nullptr;
 }
 
+// The grid sums of the Householder QR: between two grid barriers some CTAs read the sums
+// published before the first while others publish those of the second.  Barrier 0 follows
+// |W|^2, barrier j + 1 step j.
+const char* qr_sums(int nmax, bool batches, bool alternate) {
+  auto slots = [&](int b) {  // published before barrier b
+    std::vector<int> s;
+    if (b == 0) {
+      s.push_back(!batches ? 0 : alternate ? kQrNormSlot : kQrBatch - 1);
+    } else if (!batches) {
+      s.push_back(alternate ? qr_step_slot(b - 1) : 0);
+    } else {
+      const int j = b - 1, n = j % kQrBatch + 1;
+      if (n == kQrBatch || j + 1 == nmax)
+        for (int i = 0; i < n; ++i) s.push_back((alternate ? qr_batch_slot(j) : 0) + i);
+    }
+    return s;
+  };
+  for (int b = 0; b < nmax; ++b)
+    for (int read : slots(b)) {
+      if (read < 0 || read >= (batches ? kQrBatchSlots : kQrStepSlots)) return "a slot out of range";
+      for (int write : slots(b + 1))
+        if (read == write) return "a sum written over while it is read";
+    }
+  return nullptr;
+}
+
 }  // namespace
 
 int main(int argc, char** argv) {
@@ -140,6 +167,14 @@ int main(int argc, char** argv) {
           std::printf("%d CTAs: %s\n", nc, bad);
           return 0;
         }
+  }
+  if (!std::strncmp(mode, "qr", 2)) {
+    const bool batches = std::strstr(mode, "batch"), alternate = !std::strstr(mode, "single");
+    for (int nmax = 1; nmax <= 64; ++nmax)
+      if (const char* bad = qr_sums(nmax, batches, alternate)) {
+        std::printf("%d steps: %s\n", nmax, bad);
+        return 0;
+      }
   }
   std::printf("ok\n");
   return 0;

@@ -43,3 +43,17 @@ def test_mixed_splits_of_low_rank(m, n, rank, cplx):
     assert np.abs(L.conj().T @ L - np.eye(rank)).max() <= 1e-12
     P = oL.reshape(m, rank) @ oR.reshape(rank, n)
     assert np.linalg.norm(L @ R - P) <= 2e-6 * np.linalg.norm(P)
+
+
+@pytest.mark.parametrize("m, n, cplx", [(33, 190, False), (49, 174, False), (129, 133, False),
+                                        (193, 129, True), (1025, 40, False), (1100, 65, False)])
+def test_fp64_splits_whose_last_qr_batch_is_one_step(m, n, cplx):
+    """4 j + 1 columns to reduce, in registers (the rows to 1024) and streamed, where the sums of
+    the last batch follow those of the one before at once: the oracle's rank, the product to
+    1e-12 and an orthogonal factor."""
+    from tests.test_gpu_edges import check_split, matrix
+
+    rng = np.random.default_rng(m + n)
+    k = min(m, n)
+    for _ in range(4):
+        check_split(matrix(rng, m, n, np.geomspace(1.0, 1e-3, k), cplx))

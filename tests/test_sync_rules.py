@@ -23,3 +23,11 @@ def test_jacobi_block_rounds(check):
     Without the reports of receipt, the check finds the write over a copy's source."""
     assert check("jacobi") == "ok"
     assert check("jacobi-blind").endswith("a write over the source of a copy in flight")
+
+
+@pytest.mark.parametrize("kernel", ["qr-step", "qr-batch"])
+def test_householder_grid_sums(check, kernel):
+    """1 to 64 steps: no sum is written over while a slower CTA may still read it.  With one buffer
+    the check finds it: at any step, or where the last batch is a single step (5, 9, .. steps)."""
+    assert check(kernel) == "ok"
+    assert check(kernel + "-single").endswith("a sum written over while it is read")
