@@ -66,7 +66,9 @@ __global__ void __launch_bounds__(128) k_gemm(int opA, int opB, int M, int N, in
   T(*Bs)[TN + 1] = reinterpret_cast<T(*)[TN + 1]>(raw + sizeof(T) * KS * (TM + 1));
   const int tid = threadIdx.x;
   const int tx = tid % GN, ty = tid / GN;
-  const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+  // tiles along x, row by row: grid.y ends at 65535, which 16 rows a tile reach at 1 Mi
+  const int tn = (N + TN - 1) / TN;
+  const int m0 = (int)(blockIdx.x / tn) * TM, n0 = (int)(blockIdx.x % tn) * TN;
   T acc[RM][RN];
 #pragma unroll
   for (int i = 0; i < RM; ++i)
@@ -352,7 +354,7 @@ int launch_gemm(cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha,
                 const T* B, int ldb, T beta, T* C, int ldc, int nz) {
   const int kchunk = ((K + nz - 1) / nz + 15) / 16 * 16;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((N + TN - 1) / TN, (M + TM - 1) / TM, nz);
+  cfg.gridDim = dim3((unsigned)((size_t)((N + TN - 1) / TN) * ((M + TM - 1) / TM)), 1, nz);
   cfg.blockDim = dim3(128);
   cfg.stream = st;
   cudaLaunchAttribute attr[1];
@@ -362,10 +364,6 @@ int launch_gemm(cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha,
   attr[0].val.clusterDim.z = nz;
   cfg.attrs = attr;
   cfg.numAttrs = nz > 1 ? 1 : 0;
-  if (cfg.gridDim.y > 65535) {
-    set_error("gemm: M too large");
-    return SM_ERR_VALUE;
-  }
   SM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, k_gemm<T, TM, TN, RM, RN>, opA, opB, M, N, K, alpha, A, lda,
                                    B, ldb, beta, C, ldc, kchunk));
   note_launch();
@@ -385,6 +383,10 @@ int gemm(cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha, const 
   if (K == 0) {
     // C = beta C  (or zero)
     return scale_matrix<T>(st, M, N, beta, C, ldc);
+  }
+  if (M > 65535 * BM) {  // the rows of the FP32 kernel's grid: one limit for all forms
+    set_error("gemm: M too large");
+    return SM_ERR_VALUE;
   }
   // The tile and the number of slices whose fullest SM has the least to do: a CTA
   // takes TM TN kchunk / 2 clocks of its SM's FP64 pipe and some 1500 clocks of
