@@ -199,6 +199,12 @@ int sm_gemm_f64tc(void* ctx, int dtype, int opA, int opB, int M, int N, int K,
  * SM_ERR_TIMEOUT).  seemps2_gb300.batch sets it on its worker contexts. */
 int sm_ctx_set_concurrent(void* ctx, int on);
 
+/* Largest thread-block cluster (1 to 16 CTAs, default 16) that this context's FP32
+ * factorisations and tensor-core products use.  They also ask the device what it can
+ * place for this process (one that is given part of the SMs may have no room for 16):
+ * splits then take the FP64 kernels that need no cluster, products smaller clusters. */
+int sm_ctx_set_max_cluster(void* ctx, int ctas);
+
 /* Learned form (SM_PRECISION_MIXED_LEARNED) with on != 0: the predicted kept
  * rank r (or rank_hint in its place when > 0, no model needed) sizes a
  * randomized range finder (Halko, Martinsson and Tropp, SIAM Rev. 53, 2011):

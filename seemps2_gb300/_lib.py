@@ -175,6 +175,7 @@ SIGNATURES = {
     "sm_simplify_bond_caps": (C.c_int, [C.c_int, ip, C.c_int, ip, stp, ip]),
     "sm_trace_enable": (C.c_int, [vp, C.c_int]),
     "sm_trace_read": (C.c_int, [vp, ip, i64p, ip, ip, dp, dp]),
+    "sm_ctx_set_max_cluster": (C.c_int, [vp, C.c_int]),
     "sm_stats_reset": (C.c_int, [vp, C.c_int]),
     "sm_stats_read": (C.c_int, [vp, C.POINTER(sm_stats)]),
     # rank predictor (device pointers as void*, dims as a host int array)

@@ -67,6 +67,29 @@ Ctx::~Ctx() {
   if (pinned) cudaFreeHost(pinned);
 }
 
+bool Ctx::places(const void* fn, int ctas, int threads, size_t smem) {
+  if (ctas > max_cluster) return false;
+  const auto key = std::make_tuple(fn, ctas, smem);
+  const auto it = placed.find(key);
+  if (it != placed.end()) return it->second;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = ctas;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    n = 0;
+  }
+  return placed[key] = n > 0;
+}
+
 int Ctx::scratch(const std::string& name, size_t bytes, void** out) {
   bytes = std::max<size_t>(bytes, 16);
   auto it = bufs.find(name);
@@ -337,8 +360,8 @@ int sm_split_rows_f32(void* ctx, int dtype, const void* A, int m, int n, int wan
   Ctx& c = *as_ctx(ctx);
   cudaStream_t st = as_stream(stream);
   const int kw = want_u ? n : m, l = want_u ? m : n;
-  const bool fits = dtype == SM_FLOAT64 ? split_cluster_fits<double>(kw, l)
-                                        : split_cluster_fits<cplx>(kw, l);
+  const bool fits = dtype == SM_FLOAT64 ? split_cluster_fits<double>(c, kw, l)
+                                        : split_cluster_fits<cplx>(c, kw, l);
   if (!fits) {
     set_error("sm_split_rows_f32: matrix exceeds the cluster's capacity");
     return SM_ERR_VALUE;
@@ -582,6 +605,16 @@ int sm_ctx_set_range_finder(void* ctx, int on, int oversample, int power_iters, 
 int sm_ctx_set_concurrent(void* ctx, int on) {
   SM_GUARD_CTX(ctx);
   as_ctx(ctx)->concurrent = on != 0;
+  return SM_OK;
+}
+
+int sm_ctx_set_max_cluster(void* ctx, int ctas) {
+  SM_GUARD_CTX(ctx);
+  if (ctas < 1 || ctas > 16) {
+    set_error("sm_ctx_set_max_cluster: 1 to 16 CTAs");
+    return SM_ERR_VALUE;
+  }
+  as_ctx(ctx)->max_cluster = ctas;
   return SM_OK;
 }
 

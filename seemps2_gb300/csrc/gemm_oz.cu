@@ -690,6 +690,10 @@ int products(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, d
   const int tiles = kParts * tm * ((N + 63) / 64);
   int nz = 1;
   while (nz < kOzCluster && 2 * nz <= std::min(sms / tiles, nslabs)) nz *= 2;
+  if (nz > 1) SM_CHECK(raise_smem_limit(k_gemm_oz<64>, OzTile<64>::kSmem));
+  while (nz > 1 && !ctx.places(reinterpret_cast<const void*>(k_gemm_oz<64>), nz, kOzThreads,
+                               OzTile<64>::kSmem))
+    nz /= 2;  // one CTA to an SM in either width
   int slabs_per = (nslabs + nz - 1) / nz;
   const int nzo =
       nz < kOzCluster ? 1 : std::max(1, std::min(sms / (tiles * nz), slabs_per / 8));

@@ -582,15 +582,24 @@ int gemm_tc_planes(Ctx& ctx, cudaStream_t st, int M, int N, int kp, bool bf16, c
   // takes: two slabs to an accumulator, and beyond that several clusters to a tile,
   // whose sum is another launch.
   const int sms = std::max(1, ctx.num_sms);
+  const auto kernel = bf16 ? k_gemm_tc<true, OutT> : k_gemm_tc<false, OutT>;
+  const size_t smem = bf16 ? TcMode<true>::smem : TcMode<false>::smem;
+  SM_CHECK(raise_smem_limit(kernel, smem));
+  const auto placed = [&](int nz) {  // the largest cluster up to nz that finds room
+    while (nz > 1 && !ctx.places(reinterpret_cast<const void*>(kernel), nz, kTCThreads, smem)) nz /= 2;
+    return nz;
+  };
   int nz = 1, nzo = 1, kt_per;
   if (bf16) {  // ranges of two slabs and more, an accumulator each
     const int want = std::max(1, std::min(sms / tiles, ktiles / 2));
     kt_per = (ktiles + want - 1) / want;
     const int ranges = (ktiles + kt_per - 1) / kt_per;
     while (nz < kTcCluster && nz < ranges) nz *= 2;
+    nz = placed(nz);
     nzo = (ranges + nz - 1) / nz;
   } else {
     while (nz < kTcCluster && 2 * nz <= std::min(sms / tiles, ktiles)) nz *= 2;
+    nz = placed(nz);
     kt_per = (ktiles + nz - 1) / nz;
     constexpr int most = 2 * TcMode<false>::acc;
     if (nz == kTcCluster)
@@ -601,9 +610,6 @@ int gemm_tc_planes(Ctx& ctx, cudaStream_t st, int M, int N, int kp, bool bf16, c
   if (nzo > 1)
     SM_CHECK(ctx.scratch(sizeof(OutT) == 8 ? "tc.part" : "tc.part32", (size_t)nzo * M * N, &part));
   const dim3 grid((N + TN - 1) / TN, (M + TM - 1) / TM, nz * nzo);
-  const auto kernel = bf16 ? k_gemm_tc<true, OutT> : k_gemm_tc<false, OutT>;
-  const size_t smem = bf16 ? TcMode<true>::smem : TcMode<false>::smem;
-  SM_CHECK(raise_smem_limit(kernel, smem));
   SM_CHECK(cluster_launch(kernel, grid, kTCThreads, nz, smem, st, mAh, mAl, mBh, mBl, M, N, ktiles,
                           kt_per, alpha, beta, C, ldc, part, status));
   note_launch();

@@ -3,6 +3,7 @@
 
 #include <map>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include <cuda_bf16.h>
@@ -73,6 +74,8 @@ struct Ctx {
   void* pinned = nullptr;  // 64 KB of pinned host memory
   std::map<std::string, std::pair<void*, size_t>> bufs;
   std::map<const void*, int> coop_blocks;  // per-kernel co-resident CTA limit
+  int max_cluster = 16;  // CTAs of a cluster at most (sm_ctx_set_max_cluster)
+  std::map<std::tuple<const void*, int, size_t>, bool> placed;  // answers of places()
   // split trace (sm_trace_*): one record per SVD split, singular values included
   sm_stats stats{};
   bool timing = false;
@@ -85,6 +88,10 @@ struct Ctx {
   // Returns a device buffer of at least `bytes` bytes for `name`.  A buffer
   // only grows; growing it synchronises the device (cudaFree).
   int scratch(const std::string& name, size_t bytes, void** out);
+  // Whether a cluster of `ctas` CTAs of kernel `fn` (its shared-memory limit raised, its
+  // cluster size allowed) finds room on the SMs that this process is given; the device
+  // is asked once per kernel, cluster and shared memory.
+  bool places(const void* fn, int ctas, int threads, size_t smem);
   template <typename P>
   int scratch(const std::string& name, size_t count, P** out) {
     return scratch(name, count * sizeof(P), reinterpret_cast<void**>(out));
@@ -308,13 +315,14 @@ int rank_predict_dev(Ctx& ctx, cudaStream_t st, int k, const sm_strategy& strat,
 
 // --- svd_cluster_qr.cu, svd_cluster_jacobi.cu ----------------------------------
 // Whether the FP32 stage (a rank-revealing QR and a one-sided Jacobi, each in one
-// thread-block cluster) takes W (kw x l).
+// thread-block cluster) takes W (kw x l): by its size alone, and whether this process
+// can place its clusters too.
 // Splits with min(m, n) below this stay on the FP64 path in the mixed forms.
 constexpr int kMixedMinRank = 24;
 template <typename T>
 bool split_cluster_size_ok(int kw, int l);
 template <typename T>
-bool split_cluster_fits(int kw, int l);
+bool split_cluster_fits(Ctx& ctx, int kw, int l);
 // FP32 rank-revealing QR + one-sided Jacobi of W = (want_u ? A^T : A).  Writes kcap
 // rows (FP64, ld = l, zero past the iteration's rows) and their norms; ctl (zeroed by
 // the caller) receives status / sweeps / nact = rows of R kept;

@@ -2353,12 +2353,12 @@ int svd_split_mixed(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   if (k < kMixedMinRank || strat.method == SM_DO_NOT_TRUNCATE || strat.tolerance <= 0.0)
     return SM_OK;
   if constexpr (sizeof(T) != sizeof(double)) rf_k = 0;
-  if (rf_k > 0 && (rf_k >= k || rf_k > range_finder_max_k() || !split_cluster_fits<T>(l, rf_k)))
+  if (rf_k > 0 && (rf_k >= k || rf_k > range_finder_max_k() || !split_cluster_fits<T>(ctx, l, rf_k)))
     rf_k = 0;
   // the matrix the cluster factors: W (kw x l), or BH (l x rf_k)
   const int ckw = rf_k > 0 ? l : kw, cl = rf_k > 0 ? rf_k : l;
   if (rf_k > 0) qr_cap = rf_k;
-  if (rf_k == 0 && !split_cluster_fits<T>(kw, l)) return SM_OK;
+  if (rf_k == 0 && !split_cluster_fits<T>(ctx, kw, l)) return SM_OK;
   // the exact-weight rank rule resolves discarded weights down to the FP64
   // rounding of |A|^2 - kept (~ k eps |A|^2): tighter relative tolerances
   // take the FP64 path (counted as a fallback)

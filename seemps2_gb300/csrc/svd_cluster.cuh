@@ -189,13 +189,44 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
+// shared-memory limit and cluster size of a kernel of the stage
+template <typename K>
+int cl_allow(K* fn, size_t smem) {
+  SM_CHECK(raise_smem_limit(fn, smem));
+  SM_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  return SM_OK;
+}
+// one cluster of nc CTAs
+template <typename... P, typename... Q>
+int cl_launch(void (*fn)(P...), int nc, size_t smem, cudaStream_t st, Q... args) {
+  SM_CHECK(cl_allow(fn, smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(nc);
+  cfg.blockDim = dim3(kCNT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = nc;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  SM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fn, args...));
+  note_launch();
+  return SM_OK;
+}
+template <typename K>
+bool cl_places(Ctx& ctx, K* fn, int nc, size_t smem) {
+  return cl_allow(fn, smem) == SM_OK && ctx.places(reinterpret_cast<const void*>(fn), nc, kCNT, smem);
+}
+
 // ---- between the two kernels ---------------------------------------------------
 // Rows of R padded to whole 16-byte vectors of 32 lanes: R is column-major with
 // this column stride.  0: beyond the kernels' sizes.
 template <typename T>
 int qr_row_pad(int kw);
 template <typename T>
-bool qr_cluster_ok(int kw, int l);
+bool qr_cluster_ok(Ctx& ctx, int kw, int l);
 // Rank-revealing Householder QR of W = (trans ? A^T : A) (kw x l) / |W|_F: R into Rg,
 // ctl->nact = its rows, ctl->plateau = 1 if it stopped at the FP32 noise level,
 // info[0] = |W|_F^2 (FP64), info[1] the weight below the rows.
@@ -206,7 +237,7 @@ int qr_cluster(cudaStream_t st, const T* A, int n_a, int trans, int kw, int l, d
 // One-sided Jacobi on the ctl->nact (<= kmax) rows of R (length l): kcap rows (FP64,
 // times sqrt(info[0])) and their norms.
 template <typename T>
-bool jacobi_cluster_ok(int kmax, int l);
+bool jacobi_cluster_ok(Ctx& ctx, int kmax, int l);
 template <typename T>
 int jacobi_cluster(cudaStream_t st, const typename F32<T>::type* Rg, int ldk, int kmax, int l,
                    int max_sweeps, T* out_rows, double* out_nrm, int kcap, JacobiCtl* ctl,

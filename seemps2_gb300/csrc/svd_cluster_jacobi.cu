@@ -370,72 +370,54 @@ int jac_ctas(int kmax, int l, size_t* smem) {
   return 0;
 }
 
-template <typename T, int E>
-int launch_jacobi_cluster(cudaStream_t st, const typename F32<T>::type* Rg, int ldk, int kmax, int l,
-                          int max_sweeps, T* out_rows, double* out_nrm, int kcap, JacobiCtl* ctl,
-                          double* info) {
-  auto fn = k_jacobi_cluster<T, E>;
-  size_t smem = 0;
-  const int nc = jac_ctas<T>(kmax, l, &smem);
-  SM_CHECK(raise_smem_limit(fn, smem));
-  SM_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nc);
-  cfg.blockDim = dim3(kCNT);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = nc;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  const float tol2 = (float)l * FLT_EPSILON * FLT_EPSILON;
-  SM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fn, Rg, ldk, kmax, l, tol2, max_sweeps, out_rows, out_nrm,
-                                   kcap, ctl, info));
-  note_launch();
-  return SM_OK;
+// use(kernel) with the kernel for rows of length l; `none` beyond its sizes
+template <typename T, typename Use, typename R>
+R with_jacobi_kernel(int l, Use use, R none) {
+  switch (e_bucket(l)) {
+    case 4: return use(k_jacobi_cluster<T, 4>);
+    case 8: return use(k_jacobi_cluster<T, 8>);
+    case 12: return use(k_jacobi_cluster<T, 12>);
+    case 16: return use(k_jacobi_cluster<T, 16>);
+    case 24:
+      if constexpr (sizeof(T) == sizeof(double)) return use(k_jacobi_cluster<T, 24>);
+      return none;  // complex rows beyond 512 spill
+    default: return none;
+  }
 }
 
 }  // namespace
 
 template <typename T>
-bool jacobi_cluster_ok(int kmax, int l) {
-  const int e = e_bucket(l);
-  size_t smem = 0;
-  return kmax >= 1 && e != 0 && (sizeof(T) == sizeof(double) || e <= 16) &&
-         jac_ctas<T>(kmax, l, &smem) > 0;
+bool jacobi_cluster_ok(Ctx& ctx, int kmax, int l) {
+  if (kmax < 1) return false;
+  return with_jacobi_kernel<T>(
+      l,
+      [&](auto fn) {
+        size_t smem = 0;
+        const int nc = jac_ctas<T>(kmax, l, &smem);
+        return nc > 0 && cl_places(ctx, fn, nc, smem);
+      },
+      false);
 }
 
 template <typename T>
 int jacobi_cluster(cudaStream_t st, const typename F32<T>::type* Rg, int ldk, int kmax, int l,
                    int max_sweeps, T* out_rows, double* out_nrm, int kcap, JacobiCtl* ctl,
                    double* info) {
-  switch (e_bucket(l)) {
-#define SM_C(EV)                                                                                   \
-  case EV:                                                                                         \
-    return launch_jacobi_cluster<T, EV>(st, Rg, ldk, kmax, l, max_sweeps, out_rows, out_nrm, kcap, \
-                                        ctl, info)
-    SM_C(4);
-    SM_C(8);
-    SM_C(12);
-    SM_C(16);
-    case 24:
-      if constexpr (sizeof(T) == sizeof(double))  // complex rows beyond 512 spill
-        return launch_jacobi_cluster<T, 24>(st, Rg, ldk, kmax, l, max_sweeps, out_rows, out_nrm, kcap,
-                                            ctl, info);
-      break;
-#undef SM_C
-    default:
-      break;
-  }
-  set_error("mixed split: row length beyond the cluster kernel's limit");
-  return SM_ERR_VALUE;
+  const float tol2 = (float)l * FLT_EPSILON * FLT_EPSILON;
+  const int rc = with_jacobi_kernel<T>(
+      l,
+      [&](auto fn) {
+        size_t smem = 0;
+        const int nc = jac_ctas<T>(kmax, l, &smem);
+        return cl_launch(fn, nc, smem, st, Rg, ldk, kmax, l, tol2, max_sweeps, out_rows, out_nrm, kcap,
+                         ctl, info);
+      },
+      (int)SM_ERR_VALUE);
+  if (rc == SM_ERR_VALUE) set_error("mixed split: row length beyond the cluster kernel's limit");
+  return rc;
 }
 
-template bool jacobi_cluster_ok<double>(int, int);
-template bool jacobi_cluster_ok<cplx>(int, int);
 template int jacobi_cluster<double>(cudaStream_t, const float*, int, int, int, int, double*, double*,
                                     int, JacobiCtl*, double*);
 template int jacobi_cluster<cplx>(cudaStream_t, const float2*, int, int, int, int, cplx*, double*,
@@ -451,9 +433,9 @@ bool split_cluster_size_ok(int kw, int l) {
 }
 
 template <typename T>
-bool split_cluster_fits(int kw, int l) {
-  return split_cluster_size_ok<T>(kw, l) && qr_cluster_ok<T>(kw, l) &&
-         jacobi_cluster_ok<T>(std::min(kw, l), l);
+bool split_cluster_fits(Ctx& ctx, int kw, int l) {
+  return split_cluster_size_ok<T>(kw, l) && qr_cluster_ok<T>(ctx, kw, l) &&
+         jacobi_cluster_ok<T>(ctx, std::min(kw, l), l);
 }
 
 size_t split_cluster_rbuf_bytes(int kw, int l) {
@@ -479,8 +461,8 @@ int split_cluster_f32(cudaStream_t st, const T* A, int m, int n, bool want_u, do
 
 template bool split_cluster_size_ok<double>(int, int);
 template bool split_cluster_size_ok<cplx>(int, int);
-template bool split_cluster_fits<double>(int, int);
-template bool split_cluster_fits<cplx>(int, int);
+template bool split_cluster_fits<double>(Ctx&, int, int);
+template bool split_cluster_fits<cplx>(Ctx&, int, int);
 template int split_cluster_f32<double>(cudaStream_t, const double*, int, int, bool, double,
                                        double, int, double*, double*, int, JacobiCtl*, double*,
                                        int, void*, bool, const int*, bool);

@@ -495,55 +495,13 @@ int nv_bucket(int kw) {
 // the columns need
 inline int qr_ctas(int l) { return l <= 4 * kCNW ? 4 : l <= 8 * kCNW ? 8 : kCWMax; }
 
-template <typename T, int NV, int NC>
-int launch_qr(cudaStream_t st, int nc, const T* A, int n_a, int trans, int kw, int l, double thr_rel,
-              double thr_abs, typename F32<T>::type* Rg, JacobiCtl* ctl, double* info, int qr_cap,
-              const int* cap_dev, int pivot, int plateau) {
-  using F = typename F32<T>::type;
-  auto fn = k_qr_cluster<T, NV, NC>;
-  const size_t smem = (size_t)2 * kRing * (16 + NV * 512);
-  SM_CHECK(raise_smem_limit(fn, smem));
-  SM_CUDA_CHECK(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nc);
-  cfg.blockDim = dim3(kCNT);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = nc;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  SM_CUDA_CHECK(cudaLaunchKernelEx(&cfg, fn, A, n_a, trans, kw, l, thr_rel, thr_abs, Rg, ctl, info,
-                                   qr_cap, cap_dev, pivot, plateau));
-  note_launch();
-  return SM_OK;
-}
-
-}  // namespace
-
-template <typename T>
-int qr_row_pad(int kw) {
-  return nv_bucket<T>(kw) * (sizeof(T) == sizeof(double) ? 128 : 64);
-}
-
-template <typename T>
-bool qr_cluster_ok(int kw, int l) {
-  return kw >= 1 && l >= 1 && kw <= kMaxCol && std::min(kw, l) <= kMaxRows &&
-         l <= (sizeof(T) == sizeof(double) ? 768 : 512);
-}
-
-template <typename T>
-int qr_cluster(cudaStream_t st, const T* A, int n_a, int trans, int kw, int l, double thr_rel,
-               double thr_abs, typename F32<T>::type* Rg, JacobiCtl* ctl, double* info, int qr_cap,
-               const int* cap_dev, int pivot, int plateau) {
+// use(kernel, vectors per lane) with the kernel for kw rows and l columns; `none` beyond
+// its sizes
+template <typename T, typename Use, typename R>
+R with_qr_kernel(int kw, int l, Use use, R none) {
   const int nc = qr_ctas(l), cols = (l + nc * kCNW - 1) / (nc * kCNW), nv = nv_bucket<T>(kw);
-#define SM_QR(NVV, NCC)                                                                           \
-  if (nv == NVV && cols == NCC)                                                                   \
-  return launch_qr<T, NVV, NCC>(st, nc, A, n_a, trans, kw, l, thr_rel, thr_abs, Rg, ctl, info,    \
-                                qr_cap, cap_dev, pivot, plateau)
+#define SM_QR(NVV, NCC) \
+  if (nv == NVV && cols == NCC) return use(k_qr_cluster<T, NVV, NCC>, NVV)
   SM_QR(1, 1);
   SM_QR(1, 2);
   SM_QR(2, 1);
@@ -565,14 +523,45 @@ int qr_cluster(cudaStream_t st, const T* A, int n_a, int trans, int kw, int l, d
     SM_QR(16, 2);
   }
 #undef SM_QR
-  set_error("mixed split: matrix beyond the cluster QR's limits");
-  return SM_ERR_VALUE;
+  return none;
+}
+constexpr size_t qr_smem(int nv) { return (size_t)2 * kRing * (16 + nv * 512); }
+
+}  // namespace
+
+template <typename T>
+int qr_row_pad(int kw) {
+  return nv_bucket<T>(kw) * (sizeof(T) == sizeof(double) ? 128 : 64);
+}
+
+template <typename T>
+bool qr_cluster_ok(Ctx& ctx, int kw, int l) {
+  if (kw < 1 || l < 1 || kw > kMaxCol || std::min(kw, l) > kMaxRows ||
+      l > (sizeof(T) == sizeof(double) ? 768 : 512))
+    return false;
+  return with_qr_kernel<T>(
+      kw, l, [&](auto fn, int nv) { return cl_places(ctx, fn, qr_ctas(l), qr_smem(nv)); }, false);
+}
+
+template <typename T>
+int qr_cluster(cudaStream_t st, const T* A, int n_a, int trans, int kw, int l, double thr_rel,
+               double thr_abs, typename F32<T>::type* Rg, JacobiCtl* ctl, double* info, int qr_cap,
+               const int* cap_dev, int pivot, int plateau) {
+  const int rc = with_qr_kernel<T>(
+      kw, l,
+      [&](auto fn, int nv) {
+        return cl_launch(fn, qr_ctas(l), qr_smem(nv), st, A, n_a, trans, kw, l, thr_rel, thr_abs, Rg,
+                         ctl, info, qr_cap, cap_dev, pivot, plateau);
+      },
+      (int)SM_ERR_VALUE);
+  if (rc == SM_ERR_VALUE) set_error("mixed split: matrix beyond the cluster QR's limits");
+  return rc;
 }
 
 template int qr_row_pad<double>(int);
 template int qr_row_pad<cplx>(int);
-template bool qr_cluster_ok<double>(int, int);
-template bool qr_cluster_ok<cplx>(int, int);
+template bool qr_cluster_ok<double>(Ctx&, int, int);
+template bool qr_cluster_ok<cplx>(Ctx&, int, int);
 template int qr_cluster<double>(cudaStream_t, const double*, int, int, int, int, double, double,
                                 float*, JacobiCtl*, double*, int, const int*, int, int);
 template int qr_cluster<cplx>(cudaStream_t, const cplx*, int, int, int, int, double, double, float2*,

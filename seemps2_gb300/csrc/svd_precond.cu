@@ -161,7 +161,7 @@ template <typename T>
 int precondition_rows(Ctx& ctx, cudaStream_t st, T* R, int k, int l, double tol2, int use_floor,
                       double defl_rel, bool* converged) {
   *converged = false;
-  if (k < kPrecondMinRows || !split_cluster_fits<T>(l, k)) return SM_OK;
+  if (k < kPrecondMinRows || !split_cluster_fits<T>(ctx, l, k)) return SM_OK;
   const int cap = k + 32;
   const size_t kk = (size_t)k * k, kl = (size_t)k * l;
   T *rows, *X, *Xn, *M, *W, *Y;
