@@ -688,15 +688,16 @@ int products(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, d
   // a tile gets several clusters: their sum is another launch of ~4 us.
   const int sms = std::max(1, ctx.num_sms), tm = (M + OM - 1) / OM;
   const int tiles = kParts * tm * ((N + 63) / 64);
+  SM_CHECK(raise_smem_limit(k_gemm_oz<64>, OzTile<64>::kSmem));
+  int nmax = kOzCluster;  // the largest cluster that finds room, at one CTA to an SM in either width
+  while (nmax > 1 && !ctx.places(reinterpret_cast<const void*>(k_gemm_oz<64>), nmax, kOzThreads,
+                                 OzTile<64>::kSmem))
+    nmax /= 2;
   int nz = 1;
-  while (nz < kOzCluster && 2 * nz <= std::min(sms / tiles, nslabs)) nz *= 2;
-  if (nz > 1) SM_CHECK(raise_smem_limit(k_gemm_oz<64>, OzTile<64>::kSmem));
-  while (nz > 1 && !ctx.places(reinterpret_cast<const void*>(k_gemm_oz<64>), nz, kOzThreads,
-                               OzTile<64>::kSmem))
-    nz /= 2;  // one CTA to an SM in either width
+  while (nz < nmax && 2 * nz <= std::min(sms / tiles, nslabs)) nz *= 2;
   int slabs_per = (nslabs + nz - 1) / nz;
   const int nzo =
-      nz < kOzCluster ? 1 : std::max(1, std::min(sms / (tiles * nz), slabs_per / 8));
+      nz < nmax ? 1 : std::max(1, std::min(sms / (tiles * nz), slabs_per / 8));
   if (nzo > 1) slabs_per = (nslabs + nz * nzo - 1) / (nz * nzo);
   double* part = nullptr;
   if (nzo > 1) SM_CHECK(ctx.scratch("oz.part", (size_t)nzo * kParts * M * N, &part));

@@ -585,24 +585,20 @@ int gemm_tc_planes(Ctx& ctx, cudaStream_t st, int M, int N, int kp, bool bf16, c
   const auto kernel = bf16 ? k_gemm_tc<true, OutT> : k_gemm_tc<false, OutT>;
   const size_t smem = bf16 ? TcMode<true>::smem : TcMode<false>::smem;
   SM_CHECK(raise_smem_limit(kernel, smem));
-  const auto placed = [&](int nz) {  // the largest cluster up to nz that finds room
-    while (nz > 1 && !ctx.places(reinterpret_cast<const void*>(kernel), nz, kTCThreads, smem)) nz /= 2;
-    return nz;
-  };
+  int nmax = kTcCluster;  // the largest cluster that finds room
+  while (nmax > 1 && !ctx.places(reinterpret_cast<const void*>(kernel), nmax, kTCThreads, smem)) nmax /= 2;
   int nz = 1, nzo = 1, kt_per;
   if (bf16) {  // ranges of two slabs and more, an accumulator each
     const int want = std::max(1, std::min(sms / tiles, ktiles / 2));
     kt_per = (ktiles + want - 1) / want;
     const int ranges = (ktiles + kt_per - 1) / kt_per;
-    while (nz < kTcCluster && nz < ranges) nz *= 2;
-    nz = placed(nz);
+    while (nz < nmax && nz < ranges) nz *= 2;
     nzo = (ranges + nz - 1) / nz;
   } else {
-    while (nz < kTcCluster && 2 * nz <= std::min(sms / tiles, ktiles)) nz *= 2;
-    nz = placed(nz);
+    while (nz < nmax && 2 * nz <= std::min(sms / tiles, ktiles)) nz *= 2;
     kt_per = (ktiles + nz - 1) / nz;
     constexpr int most = 2 * TcMode<false>::acc;
-    if (nz == kTcCluster)
+    if (nz == nmax)
       nzo = std::max(1, std::min(sms / (tiles * nz), (kt_per + most - 1) / most));
     if (nzo > 1) kt_per = (ktiles + nz * nzo - 1) / (nz * nzo);
   }
