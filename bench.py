@@ -865,8 +865,10 @@ def main():
     _lib.stats_reset(timing=False)
     peak = fp64_peak(torch, _lib)
     # the dominant FP64 kernel of the step (event-timed per launch in this step)
-    cands = {"k_jacobi (one-sided Jacobi SVD, FP64)": ("jacobi", stt["jacobi_flops"],
-                                                      stt["jacobi_ms"], stt["jacobi_launches"]),
+    cands = {"k_jacobi, k_split_small (one-sided Jacobi SVD, FP64)":
+             ("jacobi", stt["jacobi_flops"], stt["jacobi_ms"], stt["jacobi_launches"]),
+             "FP32 start (k_qr_cluster, k_jacobi_cluster, FP64 correction products)":
+             ("start", stt["start_flops"], stt["start_ms"], stt["start_splits"]),
              "k_gemm (SIMT FP64 GEMM, split-K)": ("gemm", stt["gemm_flops"], stt["gemm_ms"],
                                                   stt["gemm_launches"])}
     kname, (tag, kfl, kms, kl) = max(cands.items(), key=lambda kv: kv[1][2])

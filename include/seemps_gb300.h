@@ -489,7 +489,7 @@ int sm_trace_read(void* ctx, int* count, int64_t* total_s, int* ranks, int* lens
  * (m >= n, x4 complex). */
 typedef struct sm_stats {
   int64_t launches;        /* kernels launched by this library */
-  int64_t jacobi_launches;
+  int64_t jacobi_launches; /* FP64 Jacobi kernels (k_jacobi, k_split_small) */
   int64_t jacobi_sweeps;   /* Jacobi sweeps summed over launches */
   int64_t gemm_launches;
   int64_t splits;          /* SVD splits */
@@ -529,6 +529,11 @@ typedef struct sm_stats {
   int64_t mixed_ns_steps;      /* Newton-Schulz steps of the mixed splits (one, or two for rows
                                   below FP32 resolution) */
   int64_t rank_predictions;    /* splits whose kept rank the predictor (or a rank hint) gave */
+  int64_t start_splits;        /* FP64 splits that took the FP32 start */
+  int64_t start_finished;      /* of those, finished without an FP64 Jacobi */
+  double start_ms;             /* event-timed (stats timing on): FP32 stage, Newton-Schulz and
+                                  correction products, which the gemm_* entries then leave out */
+  double start_flops;          /* algorithmic SVD flops of the finished ones */
 } sm_stats;
 int sm_stats_reset(void* ctx, int timing);
 int sm_stats_read(void* ctx, sm_stats* out);

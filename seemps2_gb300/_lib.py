@@ -88,6 +88,10 @@ class sm_stats(C.Structure):
         ("rf_splits", C.c_int64),
         ("mixed_ns_steps", C.c_int64),
         ("rank_predictions", C.c_int64),
+        ("start_splits", C.c_int64),
+        ("start_finished", C.c_int64),
+        ("start_ms", C.c_double),
+        ("start_flops", C.c_double),
     ]
 
 

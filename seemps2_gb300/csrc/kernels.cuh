@@ -79,7 +79,7 @@ struct Ctx {
   // split trace (sm_trace_*): one record per SVD split, singular values included
   sm_stats stats{};
   bool timing = false;
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // stats timing: around one launch or stage
   MatvecPrep mvp;
   bool trace = false;
   std::vector<int> tr_rank, tr_len;
@@ -296,8 +296,10 @@ int newton_schulz_matrix(cudaStream_t st, const T* M, int k, T* F, double* dev);
 // R <- X R (rows k x l, contiguous) with X unitary to FP64 rounding and the rows
 // close to orthogonal; `converged`: every pair passes the FP64 Jacobi's test
 // (tol2, use_floor, defl_rel as k_jacobi's), so that no Jacobi is needed.  Leaves
-// R as it is where the FP32 stage does not take the size or gives no basis.
+// R as it is where the FP32 stage gives no basis.  `takes`: the stage takes the size.
 constexpr int kPrecondMinRows = 24;
+template <typename T>
+bool precondition_takes(Ctx& ctx, int k, int l);
 template <typename T>
 int precondition_rows(Ctx& ctx, cudaStream_t st, T* R, int k, int l, double tol2, int use_floor,
                       double defl_rel, bool* converged);

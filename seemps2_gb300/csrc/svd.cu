@@ -1785,6 +1785,9 @@ int svd_split_xfree(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   else if (strat.method == SM_RELATIVE_SINGULAR_VALUE)
     use_floor = strat.tolerance >= 16.0 * std::sqrt((double)k * l) * eps;
   const double tol = std::sqrt((double)l) * DBL_EPSILON;
+  const double svd_flops = (4.0 * std::max(m, n) * (double)k * k + 8.0 * (double)k * k * k) *
+                           (sizeof(T) == sizeof(double) ? 1.0 : 4.0);
+  bool jacobi = false;  // an FP64 Jacobi ran, between ev0 and ev1
   if (small_split_fits<T>(ctx, kw, l)) {
     const size_t plain = sizeof(T) * (size_t)kw * (l | 1);
     const size_t staged = plain + small_stage_bytes<T>(k, l);
@@ -1798,10 +1801,7 @@ int svd_split_xfree(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
     if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev1, st));
     note_launch();
     SM_CUDA_CHECK(cudaGetLastError());
-    ctx.stats.jacobi_launches += k >= 2;
-    if (k >= 2)
-      ctx.stats.jacobi_flops += (4.0 * std::max(m, n) * (double)k * k + 8.0 * (double)k * k * k) *
-                                (sizeof(T) == sizeof(double) ? 1.0 : 4.0);
+    jacobi = k >= 2;
   } else {
     // Wt = W^T (l x kw): A itself for U, A^T for V; then scaled to O(1) entries
     if (want_u) {
@@ -1825,7 +1825,6 @@ int svd_split_xfree(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
       k_row_norms<T><<<(k + 7) / 8, 256, 0, st>>>(Wx, ld, k, l, nrm0, 1);
       note_launch();
       SM_CUDA_CHECK(cudaGetLastError());
-      if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev0, st));
       // the rows of R (the QR's steps; the rows below them are discarded weight)
       // through the FP32 start; the Jacobi only where that leaves pairs to rotate
       bool converged = false;
@@ -1834,17 +1833,39 @@ int svd_split_xfree(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
         SM_CUDA_CHECK(cudaMemcpyAsync(hq, qctl, sizeof(QrCtl), cudaMemcpyDeviceToHost, st));
         SM_CUDA_CHECK(cudaStreamSynchronize(st));
         const int steps = hq->steps;
-        if (hq->bar.status == 0)
-          SM_CHECK(precondition_rows<T>(ctx, st, Wx, steps, l, tol * tol, use_floor ? 1 : 0, drel,
-                                        &converged));
+        if (hq->bar.status == 0 && precondition_takes<T>(ctx, steps, l)) {
+          // its products are part of its time: they would record the same events
+          const sm_stats before = ctx.stats;
+          const bool timing = ctx.timing;
+          ctx.timing = false;
+          if (timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev0, st));
+          const int rc = precondition_rows<T>(ctx, st, Wx, steps, l, tol * tol, use_floor ? 1 : 0,
+                                              drel, &converged);
+          ctx.timing = timing;
+          SM_CHECK(rc);
+          if (timing) {
+            SM_CUDA_CHECK(cudaEventRecord(ctx.ev1, st));
+            SM_CUDA_CHECK(cudaEventSynchronize(ctx.ev1));
+            float ms = 0.f;
+            SM_CUDA_CHECK(cudaEventElapsedTime(&ms, ctx.ev0, ctx.ev1));
+            ctx.stats.start_ms += ms;
+            ctx.stats.gemm_launches = before.gemm_launches;
+            ctx.stats.gemm_flops = before.gemm_flops;
+            ctx.stats.gemm_oz_launches = before.gemm_oz_launches;
+            ctx.stats.gemm_oz_flops = before.gemm_oz_flops;
+          }
+          ctx.stats.start_splits += 1;
+          ctx.stats.start_finished += converged;
+          if (converged) ctx.stats.start_flops += svd_flops;
+        }
       }
-      if (!converged)
+      if (!converged) {
+        if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev0, st));
         SM_CHECK(run_jacobi<T>(ctx, st, Wx, ld, k, l, l, tol * tol, use_floor ? 1 : 0, drel, dabs, nrm,
                                nrm0, act, ctl));
-      if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev1, st));
-      ctx.stats.jacobi_launches += 1;
-      ctx.stats.jacobi_flops += (4.0 * std::max(m, n) * (double)k * k + 8.0 * (double)k * k * k) *
-                                (sizeof(T) == sizeof(double) ? 1.0 : 4.0);
+        if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev1, st));
+        jacobi = true;
+      }
     }
     k_row_norms<T><<<(k + 7) / 8, 256, 0, st>>>(Wx, ld, k, l, nrm, 0, wexp);
     note_launch();
@@ -1857,7 +1878,9 @@ int svd_split_xfree(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   *out = *h;
   ctx.stats.splits += 1;
   ctx.stats.jacobi_sweeps += h->sweeps;
-  if (ctx.timing && k >= 2) {
+  ctx.stats.jacobi_launches += jacobi;
+  if (jacobi) ctx.stats.jacobi_flops += svd_flops;
+  if (ctx.timing && jacobi) {
     float ms = 0.f;
     SM_CUDA_CHECK(cudaEventElapsedTime(&ms, ctx.ev0, ctx.ev1));
     ctx.stats.jacobi_ms += ms;

@@ -158,10 +158,14 @@ __global__ void __launch_bounds__(128) k_angles(const T* __restrict__ G, int k, 
 }  // namespace
 
 template <typename T>
+bool precondition_takes(Ctx& ctx, int k, int l) {
+  return k >= kPrecondMinRows && split_cluster_fits<T>(ctx, l, k);
+}
+
+template <typename T>
 int precondition_rows(Ctx& ctx, cudaStream_t st, T* R, int k, int l, double tol2, int use_floor,
                       double defl_rel, bool* converged) {
   *converged = false;
-  if (k < kPrecondMinRows || !split_cluster_fits<T>(ctx, l, k)) return SM_OK;
   const int cap = k + 32;
   const size_t kk = (size_t)k * k, kl = (size_t)k * l;
   T *rows, *X, *Xn, *M, *W, *Y;
@@ -280,6 +284,8 @@ int precondition_rows(Ctx& ctx, cudaStream_t st, T* R, int k, int l, double tol2
   return SM_OK;
 }
 
+template bool precondition_takes<double>(Ctx&, int, int);
+template bool precondition_takes<cplx>(Ctx&, int, int);
 template int precondition_rows<double>(Ctx&, cudaStream_t, double*, int, int, double, int, double,
                                        bool*);
 template int precondition_rows<cplx>(Ctx&, cudaStream_t, cplx*, int, int, double, int, double,
