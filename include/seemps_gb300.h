@@ -459,8 +459,8 @@ int sm_two_site_matvec_prepared(void* ctx, const void* H, const void* v, void* o
 
 /* At most m Lanczos steps (real FP64 basis, every new vector re-orthogonalised twice)
  * on the two-site operator from x0: the matvec of sm_two_site_matvec with `precision`,
- * or with `prepared` != 0 the prepared operator (sm_two_site_prepare with the same L and
- * R).  V (m x n, device, n = the vector's size) receives the basis, alpha and beta (host,
+ * or with `prepared` != 0 the prepared operator (sm_two_site_prepare with the same dims,
+ * L, R and precision, else SM_ERR_VALUE).  V (m x n, device, n = the vector's size) receives the basis, alpha and beta (host,
  * m each) the tridiagonal matrix; *steps <= m counts the steps up to a breakdown
  * (beta <= 1e-14 max |alpha|).  Counterpart of the eigsh call of
  * optimization/dmrg.py:15-23, whose small eigenproblem stays with the caller. */

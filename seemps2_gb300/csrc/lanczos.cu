@@ -129,6 +129,14 @@ int lanczos_run(Ctx& ctx, cudaStream_t st, const int* d, const double* L, const 
     set_error("lanczos: the operator must be square");
     return SM_ERR_VALUE;
   }
+  if (prepared) {  // its matvec goes by its own sizes and environments
+    const MatvecPrep& mp = ctx.mvp;
+    const int own[8] = {mp.a, mp.c, mp.b, mp.p1, mp.p2, mp.e, mp.g, mp.f};
+    if (mp.precision != precision || mp.L != L || mp.R != R || !std::equal(own, own + 8, d)) {
+      set_error("lanczos: the context holds another prepared operator (sm_two_site_prepare)");
+      return SM_ERR_VALUE;
+    }
+  }
   const int n = (int)n64;
   m = std::max(1, std::min(m, n));
   const int nb = (n + kChunk - 1) / kChunk, ub = (n + kLanNT - 1) / kLanNT;

@@ -1,0 +1,50 @@
+"""The Lanczos entry's checks and its end at an invariant subspace (GPU required)."""
+
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA GPU", allow_module_level=True)
+
+from seemps2_gb300 import _lib, dmrg  # noqa: E402
+
+
+def operator(chi, seed=0):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    r = lambda *s: torch.randn(*s, dtype=torch.float64, device="cuda", generator=g)
+    return r(chi, 3, chi), r(3, 2, 2, 2, 2, 3), r(chi, 3, chi)
+
+
+def lanczos(L, H, R, precision, prepared, m=4):
+    a, c, b = L.shape
+    g, e, f = R.shape
+    n = b * 4 * f
+    x0 = torch.ones(n, dtype=torch.float64, device="cuda")
+    V = torch.empty((m, n), dtype=torch.float64, device="cuda")
+    alpha, beta, steps = (C.c_double * m)(), (C.c_double * m)(), C.c_int()
+    _lib.check(_lib.load().sm_two_site_lanczos(
+        _lib.context(), _lib.int_array([a, c, b, 2, 2, e, g, f]), _lib.ptr(L), _lib.ptr(H), _lib.ptr(R),
+        _lib.ptr(x0), m, dmrg.PRECISIONS[precision], prepared, _lib.ptr(V), alpha, beta, C.byref(steps),
+        _lib.stream_handle()))
+    return steps.value
+
+
+def test_prepared_operator_has_to_be_the_one():
+    """Another shape, other environments of the same shape, another precision: refused before any
+    launch; the right one runs."""
+    L, H, R = operator(16)
+    op = dmrg.TwoSiteOperator(L, H, R, "bf16")
+    assert lanczos(L, H, R, "bf16", 1) == 4
+    for other, precision in [(operator(8), "bf16"), (operator(16, seed=1), "bf16"), ((L, H, R), "tf32x3"),
+                             ((L, H, R), "fp64")]:
+        _lib.stats_reset()
+        with pytest.raises(ValueError, match="another prepared operator"):
+            lanczos(*other, precision, 1)
+        assert _lib.stats_read()["launches"] == 0
+    op.ensure_prepared()
+    assert lanczos(L, H, R, "bf16", 1) == 4
