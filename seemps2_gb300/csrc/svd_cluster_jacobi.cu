@@ -28,7 +28,10 @@
 //     while its place is filled from below), and a copy is known to have read its
 //     source only where it arrives: whoever has received a round's rows tells the CTAs
 //     that write over their sources (an mbarrier each, sync_rules.h), which wait for it
-//     a whole block round later.
+//     a whole block round later.  A warp without a row tells them where there is one: the
+//     arrivals release to the cluster, which held up the round when a warp of the pairs
+//     made them (nine sweeps on 173 rows of 256: 0.737 ms, 0.690 so; seven on 76 of 128:
+//     0.223 and 0.203).
 // The cluster meets once per sweep, to agree on that flag.  A sweep takes 29 us on 64
 // rows of 64, 61 us on 153 rows of 256 and 206 us on 337 rows of 512 (with 16 CTAs
 // always, three sums per pair, copies through mailboxes and a cluster barrier per
@@ -206,9 +209,15 @@ __global__ void __launch_bounds__(kCNT, 1)
   const JacBlock tdst = jac_dest(rank, 0, nc), bdst = jac_dest(rank, 1, nc);
   const bool top_stays = tdst.cta == rank;
   const uint32_t incoming = (top_stays ? 1u : 2u) * blk;
-  const int report0 = jac_report(rank, 0, nc), report1 = jac_report(rank, 1, nc);
-  const bool reported = jac_reports(rank, nc) > 0;
   bool timeout = false;
+  const int report = lane < 2 ? jac_report(rank, lane, nc) : -1;
+  const bool reports = jac_report(rank, 0, nc) >= 0 || jac_report(rank, 1, nc) >= 0;
+  const int reporter = r < kCNW ? r : 0;
+  // the rows of round gr are here
+  auto tell = [&](unsigned int gr) {
+    if (report >= 0 && !timeout) cl_mbar_arrive(cl_map(cl_smem(&sh.clear[gr & 1]), report));
+  };
+  const bool reported = jac_reports(rank, nc) > 0;
   int status = DEV_NOT_CONVERGED, sweeps = max_sweeps;
   unsigned int g = 0;  // block rounds so far; the active buffers have parity g & 1
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
@@ -292,12 +301,14 @@ __global__ void __launch_bounds__(kCNT, 1)
                   cl_map(bar, bdst.cta));
         }
         if (!timeout && !cl_mbar_wait(&sh.bar[ap], (g >> 1) & 1)) timeout = true;
-        if (tid == 0 && !timeout) {
-          const uint32_t clear = cl_smem(&sh.clear[ap]);
-          if (report0 >= 0) cl_mbar_arrive(cl_map(clear, report0));
-          if (report1 >= 0) cl_mbar_arrive(cl_map(clear, report1));
-        }
+        if (warp == reporter) tell(g);
       }
+    } else if (warp == reporter && reports) {
+      for (int br = 0; br < 2 * nc - 1; ++br, ++g) {
+        if (lane < 2 && !timeout && !cl_mbar_wait(&sh.bar[g & 1], (g >> 1) & 1)) timeout = true;
+        tell(g);
+      }
+      __syncwarp();
     } else {
       g += 2 * nc - 1;
     }
