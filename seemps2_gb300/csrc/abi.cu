@@ -62,6 +62,8 @@ const char* last_error() { return g_error.c_str(); }
 Ctx::~Ctx() {
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
+  for (cudaEvent_t e : lan)
+    if (e) cudaEventDestroy(e);
   for (auto& kv : bufs)
     if (kv.second.first) cudaFree(kv.second.first);
   if (pinned) cudaFreeHost(pinned);

@@ -80,6 +80,7 @@ struct Ctx {
   sm_stats stats{};
   bool timing = false;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;  // stats timing: around one launch or stage
+  cudaEvent_t lan[2] = {};  // ends of the last Lanczos steps
   MatvecPrep mvp;
   bool trace = false;
   std::vector<int> tr_rank, tr_len;

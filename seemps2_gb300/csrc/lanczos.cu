@@ -3,11 +3,12 @@
 // Step j: w = H V[j]; the overlaps of w with all vectors so far are taken out twice
 // (classical Gram-Schmidt, FP64), alpha_j is the first pass's own, beta_j = |w|, and
 // V[j + 1] = w / beta_j.  The reference calls ARPACK for this (optimization/dmrg.py:
-// 15-23).  The host reads the alphas and betas once, after the last step; a run that
-// broke down (an invariant subspace) is cut at that step then, the vectors past it
-// being unused.  A step is the matvec and five kernels; with a dozen calls from Python
-// and two reads of a scalar per step, 30 steps at bond 108 took 160 us a step beyond
-// the matvec's kernels.
+// 15-23).  The kernels store the alphas and betas in host memory too, and before the host
+// issues a step it looks at the one two before: a run that breaks down (an invariant
+// subspace: a start that is an eigenvector, a small block) ends there, with one
+// unused step issued, and the device has a step to do while the host issues the next.  A step is the matvec
+// and five kernels; with a dozen calls from Python and two reads of a scalar per step,
+// 30 steps at bond 108 took 160 us a step beyond the matvec's kernels.
 #include <algorithm>
 #include <cmath>
 
@@ -19,17 +20,20 @@ namespace {
 
 constexpr int kChunk = 512;   // vector elements per block of the overlaps
 constexpr int kLanNT = 256;
+constexpr double kBreakdown = 1e-14;  // beta of an invariant subspace, relative to the alphas
+constexpr int kLead = 2;          // a step is issued once the beta of the kLead-th before it is seen
+constexpr size_t kLanPinned = 60 * 1024;  // their alphas and betas in the pinned block (bytes)
 
 // Overlaps coef[i] = V[i] . w, i < rows: block b holds one chunk of w in shared
 // memory, warp k takes rows k, k + 8, ..; the last block to finish adds the blocks'
-// parts in order and stores coef[rows - 1] to *alpha too (if given).  A lane adds 16
+// parts in order and stores coef[rows - 1] to *alpha and *host too (if given).  A lane adds 16
 // products before the warp's five shuffle sums: each FP64 instruction costs its warp
 // 64 clocks whether it adds products or partial sums.
 __global__ void __launch_bounds__(kLanNT) k_lan_dots(const double* __restrict__ V, int rows, int n,
                                                      const double* __restrict__ w,
                                                      double* __restrict__ part,
                                                      double* __restrict__ coef, double* alpha,
-                                                     unsigned int* done) {
+                                                     double* host, unsigned int* done) {
   __shared__ double ws[kChunk];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -57,18 +61,19 @@ __global__ void __launch_bounds__(kLanNT) k_lan_dots(const double* __restrict__ 
     for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
     if (lane == 0) {
       coef[i] = a;
-      if (alpha && i == rows - 1) *alpha = a;
+      if (alpha && i == rows - 1) *alpha = *host = a;
     }
   }
   if (threadIdx.x == 0) *done = 0u;
 }
 
-// w -= sum_i coef[i] V[i]; with `beta`, also *beta = |w| (the last block adds the
+// w -= sum_i coef[i] V[i]; with `beta`, also *beta = *host = |w| (the last block adds the
 // blocks' sums of squares in order).
 __global__ void __launch_bounds__(kLanNT) k_lan_update(const double* __restrict__ V, int rows, int n,
                                                        const double* __restrict__ coef,
                                                        double* __restrict__ w, double* __restrict__ part,
-                                                       double* beta, unsigned int* done) {
+                                                       double* beta, double* host,
+                                                       unsigned int* done) {
   __shared__ double red[kLanNT / 32];
   __shared__ bool last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -106,7 +111,7 @@ __global__ void __launch_bounds__(kLanNT) k_lan_update(const double* __restrict_
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
   if (lane == 0) {
-    *beta = sqrt(t);
+    *beta = *host = sqrt(t);
     *done = 0u;
   }
 }
@@ -149,23 +154,40 @@ int lanczos_run(Ctx& ctx, cudaStream_t st, const int* d, const double* L, const 
   SM_CHECK(ctx.scratch("lan.done", 1, &done));
   SM_CUDA_CHECK(cudaMemsetAsync(done, 0, sizeof(unsigned int), st));
   const int sb = std::min(ub, 1024);
+  for (cudaEvent_t& e : ctx.lan)
+    if (!e) SM_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  // [step % kLead][alpha, beta], and |x0|
+  volatile double* seen = reinterpret_cast<double*>(static_cast<char*>(ctx.pinned) + kLanPinned);
+  double* seen_dev = const_cast<double*>(seen);
+  int run = 0;  // steps issued
+  double largest = 0.0;
   // V[0] = x0 / |x0|: no vectors to take out, the norm alone
   SM_CUDA_CHECK(cudaMemcpyAsync(w, x0, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-  k_lan_update<<<ub, kLanNT, 0, st>>>(V, 0, n, coef, w, part, ab + 2 * m, done);
+  k_lan_update<<<ub, kLanNT, 0, st>>>(V, 0, n, coef, w, part, ab + 2 * m,
+                                      seen_dev + 2 * kLead, done);
   k_lan_scale<<<sb, kLanNT, 0, st>>>(w, n, ab + 2 * m, V);
   note_launch(2);
   for (int j = 0; j < m; ++j) {
+    double* slot = seen_dev + 2 * (j % kLead);
+    if (j >= kLead) {
+      SM_CUDA_CHECK(cudaEventSynchronize(ctx.lan[j % kLead]));
+      largest = std::max(largest, std::fabs(seen[2 * (j % kLead)]));
+      if (seen[2 * (j % kLead) + 1] <= kBreakdown * largest) break;
+    }
+    run = j + 1;
     const double* q = V + (size_t)j * n;
     if (prepared) SM_CHECK(two_site_matvec_prepared(ctx, st, H, q, w));
     else
       SM_CHECK(two_site_matvec<double>(ctx, st, d[0], d[1], d[2], d[3], d[4], d[5], d[6], d[7], L, H, R,
                                        q, w, precision));
     for (int pass = 0; pass < 2; ++pass) {
-      k_lan_dots<<<nb, kLanNT, 0, st>>>(V, j + 1, n, w, part, coef, pass ? nullptr : ab + j, done);
+      k_lan_dots<<<nb, kLanNT, 0, st>>>(V, j + 1, n, w, part, coef, pass ? nullptr : ab + j, slot,
+                                        done);
       k_lan_update<<<ub, kLanNT, 0, st>>>(V, j + 1, n, coef, w, part, pass ? ab + m + j : nullptr,
-                                          done);
+                                          slot + 1, done);
     }
     note_launch(4);
+    SM_CUDA_CHECK(cudaEventRecord(ctx.lan[j % kLead], st));
     if (j + 1 < m) {
       k_lan_scale<<<sb, kLanNT, 0, st>>>(w, n, ab + m + j, V + (size_t)(j + 1) * n);
       note_launch();
@@ -181,12 +203,12 @@ int lanczos_run(Ctx& ctx, cudaStream_t st, const int* d, const double* L, const 
   }
   if (prepared || precision != SM_MATVEC_FP64) SM_CHECK(tc_status_check(ctx, st));
   double amax = 0.0;
-  for (int j = 0; j < m; ++j) {
+  for (int j = 0; j < run; ++j) {
     alpha[j] = h[j];
     beta[j] = h[m + j];
     *steps = j + 1;
     amax = std::max(amax, std::fabs(h[j]));
-    if (beta[j] <= 1e-14 * amax) break;  // an invariant subspace: the Ritz pair is exact
+    if (beta[j] <= kBreakdown * amax) break;  // an invariant subspace: the Ritz pair is exact
   }
   return SM_OK;
 }

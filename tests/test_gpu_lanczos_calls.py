@@ -48,3 +48,26 @@ def test_prepared_operator_has_to_be_the_one():
         assert _lib.stats_read()["launches"] == 0
     op.ensure_prepared()
     assert lanczos(L, H, R, "bf16", 1) == 4
+
+
+@pytest.mark.parametrize("precision, spread", [("fp64", False), ("fp64", True), ("fp64tc", True), ("bf16", False)])
+def test_run_ends_at_an_invariant_subspace(precision, spread):
+    """A diagonal operator of three values: a start that is an eigenvector and one that reaches
+    three vectors. Of thirty steps asked for no more are issued than of two beyond those."""
+    chi = 24
+    eye = torch.eye(chi, dtype=torch.float64, device="cuda").reshape(chi, 1, chi)
+    H = np.zeros((1, 2, 2, 2, 2, 1))
+    for k, v in enumerate([-1.0, 0.5, 2.0, 2.0]):
+        H[0, k // 2, k // 2, k % 2, k % 2, 0] = v
+    start, steps = np.random.default_rng(0).normal(size=(chi, 2, 2, chi)), 3
+    if not spread:
+        start, steps = np.zeros_like(start), 1
+        start[3, 0, 0, 5] = 1.0
+    launches = []
+    for krylov in (steps + 2, 30):
+        _lib.stats_reset()
+        lam, _, total = dmrg.lanczos_ground_state(eye, H, eye, start, krylov=krylov, precision=precision)
+        launches.append(_lib.stats_read()["launches"])
+        assert total == steps
+        assert abs(lam + 1.0) <= 1e-12
+    assert launches[1] <= launches[0]
