@@ -1992,6 +1992,7 @@ constexpr int kMixedRefine = 2;    // refinement steps
 constexpr double kMixedBlind = 1e-4;  // smallest kept s / s_max the FP32 stage resolves
 constexpr double kMixedCutAmp = 1e-6;  // largest kept/dropped coupling (angle s_i / |A|)
 constexpr double kMixedMinTol = 1e-14;   // smallest relative-norm tolerance taken in mixed
+constexpr double kMixedPlateauMin = 9.9e-15;  // QR threshold (of |A|^2) that the exact weight resolves
 constexpr double kMixedRowFloor = 1e-12;  // FP32 rows lighter than this times |A|_F are dropped
 constexpr double kMixedOrthMax = 0.25;    // largest |V V^H - I| entry a Newton-Schulz step takes
 constexpr double kMixedNsOne = 3e-7;      // deviation after which one step reaches 1.4e-13
@@ -2449,7 +2450,7 @@ int svd_split_mixed(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
     if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev0, st));
     SM_CHECK(split_cluster_f32<T>(st, A, m, n, want_u, thr_rel, thr_abs, 40, rows, nrm, kcap, ctl,
                                   info, qr_cap, rbuf, true, cap_dev,
-                                  exact && qr_cap < std::min(m, n)));
+                                  exact && thr_rel >= kMixedPlateauMin && qr_cap < std::min(m, n)));
     if (ctx.timing) SM_CUDA_CHECK(cudaEventRecord(ctx.ev1, st));
   }
   struct Head {
@@ -2654,9 +2655,12 @@ int svd_split_mixed(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const s
   // a capped QR that left weight the rank may need: more than 1% of what the
   // tolerance allows (and more than 1e-12 of |A|^2) outside the rows' span,
   // computed exactly after the refinement
-  // (a stop at the noise level: more than 1e-13, well above FP64's rounding of the sum)
-  const bool missed = capped && hs[5] > std::max(hc.plateau ? 1e-13 : 1e-12,
-                                                 1e-2 * strat.tolerance) * norm2;
+  // (a QR without a cap that stopped at the noise level: more than its own threshold,
+  // as if it had gone on to it)
+  const double outside = !hc.plateau                ? std::max(1e-12, 1e-2 * strat.tolerance)
+                         : qr_cap > 0 && qr_cap < k ? std::max(1e-13, 1e-2 * strat.tolerance)
+                                                    : thr_rel;
+  const bool missed = capped && hs[5] > outside * norm2;
   const bool coupled = !(cut_angle <= kMixedCutAmp);
   const bool over_tol = r.err2 > allowed_discard(strat, norm2, s0, k, D) * (1.0 + 1e-12);
   const bool over = D < strat.max_bond_dimension && D < k && over_tol;
