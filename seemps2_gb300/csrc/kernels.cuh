@@ -288,11 +288,6 @@ int svd_split(Ctx& ctx, cudaStream_t st, const T* A, int m, int n, const sm_stra
               int left_mode, T* left, int right_mode, T* right, double* s_out,
               SplitResult* res);
 
-// F = 1.5 I - 0.5 M (F may be M), the Newton-Schulz factor of M = V V^H (k x k), and
-// *dev = max(*dev, the largest entry of |M - I|).
-template <typename T>
-int newton_schulz_matrix(cudaStream_t st, const T* M, int k, T* F, double* dev);
-
 // --- svd_precond.cu ----------------------------------------------------------
 // R <- X R (rows k x l, contiguous) with X unitary to FP64 rounding and the rows
 // close to orthogonal; `converged`: every pair passes the FP64 Jacobi's test

@@ -1317,7 +1317,7 @@ __device__ __forceinline__ float sum8(float x) {
   return x + __shfl_xor_sync(0xffffffffu, x, 1);
 }
 
-// a / b and 1 / sqrt(a) to a few FP32 roundings (the angle of an FP32 rotation)
+// a / b to a few FP32 roundings (the angle of an FP32 rotation)
 __device__ __forceinline__ float div_fast(float a, float b) { return __fdividef(a, b); }
 
 // One pair of FP32 rows [R | X] on 8 lanes: rotates them (all of l + k entries) if their
@@ -2347,16 +2347,6 @@ double allowed_discard(const sm_strategy& st, double norm2, double s0, int k, in
 }
 
 }  // namespace
-
-template <typename T>
-int newton_schulz_matrix(cudaStream_t st, const T* M, int k, T* F, double* dev) {
-  k_ns_matrix<T><<<grid_for((size_t)k * k), 256, 0, st>>>(M, k, F, dev, 0);
-  note_launch();
-  SM_CUDA_CHECK(cudaGetLastError());
-  return SM_OK;
-}
-template int newton_schulz_matrix<double>(cudaStream_t, const double*, int, double*, double*);
-template int newton_schulz_matrix<cplx>(cudaStream_t, const cplx*, int, cplx*, double*);
 
 // rf_k > 0 (real operands): instead of factoring W, the cluster factors
 // BH = W^T Q (l x rf_k) of a randomized range finder (rangefinder.cu) sized by

@@ -21,9 +21,9 @@
 //      pairs: usually two steps and one closing test;
 //   4. where pairs are left whose angle is not small (singular values below
 //      the FP32 resolution of the first pass, nearly equal ones), the FP32
-//      stage runs once or twice more on the graded W, where it takes one or two
-//      sweeps and resolves the next 5..6 decades; what is left after that is
-//      the FP64 Jacobi's, which starts from W and needs few sweeps.
+//      stage runs again on the graded W (up to three times), where it takes one
+//      or two sweeps and resolves the next 5..6 decades; what is left after that
+//      is the FP64 Jacobi's, which starts from W and needs few sweeps.
 //
 // The closing test is the Jacobi's convergence test on every pair of rows, so
 // a caller that gets `converged` needs no Jacobi at all.
@@ -40,7 +40,7 @@ namespace {
 constexpr double kAngleMax = 1e-2;   // largest angle a correction step takes
 constexpr double kAngleSafe = 1e-3;  // ... before another FP32 pass (larger ones are noise then)
 constexpr double kAngleInf = 0.05;   // |E|_inf above which the FP32 stage runs again
-constexpr double kDevDone = 2e-8;    // |X X^H - I| that one Newton-Schulz step takes to rounding
+constexpr double kDevDone = 2e-8;    // |X X^H - I|_inf that one Newton-Schulz step takes to rounding
 constexpr double kDevMax = 0.9;      // ... that a step still reduces
 constexpr int kLevels = 4;           // FP32 passes at most
 constexpr int kSteps = 12;           // correction steps at most
@@ -48,7 +48,7 @@ constexpr int kTaylor = 8;           // terms of exp(E) at most
 
 // What the host reads after a test.
 struct PrecondStat {
-  double dev;           // largest entry of |X X^H - I| before the last Newton-Schulz step
+  double dev;           // |X X^H - I|_inf before the last Newton-Schulz step
   double einf;          // largest row sum of |E|
   unsigned int viol;    // pairs that the Jacobi would rotate
   unsigned int left;    // ... of them without a small angle
@@ -85,6 +85,31 @@ __global__ void __launch_bounds__(128) k_rows_to_basis(const T* __restrict__ row
   if (threadIdx.x == 0 && !(nb > 0.0)) atomicAdd(&stat->missing, 1);
   for (int x = threadIdx.x; x < k; x += blockDim.x)
     X[(size_t)p * k + x] = S<T>::scale(S<T>::conj(rows[(size_t)b * k + x]), inv);
+}
+
+// M <- 1.5 I - 0.5 M, the Newton-Schulz factor of M = X X^H: block i takes row i and
+// *dev = max(*dev, |M - I|_inf).  A row sum bounds the spectral deviation, which the
+// largest entry does not: k entries of 2e-8 in phase are one of k 2e-8, whose square a
+// step leaves behind.
+template <typename T>
+__global__ void __launch_bounds__(128) k_newton_schulz(T* M, int k, double* dev) {
+  __shared__ double red[4];
+  const int i = blockIdx.x;
+  double sum = 0.0;
+  for (int j = threadIdx.x; j < k; j += blockDim.x) {
+    T& m = M[(size_t)i * k + j];
+    const T d = i == j ? m - S<T>::one() : m;
+    sum += sqrt(S<T>::abs2(d));
+    m = S<T>::scale(d, -0.5);
+    if (i == j) m = m + S<T>::one();
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0)  // without its sign bit a NaN counts as the largest
+    atomicMax(reinterpret_cast<unsigned long long*>(dev),
+              (unsigned long long)__double_as_longlong(fabs(red[0] + red[1] + red[2] + red[3])));
 }
 
 // E and the verdict from G = W W^H: block i takes row i.  The test is the
@@ -195,7 +220,9 @@ int precondition_rows(Ctx& ctx, cudaStream_t st, T* R, int k, int l, double tol2
   auto newton_schulz = [&]() -> int {
     SM_CUDA_CHECK(cudaMemsetAsync(&stat->dev, 0, sizeof(double), st));
     SM_CHECK(gemm_ctx<T>(ctx, st, SM_OP_N, SM_OP_C, k, k, k, one, X, k, X, k, zero, M, k));
-    SM_CHECK(newton_schulz_matrix<T>(st, M, k, M, &stat->dev));
+    k_newton_schulz<T><<<k, 128, 0, st>>>(M, k, &stat->dev);
+    note_launch();
+    SM_CUDA_CHECK(cudaGetLastError());
     SM_CHECK(gemm_ctx<T>(ctx, st, SM_OP_N, SM_OP_N, k, k, k, one, M, k, X, k, zero, Xn, k));
     std::swap(X, Xn);
     return SM_OK;
