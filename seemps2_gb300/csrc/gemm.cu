@@ -13,6 +13,7 @@
 #include <cmath>
 
 #include "kernels.cuh"
+#include "tile_rules.h"
 
 namespace cg = cooperative_groups;
 
@@ -372,9 +373,11 @@ int launch_gemm(cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha,
 
 }  // namespace
 
+namespace {
 template <typename T>
-int gemm(cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha, const T* A, int lda,
-         const T* B, int ldb, T beta, T* C, int ldc) {
+int gemm(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha, const T* A,
+         int lda, const T* B, int ldb, T beta, T* C, int ldc) {
+  const int sms = std::max(1, ctx.num_sms);
   if (M < 0 || N < 0 || K < 0) {
     set_error("gemm: negative size");
     return SM_ERR_VALUE;
@@ -388,33 +391,14 @@ int gemm(cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha, const 
     set_error("gemm: M too large");
     return SM_ERR_VALUE;
   }
-  // The tile and the number of slices whose fullest SM has the least to do: a CTA
-  // takes TM TN kchunk / 2 clocks of its SM's FP64 pipe and some 1500 clocks of
-  // loads and stores that only further CTAs hide, the slices' sum as much again.
-  // (130 x 130 x 256: 25 tiles of 32 in 6 slices, 150 CTAs, against 8 slices, 200
-  // CTAs on 152 SMs: 22 us.)
-  const int sms = 152;
-  double best = 0.0;
-  int best_t = 0, best_z = 1;
-  for (int t = 16; t <= 32; t += 16) {
-    const double tiles = (double)((M + t - 1) / t) * ((N + t - 1) / t);
-    for (int nz = 1; nz <= 8 && (nz == 1 || K > 16 * (nz - 1)); ++nz) {
-      const int kc = ((K + nz - 1) / nz + 15) / 16 * 16;
-      const double cta = 0.5 * t * t * kc * (sizeof(T) == sizeof(double) ? 1.0 : 4.0) + 1500.0;
-      const double cost = std::ceil(tiles * nz / sms) * cta + (nz > 1 ? 1500.0 : 0.0);
-      if (best_t == 0 || cost < best) {
-        best = cost;
-        best_t = t;
-        best_z = nz;
-      }
-    }
-  }
-  if (best_t == 16)
+  const GemmCut cut = gemm_cut(M, N, K, sizeof(T) != sizeof(double), sms);
+  if (cut.tile == 16)
     return launch_gemm<T, 16, 16, 1, 2>(st, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc,
-                                        best_z);
+                                        cut.slices);
   return launch_gemm<T, 32, 32, 2, 4>(st, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc,
-                                      best_z);
+                                      cut.slices);
 }
+}  // namespace
 
 // K slices of the FP32 kernel for an M x N x K product on `sms` SMs: enough CTAs
 // for about two waves, each slice at least 64 deep; 1 = no split.
@@ -448,7 +432,7 @@ bool slices_pay(int M, int N, int K) {
 template <typename T>
 int gemm_ctx_sel(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha,
                  const T* A, int lda, const T* B, int ldb, T beta, T* C, int ldc, bool allow_tc) {
-  if (M == 0 || N == 0 || K == 0) return gemm<T>(st, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+  if (M == 0 || N == 0 || K == 0) return gemm<T>(ctx, st, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
   if constexpr (sizeof(T) == sizeof(double)) {
     // mixed forms: FP64-accurate products on the BF16 tensor cores
     if (allow_tc && ctx.precision != SM_PRECISION_FP64 && ctx.fp64_tc && slices_pay<T>(M, N, K)) {
@@ -506,7 +490,7 @@ int gemm_ctx_sel(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int 
     return SM_OK;
   }
   auto run = [&]() -> int {
-    return gemm<T>(st, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+    return gemm<T>(ctx, st, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
   };
   if (!ctx.timing) return run();
   SM_CUDA_CHECK(cudaEventRecord(ctx.ev0, st));
@@ -522,7 +506,7 @@ int gemm_ctx_sel(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int 
 template <typename T>
 int gemm_ctx_f32(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha,
                  const T* A, int lda, const T* B, int ldb, T beta, T* C, int ldc) {
-  if (M == 0 || N == 0 || K == 0) return gemm<T>(st, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+  if (M == 0 || N == 0 || K == 0) return gemm<T>(ctx, st, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
   ctx.stats.gemm32_launches += 1;
   ctx.stats.gemm32_flops += 2.0 * M * N * K * (sizeof(T) == sizeof(double) ? 1.0 : 4.0);
   if constexpr (sizeof(T) == sizeof(double)) {
@@ -607,10 +591,5 @@ template int gemm_ctx_sel<cplx>(Ctx&, cudaStream_t, int, int, int, int, int, cpl
                                 int, const cplx*, int, cplx, cplx*, int, bool);
 template int gemm_ctx<cplx>(Ctx&, cudaStream_t, int, int, int, int, int, cplx, const cplx*, int,
                             const cplx*, int, cplx, cplx*, int);
-
-template int gemm<double>(cudaStream_t, int, int, int, int, int, double, const double*, int,
-                          const double*, int, double, double*, int);
-template int gemm<cplx>(cudaStream_t, int, int, int, int, int, cplx, const cplx*, int,
-                        const cplx*, int, cplx, cplx*, int);
 
 }  // namespace sm

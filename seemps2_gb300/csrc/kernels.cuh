@@ -158,9 +158,6 @@ int gemm_ctx(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, T
 template <typename T>
 int gemm_ctx_sel(Ctx& ctx, cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha,
                  const T* A, int lda, const T* B, int ldb, T beta, T* C, int ldc, bool allow_tc);
-template <typename T>
-int gemm(cudaStream_t st, int opA, int opB, int M, int N, int K, T alpha, const T* A, int lda,
-         const T* B, int ldb, T beta, T* C, int ldc);
 // Same contract with FP32 arithmetic (FP64 operands rounded on load, FP32
 // accumulation): the contractions of the mixed forms.
 template <typename T>

@@ -23,6 +23,7 @@
 #include <cuda_bf16.h>
 
 #include "kernels.cuh"
+#include "tile_rules.h"
 
 namespace cg = cooperative_groups;
 
@@ -215,12 +216,10 @@ inline int blocks_for(size_t n) {
 }
 
 template <int OPA, int OPB, int EPI>
-int sgemm(cudaStream_t st, int M, int N, int K, const float* A, int lda, const float* B, int ldb,
+int sgemm(Ctx& ctx, cudaStream_t st, int M, int N, int K, const float* A, int lda, const float* B, int ldb,
           float* C, int ldc, const Epi& ep) {
   const long tiles = (long)((N + TS - 1) / TS) * ((M + TS - 1) / TS);
-  // slices of at least one slab, until two CTAs per SM
-  int nz = 1;
-  while (nz < 8 && tiles * nz < 304 && K > TS * nz) nz *= 2;
+  const int nz = sgemm_slices(tiles, K, TS, std::max(1, ctx.num_sms));
   const int kchunk = ((K + nz - 1) / nz + TS - 1) / TS * TS;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((M + TS - 1) / TS, (N + TS - 1) / TS, nz);  // N <= 4096
@@ -423,7 +422,7 @@ int sm_mlp_forward(void* ctx, int n_layers, const int* dims, const float* params
     ep.act = A;
     ep.hidden = k + 1 < n_layers;
     ep.out = ep.hidden ? nullptr : Y;
-    SM_CHECK((sgemm<0, 1, EPI_LAYER>(st, batch, dout, di, in, di, W, di, Z, dout, ep)));
+    SM_CHECK((sgemm<0, 1, EPI_LAYER>(*mctx(ctx), st, batch, dout, di, in, di, W, di, Z, dout, ep)));
     in = A;
     po += (size_t)dout * di + dout;
     co += 2 * (size_t)batch * dout;
@@ -464,12 +463,12 @@ int sm_mlp_backward(void* ctx, int n_layers, const int* dims, const float* param
     const float* in = k == 0 ? X : cache + co[k - 1] + (size_t)batch * dims[k];  // A_{k-1}
     Epi ep;
     ep.colsum = gb;
-    SM_CHECK((sgemm<1, 0, EPI_DW>(st, dout, di, batch, dZ, dout, in, di, gW, di, ep)));  // dZ^T X
+    SM_CHECK((sgemm<1, 0, EPI_DW>(c, st, dout, di, batch, dZ, dout, in, di, gW, di, ep)));  // dZ^T X
     if (k > 0) {  // dZ of the layer below = (dZ W) gelu'(Z)
       Epi ed;
       ed.z = cache + co[k - 1];
       float* g = dZ == g0 ? g1 : g0;
-      SM_CHECK((sgemm<0, 0, EPI_DA>(st, batch, di, dout, dZ, dout, W, di, g, di, ed)));
+      SM_CHECK((sgemm<0, 0, EPI_DA>(c, st, batch, di, dout, dZ, dout, W, di, g, di, ed)));
       dZ = g;
     }
   }
