@@ -41,7 +41,11 @@ constexpr double kAngleMax = 1e-2;   // largest angle a correction step takes
 constexpr double kAngleSafe = 1e-3;  // ... before another FP32 pass (larger ones are noise then)
 constexpr double kAngleInf = 0.05;   // |E|_inf above which the FP32 stage runs again
 constexpr double kDevDone = 2e-8;    // |X X^H - I|_inf that one Newton-Schulz step takes to rounding
-constexpr double kDevMax = 0.9;      // ... that a step still reduces
+constexpr double kDevMax = 0.9;      // largest entry of X X^H - I from which no step is tried
+// Newton-Schulz steps at most after the first: nearly parallel rows (an entry of 0.9) are
+// eleven steps from rounding.  Of 488 splits in eight chains of bond 256, 42 went to the
+// FP64 Jacobi with eight steps (~19 ms each against 0.1 a step), 38 with twelve.
+constexpr int kNewtonSteps = 12;
 constexpr int kLevels = 4;           // FP32 passes at most
 constexpr int kSteps = 12;           // correction steps at most
 constexpr int kTaylor = 8;           // terms of exp(E) at most
@@ -49,6 +53,7 @@ constexpr int kTaylor = 8;           // terms of exp(E) at most
 // What the host reads after a test.
 struct PrecondStat {
   double dev;           // |X X^H - I|_inf before the last Newton-Schulz step
+  double entry;         // and its largest entry
   double einf;          // largest row sum of |E|
   unsigned int viol;    // pairs that the Jacobi would rotate
   unsigned int left;    // ... of them without a small angle
@@ -87,29 +92,44 @@ __global__ void __launch_bounds__(128) k_rows_to_basis(const T* __restrict__ row
     X[(size_t)p * k + x] = S<T>::scale(S<T>::conj(rows[(size_t)b * k + x]), inv);
 }
 
-// M <- 1.5 I - 0.5 M, the Newton-Schulz factor of M = X X^H: block i takes row i and
-// *dev = max(*dev, |M - I|_inf).  A row sum bounds the spectral deviation, which the
-// largest entry does not: k entries of 2e-8 in phase are one of k 2e-8, whose square a
-// step leaves behind.
+// M <- 1.5 I - 0.5 M, the Newton-Schulz factor of M = X X^H: block i takes row i; the
+// largest row sum and entry of |M - I| go to *stat.  The row sum says when to stop: it
+// bounds the spectral deviation, which the largest entry does not (k entries of 2e-8 in
+// phase are one of k 2e-8, whose square a step leaves behind).
 template <typename T>
-__global__ void __launch_bounds__(128) k_newton_schulz(T* M, int k, double* dev) {
-  __shared__ double red[4];
+__global__ void __launch_bounds__(128) k_newton_schulz(T* M, int k, PrecondStat* stat) {
+  __shared__ double red[4], top[4];
   const int i = blockIdx.x;
-  double sum = 0.0;
+  double sum = 0.0, worst = 0.0;
   for (int j = threadIdx.x; j < k; j += blockDim.x) {
     T& m = M[(size_t)i * k + j];
     const T d = i == j ? m - S<T>::one() : m;
-    sum += sqrt(S<T>::abs2(d));
+    const double a = sqrt(S<T>::abs2(d));
+    sum += a;
+    worst = a > worst ? a : worst;  // a NaN shows in the sum
     m = S<T>::scale(d, -0.5);
     if (i == j) m = m + S<T>::one();
   }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
+  for (int o = 16; o > 0; o >>= 1) {
+    sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const double a = __shfl_xor_sync(0xffffffffu, worst, o);
+    worst = a > worst ? a : worst;
+  }
+  if ((threadIdx.x & 31) == 0) {
+    red[threadIdx.x >> 5] = sum;
+    top[threadIdx.x >> 5] = worst;
+  }
   __syncthreads();
-  if (threadIdx.x == 0)  // without its sign bit a NaN counts as the largest
-    atomicMax(reinterpret_cast<unsigned long long*>(dev),
-              (unsigned long long)__double_as_longlong(fabs(red[0] + red[1] + red[2] + red[3])));
+  if (threadIdx.x != 0) return;
+  for (int w = 1; w < 4; ++w) worst = top[w] > worst ? top[w] : worst;
+  // without its sign bit a NaN counts as the largest
+  auto most = [](double* at, double x) {
+    atomicMax(reinterpret_cast<unsigned long long*>(at),
+              (unsigned long long)__double_as_longlong(fabs(x)));
+  };
+  most(&stat->dev, red[0] + red[1] + red[2] + red[3]);
+  most(&stat->entry, worst);
 }
 
 // E and the verdict from G = W W^H: block i takes row i.  The test is the
@@ -216,11 +236,11 @@ int precondition_rows(Ctx& ctx, cudaStream_t st, T* R, int k, int l, double tol2
     SM_CUDA_CHECK(cudaStreamSynchronize(st));
     return SM_OK;
   };
-  // one Newton-Schulz step; stat->dev = the deviation it started from
+  // one Newton-Schulz step; stat->dev and entry: the deviation it started from
   auto newton_schulz = [&]() -> int {
-    SM_CUDA_CHECK(cudaMemsetAsync(&stat->dev, 0, sizeof(double), st));
+    SM_CUDA_CHECK(cudaMemsetAsync(&stat->dev, 0, 2 * sizeof(double), st));
     SM_CHECK(gemm_ctx<T>(ctx, st, SM_OP_N, SM_OP_C, k, k, k, one, X, k, X, k, zero, M, k));
-    k_newton_schulz<T><<<k, 128, 0, st>>>(M, k, &stat->dev);
+    k_newton_schulz<T><<<k, 128, 0, st>>>(M, k, stat);
     note_launch();
     SM_CUDA_CHECK(cudaGetLastError());
     SM_CHECK(gemm_ctx<T>(ctx, st, SM_OP_N, SM_OP_N, k, k, k, one, M, k, X, k, zero, Xn, k));
@@ -273,10 +293,11 @@ int precondition_rows(Ctx& ctx, cudaStream_t st, T* R, int k, int l, double tol2
     note_launch();
     SM_CUDA_CHECK(cudaGetLastError());
     SM_CHECK(newton_schulz());
-    for (int ns = 0; ns < 8; ++ns) {
+    for (int ns = 0; ns < kNewtonSteps; ++ns) {
       SM_CHECK(newton_schulz());
       SM_CHECK(read());
-      if (h->status != 0 || h->missing != 0 || !(h->dev <= kDevMax)) return SM_OK;
+      if (h->status != 0 || h->missing != 0 || !(h->entry <= kDevMax) || !(h->dev <= DBL_MAX))
+        return SM_OK;
       if (h->dev <= kDevDone) {
         *ok = true;
         break;
