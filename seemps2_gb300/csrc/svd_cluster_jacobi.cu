@@ -24,22 +24,26 @@
 //     its new blocks: no cluster barrier.  Two buffers per block are enough: a CTA
 //     has sent round g's rows only after all its warps are done with the buffers of
 //     round g - 1, and its neighbours send into those only after they have received
-//     rows of it.  Those are not always the rows whose place they take (a top goes up
-//     while its place is filled from below), and a copy is known to have read its
-//     source only where it arrives: whoever has received a round's rows tells the CTAs
-//     that write over their sources (an mbarrier each, sync_rules.h), which wait for it
-//     a whole block round later.  A warp without a row tells them where there is one: the
-//     arrivals release to the cluster, which held up the round when a warp of the pairs
-//     made them (nine sweeps on 173 rows of 256: 0.737 ms, 0.690 so; seven on 76 of 128:
-//     0.223 and 0.203).
-// The cluster meets once per sweep, to agree on that flag.  A sweep takes 29 us on 64
-// rows of 64, 61 us on 153 rows of 256 and 206 us on 337 rows of 512 (with 16 CTAs
+//     rows of it.  The rows leave from two more buffers per block, free again two rounds
+//     later: by then the CTA has received rows that its neighbours sent after they had
+//     its own.  Where shared memory holds four buffers a block only, they leave from the
+//     round's own.  These are written over a round later, by a neighbour that need not
+//     have received them (a top goes up while its place is filled from below), and a
+//     copy is known to have read its source only where it arrives: whoever has received
+//     a round's rows tells the CTAs that write over their sources (an mbarrier each,
+//     sync_rules.h).  Reports cost up to a tenth: a sweep on 153 rows of 256 takes 63 us
+//     with the buffers apart and 68 with reports, on 256 rows 100 and 107, on 337 rows of
+//     512 210 and 217.  (They are made by a warp without a row where there is one, 4 to
+//     10 % less than by a warp of the pairs: their arrivals release to the cluster.)
+// The cluster meets once per sweep, to agree on that flag.  A sweep takes 21 us on 64
+// rows of 64, 63 us on 153 rows of 256 and 210 us on 337 rows of 512 (with 16 CTAs
 // always, three sums per pair, copies through mailboxes and a cluster barrier per
 // block round: 56, 93 and 268 us).
 #include <cooperative_groups.h>
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 #include "svd_cluster.cuh"
 #include "sync_rules.h"
@@ -76,7 +80,7 @@ __device__ __forceinline__ void pair_barrier(int warps) {  // the warps that hol
 template <typename T, int E>
 __global__ void __launch_bounds__(kCNT, 1)
     k_jacobi_cluster(const typename F32<T>::type* __restrict__ Rg, int ldk, int kmax, int l,
-                     float tol2, int max_sweeps, T* __restrict__ out_rows,
+                     float tol2, int max_sweeps, uint32_t smem, T* __restrict__ out_rows,
                      double* __restrict__ out_nrm, int kcap, JacobiCtl* ctl,
                      double* __restrict__ info) {
   using F = typename F32<T>::type;
@@ -94,6 +98,8 @@ __global__ void __launch_bounds__(kCNT, 1)
   if (ctl->status != 0) return;  // the QR gave up (every CTA reads the same word)
   const int r = max(1, (keff + 2 * nc - 1) / (2 * nc));
   const uint32_t blk = (uint32_t)r * kRowBytes;
+  // where a round's rows are copied from, behind its buffers: others, or themselves
+  const bool apart = 8 * blk <= smem;
   // block buffers [top / bottom][parity]
   auto buf = [&](int half, int par) -> unsigned char* {
     return jac_raw + (size_t)(half * 2 + par) * blk;
@@ -205,21 +211,81 @@ __global__ void __launch_bounds__(kCNT, 1)
     }
     return true;
   };
-  // where the blocks go, and whom this CTA and who to it reports a round's receipt
+  // where the blocks go
   const JacBlock tdst = jac_dest(rank, 0, nc), bdst = jac_dest(rank, 1, nc);
   const bool top_stays = tdst.cta == rank;
   const uint32_t incoming = (top_stays ? 1u : 2u) * blk;
   bool timeout = false;
-  const int report = lane < 2 ? jac_report(rank, lane, nc) : -1;
-  const bool reports = jac_report(rank, 0, nc) >= 0 || jac_report(rank, 1, nc) >= 0;
-  const int reporter = r < kCNW ? r : 0;
   // the rows of round gr are here
   auto tell = [&](unsigned int gr) {
+    const int report = lane < 2 ? jac_report(rank, lane, nc) : -1;
     if (report >= 0 && !timeout) cl_mbar_arrive(cl_map(cl_smem(&sh.clear[gr & 1]), report));
   };
-  const bool reported = jac_reports(rank, nc) > 0;
-  int status = DEV_NOT_CONVERGED, sweeps = max_sweeps;
   unsigned int g = 0;  // block rounds so far; the active buffers have parity g & 1
+  // A sweep's block rounds for the warps that hold rows, in one of the two ways to send
+  // them (compiled apart: the one's registers and branches would slow the other).
+  auto block_rounds = [&](auto way) {
+    constexpr bool kApart = decltype(way)::value;
+    const uint32_t out = kApart ? 4 * blk : 0;
+    const bool reported = !kApart && jac_reports(rank, nc) > 0;
+    for (int br = 0; br < 2 * nc - 1; ++br, ++g) {
+      const int ap = g & 1, np = ap ^ 1;
+      if (tid == 0) cl_mbar_expect(&sh.bar[ap], incoming);
+      const uint32_t B = adr(1, ap), nB = cl_smem(sh.nB[ap]);
+      f2_t tr[NU], v[NU];
+      load_row(adr(0, ap) + (uint32_t)warp * kRowBytes, tr);
+      load_row(B + (uint32_t)warp * kRowBytes, v);
+      float a = norm2_of(tr);
+      {
+        const float b = norm2_of(v);
+        if (lane == 0) cl_sts(nB + 4u * warp, b);
+      }
+      pair_barrier(r);
+      uint32_t brow = B + (uint32_t)warp * kRowBytes, nb = nB + 4u * warp;
+      const uint32_t bend = B + blk;
+#pragma unroll 1
+      for (int t = r; t > 0; --t) {
+        load_row(brow, v);
+        float b = cl_lds(nb);
+        const bool rot = rotate(tr, v, a, b);
+        if (t == 1) break;
+        if (rot) {
+          store_row(brow, v);
+          if (lane == 0) cl_sts(nb, b);
+        }
+        pair_barrier(r);
+        brow += kRowBytes;
+        nb += 4;
+        if (brow == bend) {
+          brow = B;
+          nb = nB;
+        }
+      }
+      // Both rows to where they meet next, one bulk copy each.  CTA 0's top and the
+      // last CTA's top (its own bottom next) stay in the CTA: plain stores of the warp
+      // that reads them first.
+      const uint32_t trow = adr(0, ap) + out + (uint32_t)warp * kRowBytes;
+      store_row(brow + out, v);
+      if (!top_stays) store_row(trow, tr);
+      cl_bulk_fence();
+      // without buffers apart those written now were the sources of the round before
+      if (reported && g > 0 && !timeout && !cl_mbar_wait(&sh.clear[np], ((g - 1) >> 1) & 1))
+        timeout = true;
+      __syncwarp();
+      if (top_stays) store_row(adr(tdst.half, np) + (uint32_t)warp * kRowBytes, tr);
+      if (lane == 0 && !timeout) {
+        const uint32_t bar = cl_smem(&sh.bar[ap]);
+        if (!top_stays)
+          cl_bulk(cl_map(adr(tdst.half, np) + (uint32_t)warp * kRowBytes, tdst.cta), trow, kRowBytes,
+                  cl_map(bar, tdst.cta));
+        cl_bulk(cl_map(adr(bdst.half, np) + (brow - B), bdst.cta), brow + out, kRowBytes,
+                cl_map(bar, bdst.cta));
+      }
+      if (!timeout && !cl_mbar_wait(&sh.bar[ap], (g >> 1) & 1)) timeout = true;
+      if (!kApart && r == kCNW && warp == 0) tell(g);
+    }
+  };
+  int status = DEV_NOT_CONVERGED, sweeps = max_sweeps;
   for (int sweep = 0; sweep < max_sweeps; ++sweep) {
     wide = false;
     // pairs inside each block (circle method over r positions, padded to even)
@@ -247,63 +313,9 @@ __global__ void __launch_bounds__(kCNT, 1)
       }
     }
     if (warp < r) {
-      for (int br = 0; br < 2 * nc - 1; ++br, ++g) {
-        const int ap = g & 1, np = ap ^ 1;
-        if (tid == 0) cl_mbar_expect(&sh.bar[ap], incoming);
-        const uint32_t B = adr(1, ap), nB = cl_smem(sh.nB[ap]);
-        f2_t tr[NU], v[NU];
-        load_row(adr(0, ap) + (uint32_t)warp * kRowBytes, tr);
-        load_row(B + (uint32_t)warp * kRowBytes, v);
-        float a = norm2_of(tr);
-        {
-          const float b = norm2_of(v);
-          if (lane == 0) cl_sts(nB + 4u * warp, b);
-        }
-        pair_barrier(r);
-        uint32_t brow = B + (uint32_t)warp * kRowBytes, nb = nB + 4u * warp;
-        const uint32_t bend = B + blk;
-#pragma unroll 1
-        for (int t = r; t > 0; --t) {
-          load_row(brow, v);
-          float b = cl_lds(nb);
-          const bool rot = rotate(tr, v, a, b);
-          if (t == 1) break;
-          if (rot) {
-            store_row(brow, v);
-            if (lane == 0) cl_sts(nb, b);
-          }
-          pair_barrier(r);
-          brow += kRowBytes;
-          nb += 4;
-          if (brow == bend) {
-            brow = B;
-            nb = nB;
-          }
-        }
-        // Both rows to where they meet next, one bulk copy each from their places in
-        // the round's buffers.  CTA 0's top and the last CTA's top (its own bottom
-        // next) stay in the CTA: plain stores of the warp that reads them first.
-        const uint32_t trow = adr(0, ap) + (uint32_t)warp * kRowBytes;
-        store_row(brow, v);
-        if (!top_stays) store_row(trow, tr);
-        cl_bulk_fence();
-        // the buffers written now were the sources of the round before
-        if (reported && g > 0 && !timeout && !cl_mbar_wait(&sh.clear[np], ((g - 1) >> 1) & 1))
-          timeout = true;
-        __syncwarp();
-        if (top_stays) store_row(adr(tdst.half, np) + (uint32_t)warp * kRowBytes, tr);
-        if (lane == 0 && !timeout) {
-          const uint32_t bar = cl_smem(&sh.bar[ap]);
-          if (!top_stays)
-            cl_bulk(cl_map(adr(tdst.half, np) + (uint32_t)warp * kRowBytes, tdst.cta), trow, kRowBytes,
-                    cl_map(bar, tdst.cta));
-          cl_bulk(cl_map(adr(bdst.half, np) + (brow - B), bdst.cta), brow, kRowBytes,
-                  cl_map(bar, bdst.cta));
-        }
-        if (!timeout && !cl_mbar_wait(&sh.bar[ap], (g >> 1) & 1)) timeout = true;
-        if (warp == reporter) tell(g);
-      }
-    } else if (warp == reporter && reports) {
+      if (apart) block_rounds(std::true_type());
+      else block_rounds(std::false_type());
+    } else if (!apart && warp == r && (jac_report(rank, 0, nc) >= 0 || jac_report(rank, 1, nc) >= 0)) {
       for (int br = 0; br < 2 * nc - 1; ++br, ++g) {
         if (lane < 2 && !timeout && !cl_mbar_wait(&sh.bar[g & 1], (g >> 1) & 1)) timeout = true;
         tell(g);
@@ -368,15 +380,18 @@ inline int e_bucket(int l) {
   return 0;
 }
 
+constexpr size_t kJacSmem = 225 * 1024;
+
 // CTAs for kmax rows of length l: the fewest whose blocks have at most 8 rows, 16
-// CTAs with up to 16 rows beyond that, if the four block buffers fit shared memory
-// (0: they do not)
+// CTAs with up to 16 rows beyond that, if four block buffers fit shared memory (0: they
+// do not); *smem: that of eight, or all there is
 template <typename T>
 int jac_ctas(int kmax, int l, size_t* smem) {
   for (int nc : {2, 4, 8, 16}) {
     const size_t r = (size_t)std::max(1, (kmax + 2 * nc - 1) / (2 * nc));
-    *smem = 4 * r * 32 * e_bucket(l) * sizeof(typename F32<T>::type);
-    if ((r <= 8 || (nc == 16 && r <= 16)) && *smem <= 225 * 1024) return nc;
+    const size_t block = r * 32 * e_bucket(l) * sizeof(typename F32<T>::type);
+    *smem = std::min(8 * block, kJacSmem);
+    if ((r <= 8 || (nc == 16 && r <= 16)) && 4 * block <= kJacSmem) return nc;
   }
   return 0;
 }
@@ -421,8 +436,8 @@ int jacobi_cluster(cudaStream_t st, const typename F32<T>::type* Rg, int ldk, in
       [&](auto fn) {
         size_t smem = 0;
         const int nc = jac_ctas<T>(kmax, l, &smem);
-        return cl_launch(fn, nc, smem, st, Rg, ldk, kmax, l, tol2, max_sweeps, out_rows, out_nrm, kcap,
-                         ctl, info);
+        return cl_launch(fn, nc, smem, st, Rg, ldk, kmax, l, tol2, max_sweeps, (uint32_t)smem, out_rows,
+                         out_nrm, kcap, ctl, info);
       },
       (int)SM_ERR_VALUE);
   if (rc == SM_ERR_VALUE) set_error("mixed split: row length beyond the cluster kernel's limit");

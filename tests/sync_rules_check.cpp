@@ -1,5 +1,6 @@
 // Runs the rules of csrc/sync_rules.h through random orders of events; prints "ok" or
-// what went wrong. "jacobi-blind" leaves the reports out, "qr-step-single" and
+// what went wrong. "jacobi-outs" sends from buffers apart instead of
+// reporting, "jacobi-blind" does neither, "qr-step-single" and
 // "qr-batch-single" keep one buffer for the sums.
 #include <cstdio>
 #include <cstring>
@@ -46,8 +47,9 @@ struct Copy {
 
 // The block rounds of k_jacobi_cluster, one row to a block: every CTA's steps in order,
 // the copies delivered whenever the order of events likes.
-// The reports are a warp's of their own (`apart`) or the last of a round's steps.
-const char* jacobi(int nc, int rounds, bool reports, bool apart, unsigned seed) {
+// `outs`: the copies leave from buffers of their own, two to a block, and nothing is
+// reported. Else the reports are made by a warp of its own (`apart`) or last in a round.
+const char* jacobi(int nc, int rounds, bool reports, bool outs, bool apart, unsigned seed) {
   std::mt19937 rng(seed);
   struct Cta {
     int g = 0, step = 0, told = 0;
@@ -56,9 +58,11 @@ const char* jacobi(int nc, int rounds, bool reports, bool apart, unsigned seed) 
   std::vector<Cta> c(nc);
   for (int k = 0; k < nc; ++k)
     for (int p = 0; p < 2; ++p) c[k].clear[p].init(jac_reports(k, nc) > 0 ? jac_reports(k, nc) : 1);
-  std::vector<std::vector<int>> block[2];  // [half][cta][parity]: which block lies there
+  // [half][cta][parity]: which block lies there
+  std::vector<std::vector<std::vector<int>>> block(2);
   for (int h = 0; h < 2; ++h)
     for (int k = 0; k < nc; ++k) block[h].push_back({h ? 2 * nc - 1 - k : k, -1});
+  auto sent = block;  // the buffers apart
   std::vector<Copy> flight;
   std::vector<int> met(4 * nc * nc, 0);
   const bool slow = rng() % 2;  // prefer the CTAs over the copies
@@ -83,7 +87,7 @@ const char* jacobi(int nc, int rounds, bool reports, bool apart, unsigned seed) 
       const size_t i = rng() % flight.size();
       const Copy f = flight[i];
       flight.erase(flight.begin() + i);
-      block[f.dst_half][f.dst][f.par ^ 1] = block[f.src_half][f.src][f.par];
+      block[f.dst_half][f.dst][f.par ^ 1] = (outs ? sent : block)[f.src_half][f.src][f.par];
       c[f.dst].bar[f.par].complete();
       continue;
     }
@@ -114,11 +118,13 @@ const char* jacobi(int nc, int rounds, bool reports, bool apart, unsigned seed) 
         const JacBlock s = jac_source(d.cta, d.half, nc);
         if (s.cta != k || s.half != h) return "jac_source does not undo jac_dest";
         for (const Copy& f : flight)
-          if (f.src == d.cta && f.src_half == d.half && f.par == np)
+          if (outs ? f.src == k && f.src_half == h && f.par == ap
+                   : f.src == d.cta && f.src_half == d.half && f.par == np)
             return "a write over the source of a copy in flight";
+        sent[h][k][ap] = block[h][k][ap];
         // its CTA is done with it once it has sent the rows of the round before
         const Cta& y = c[d.cta];
-        if (d.cta != k && (y.g < x.g - 1 || (y.g == x.g - 1 && y.step < 3))) 
+        if (d.cta != k && (y.g < x.g - 1 || (y.g == x.g - 1 && y.step < 3)))
           return "a write into a buffer in use";
         if (d.cta == k) block[d.half][k][np] = block[h][k][ap];
         else flight.push_back({k, h, d.cta, d.half, ap});
@@ -171,10 +177,10 @@ const char* qr_sums(int nmax, bool batches, bool alternate) {
 int main(int argc, char** argv) {
   const char* mode = argc > 1 ? argv[1] : "";
   if (!std::strncmp(mode, "jacobi", 6)) {
-    const bool reports = std::strcmp(mode, "jacobi-blind") != 0;
+    const bool outs = !std::strcmp(mode, "jacobi-outs"), reports = !std::strcmp(mode, "jacobi");
     for (int nc = 2; nc <= 16; ++nc)
       for (unsigned seed = 0; seed < 120; ++seed)
-        if (const char* bad = jacobi(nc, 3 * (2 * nc - 1), reports, seed % 2, seed)) {
+        if (const char* bad = jacobi(nc, 3 * (2 * nc - 1), reports, outs, reports && seed % 2, seed)) {
           std::printf("%d CTAs: %s\n", nc, bad);
           return 0;
         }

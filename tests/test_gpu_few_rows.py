@@ -57,3 +57,11 @@ def test_fp64_splits_whose_last_qr_batch_is_one_step(m, n, cplx):
     k = min(m, n)
     for _ in range(4):
         check_split(matrix(rng, m, n, np.geomspace(1.0, 1e-3, k), cplx))
+
+
+@pytest.mark.parametrize("m, n, rank, cplx", [(512, 512, 430, False), (512, 500, 470, False), (512, 512, 490, False),
+                                              (512, 512, 200, True), (512, 512, 300, True), (300, 512, 296, False)])
+def test_mixed_splits_of_many_rows(m, n, rank, cplx):
+    """Where shared memory has no room to send a round's rows from buffers apart (beyond 448 real
+    rows of 512, 224 complex ones), with and without a warp to spare, and just below."""
+    test_mixed_splits_of_low_rank(m, n, rank, cplx)

@@ -19,9 +19,11 @@ def check(tmp_path_factory):
 
 def test_jacobi_block_rounds(check):
     """Clusters of 2 to 16 CTAs, three sweeps: every pair of blocks meets once a sweep, no block is
-    written over while a copy of it may be in flight or its CTA works on it, and every wait ends.
-    Without the reports of receipt, the check finds the write over a copy's source."""
+    written over while a copy of it may be in flight or its CTA works on it, and every wait ends,
+    with reports of receipt or with buffers apart for what is sent. Without either, the check finds
+    the write over a copy's source."""
     assert check("jacobi") == "ok"
+    assert check("jacobi-outs") == "ok"
     assert check("jacobi-blind").endswith("a write over the source of a copy in flight")
 
 
