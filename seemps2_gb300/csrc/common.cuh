@@ -91,7 +91,7 @@ enum DevStatus : int {
   DEV_NONFINITE = 4,
 };
 
-// Bounded spin limit for every device-side wait (about a second with backoff).
+// Bounded number of polls of every grid barrier (a few seconds of round trips to L2).
 constexpr long long kSpinLimit = 1LL << 23;
 
 }  // namespace sm

@@ -1284,12 +1284,16 @@ constexpr size_t kStageBytes = 220 * 1024;  // shared memory with the FP32 stage
 constexpr double kSmallWork = 2e5, kSmallWorkPrecond = 5e4;
 
 // Fits the kernel: W (kw x l) with its odd row stride in shared memory, and no more work
-// than the other path's latencies leave time for.  Against the FP32 start: 24 rows 0.31
-// ms here and 0.49 there, 32 rows 0.41 and 0.54 (spanning 1e-12 0.59 and 0.98, in groups
-// of equal values 0.48 and 1.29); before the rows went to registers 40 rows 0.77 and 0.60,
-// 48 rows 1.10 and 0.65, complex 24 rows 0.53 and 0.58, 32 rows 0.80 and 0.66.  A
-// context that shares the device has no grid for the FP64 QR before that start and
-// keeps the larger limit.
+// than the other path's latencies leave time for.  Against the FP32 start, calls on square
+// matrices of values down to 0.03 / down to 1e-12 / in groups of eight equal ones, in ms:
+//   32 rows 0.41 and 0.54 / 0.59 and 0.98 / 0.48 and 1.29;  38 rows 0.66 and 0.61 / 0.88
+//   and 1.04 / 0.81 and 1.40;  44 rows 0.83 and 0.64 / 1.10 and 1.06 / 1.08 and 1.51;  48
+//   rows 0.98 and 0.66 / 1.32 and 1.09 / 1.17 and 1.67;  complex 28 rows 0.63 and 0.64 /
+//   0.87 and 1.10 / 0.78 and 1.49;  32 rows 0.75 and 0.68 / 1.06 and 1.18 / 0.98 and 1.64;
+//   36 rows 1.17 and 0.72 / 1.65 and 1.24 / 1.66 and 1.81.
+// The size alone is known beforehand, so the line (36 rows, complex 27) lies where the
+// first kind, most splits of a sweep, changes sides.  A context that shares the device has
+// no grid for the FP64 QR before that start and keeps the larger limit.
 template <typename T>
 bool small_split_fits(const Ctx& ctx, int kw, int l) {
   const int k = std::min(kw, l);
