@@ -37,6 +37,7 @@ struct H12Shared {
   short in[kH12Out][kH12In];
   int cnt[kH12Out];
 };
+__device__ __forceinline__ bool h12_zero(float x) { return x == 0.f; }
 __device__ __forceinline__ bool h12_zero(double x) { return x == 0.0; }
 __device__ __forceinline__ bool h12_zero(cplx x) { return x.re == 0.0 && x.im == 0.0; }
 template <typename T>
@@ -63,16 +64,16 @@ __device__ __forceinline__ void h12_sums(const V* __restrict__ X1, const T* __re
       for (int j = 0; j < ni; j += 32) {
         const int i = i0 + j + lane;
         bool put = false;
-        T h{};
+        V h{};
         if (j + lane < ni) {
           const int c = i / (p1 * p2), k = i / p2 % p1, l = i % p2;
-          h = H[((((size_t)(c * p1 + ko) * p1 + k) * p2 + lo) * p2 + l) * E + d0 + warp];
-          put = !h12_zero(h);
+          h12_put(h, H[((((size_t)(c * p1 + ko) * p1 + k) * p2 + lo) * p2 + l) * E + d0 + warp]);
+          put = !h12_zero(h);  // as multiplied: 1e-60 is zero in FP32
         }
         const unsigned m = __ballot_sync(0xffffffffu, put);
         if (put) {
           const int at = n + __popc(m & ((1u << lane) - 1u));
-          h12_put(sh.h[warp][at], h);
+          sh.h[warp][at] = h;
           sh.in[warp][at] = (short)(j + lane);
         }
         n += __popc(m);

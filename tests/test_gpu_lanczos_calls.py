@@ -71,3 +71,15 @@ def test_run_ends_at_an_invariant_subspace(precision, spread):
         assert total == steps
         assert abs(lam + 1.0) <= 1e-12
     assert launches[1] <= launches[0]
+
+
+@pytest.mark.parametrize("precision", ["bf16", "tf32x3"])
+def test_mpo_entries_that_vanish_in_fp32(precision):
+    """An MPO entry of 1e-60 meets products beyond the FP32 range: nothing is added, no NaN."""
+    chi = 160
+    L = torch.full((chi, 3, chi), 10.0, dtype=torch.float64, device="cuda")
+    H = torch.zeros((3, 2, 2, 2, 2, 3), dtype=torch.float64, device="cuda")
+    H[0, 0, 0, 0, 0, 0] = 1e-60
+    op = dmrg.TwoSiteOperator(L, H, L, precision)
+    out = op.matvec(torch.full((chi, 2, 2, chi), 1e38, dtype=torch.float64, device="cuda"))
+    assert (out == 0).all()
