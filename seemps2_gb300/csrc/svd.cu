@@ -1279,9 +1279,19 @@ constexpr size_t kSmallBytes = 160 * 1024;  // W in shared memory at most
 // 24 0.50 and 0.75 ms.
 constexpr int kStageRows = 8;
 constexpr size_t kStageBytes = 220 * 1024;  // shared memory with the FP32 stage's at most
-// Work (k^2 l) up to which one CTA is the faster: against the grid's Jacobi, and against
-// the FP32 start (svd_precond.cu) where that takes over.
+// Work (k^2 l) up to which one CTA is the faster: against one CTA of the grid's kernels (a
+// context that shares the device), and against the FP32 start (svd_precond.cu).
 constexpr double kSmallWork = 2e5, kSmallWorkPrecond = 5e4;
+// Below kPrecondMinRows rows of R the other side is the grid's QR and Jacobi, which spread
+// a row over many SMs; one CTA takes rows of up to this length (complex half of it).  Right
+// splits of k x l matrices, values down to 0.003 / to 1e-12, ms here and there: 8 x 128 0.23
+// and 0.29 / 0.24 and 0.27, 8 x 192 0.27 and 0.31 / 0.28 and 0.27, 8 x 512 0.51 and 0.33 /
+// 0.55 and 0.30; 16 x 128 0.41 and 0.54 / 0.51 and 0.50, 16 x 192 0.52 and 0.56 / 0.64 and
+// 0.51, 16 x 512 1.04 and 0.58 / 1.35 and 0.56; 2 x 384 0.14 and 0.15, 2 x 768 0.18 and
+// 0.15; 1 x 768 0.15 and 0.17; complex 16 x 64 0.48 and 0.66 / 0.62 and 0.62, 16 x 128 0.74
+// and 0.67 / 1.00 and 0.61.  (Long columns cost little: the left split of 16 x 512, whose R
+// is 16 x 16, 0.39 and 0.57.)
+constexpr int small_row_limit(int k) { return k == 1 ? 640 : k == 2 ? 384 : 160; }
 
 // Fits the kernel: W (kw x l) with its odd row stride in shared memory, and no more work
 // than the other path's latencies leave time for.  Against the FP32 start, calls on square
@@ -1299,9 +1309,9 @@ bool small_split_fits(const Ctx& ctx, int kw, int l) {
   const int k = std::min(kw, l);
   const bool cplx_t = sizeof(T) != sizeof(double);
   const double work = (double)k * k * l;
-  const bool fast = k < kPrecondMinRows || ctx.concurrent
-                        ? work * (cplx_t ? 4.0 : 1.0) <= kSmallWork
-                        : work * (cplx_t ? 2.5 : 1.0) <= kSmallWorkPrecond;
+  const bool fast = ctx.concurrent          ? work * (cplx_t ? 4.0 : 1.0) <= kSmallWork
+                    : k < kPrecondMinRows ? l * (cplx_t ? 2 : 1) <= small_row_limit(k)
+                                          : work * (cplx_t ? 2.5 : 1.0) <= kSmallWorkPrecond;
   return k <= kSmallRows && fast && sizeof(T) * (size_t)kw * (l | 1) <= kSmallBytes;
 }
 
