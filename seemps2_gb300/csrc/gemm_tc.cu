@@ -596,6 +596,10 @@ int gemm_tc_planes(Ctx& ctx, cudaStream_t st, int M, int N, int kp, bool bf16, c
     nzo = (ranges + nz - 1) / nz;
   } else {
     while (nz < nmax && 2 * nz <= std::min(sms / tiles, ktiles)) nz *= 2;
+    // Two CTAs share a tile from more slabs on than one's accumulators take two of: a call
+    // of 1200 x 69 x 85 takes 40 us in one CTA a tile and 50 in two, 1024 x 1024 x 256 46
+    // and 52 (x 512 52 and 56, x 1024 75 and 68).
+    if (nz == 2 && ktiles <= 2 * TcMode<false>::acc) nz = 1;
     kt_per = (ktiles + nz - 1) / nz;
     constexpr int most = 2 * TcMode<false>::acc;
     if (nz == nmax)

@@ -36,3 +36,15 @@ def test_beyond_the_row_limit():
     A = torch.ones(65535 * 64 + 1, 2, dtype=torch.float64, device="cuda")
     with pytest.raises(ValueError, match="M too large"):
         core._gemm(A, 0, torch.ones(2, 2, dtype=torch.float64, device="cuda"), 0)
+
+
+@pytest.mark.parametrize("K", [33, 64, 96, 250, 257, 300])
+@pytest.mark.parametrize("M, N", [(1200, 69), (1024, 1024)])
+def test_tf32_products_of_few_slabs(M, N, K):
+    """One or two CTAs to a tile of a few slabs of K: 2e-6 of the norm, as the others."""
+    from tests.test_gpu_tc import _gemm_f32
+
+    rng = np.random.default_rng(M + K)
+    A, B = rng.normal(size=(M, K)), rng.normal(size=(K, N))
+    ref = A @ B
+    assert np.linalg.norm(_gemm_f32("N", "N", A, B, M, N, K) - ref) <= 2e-6 * np.linalg.norm(ref)
